@@ -1,0 +1,656 @@
+// The Python-facing calls of the library: argument checks, allocation, stream lookup and the C ABI call, and the
+// differentiable forms of the two ops as native autograd nodes.  Everything here is host work per call; it bounds every
+// layer that runs for less than a few tens of microseconds, which is why it is not Python (one image through the
+// 64 x 64 x 56 x 56 layer took 24 us to enqueue from Python for 12 us of kernel).  The arithmetic, and every decision about
+// how a shape is computed, stays behind include/winograd2x2_b200.h.
+#include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/autograd/saved_variable.h>
+
+#include "../../include/winograd2x2_b200.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+PyObject *g_error = nullptr;     // wg2x2.Wg2x2Error, handed over by set_error
+
+// ---------------------------------------------------------------------------------------
+// Errors: the types and texts that the callers of the Python functions see
+// ---------------------------------------------------------------------------------------
+void check(int status, const char *what)
+{
+    if (status == WG2X2_OK) return;
+    pybind11::gil_scoped_acquire gil;      // also reached from the autograd engine's threads
+    PyObject *e = g_error ? PyObject_CallFunction(g_error, "is", status, what) : nullptr;
+    if (e) {
+        PyErr_SetObject(g_error, e);
+        Py_DECREF(e);
+    } else if (!PyErr_Occurred()) {
+        PyErr_Format(PyExc_RuntimeError, "%s: status %d", what, status);
+    }
+    python_error err;                      // carries the exception over to whichever thread reports it
+    err.persist();
+    throw std::move(err);
+}
+[[noreturn]] void value_error(const std::string &msg) { TORCH_CHECK_VALUE(false, msg); __builtin_unreachable(); }
+[[noreturn]] void type_error(const std::string &msg) { throw torch::TypeError(msg); }
+[[noreturn]] void not_a_tensor(const char *name) { type_error(std::string(name) + " must be a contiguous float32 CUDA tensor"); }
+
+void require(const Tensor &t, const char *name)
+{
+    if (!(t.is_cuda() && t.scalar_type() == at::kFloat && t.is_contiguous()))
+        not_a_tensor(name);
+}
+std::string shape_text(at::IntArrayRef s)
+{
+    std::string o = "(";
+    for (size_t i = 0; i < s.size(); ++i) o += (i ? ", " : "") + std::to_string(s[i]);
+    return o + (s.size() == 1 ? ",)" : ")");
+}
+
+// a float32 CUDA tensor argument; `None` gives an undefined tensor where that is allowed
+Tensor arg(PyObject *o, const char *name, bool optional = false)
+{
+    if (optional && o == Py_None) return Tensor();
+    if (!THPVariable_Check(o)) not_a_tensor(name);
+    const Tensor &t = THPVariable_Unpack(o);
+    require(t, name);
+    return t;
+}
+Tensor arg_shaped(PyObject *o, at::IntArrayRef shape, const char *name)
+{
+    Tensor t = arg(o, name, true);
+    if (t.defined() && t.sizes() != shape)
+        value_error(std::string(name) + " has shape " + shape_text(t.sizes()) + ", expected " + shape_text(shape));
+    return t;
+}
+// a tensor whose memory is used as it is: an output or a workspace of the caller
+Tensor arg_raw(PyObject *o, const char *name)
+{
+    if (o == Py_None) return Tensor();
+    if (!THPVariable_Check(o)) type_error(std::string(name) + " must be a tensor");
+    return THPVariable_Unpack(o);
+}
+int arg_int(PyObject *o)
+{
+    const long v = PyLong_AsLong(o);
+    if (v == -1 && PyErr_Occurred()) throw python_error();
+    return (int)v;
+}
+bool arg_bool(PyObject *o)
+{
+    const int v = PyObject_IsTrue(o);
+    if (v < 0) throw python_error();
+    return v != 0;
+}
+int arg_int_or(PyObject *o, int otherwise) { return o == Py_None ? otherwise : arg_int(o); }
+
+void need_dims(const Tensor &t, int dims, const char *name)
+{
+    if (t.dim() != dims) value_error(std::string(name) + " must have " + std::to_string(dims) + " dimensions, got " + shape_text(t.sizes()));
+}
+
+struct Img { int64_t B, H, W, C; };
+Img img_of(const Tensor &t, int layout, const char *name)
+{
+    need_dims(t, 4, name);
+    const auto s = t.sizes();
+    return layout == WG2X2_NHWC ? Img{s[0], s[1], s[2], s[3]} : Img{s[0], s[2], s[3], s[1]};
+}
+std::array<int64_t, 4> img_shape(int64_t B, int64_t H, int64_t W, int64_t C, int layout)
+{
+    if (layout == WG2X2_NHWC) return {B, H, W, C};
+    return {B, C, H, W};
+}
+
+// The opaque buffer of prepare_weights for exactly (C, K): the kernels build their TMA maps over it from C and K alone, so
+// a buffer made for other sizes would be read past its end.
+Tensor arg_prepared(PyObject *o, int64_t C, int64_t K)
+{
+    if (!THPVariable_Check(o)) type_error("prepared must be the buffer returned by prepare_weights");
+    const Tensor &t = THPVariable_Unpack(o);
+    if (!t.is_cuda() || t.scalar_type() != at::kByte) type_error("prepared must be the buffer returned by prepare_weights");
+    static PyObject *ck_name = PyUnicode_InternFromString("_wg_ck");
+    if (PyObject *ck = PyObject_GetAttr(o, ck_name)) {
+        long c = 0, k = 0;
+        const bool pair = PyTuple_Check(ck) && PyTuple_GET_SIZE(ck) == 2;
+        if (pair) { c = PyLong_AsLong(PyTuple_GET_ITEM(ck, 0)); k = PyLong_AsLong(PyTuple_GET_ITEM(ck, 1)); }
+        Py_DECREF(ck);
+        if (pair && (c != C || k != K))
+            value_error("prepared weights are for (C, K) = (" + std::to_string(c) + ", " + std::to_string(k) + "), the call has (" +
+                        std::to_string(C) + ", " + std::to_string(K) + ")");
+    } else {
+        PyErr_Clear();
+    }
+    if ((size_t)t.numel() < wg2x2_prepared_weights_bytes((int)C, (int)K))
+        value_error("prepared weight buffer too small for C=" + std::to_string(C) + " K=" + std::to_string(K));
+    return t;
+}
+
+// ---------------------------------------------------------------------------------------
+// Memory and launch context
+// ---------------------------------------------------------------------------------------
+const float *cptr(const Tensor &t) { return t.defined() ? static_cast<const float *>(t.data_ptr()) : nullptr; }
+float *ptr(const Tensor &t) { return t.defined() ? static_cast<float *>(t.data_ptr()) : nullptr; }
+
+Tensor new_float(at::IntArrayRef shape, const Tensor &like)
+{
+    return Tensor(at::detail::empty_cuda(shape, at::kFloat, like.device(), std::nullopt));
+}
+
+// Scratch memory of one call: from torch's caching allocator, whose blocks belong to the stream they were taken on, so that
+// the block may be handed on while the kernels that use it are still queued.
+struct Scratch {
+    c10::DataPtr block;
+    size_t bytes = 0;
+    void take(size_t n)
+    {
+        if (!n) return;
+        block = c10::cuda::CUDACachingAllocator::get()->allocate(n);
+        bytes = n;
+    }
+    void *get() const { return block.get(); }
+};
+
+// The tensor's device, current, and its current stream
+struct OnDevice {
+    c10::cuda::CUDAGuard guard;
+    void *stream;
+    explicit OnDevice(const Tensor &t) : guard(t.device()), stream(c10::cuda::getCurrentCUDAStream(t.device().index()).stream()) {}
+};
+
+// ---------------------------------------------------------------------------------------
+// The ops
+// ---------------------------------------------------------------------------------------
+Tensor imtrans_fwd(const Tensor &x, bool relu, int layout, const Tensor &out, const Tensor &in_scale, const Tensor &in_shift)
+{
+    const Img d = img_of(x, layout, "x");
+    OnDevice on(x);
+    Tensor V = out.defined() ? out : new_float({16, d.B, (d.H + 1) / 2, (d.W + 1) / 2, d.C}, x);
+    if (in_scale.defined())
+        check(wg2x2_imtrans_fwd_affine(cptr(x), cptr(in_scale), cptr(in_shift), ptr(V), d.B, d.H, d.W, d.C, layout, relu, on.stream),
+              "wg2x2_imtrans_fwd_affine");
+    else
+        check(wg2x2_imtrans_fwd(cptr(x), ptr(V), d.B, d.H, d.W, d.C, layout, relu, on.stream), "wg2x2_imtrans_fwd");
+    return V;
+}
+
+Tensor imtrans_bwd(const Tensor &dV, int64_t H, int64_t W, const Tensor &V_relu, int layout)
+{
+    need_dims(dV, 5, "dV");
+    const int64_t B = dV.size(1), nH = dV.size(2), nW = dV.size(3), C = dV.size(4);
+    if ((H + 1) / 2 != nH || (W + 1) / 2 != nW) value_error("H, W do not match the tile grid of dV");
+    OnDevice on(dV);
+    Tensor dX = new_float(img_shape(B, H, W, C, layout), dV);
+    check(wg2x2_imtrans_bwd(cptr(dV), cptr(V_relu), ptr(dX), B, H, W, C, layout, on.stream), "wg2x2_imtrans_bwd");
+    return dX;
+}
+
+Tensor conv_fwd(const Tensor &V, const Tensor &Wt, int out_h, int out_w, int layout, int math, const Tensor &out, const Tensor &workspace)
+{
+    need_dims(V, 5, "V");
+    const int64_t B = V.size(1), nH = V.size(2), nW = V.size(3), C = V.size(4);
+    if (Wt.dim() != 3 || Wt.size(0) != 16 || Wt.size(1) != C) value_error("Wt must be (16, C, K)");
+    const int64_t K = Wt.size(2);
+    if (out_h < 0) out_h = (int)(2 * nH);
+    if (out_w < 0) out_w = (int)(2 * nW);
+    OnDevice on(V);
+    Tensor Y = out.defined() ? out : new_float(img_shape(B, out_h, out_w, K, layout), V);
+    Scratch ws;
+    void *wp = nullptr;
+    size_t wn = 0;
+    if (workspace.defined()) { wp = workspace.data_ptr(); wn = (size_t)workspace.numel(); }
+    else { ws.take(wg2x2_conv_fwd_workspace_bytes(B, nH, nW, C, K, math)); wp = ws.get(); wn = ws.bytes; }
+    check(wg2x2_conv_fwd(cptr(V), cptr(Wt), ptr(Y), B, nH, nW, C, K, out_h, out_w, layout, math, wp, wn, on.stream), "wg2x2_conv_fwd");
+    return Y;
+}
+
+std::pair<Tensor, Tensor> conv_bwd(const Tensor &V, const Tensor &Wt, const Tensor &dY, const Tensor &mask, int layout, bool relu, int math,
+                                   bool need_dV, bool need_dW)
+{
+    need_dims(V, 5, "V");
+    const int64_t B = V.size(1), nH = V.size(2), nW = V.size(3), C = V.size(4);
+    need_dims(Wt, 3, "Wt");
+    const int64_t K = Wt.size(2);
+    const Img d = img_of(dY, layout, "dY");
+    if (d.B != B || d.C != K || (d.H + 1) / 2 != nH || (d.W + 1) / 2 != nW) value_error("dY does not match V / Wt");
+    OnDevice on(V);
+    Tensor dV, dW;
+    if (need_dV) dV = new_float(V.sizes(), V);
+    if (need_dW) dW = new_float(Wt.sizes(), V);
+    Scratch ws;
+    ws.take(wg2x2_conv_bwd_workspace_bytes(B, d.H, d.W, C, K, math, need_dW));
+    check(wg2x2_conv_bwd(cptr(V), cptr(Wt), cptr(dY), cptr(mask), ptr(dV), ptr(dW), B, d.H, d.W, C, K, layout, relu, math, ws.get(), ws.bytes,
+                         on.stream),
+          "wg2x2_conv_bwd");
+    return {dV, dW};
+}
+
+// ---------------------------------------------------------------------------------------
+// Autograd nodes of the two ops (the reference pairs each op with its gradient op by RegisterGradient:
+// winograd2x2_imTrans.py:29-33, winograd2x2_conv.py:32-36)
+// ---------------------------------------------------------------------------------------
+struct ImTransBackward : public torch::autograd::Node {
+    SavedVariable V_;          // post-ReLU output, kept only where the ReLU was applied
+    int64_t H = 0, W = 0;
+    int layout = 0;
+    bool relu = false;
+    std::string name() const override { return "Winograd2x2ImTransBackward"; }
+    void release_variables() override { V_.reset_data(); }
+    variable_list apply(variable_list &&grads) override
+    {
+        if (!grads[0].defined()) return {Tensor()};
+        Tensor V = relu ? V_.unpack(shared_from_this()) : Tensor();
+        const Tensor g = grads[0].contiguous();
+        require(g, "dV");
+        return {imtrans_bwd(g, H, W, V, layout)};
+    }
+};
+
+struct ConvBackward : public torch::autograd::Node {
+    SavedVariable I_, W_;
+    int layout = 0, math = 0;
+    std::string name() const override { return "Winograd2x2ConvBackward"; }
+    void release_variables() override { I_.reset_data(); W_.reset_data(); }
+    variable_list apply(variable_list &&grads) override
+    {
+        if (!grads[0].defined()) return {Tensor(), Tensor()};
+        const bool dI = task_should_compute_output(0), dW = task_should_compute_output(1);
+        const Tensor g = grads[0].contiguous();
+        require(g, "dY");
+        auto r = conv_bwd(I_.unpack(), W_.unpack(), g, Tensor(), layout, false, math, dI, dW);
+        return {r.first, r.second};
+    }
+};
+
+template <class N>
+std::shared_ptr<N> new_node(torch::autograd::edge_list edges)
+{
+    std::shared_ptr<N> n(new N(), torch::autograd::deleteNode);
+    n->set_next_edges(std::move(edges));
+    return n;
+}
+
+Tensor imtrans_op(const Tensor &in, bool relu, int layout)
+{
+    const Tensor I = in.contiguous();
+    require(I, "x");
+    Tensor V = imtrans_fwd(I, relu, layout, Tensor(), Tensor(), Tensor());
+    if (torch::autograd::compute_requires_grad(I)) {
+        auto n = new_node<ImTransBackward>(torch::autograd::collect_next_edges(I));
+        const Img d = img_of(I, layout, "x");
+        n->H = d.H; n->W = d.W; n->layout = layout; n->relu = relu;
+        torch::autograd::set_history(V, n);
+        if (relu) n->V_ = SavedVariable(V, true);
+    }
+    return V;
+}
+
+Tensor conv_op(const Tensor &in, const Tensor &win, int out_h, int out_w, int layout, int math)
+{
+    const Tensor I = in.contiguous(), Wt = win.contiguous();
+    require(I, "V");
+    require(Wt, "Wt");
+    Tensor Y = conv_fwd(I, Wt, out_h, out_w, layout, math, Tensor(), Tensor());
+    if (torch::autograd::compute_requires_grad(I, Wt)) {
+        auto n = new_node<ConvBackward>(torch::autograd::collect_next_edges(I, Wt));
+        n->layout = layout; n->math = math;
+        n->I_ = SavedVariable(I, false);
+        n->W_ = SavedVariable(Wt, false);
+        torch::autograd::set_history(Y, n);
+    }
+    return Y;
+}
+
+// ---------------------------------------------------------------------------------------
+// Python entry points (positional arguments, all given; the keyword forms and defaults are in ops.py)
+// ---------------------------------------------------------------------------------------
+void want(Py_ssize_t got, Py_ssize_t n)
+{
+    if (got != n) type_error("expected " + std::to_string(n) + " arguments, got " + std::to_string(got));
+}
+#define WG_ARGS PyObject *, PyObject *const *a, Py_ssize_t n
+// The GIL is given up while a call allocates and launches, as a foreign call would do it
+#define WG_NOGIL pybind11::gil_scoped_release nogil
+
+PyObject *py_set_error(PyObject *, PyObject *cls)
+{
+    Py_XINCREF(cls);
+    Py_XSETREF(g_error, cls);
+    Py_RETURN_NONE;
+}
+
+// x, relu, layout, out, in_scale, in_shift
+PyObject *py_imtrans_fwd(WG_ARGS)
+{
+    HANDLE_TH_ERRORS
+    want(n, 6);
+    const Tensor x = arg(a[0], "x");
+    const bool relu = arg_bool(a[1]);
+    const int layout = arg_int(a[2]);
+    const Tensor out = arg_raw(a[3], "out");
+    Tensor sc, sh;
+    if (a[4] != Py_None) { sc = arg(a[4], "in_scale"); sh = arg(a[5], "in_shift"); }
+    Tensor V;
+    { WG_NOGIL; V = imtrans_fwd(x, relu, layout, out, sc, sh); }
+    return THPVariable_Wrap(V);
+    END_HANDLE_TH_ERRORS
+}
+
+// dV, H, W, V_relu, layout
+PyObject *py_imtrans_bwd(WG_ARGS)
+{
+    HANDLE_TH_ERRORS
+    want(n, 5);
+    const Tensor dV = arg(a[0], "dV");
+    const int H = arg_int(a[1]), W = arg_int(a[2]);
+    const Tensor Vr = arg(a[3], "V_relu", true);
+    const int layout = arg_int(a[4]);
+    Tensor dX;
+    { WG_NOGIL; dX = imtrans_bwd(dV, H, W, Vr, layout); }
+    return THPVariable_Wrap(dX);
+    END_HANDLE_TH_ERRORS
+}
+
+// V, Wt, out_h, out_w, layout, math, out, workspace
+PyObject *py_conv_fwd(WG_ARGS)
+{
+    HANDLE_TH_ERRORS
+    want(n, 8);
+    const Tensor V = arg(a[0], "V"), Wt = arg(a[1], "Wt");
+    const int oh = arg_int_or(a[2], -1), ow = arg_int_or(a[3], -1), layout = arg_int(a[4]), math = arg_int(a[5]);
+    const Tensor out = arg_raw(a[6], "out"), ws = arg_raw(a[7], "workspace");
+    Tensor Y;
+    { WG_NOGIL; Y = conv_fwd(V, Wt, oh, ow, layout, math, out, ws); }
+    return THPVariable_Wrap(Y);
+    END_HANDLE_TH_ERRORS
+}
+
+// V, prepared, K, out_h, out_w, layout, out, out_scale, out_shift, residual, workspace, wide
+PyObject *py_conv_fwd_prepared(WG_ARGS)
+{
+    HANDLE_TH_ERRORS
+    want(n, 12);
+    const Tensor V = arg(a[0], "V");
+    need_dims(V, 5, "V");
+    const int64_t B = V.size(1), nH = V.size(2), nW = V.size(3), C = V.size(4), K = arg_int(a[2]);
+    const Tensor prep = arg_prepared(a[1], C, K);
+    const int oh = arg_int_or(a[3], (int)(2 * nH)), ow = arg_int_or(a[4], (int)(2 * nW)), layout = arg_int(a[5]);
+    const auto ys = img_shape(B, oh, ow, K, layout);
+    Tensor Y = arg_shaped(a[6], ys, "out");
+    const Tensor sc = arg_shaped(a[7], {K}, "out_scale"), sh = arg_shaped(a[8], {K}, "out_shift"), res = arg_shaped(a[9], ys, "residual");
+    const Tensor uws = arg_raw(a[10], "workspace");
+    const bool wide = arg_bool(a[11]);
+    {
+        WG_NOGIL;
+        OnDevice on(V);
+        if (!Y.defined()) Y = new_float(ys, V);
+        const size_t nws = wide ? wg2x2_conv_fwd_prepared_workspace_bytes(B, nH, nW, C, K) : 0;
+        if (nws) {       // many channels: products as wide GEMMs into scratch memory, then the output transform
+            Scratch ws;
+            void *wp;
+            size_t wn;
+            if (uws.defined() && (size_t)uws.numel() >= nws) { wp = uws.data_ptr(); wn = (size_t)uws.numel(); }
+            else { ws.take(nws); wp = ws.get(); wn = nws; }
+            check(wg2x2_conv_fwd_prepared_ws(cptr(V), prep.data_ptr(), ptr(Y), B, nH, nW, C, K, oh, ow, layout, cptr(sc), cptr(sh), cptr(res),
+                                             wp, wn, on.stream),
+                  "wg2x2_conv_fwd_prepared_ws");
+        } else if (!sc.defined() && !res.defined()) {
+            check(wg2x2_conv_fwd_prepared(cptr(V), prep.data_ptr(), ptr(Y), B, nH, nW, C, K, oh, ow, layout, on.stream), "wg2x2_conv_fwd_prepared");
+        } else {
+            check(wg2x2_conv_fwd_prepared_fused(cptr(V), prep.data_ptr(), ptr(Y), B, nH, nW, C, K, oh, ow, layout, cptr(sc), cptr(sh), cptr(res),
+                                                on.stream),
+                  "wg2x2_conv_fwd_prepared_fused");
+        }
+    }
+    return THPVariable_Wrap(Y);
+    END_HANDLE_TH_ERRORS
+}
+
+// V, Wt, dY, mask, layout, relu, math, need_dV, need_dW
+PyObject *py_conv_bwd(WG_ARGS)
+{
+    HANDLE_TH_ERRORS
+    want(n, 9);
+    const Tensor V = arg(a[0], "V"), Wt = arg(a[1], "Wt"), dY = arg(a[2], "dY"), mask = arg(a[3], "mask", true);
+    const int layout = arg_int(a[4]);
+    const bool relu = arg_bool(a[5]);
+    const int math = arg_int(a[6]);
+    const bool ndv = arg_bool(a[7]), ndw = arg_bool(a[8]);
+    std::pair<Tensor, Tensor> r;
+    { WG_NOGIL; r = conv_bwd(V, Wt, dY, mask, layout, relu, math, ndv, ndw); }
+    PyObject *t = PyTuple_New(2);
+    if (!t) throw python_error();
+    PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(r.first));       // an undefined tensor wraps to None
+    PyTuple_SET_ITEM(t, 1, THPVariable_Wrap(r.second));
+    return t;
+    END_HANDLE_TH_ERRORS
+}
+
+// x, Wt, relu, layout, math, keep_V, out, workspace
+PyObject *py_layer_fwd(WG_ARGS)
+{
+    HANDLE_TH_ERRORS
+    want(n, 8);
+    const Tensor x = arg(a[0], "x"), Wt = arg(a[1], "Wt");
+    const bool relu = arg_bool(a[2]);
+    const int layout = arg_int(a[3]), math = arg_int(a[4]);
+    const bool keep = arg_bool(a[5]);
+    const Img d = img_of(x, layout, "x");
+    if (Wt.dim() != 3 || Wt.size(0) != 16 || Wt.size(1) != d.C) value_error("Wt must be (16, C, K)");
+    const int64_t K = Wt.size(2);
+    Tensor Y = arg_raw(a[6], "out"), V;
+    const Tensor uws = arg_raw(a[7], "workspace");
+    {
+        WG_NOGIL;
+        OnDevice on(x);
+        if (!Y.defined()) Y = new_float(img_shape(d.B, d.H, d.W, K, layout), x);
+        if (keep) V = new_float({16, d.B, (d.H + 1) / 2, (d.W + 1) / 2, d.C}, x);
+        Scratch ws;
+        void *wp;
+        size_t wn;
+        if (uws.defined()) { wp = uws.data_ptr(); wn = (size_t)uws.numel(); }
+        else { ws.take(wg2x2_layer_fwd_workspace_bytes(d.B, d.H, d.W, d.C, K, math, keep)); wp = ws.get(); wn = ws.bytes; }
+        check(wg2x2_layer_fwd(cptr(x), cptr(Wt), ptr(Y), ptr(V), d.B, d.H, d.W, d.C, K, layout, relu, math, wp, wn, on.stream), "wg2x2_layer_fwd");
+    }
+    if (!keep) return THPVariable_Wrap(Y);
+    PyObject *t = PyTuple_New(2);
+    if (!t) throw python_error();
+    PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(Y));
+    PyTuple_SET_ITEM(t, 1, THPVariable_Wrap(V));
+    return t;
+    END_HANDLE_TH_ERRORS
+}
+
+// x, prepared, K, relu, layout, out, V_scratch, out_scale, out_shift, residual, workspace
+PyObject *py_layer_fwd_prepared(WG_ARGS)
+{
+    HANDLE_TH_ERRORS
+    want(n, 11);
+    const Tensor x = arg(a[0], "x");
+    const int layout = arg_int(a[4]);
+    const Img d = img_of(x, layout, "x");
+    const int64_t K = arg_int(a[2]);
+    const Tensor prep = arg_prepared(a[1], d.C, K);
+    const bool relu = arg_bool(a[3]);
+    const auto ys = img_shape(d.B, d.H, d.W, K, layout);
+    Tensor Y = arg_shaped(a[5], ys, "out");
+    const Tensor sc = arg_shaped(a[7], {K}, "out_scale"), sh = arg_shaped(a[8], {K}, "out_shift"), res = arg_shaped(a[9], ys, "residual");
+    const Tensor V = arg_shaped(a[6], {16, d.B, (d.H + 1) / 2, (d.W + 1) / 2, d.C}, "V_scratch");
+    const Tensor uws = arg_raw(a[10], "workspace");
+    {
+        WG_NOGIL;
+        OnDevice on(x);
+        if (!Y.defined()) Y = new_float(ys, x);
+        Scratch vs, ws;
+        const size_t nws = wg2x2_layer_fwd_prepared_workspace_bytes(d.B, d.H, d.W, d.C, K);
+        float *vp = ptr(V);
+        if (!vp && (nws || !wg2x2_layer_fwd_fused_supported(d.B, d.H, d.W, d.C, K, layout))) {
+            vs.take(sizeof(float) * 16 * (size_t)d.B * ((d.H + 1) / 2) * ((d.W + 1) / 2) * d.C);
+            vp = static_cast<float *>(vs.get());
+        }
+        void *wp = nullptr;
+        if (nws) {
+            if (uws.defined() && (size_t)uws.numel() >= nws) wp = uws.data_ptr();
+            else { ws.take(nws); wp = ws.get(); }
+        }
+        check(wg2x2_layer_fwd_prepared_ws(cptr(x), prep.data_ptr(), ptr(Y), vp, d.B, d.H, d.W, d.C, K, layout, relu, cptr(sc), cptr(sh), cptr(res),
+                                          wp, nws, on.stream),
+              "wg2x2_layer_fwd_prepared_ws");
+    }
+    return THPVariable_Wrap(Y);
+    END_HANDLE_TH_ERRORS
+}
+
+// x, prepared, K, relu, out, out_scale, out_shift, residual, in_scale, in_shift
+PyObject *py_layer_fwd_fused(WG_ARGS)
+{
+    HANDLE_TH_ERRORS
+    want(n, 10);
+    const Tensor x = arg(a[0], "x");
+    const Img d = img_of(x, WG2X2_NCHW, "x");
+    const int64_t K = arg_int(a[2]);
+    const Tensor prep = arg_prepared(a[1], d.C, K);
+    const bool relu = arg_bool(a[3]);
+    const auto ys = img_shape(d.B, d.H, d.W, K, WG2X2_NCHW);
+    Tensor Y = arg_shaped(a[4], ys, "out");
+    const Tensor sc = arg_shaped(a[5], {K}, "out_scale"), sh = arg_shaped(a[6], {K}, "out_shift"), res = arg_shaped(a[7], ys, "residual");
+    const Tensor isc = arg_shaped(a[8], {d.C}, "in_scale"), ish = arg_shaped(a[9], {d.C}, "in_shift");
+    {
+        WG_NOGIL;
+        OnDevice on(x);
+        if (!Y.defined()) Y = new_float(ys, x);
+        if (!isc.defined() && !ish.defined())
+            check(wg2x2_layer_fwd_fused(cptr(x), prep.data_ptr(), ptr(Y), d.B, d.H, d.W, d.C, K, relu, cptr(sc), cptr(sh), cptr(res), on.stream),
+                  "wg2x2_layer_fwd_fused");
+        else
+            check(wg2x2_layer_fwd_fused_affine(cptr(x), prep.data_ptr(), ptr(Y), d.B, d.H, d.W, d.C, K, relu, cptr(isc), cptr(ish), cptr(sc),
+                                               cptr(sh), cptr(res), on.stream),
+                  "wg2x2_layer_fwd_fused_affine");
+    }
+    return THPVariable_Wrap(Y);
+    END_HANDLE_TH_ERRORS
+}
+
+PyObject *pair_or_one(const Tensor &y, const Tensor &yr)
+{
+    if (!yr.defined()) return THPVariable_Wrap(y);
+    PyObject *t = PyTuple_New(2);
+    if (!t) throw python_error();
+    PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(y));
+    PyTuple_SET_ITEM(t, 1, THPVariable_Wrap(yr));
+    return t;
+}
+
+// x, with_relu, relu_scale, relu_shift
+PyObject *py_maxpool(WG_ARGS)
+{
+    HANDLE_TH_ERRORS
+    want(n, 4);
+    if (!THPVariable_Check(a[0])) not_a_tensor("x");
+    const Tensor x = THPVariable_Unpack(a[0]);
+    const Img d = img_of(x, WG2X2_NCHW, "x");
+    const bool nhwc = !x.is_contiguous() && x.is_contiguous(at::MemoryFormat::ChannelsLast) && x.is_cuda() && x.scalar_type() == at::kFloat;
+    if (!nhwc) require(x, "x");
+    const bool with_relu = arg_bool(a[1]);
+    const Tensor sc = arg_shaped(a[2], {d.C}, "relu_scale"), sh = arg_shaped(a[3], {d.C}, "relu_shift");
+    Tensor y, yr;
+    {
+        WG_NOGIL;
+        OnDevice on(x);
+        y = new_float({d.B, d.C, (d.H + 1) / 2, (d.W + 1) / 2}, x);
+        if (with_relu) yr = new_float(y.sizes(), x);
+        if (nhwc)
+            check(wg2x2_maxpool3x3s2_same_nhwc_in(cptr(x), ptr(y), ptr(yr), cptr(sc), cptr(sh), d.B, d.C, d.H, d.W, on.stream),
+                  "wg2x2_maxpool3x3s2_same_nhwc_in");
+        else
+            check(wg2x2_maxpool3x3s2_same(cptr(x), ptr(y), ptr(yr), cptr(sc), cptr(sh), d.B, d.C, d.H, d.W, on.stream), "wg2x2_maxpool3x3s2_same");
+    }
+    return pair_or_one(y, yr);
+    END_HANDLE_TH_ERRORS
+}
+
+// x, prepared, with_relu, relu_scale, relu_shift (sizes checked by the caller)
+PyObject *py_stem_pool(WG_ARGS)
+{
+    HANDLE_TH_ERRORS
+    want(n, 5);
+    const Tensor x = arg(a[0], "x");
+    const Img d = img_of(x, WG2X2_NCHW, "x");
+    const Tensor prep = arg_shaped(a[1], {(int64_t)wg2x2_stem_prepared_floats()}, "prepared");
+    const bool with_relu = arg_bool(a[2]);
+    const Tensor sc = arg_shaped(a[3], {64}, "relu_scale"), sh = arg_shaped(a[4], {64}, "relu_shift");
+    Tensor y, yr;
+    {
+        WG_NOGIL;
+        OnDevice on(x);
+        y = new_float({d.B, 64, d.H / 4, d.W / 4}, x);
+        if (with_relu) yr = new_float(y.sizes(), x);
+        check(wg2x2_stem7x7s2_pool(cptr(x), cptr(prep), ptr(y), ptr(yr), cptr(sc), cptr(sh), d.B, d.H, d.W, on.stream), "wg2x2_stem7x7s2_pool");
+    }
+    return pair_or_one(y, yr);
+    END_HANDLE_TH_ERRORS
+}
+
+// I, relu, layout: differentiable
+PyObject *py_imtrans_op(WG_ARGS)
+{
+    HANDLE_TH_ERRORS
+    want(n, 3);
+    if (!THPVariable_Check(a[0])) not_a_tensor("x");
+    const Tensor I = THPVariable_Unpack(a[0]);
+    const bool relu = arg_bool(a[1]);
+    const int layout = arg_int(a[2]);
+    Tensor V;
+    { WG_NOGIL; V = imtrans_op(I, relu, layout); }
+    return THPVariable_Wrap(V);
+    END_HANDLE_TH_ERRORS
+}
+
+// I, W, out_h, out_w, layout, math: differentiable
+PyObject *py_conv_op(WG_ARGS)
+{
+    HANDLE_TH_ERRORS
+    want(n, 6);
+    if (!THPVariable_Check(a[0])) not_a_tensor("V");
+    if (!THPVariable_Check(a[1])) not_a_tensor("Wt");
+    const Tensor I = THPVariable_Unpack(a[0]), Wt = THPVariable_Unpack(a[1]);
+    const int oh = arg_int_or(a[2], -1), ow = arg_int_or(a[3], -1), layout = arg_int(a[4]), math = arg_int(a[5]);
+    Tensor Y;
+    { WG_NOGIL; Y = conv_op(I, Wt, oh, ow, layout, math); }
+    return THPVariable_Wrap(Y);
+    END_HANDLE_TH_ERRORS
+}
+
+#define WG_FN(name, fn) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(fn)), METH_FASTCALL, nullptr}
+PyMethodDef methods[] = {
+    {"set_error", py_set_error, METH_O, nullptr},
+    WG_FN("imtrans_fwd", py_imtrans_fwd),
+    WG_FN("imtrans_bwd", py_imtrans_bwd),
+    WG_FN("conv_fwd", py_conv_fwd),
+    WG_FN("conv_fwd_prepared", py_conv_fwd_prepared),
+    WG_FN("conv_bwd", py_conv_bwd),
+    WG_FN("layer_fwd", py_layer_fwd),
+    WG_FN("layer_fwd_prepared", py_layer_fwd_prepared),
+    WG_FN("layer_fwd_fused", py_layer_fwd_fused),
+    WG_FN("maxpool", py_maxpool),
+    WG_FN("stem_pool", py_stem_pool),
+    WG_FN("imtrans_op", py_imtrans_op),
+    WG_FN("conv_op", py_conv_op),
+    {nullptr, nullptr, 0, nullptr},
+};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__native() { return PyModule_Create(&module); }

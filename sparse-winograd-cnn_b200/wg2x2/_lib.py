@@ -73,6 +73,12 @@ for _name, (_res, _args) in _SIGS.items():
 EXPORTS = tuple(_SIGS)
 
 
+NATIVE_PATH = os.path.join(_HERE, "_native.so")
+if not os.path.exists(NATIVE_PATH):
+    raise ImportError("%s not found; build it with `python %s`. There is no fallback path."
+                      % (NATIVE_PATH, os.path.join(os.path.dirname(_HERE), "build.py")))
+
+
 def check(status, what):
     if status != OK:
         raise Wg2x2Error(status, what)
