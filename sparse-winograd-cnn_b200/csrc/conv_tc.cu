@@ -634,7 +634,11 @@ static CUresult encode_cached(CUtensorMap *map, CUtensorMapDataType dtype, cuuin
         if (cache[e].used && memcmp(&cache[e].key, &k, sizeof(k)) == 0) { *map = cache[e].map; return CUDA_SUCCESS; }
     EncodeTiledFn fn = encode_fn_raw();
     if (!fn) return CUDA_ERROR_NOT_SUPPORTED;
-    const CUresult r = fn(map, dtype, rank, ptr, dims, strides, box, estr, il, sw, promo, oob);
+    CUresult r = fn(map, dtype, rank, ptr, dims, strides, box, estr, il, sw, promo, oob);
+    // a driver call on a thread that has not yet run anything on the device finds no context (an autograd thread whose
+    // first call is this one): have the runtime bind it and ask again
+    if ((r == CUDA_ERROR_INVALID_CONTEXT || r == CUDA_ERROR_NOT_INITIALIZED) && cudaFree(nullptr) == cudaSuccess)
+        r = fn(map, dtype, rank, ptr, dims, strides, box, estr, il, sw, promo, oob);
     if (r == CUDA_SUCCESS) {
         Entry &en = cache[next];
         next = (next + 1) % kEntries;
@@ -643,6 +647,33 @@ static CUresult encode_cached(CUtensorMap *map, CUtensorMapDataType dtype, cuuin
     return r;
 }
 static EncodeTiledFn encode_fn() { return encode_fn_raw() ? &encode_cached : nullptr; }
+
+// Dense fp32 map with unit element strides, for the kernels of the other source files
+bool tensor_map_f32(CUtensorMap *map, int rank, const float *ptr, const cuuint64_t *dims, const cuuint64_t *strides, const cuuint32_t *box,
+                    CUtensorMapSwizzle swizzle)
+{
+    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    EncodeTiledFn fn = encode_fn();
+    return fn && fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, (cuuint32_t)rank, const_cast<float *>(ptr), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// The status word of the current device, for those kernels' bounded waits (NULL: it cannot be had)
+unsigned int *tc_status_word()
+{
+    static std::atomic<unsigned int *> known[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+    unsigned int *p = known[dev].load(std::memory_order_acquire);
+    if (!p) {
+        void *a = nullptr;
+        if (cudaGetSymbolAddress(&a, g_tc_status) != cudaSuccess) return nullptr;
+        p = static_cast<unsigned int *>(a);
+        known[dev].store(p, std::memory_order_release);
+    }
+    return p;
+}
+uint32_t tc_wait_limit() { return wait_limit(); }
 
 // 3-D map over a (16, rows, C) fp32 tensor, C contiguous: box = 32 x box_rows x 1, 128-B swizzle,
 // out-of-range elements read as zero.
