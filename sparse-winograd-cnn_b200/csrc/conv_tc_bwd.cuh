@@ -51,42 +51,53 @@ __global__ void __launch_bounds__(256) conv_dm_nhwc_kernel(const float *__restri
                 make_float4(round_tf32(m0[i][j]), round_tf32(m1[i][j]), round_tf32(m2[i][j]), round_tf32(m3[i][j]));
 }
 
-// NCHW: a CTA stages a band of 2R rows of dY for 32 channels (one contiguous run per channel), then walks
-// tiles with lane = channel so that the plane stores are contiguous along K.  Any layout/width: R >= 1.
+// NCHW: a CTA stages a band of 2R rows of dY (or two rows of a segment of S tiles) for 32 channels, then walks tiles with
+// lane = channel so that the plane stores are contiguous along K.  Any layout/width: R >= 1.
+template <bool SEG>
 __global__ void __launch_bounds__(256) conv_dm_nchw_kernel(const float *__restrict__ dY, float *__restrict__ dM, long long P, int nH,
-                                                             int nW, int H, int W, int K, int R, int nbands, int pitch)
+                                                             int nW, int H, int W, int K, int R, int nbands, int S_, int nsegs, int pitch)
 {
     extern __shared__ float S[];
-    const int band = blockIdx.x % nbands;
-    const int b = blockIdx.x / nbands;
+    int bb = blockIdx.x;
+    const int seg = SEG ? bb % nsegs : 0;
+    if (SEG) bb /= nsegs;
+    const int band = bb % nbands;
+    const int b = bb / nbands;
     const int k0 = blockIdx.y * 32;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int th0 = band * R;
     const int rows_tile = min(R, nH - th0);
+    const int tw0 = SEG ? seg * S_ : 0, ns = SEG ? min(S_, nW - tw0) : nW;
+    const int w0 = 2 * tw0, SW = SEG ? min(2 * ns, W - w0) : W;      // pixels of a staged row
     const int lo = 2 * th0, hi = min(2 * th0 + 2 * rows_tile, H);
-    const int nfill = (hi - lo) * W;
+    const int nfill = (hi - lo) * SW;
     for (int kk = warp; kk < 32; kk += 8) {
         if (k0 + kk >= K) break;
-        const float *src = dY + (((long long)b * K + k0 + kk) * H + lo) * W;
+        const float *src = dY + (((long long)b * K + k0 + kk) * H + lo) * W + w0;
         float *dst = S + kk * pitch;
-        for (int i = lane; i < nfill; i += 32) dst[i] = __ldg(src + i);
+        if (!SEG) {
+            for (int i = lane; i < nfill; i += 32) dst[i] = __ldg(src + i);
+        } else {                                             // two rows of a segment
+            for (int i = lane; i < nfill; i += 32) dst[i] = __ldg(src + (i >= SW ? W + i - SW : i));
+        }
     }
     __syncthreads();
     if (k0 + lane >= K) return;
     const float *Sk = S + lane * pitch;
-    for (int q = warp; q < rows_tile * nW; q += 8) {
-        const int tr = q / nW, tw = q - tr * nW;
+#pragma unroll 1
+    for (int q = warp; q < rows_tile * ns; q += 8) {
+        const int tr = q / ns, tl = q - tr * ns;
         float g[2][2];
 #pragma unroll
         for (int a = 0; a < 2; ++a)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                const int h = lo + 2 * tr + a, w = 2 * tw + e;
-                g[a][e] = (h < H && w < W) ? Sk[(2 * tr + a) * W + w] : 0.f;
+                const int h = lo + 2 * tr + a, w = 2 * tl + e;
+                g[a][e] = (h < H && w < SW) ? Sk[(2 * tr + a) * SW + w] : 0.f;
             }
         float m[4][4];
         a_g_at(g[0][0], g[0][1], g[1][0], g[1][1], m);
-        const long long p = ((long long)b * nH + th0 + tr) * nW + tw;
+        const long long p = ((long long)b * nH + th0 + tr) * nW + tw0 + tl;
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -214,16 +225,17 @@ static int launch_dm(const float *dY, float *dM, int B, int H, int W, int K, int
             return WG2X2_ERR_LAUNCH;
         conv_dm_nchw_vec_kernel<32><<<grid, 256, smem, st>>>(dY, dM, P, nH, nW, H, W, K, R, nbands, pitch);
     } else {
-        int R = 384 / (2 * W);
-        if (R < 1) R = 1;
-        if (R > nH) R = nH;
-        const int nbands = cdiv(nH, R);
-        const int pitch = (2 * R * W) | 1;
+        const BandCut cut = cut_bands(nH, nW, (long long)B * cdiv(K, 32), 384 / (2 * W));
+        const int pitch = (2 * cut.R * (cut.nsegs == 1 ? W : 2 * cut.S)) | 1;
         const int smem = 32 * pitch * (int)sizeof(float);
-        if ((long long)B * nbands > 0x7fffffffLL || smem > 200 * 1024) return WG2X2_ERR_UNSUPPORTED;
-        if (cudaFuncSetAttribute(conv_dm_nchw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-            return WG2X2_ERR_LAUNCH;
-        conv_dm_nchw_kernel<<<dim3((unsigned)(B * nbands), cdiv(K, 32)), 256, smem, st>>>(dY, dM, P, nH, nW, H, W, K, R, nbands, pitch);
+        const long long blocks = (long long)B * cut.nbands * cut.nsegs;
+        if (blocks > 0x7fffffffLL || smem > 200 * 1024) return WG2X2_ERR_UNSUPPORTED;
+        auto launch = [&](auto kernel) -> bool {
+            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return false;
+            kernel<<<dim3((unsigned)blocks, cdiv(K, 32)), 256, smem, st>>>(dY, dM, P, nH, nW, H, W, K, cut.R, cut.nbands, cut.S, cut.nsegs, pitch);
+            return true;
+        };
+        if (!(cut.nsegs == 1 ? launch(conv_dm_nchw_kernel<false>) : launch(conv_dm_nchw_kernel<true>))) return WG2X2_ERR_LAUNCH;
     }
     return launch_status();
 }

@@ -412,10 +412,10 @@ __global__ void __launch_bounds__(256) imtrans_bwd_nchw_kernel(const float *__re
 // all the block's channels.  VEC = 4 reads dV (and the ReLU mask) with 16-byte loads: LC = 32 lanes along the
 // channels (128 per block, 512 bytes per request) where such a band fits four blocks per SM, else LC = 16 (64
 // channels per block, the two halves of a warp on two tiles at once).
-template <int VEC, int LC, bool MASK>
+template <int VEC, int LC, bool MASK, bool SEG>
 __global__ void __launch_bounds__(256, 4) imtrans_bwd_nchw_band_kernel(const float *__restrict__ dV, const float *__restrict__ Vm,
                                                                          float *__restrict__ dX, int B, int H, int W, int C, int nH,
-                                                                         int nW, int R, int nbands, int pitch)
+                                                                         int nW, int R, int nbands, int S, int nsegs, int pitch)
 {
     using T = typename Vec<VEC>::type;
     constexpr int CB = LC * VEC;             // channels per block
@@ -434,18 +434,22 @@ __global__ void __launch_bounds__(256, 4) imtrans_bwd_nchw_band_kernel(const flo
         c0 = (int)(blockIdx.x % ncb) * CB;
         bb = blockIdx.x / ncb;
     }
+    const int seg = SEG ? bb % nsegs : 0;
+    if (SEG) bb /= nsegs;
     const int band = bb % nbands;
     const int b = bb / nbands;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int lc = lane % LC, lq = lane / LC;
     const int th0 = band * R;
     const int rows_blk = min(R, nH - th0);
+    const int tw0 = SEG ? seg * S : 0, ns = SEG ? min(S, nW - tw0) : nW;   // tile columns of the block
+    const int OW = SEG ? min(2 * ns, W - 2 * tw0) : W;                     // pixels of an output row
     const int CV = C / VEC;
     const long long plane = (long long)B * nH * nW * CV;
     const bool c_ok = c0 + VEC * lc < C;
 #pragma unroll 1
-    for (int q = warp * QW + lq; q < rows_blk * nW; q += 8 * QW) {
-        const int br = q / nW, bw = q - br * nW;
+    for (int q = warp * QW + lq; q < rows_blk * ns; q += 8 * QW) {
+        const int br = q / ns, bl = q - br * ns, bw = tw0 + bl;
         T out[2][2];
 #pragma unroll
         for (int a = 0; a < 2; ++a)
@@ -459,13 +463,13 @@ __global__ void __launch_bounds__(256, 4) imtrans_bwd_nchw_band_kernel(const flo
 #pragma unroll
             for (int e = 0; e < 2; ++e)
                 if (2 * bw + e < W) {
-                    float *o = O + VEC * lc * pitch + (2 * br + a) * W + 2 * bw + e;
+                    float *o = O + VEC * lc * pitch + (2 * br + a) * OW + 2 * bl + e;
                     put_lanes(o, pitch, out[a][e]);
                 }
     }
     __syncthreads();
     const int lo = 2 * th0, hi = min(2 * th0 + 2 * rows_blk, H);
-    const int n = (hi - lo) * W;
+    const int n = (hi - lo) * OW;
     const int nch = min(CB, C - c0);
     if (n == H * W) {
         // the block's channels are one run of nch * H * W floats
@@ -478,7 +482,11 @@ __global__ void __launch_bounds__(256, 4) imtrans_bwd_nchw_band_kernel(const flo
         for (int cc = warp; cc < nch; cc += 8) {
             float *dst = dX + (((long long)b * C + c0 + cc) * H + lo) * W;
             const float *src = O + cc * pitch;
-            for (int i = lane; i < n; i += 32) dst[i] = src[i];
+            if (!SEG) {
+                for (int i = lane; i < n; i += 32) dst[i] = src[i];
+            } else {                                         // two rows of a segment
+                for (int i = lane; i < n; i += 32) dst[(i >= OW ? W : 0) + 2 * tw0 + (i >= OW ? i - OW : i)] = src[i];
+            }
         }
     }
 }
@@ -802,24 +810,24 @@ int imtrans_bwd(const float *dV, const float *Vm, float *dX, int B, int H, int W
             const bool wide = vec_ok && C >= 128 && 2 * W <= kBandFloats / 4 && ctas(128, kBandFloats / 4) >= fill;
             const bool vec = wide || (vec_ok && ctas(64, kBandFloats / 2) >= fill);
             const int cb = wide ? 128 : (vec ? 64 : 32);
-            int R = (wide ? kBandFloats / 4 : (vec ? kBandFloats / 2 : kBandFloats)) / (2 * W);
-            if (R < 1) R = 1;
-            if (R > nH) R = nH;
-            const int nbands = cdiv(nH, R);
-            R = cdiv(nH, nbands);                              // bands of even height
-            const int pitch = (2 * R * W) | 1;
+            const int max_rows = (wide ? kBandFloats / 4 : (vec ? kBandFloats / 2 : kBandFloats)) / (2 * W);
+            const BandCut cut = cut_bands(nH, nW, (long long)B * cdiv(C, cb), max_rows);
+            const int pitch = (2 * cut.R * (cut.nsegs == 1 ? W : 2 * cut.S)) | 1;
             const int smem = cb * pitch * (int)sizeof(float);
-            if ((long long)B * nbands * cdiv(C, cb) > 0x7fffffffLL || cdiv(C, cb) > 65535) return WG2X2_ERR_UNSUPPORTED;
-            const dim3 grid = Vm ? dim3((unsigned)(B * nbands), cdiv(C, cb)) : dim3((unsigned)(B * nbands * cdiv(C, cb)));
+            const long long blocks = (long long)B * cut.nbands * cut.nsegs;
+            if (blocks * cdiv(C, cb) > 0x7fffffffLL || cdiv(C, cb) > 65535) return WG2X2_ERR_UNSUPPORTED;
+            const dim3 grid = Vm ? dim3((unsigned)blocks, cdiv(C, cb)) : dim3((unsigned)(blocks * cdiv(C, cb)));
             auto launch = [&](auto kernel) -> bool {
                 if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return false;
-                kernel<<<grid, 256, smem, st>>>(dV, Vm, dX, B, H, W, C, nH, nW, R, nbands, pitch);
+                kernel<<<grid, 256, smem, st>>>(dV, Vm, dX, B, H, W, C, nH, nW, cut.R, cut.nbands, cut.S, cut.nsegs, pitch);
                 return true;
             };
+            // (the kernels with wider blocks are only taken where those already fill the GPU: they have no segments)
             const bool launched =
-                wide ? (Vm ? launch(imtrans_bwd_nchw_band_kernel<4, 32, true>) : launch(imtrans_bwd_nchw_band_kernel<4, 32, false>))
-                : vec ? (Vm ? launch(imtrans_bwd_nchw_band_kernel<4, 16, true>) : launch(imtrans_bwd_nchw_band_kernel<4, 16, false>))
-                      : (Vm ? launch(imtrans_bwd_nchw_band_kernel<1, 32, true>) : launch(imtrans_bwd_nchw_band_kernel<1, 32, false>));
+                wide ? (Vm ? launch(imtrans_bwd_nchw_band_kernel<4, 32, true, false>) : launch(imtrans_bwd_nchw_band_kernel<4, 32, false, false>))
+                : vec ? (Vm ? launch(imtrans_bwd_nchw_band_kernel<4, 16, true, false>) : launch(imtrans_bwd_nchw_band_kernel<4, 16, false, false>))
+                : cut.nsegs == 1 ? (Vm ? launch(imtrans_bwd_nchw_band_kernel<1, 32, true, false>) : launch(imtrans_bwd_nchw_band_kernel<1, 32, false, false>))
+                                 : (Vm ? launch(imtrans_bwd_nchw_band_kernel<1, 32, true, true>) : launch(imtrans_bwd_nchw_band_kernel<1, 32, false, true>));
             if (!launched) return WG2X2_ERR_LAUNCH;
             return launch_status();
         }

@@ -73,17 +73,6 @@ __device__ __forceinline__ void a_g_at(float g00, float g01, float g10, float g1
         dm[i][3] = -u[i][1];
     }
 }
-// one Winograd row i of the above (j = 0..3), used by kernels that walk the rows in turn
-__device__ __forceinline__ void a_g_at_row(int i, float g00, float g01, float g10, float g11, float (&dm)[4])
-{
-    float u0, u1;
-    if (i == 0)      { u0 = g00;        u1 = g01; }
-    else if (i == 1) { u0 = g00 + g10;  u1 = g01 + g11; }
-    else if (i == 2) { u0 = g00 - g10;  u1 = g01 - g11; }
-    else             { u0 = -g10;       u1 = -g11; }
-    dm[0] = u0; dm[1] = u0 + u1; dm[2] = u0 - u1; dm[3] = -u1;
-}
-
 // B^T as compile-time coefficients (for the gather in the input-transform gradient)
 __host__ __device__ constexpr int bt_coef(int i, int y)
 {
@@ -91,6 +80,29 @@ __host__ __device__ constexpr int bt_coef(int i, int y)
          : (i == 1) ? ((y == 1 || y == 2) ? 1 : 0)
          : (i == 2) ? (y == 1 ? -1 : (y == 2 ? 1 : 0))
                     : (y == 1 ? 1 : (y == 3 ? -1 : 0));
+}
+
+// How the NCHW kernels that walk tiles with lane = channel cut an image: bands of R tile rows, and, where a band is a single
+// row, segments of S tiles along it.  `blocks`: CTAs per band (images x channel blocks).  A small problem is cut until the
+// grid gives every SM a few CTAs (a warp's tiles are a serial chain of loads: 3 x 27 x 27 x 32 channels took 25 us in 6 CTAs,
+// whatever the bytes); eight warps share a block's tiles, so segments end at 8.
+struct BandCut {
+    int R, nbands, S, nsegs;
+};
+inline BandCut cut_bands(int nH, int nW, long long blocks, int max_rows)
+{
+    BandCut c;
+    c.R = max_rows < 1 ? 1 : (max_rows > nH ? nH : max_rows);
+    while (c.R > 1 && blocks * cdiv(nH, c.R) < 3LL * kNumSMs) --c.R;
+    c.nbands = cdiv(nH, c.R);
+    c.R = cdiv(nH, c.nbands);                 // bands of even height
+    c.nbands = cdiv(nH, c.R);
+    c.nsegs = 1;
+    if (c.R == 1)
+        while (cdiv(nW, c.nsegs) > 8 && blocks * c.nbands * c.nsegs < 3LL * kNumSMs) ++c.nsegs;
+    c.S = cdiv(nW, c.nsegs);
+    c.nsegs = cdiv(nW, c.S);
+    return c;
 }
 
 inline int launch_status()
