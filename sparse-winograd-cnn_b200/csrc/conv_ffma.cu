@@ -298,6 +298,7 @@ __global__ void __launch_bounds__(kFfThreads, 1) conv_fwd_ffma_kernel(const __gr
                                                                        const float *__restrict__ Wt, float *__restrict__ Y, FfGrid g, int C,
                                                                        int K, FfWait wt)
 {
+    after_previous_kernel(V, Wt, Y);
     using T = FfTile<MT>;
     uint32_t bar;
     float *smem = ff_shared(bar);
@@ -460,6 +461,7 @@ __global__ void __launch_bounds__(kFfThreads, 1) conv_dv_ffma_kernel(const __gri
                                                                       const float *__restrict__ Wt, const float *__restrict__ dY,
                                                                       float *__restrict__ dV, FfGrid g, int C, int K, int relu, FfWait wt)
 {
+    after_previous_kernel(Vsaved, Wt, dY, dV);
     using T = FfTile<MT>;
     uint32_t bar;
     float *As = ff_shared(bar), *Bs = As + 2 * kFfWarps * T::A, *raw = Bs + 2 * kFfWarps * kFfB;
@@ -553,6 +555,7 @@ __global__ void __launch_bounds__(kFfThreads, 1) conv_dw_ffma_kernel(const __gri
                                                                       float *__restrict__ out, FfGrid g, int C, int K, int chunks_per_split,
                                                                       int direct, FfWait wt)
 {
+    after_previous_kernel(V, dY, mask, out);
     using T = FfTile<MT>;
     uint32_t bar;
     float *As = ff_shared(bar), *Bs = As + 2 * kFfWarps * T::A, *raw = Bs + 2 * kFfWarps * kFfB;
@@ -629,6 +632,7 @@ __global__ void __launch_bounds__(kFfThreads, 1) conv_dw_ffma_kernel(const __gri
 __global__ void __launch_bounds__(256) conv_dw_reduce_kernel(const float *__restrict__ partial, const float *__restrict__ mask,
                                                                float *__restrict__ dW, long long n, int splits)
 {
+    after_previous_kernel(partial, mask, dW);
     for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += (long long)gridDim.x * blockDim.x) {
         float s = 0.f;
         for (int sp = 0; sp < splits; ++sp) s += partial[(long long)sp * n + idx];
@@ -640,7 +644,7 @@ __global__ void __launch_bounds__(256) conv_dw_reduce_kernel(const float *__rest
 void dw_reduce_launch(const float *partial, const float *mask, float *dW, long long n, int splits, cudaStream_t st)
 {
     const int blocks = (int)min((long long)kNumSMs * 8, cdivll(n, 256));
-    conv_dw_reduce_kernel<<<blocks, 256, 0, st>>>(partial, mask, dW, n, splits);
+    launch(conv_dw_reduce_kernel, dim3((unsigned)blocks), 256, 0, st, partial, mask, dW, n, splits);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -664,14 +668,6 @@ bool tensor_map_f32(CUtensorMap *map, int rank, const float *ptr, const cuuint64
 unsigned int *tc_status_word();
 uint32_t tc_wait_limit();
 static FfWait ff_wait_args() { return FfWait{tc_status_word(), tc_wait_limit()}; }
-
-template <typename Kernel, typename... Args>
-static int ff_launch(Kernel kernel, dim3 grid, int smem, cudaStream_t st, Args... args)
-{
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return WG2X2_ERR_LAUNCH;
-    kernel<<<grid, kFfThreads, smem, st>>>(args...);
-    return launch_status();
-}
 
 // A (16, rows, cols) matrix, columns contiguous: box of box_cols x box_rows of one position
 static bool ff_map(CUtensorMap *m, const float *p, long long cols, long long rows, int box_cols, int box_rows, CUtensorMapSwizzle swizzle)
@@ -697,7 +693,7 @@ int conv_fwd_ffma(const float *V, const float *Wt, float *Y, int B, int nH, int 
         return WG2X2_ERR_LAUNCH;
     const FfWait wt = ff_wait_args();
     if (!wt.status) return WG2X2_ERR_LAUNCH;
-#define WG_FF(MT, VEC, L) ff_launch(conv_fwd_ffma_kernel<MT, VEC, L>, grid, FfTile<MT>::kFwdBytes, st, mapV, mapW, V, Wt, Y, g, C, K, wt)
+#define WG_FF(MT, VEC, L) launch(conv_fwd_ffma_kernel<MT, VEC, L>, grid, kFfThreads, FfTile<MT>::kFwdBytes, st, mapV, mapW, V, Wt, Y, g, C, K, wt)
 #define WG_FF_L(MT, VEC) (layout == WG2X2_NHWC ? WG_FF(MT, VEC, WG2X2_NHWC) : WG_FF(MT, VEC, WG2X2_NCHW))
 #define WG_FF_V(MT) (vec ? WG_FF_L(MT, true) : WG_FF_L(MT, false))
     return mt == 8 ? WG_FF_V(8) : mt == 4 ? WG_FF_V(4) : WG_FF_V(2);
@@ -716,7 +712,7 @@ int conv_dv_ffma(const float *V, const float *Wt, const float *dY, float *dV, in
     if (vec && !ff_map(&mapW, Wt, K, C, kFfKC, kFfN, CU_TENSOR_MAP_SWIZZLE_64B)) return WG2X2_ERR_LAUNCH;
     const FfWait wt = ff_wait_args();
     if (!wt.status) return WG2X2_ERR_LAUNCH;
-#define WG_FF(MT, VEC, L) ff_launch(conv_dv_ffma_kernel<MT, VEC, L>, grid, FfTile<MT>::kDvBytes, st, mapW, V, Wt, dY, dV, g, C, K, relu, wt)
+#define WG_FF(MT, VEC, L) launch(conv_dv_ffma_kernel<MT, VEC, L>, grid, kFfThreads, FfTile<MT>::kDvBytes, st, mapW, V, Wt, dY, dV, g, C, K, relu, wt)
     return mt == 8 ? WG_FF_V(8) : mt == 4 ? WG_FF_V(4) : WG_FF_V(2);
 #undef WG_FF
 }
@@ -760,7 +756,7 @@ int conv_dw_ffma(const float *V, const float *dY, const float *mask, float *dW, 
     if (vec && !ff_map(&mapV, V, C, g.P, 8 * mt, kFfKC, CU_TENSOR_MAP_SWIZZLE_NONE)) return WG2X2_ERR_LAUNCH;
     const FfWait wt = ff_wait_args();
     if (!wt.status) return WG2X2_ERR_LAUNCH;
-#define WG_FF(MT, VEC, L) ff_launch(conv_dw_ffma_kernel<MT, VEC, L>, grid, FfTile<MT>::kDwBytes, st, mapV, V, dY, mask, out, g, C, K, cps, direct, wt)
+#define WG_FF(MT, VEC, L) launch(conv_dw_ffma_kernel<MT, VEC, L>, grid, kFfThreads, FfTile<MT>::kDwBytes, st, mapV, V, dY, mask, out, g, C, K, cps, direct, wt)
     const int s = mt == 8 ? WG_FF_V(8) : mt == 4 ? WG_FF_V(4) : WG_FF_V(2);
 #undef WG_FF
 #undef WG_FF_L

@@ -200,6 +200,7 @@ __host__ __device__ constexpr uint32_t make_idesc_tf32(int M, int N)
 __global__ void __launch_bounds__(256) pack_weights_kernel(const float *__restrict__ Wt, float *__restrict__ Wp,
                                                              unsigned long long *__restrict__ masks, int C, int K, int nKB, int nCC)
 {
+    after_previous_kernel(Wt, Wp, masks);
     __shared__ float tile[32][33];
     __shared__ int any;
     const int t = blockIdx.z;
@@ -285,6 +286,8 @@ conv_fwd_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr_slot, 0);
+    // (set-up touched no global memory; from here on the kernel reads and writes it)
+    wait_for_previous_kernel(kNumSMs / 2);
 
     const int nCC = prm.nCC;
 
@@ -714,7 +717,7 @@ int weights_prepare(const float *Wt, int C, int K, void *prepared, size_t bytes,
     if (cudaMemsetAsync(masks, nCC <= 64 ? 0 : 0xFF, (size_t)16 * nKB * sizeof(unsigned long long), st) != cudaSuccess)
         return WG2X2_ERR_LAUNCH;
     dim3 grid(cdiv(K, 32), cdiv(C, 32), 16);
-    pack_weights_kernel<<<grid, 256, 0, st>>>(Wt, Wp, masks, C, K, nKB, nCC);
+    launch(pack_weights_kernel, grid, 256, 0, st, Wt, Wp, masks, C, K, nKB, nCC);
     return launch_status();
 }
 
@@ -754,18 +757,10 @@ static int tc_launch(int layout, const float *A, const float *Bop, const unsigne
     if (!make_map(&mapA, A, contr, P, kBlockM)) return WG2X2_ERR_LAUNCH;
     if (!make_map(&mapB, Bop, contr, ncols, kBlockN)) return WG2X2_ERR_LAUNCH;
     const int grid = prm.units < kNumSMs ? prm.units : kNumSMs;
-#define WG_TC_LAUNCH(L, X)                                                                                              \
-    do {                                                                                                                \
-        if (cudaFuncSetAttribute(conv_fwd_tc_kernel<L, X>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) !=  \
-            cudaSuccess)                                                                                                \
-            return WG2X2_ERR_LAUNCH;                                                                                    \
-        conv_fwd_tc_kernel<L, X><<<grid, kFwdThreads, kSmemBytes, st>>>(mapA, mapB, prm);                               \
-    } while (0)
     const bool extras = out_scale || residual;
-    if (layout == WG2X2_NHWC) { if (extras) WG_TC_LAUNCH(WG2X2_NHWC, true); else WG_TC_LAUNCH(WG2X2_NHWC, false); }
-    else                      { if (extras) WG_TC_LAUNCH(WG2X2_NCHW, true); else WG_TC_LAUNCH(WG2X2_NCHW, false); }
-#undef WG_TC_LAUNCH
-    return launch_status();
+    auto *kernel = layout == WG2X2_NHWC ? (extras ? conv_fwd_tc_kernel<WG2X2_NHWC, true> : conv_fwd_tc_kernel<WG2X2_NHWC, false>)
+                                        : (extras ? conv_fwd_tc_kernel<WG2X2_NCHW, true> : conv_fwd_tc_kernel<WG2X2_NCHW, false>);
+    return launch(kernel, dim3((unsigned)grid), kFwdThreads, kSmemBytes, st, mapA, mapB, prm);
 }
 
 int conv_fwd_tc_prepared(const float *V, const void *prepared, float *Y, int B, int nH, int nW, int C, int K, int outH, int outW,

@@ -23,6 +23,7 @@ __device__ __forceinline__ float round_tf32(float x)
 __global__ void __launch_bounds__(256) conv_dm_nhwc_kernel(const float *__restrict__ dY, float *__restrict__ dM, long long P, int nH,
                                                              int nW, int H, int W, int K)
 {
+    after_previous_kernel(dY, dM);
     const int KV = K >> 2;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= P * KV) return;
@@ -57,6 +58,7 @@ template <bool SEG>
 __global__ void __launch_bounds__(256) conv_dm_nchw_kernel(const float *__restrict__ dY, float *__restrict__ dM, long long P, int nH,
                                                              int nW, int H, int W, int K, int R, int nbands, int S_, int nsegs, int pitch)
 {
+    after_previous_kernel(dY, dM);
     extern __shared__ float S[];
     int bb = blockIdx.x;
     const int seg = SEG ? bb % nsegs : 0;
@@ -113,6 +115,7 @@ template <int LC>
 __global__ void __launch_bounds__(256, 3) conv_dm_nchw_vec_kernel(const float *__restrict__ dY, float *__restrict__ dM, long long P, int nH,
                                                                     int nW, int H, int W, int K, int R, int nbands, int pitch)
 {
+    after_previous_kernel(dY, dM);
     constexpr int CB = 4 * LC, QW = 32 / LC;
     extern __shared__ float S[];
     const int band = blockIdx.x % nbands;
@@ -175,6 +178,7 @@ __global__ void __launch_bounds__(256, 3) conv_dm_nchw_vec_kernel(const float *_
 __global__ void __launch_bounds__(256) round_and_map_kernel(const float *__restrict__ Wt, float *__restrict__ Wr,
                                                               unsigned long long *__restrict__ map, int C, int K, int nKB, int nCC)
 {
+    after_previous_kernel(Wt, Wr, map);
     const int kb = blockIdx.x, cc = blockIdx.y, t = blockIdx.z;
     int nz = 0;
     if ((K & 3) == 0 && ((reinterpret_cast<uintptr_t>(Wt) | reinterpret_cast<uintptr_t>(Wr)) & 15u) == 0) {
@@ -210,7 +214,7 @@ static int launch_dm(const float *dY, float *dM, int B, int H, int W, int K, int
     const int nH = (H + 1) / 2, nW = (W + 1) / 2;
     const long long P = (long long)B * nH * nW;
     if (layout == WG2X2_NHWC) {
-        conv_dm_nhwc_kernel<<<(unsigned)cdivll(P * (K / 4), 256), 256, 0, st>>>(dY, dM, P, nH, nW, H, W, K);
+        launch(conv_dm_nhwc_kernel, dim3((unsigned)cdivll(P * (K / 4), 256)), 256, 0, st, dY, dM, P, nH, nW, H, W, K);
     } else if (K % 4 == 0 && K >= 128 && 2 * nH * W <= 96 && (reinterpret_cast<uintptr_t>(dM) & 15u) == 0 &&
                (long long)B * cdiv(K, 128) >= 4LL * kNumSMs) {
         // Four channels per lane, 128 per CTA, where the whole image is one small band and the CTAs fill the GPU
@@ -221,21 +225,15 @@ static int launch_dm(const float *dY, float *dM, int B, int H, int W, int K, int
         const int smem = 128 * pitch * (int)sizeof(float);
         if ((long long)B > 0x7fffffffLL || cdiv(K, 128) > 65535) return WG2X2_ERR_UNSUPPORTED;
         const dim3 grid((unsigned)B, cdiv(K, 128));
-        if (cudaFuncSetAttribute(conv_dm_nchw_vec_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-            return WG2X2_ERR_LAUNCH;
-        conv_dm_nchw_vec_kernel<32><<<grid, 256, smem, st>>>(dY, dM, P, nH, nW, H, W, K, R, nbands, pitch);
+        launch(conv_dm_nchw_vec_kernel<32>, dim3(grid), 256, smem, st, dY, dM, P, nH, nW, H, W, K, R, nbands, pitch);
     } else {
         const BandCut cut = cut_bands(nH, nW, (long long)B * cdiv(K, 32), 384 / (2 * W));
         const int pitch = (2 * cut.R * (cut.nsegs == 1 ? W : 2 * cut.S)) | 1;
         const int smem = 32 * pitch * (int)sizeof(float);
         const long long blocks = (long long)B * cut.nbands * cut.nsegs;
         if (blocks > 0x7fffffffLL || smem > 200 * 1024) return WG2X2_ERR_UNSUPPORTED;
-        auto launch = [&](auto kernel) -> bool {
-            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return false;
-            kernel<<<dim3((unsigned)blocks, cdiv(K, 32)), 256, smem, st>>>(dY, dM, P, nH, nW, H, W, K, cut.R, cut.nbands, cut.S, cut.nsegs, pitch);
-            return true;
-        };
-        if (!(cut.nsegs == 1 ? launch(conv_dm_nchw_kernel<false>) : launch(conv_dm_nchw_kernel<true>))) return WG2X2_ERR_LAUNCH;
+        launch(cut.nsegs == 1 ? conv_dm_nchw_kernel<false> : conv_dm_nchw_kernel<true>, dim3((unsigned)blocks, cdiv(K, 32)), 256, smem, st, dY, dM,
+               P, nH, nW, H, W, K, cut.R, cut.nbands, cut.S, cut.nsegs, pitch);
     }
     return launch_status();
 }
@@ -397,6 +395,8 @@ conv_grad_gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr_slot, 0);
+    // (set-up touched no global memory; from here on the kernel reads and writes it)
+    wait_for_previous_kernel(kNumSMs / 2);
 
     const int N = prm.N;
     // unit -> (split, t, row block, column block); column block fastest so that neighbouring CTAs share the A tile in L2
@@ -731,13 +731,11 @@ static int gg_launch(const CUtensorMap &mapA, const CUtensorMap &mapB, GgParams 
         p2.nRB = cdiv(prm.nRB, 2);
         p2.units = prm.units / prm.nRB * p2.nRB;
         const int pairs = p2.units < nclusters ? p2.units : nclusters;
-        conv_grad_gemm_tc2_kernel<KIND><<<2 * pairs, kTcThreads, kGg2SmemBytes, st>>>(mapA, mapB_half ? *mapB_half : mapB, mapOut, p2);
+        launch(conv_grad_gemm_tc2_kernel<KIND>, dim3(2 * pairs), kTcThreads, kGg2SmemBytes, st, mapA, mapB_half ? *mapB_half : mapB, mapOut, p2);
         return launch_status();
     }
-    if (cudaFuncSetAttribute(conv_grad_gemm_tc_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGgSmemBytes) != cudaSuccess)
-        return WG2X2_ERR_LAUNCH;
     const int grid = prm.units < kNumSMs ? prm.units : kNumSMs;
-    conv_grad_gemm_tc_kernel<KIND><<<grid, kTcThreads, kGgSmemBytes, st>>>(mapA, mapB, mapOut, prm);
+    launch(conv_grad_gemm_tc_kernel<KIND>, dim3((unsigned)grid), kTcThreads, kGgSmemBytes, st, mapA, mapB, mapOut, prm);
     return launch_status();
 }
 
@@ -778,7 +776,7 @@ int conv_dv_tc(const float *V, const float *Wt, const float *dM, float *Wr, unsi
     const int nKB = cdiv(K, 64), nCC = cdiv(C, 32);
     if (nCC > 65535) return WG2X2_ERR_UNSUPPORTED;
     if (cudaMemsetAsync(map, nCC <= 64 ? 0 : 0xFF, (size_t)16 * nKB * sizeof(unsigned long long), st) != cudaSuccess) return WG2X2_ERR_LAUNCH;
-    round_and_map_kernel<<<dim3(nKB, nCC, 16), 256, 0, st>>>(Wt, Wr, map, C, K, nKB, nCC);
+    launch(round_and_map_kernel, dim3(nKB, nCC, 16), 256, 0, st, Wt, Wr, map, C, K, nKB, nCC);
     if (launch_status() != WG2X2_OK) return WG2X2_ERR_LAUNCH;
     GgParams prm;
     prm.rows = P; prm.cols = C; prm.contr = K;
@@ -849,6 +847,7 @@ struct OutExtras {
 __global__ void __launch_bounds__(256) out_transform_nhwc_kernel(const float *__restrict__ M, float *__restrict__ Y, long long P,
                                                                    int nH, int nW, int K, int outH, int outW, OutExtras ex)
 {
+    after_previous_kernel(M, Y, ex.scale, ex.shift, ex.residual);
     const int KV = K >> 2;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= P * KV) return;
@@ -893,6 +892,7 @@ __global__ void __launch_bounds__(256) out_transform_nchw_kernel(const float *__
                                                                    int nH, int nW, int K, int outH, int outW, int R, int nbands,
                                                                    int pitch, OutExtras ex)
 {
+    after_previous_kernel(M, Y, ex.scale, ex.shift, ex.residual);
     extern __shared__ float O[];
     const int band = blockIdx.x % nbands;
     const int b = blockIdx.x / nbands;
@@ -974,7 +974,7 @@ int conv_fwd_tc_wide(const float *V, const void *prepared, float *Y, int B, int 
     if (s != WG2X2_OK) return s;
     OutExtras ex{out_scale, out_shift, residual};
     if (layout == WG2X2_NHWC) {
-        out_transform_nhwc_kernel<<<(unsigned)cdivll(P * (K / 4), 256), 256, 0, st>>>(M, Y, P, nH, nW, K, outH, outW, ex);
+        launch(out_transform_nhwc_kernel, dim3((unsigned)cdivll(P * (K / 4), 256)), 256, 0, st, M, Y, P, nH, nW, K, outH, outW, ex);
     } else {
         int R = 384 / (2 * outW);
         if (R < 1) R = 1;
@@ -986,9 +986,7 @@ int conv_fwd_tc_wide(const float *V, const void *prepared, float *Y, int B, int 
         const int pitch = (2 * R * outW) | 1;
         const int smem = 32 * pitch * (int)sizeof(float);
         if ((long long)B * nbands > 0x7fffffffLL || smem > 200 * 1024) return WG2X2_ERR_UNSUPPORTED;
-        if (cudaFuncSetAttribute(out_transform_nchw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-            return WG2X2_ERR_LAUNCH;
-        out_transform_nchw_kernel<<<dim3((unsigned)(B * nbands), cdiv(K, 32)), 256, smem, st>>>(M, Y, P, nH, nW, K, outH, outW, R,
+        launch(out_transform_nchw_kernel, dim3((unsigned)(B * nbands), cdiv(K, 32)), 256, smem, st, M, Y, P, nH, nW, K, outH, outW, R,
                                                                                                  nbands, pitch, ex);
     }
     return launch_status();

@@ -904,26 +904,7 @@ int layer_fwd_fused(const float *X, const void *prepared, float *Y, int B, int H
     const int rounds = cdiv(p.units, kNumSMs);
     const int grid = cdiv(p.units, rounds);
     const bool extras = out_scale != nullptr, affine = in_scale != nullptr;
-    // Back-to-back layers: the next launch's scheduling and set-up overlap this kernel's tail (programmatic dependent
-    // launch; the kernel waits for its predecessor before its first global access).  Not while a graph is being
-    // captured, and WG2X2_PDL=0 in the environment turns it off.
-    static const bool pdl_env = [] { const char *e = getenv("WG2X2_PDL"); return !(e && e[0] == '0'); }();
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) return WG2X2_ERR_LAUNCH;
-    const bool pdl = pdl_env && capturing == cudaStreamCaptureStatusNone;
-    auto launch = [&](auto kernel) -> bool {
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFuSmemBytes) != cudaSuccess) return false;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)grid); cfg.blockDim = dim3((unsigned)kFuThreads);
-        cfg.dynamicSmemBytes = kFuSmemBytes; cfg.stream = st;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr; cfg.numAttrs = pdl ? 1 : 0;
-        return cudaLaunchKernelEx(&cfg, kernel, mapX1, mapX2, mapW, mapW2, mapY, p) == cudaSuccess;
-    };
-    const bool launched = extras ? (affine ? launch(layer_fwd_fused_kernel<true, true>) : launch(layer_fwd_fused_kernel<true, false>))
-                                 : (affine ? launch(layer_fwd_fused_kernel<false, true>) : launch(layer_fwd_fused_kernel<false, false>));
-    if (!launched) return WG2X2_ERR_LAUNCH;
-    return launch_status();
+    auto *kernel = extras ? (affine ? layer_fwd_fused_kernel<true, true> : layer_fwd_fused_kernel<true, false>)
+                          : (affine ? layer_fwd_fused_kernel<false, true> : layer_fwd_fused_kernel<false, false>);
+    return launch(kernel, dim3((unsigned)grid), kFuThreads, kFuSmemBytes, st, mapX1, mapX2, mapW, mapW2, mapY, p);
 }

@@ -119,6 +119,8 @@ conv_grad_gemm_tc2_kernel(const __grid_constant__ CUtensorMap mapA, const __grid
     cluster_sync_all();    // the partner's barriers exist before anything is signalled into them
     tc_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr_slot, 0);
+    // (set-up touched no global memory; from here on the kernel reads and writes it)
+    wait_for_previous_kernel(kNumSMs / 2);
 
     const int N = prm.N, NH = prm.N >> 1;          // each CTA holds half of the B tile's columns
     const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;

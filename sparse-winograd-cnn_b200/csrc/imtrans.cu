@@ -34,6 +34,7 @@ __global__ void __launch_bounds__(256) imtrans_fwd_nhwc_kernel(const float *__re
                                                                  int B, int H, int W, int C, int nH, int nW, int relu,
                                                                  const float *__restrict__ scale, const float *__restrict__ shift)
 {
+    after_previous_kernel(X, V, scale, shift);
     using T = typename Vec<VEC>::type;
     const int CV = C / VEC;
     const long long total = (long long)B * nH * nW * CV;
@@ -90,6 +91,7 @@ __global__ void __launch_bounds__(256) imtrans_fwd_nchw_kernel(const float *__re
                                                                  int B, int H, int W, int C, int nH, int nW, int relu,
                                                                  const float *__restrict__ scale, const float *__restrict__ shift)
 {
+    after_previous_kernel(X, V, scale, shift);
     __shared__ float S[kCCH * kChanPitch];
     const int nseg = cdiv(nW, kTSEG);
     int bx = blockIdx.x;
@@ -153,6 +155,7 @@ __global__ void __launch_bounds__(256) imtrans_fwd_nchw_band_kernel(const float 
                                                                       int R, int nbands, int pitch,
                                                                       const float *__restrict__ scale, const float *__restrict__ shift)
 {
+    after_previous_kernel(X, V, scale, shift);
     extern __shared__ float S[];   // [32 channels][pitch]
     const int band = blockIdx.x % nbands;
     const int b = blockIdx.x / nbands;
@@ -213,6 +216,7 @@ __global__ void __launch_bounds__(256, 3) imtrans_fwd_nchw_vec_kernel(const floa
                                                                         int R, int nbands, int pitch,
                                                                         const float *__restrict__ scale, const float *__restrict__ shift)
 {
+    after_previous_kernel(X, V, scale, shift);
     constexpr int CB = 4 * LC, QW = 32 / LC;
     extern __shared__ float S[];   // [CB channels][pitch]
     const int band = blockIdx.x % nbands;
@@ -342,6 +346,7 @@ template <int VEC, bool MASK>
 __global__ void __launch_bounds__(256) imtrans_bwd_nhwc_kernel(const float *__restrict__ dV, const float *__restrict__ Vm,
                                                                  float *__restrict__ dX, int B, int H, int W, int C, int nH, int nW)
 {
+    after_previous_kernel(dV, Vm, dX);
     using T = typename Vec<VEC>::type;
     const int CV = C / VEC;
     const long long total = (long long)B * nH * nW * CV;
@@ -371,6 +376,7 @@ template <bool MASK>
 __global__ void __launch_bounds__(256) imtrans_bwd_nchw_kernel(const float *__restrict__ dV, const float *__restrict__ Vm,
                                                                  float *__restrict__ dX, int B, int H, int W, int C, int nH, int nW)
 {
+    after_previous_kernel(dV, Vm, dX);
     constexpr int OP = 2 * kTSEG + 1;  // 65: odd pitch per (c,a) row
     __shared__ float O[kCCH * 2 * OP];
     const int nseg = cdiv(nW, kTSEG);
@@ -417,6 +423,7 @@ __global__ void __launch_bounds__(256, 4) imtrans_bwd_nchw_band_kernel(const flo
                                                                          float *__restrict__ dX, int B, int H, int W, int C, int nH,
                                                                          int nW, int R, int nbands, int S, int nsegs, int pitch)
 {
+    after_previous_kernel(dV, Vm, dX);
     using T = typename Vec<VEC>::type;
     constexpr int CB = LC * VEC;             // channels per block
     constexpr int QW = 32 / LC;              // tiles a warp works on at once
@@ -504,6 +511,7 @@ __global__ void __launch_bounds__(256) imtrans_bwd_nchw_image_kernel(const float
                                                                        float *__restrict__ dX, int B, int H, int W, int C, int nH, int nW,
                                                                        int CB, int pitch)
 {
+    after_previous_kernel(dV, Vm, dX);
     extern __shared__ float O[];                   // [CB][pitch]
     const int b = blockIdx.x, c0 = blockIdx.y * CB;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -603,6 +611,7 @@ __global__ void __launch_bounds__(256, 4) imtrans_bwd_nchw_image2_kernel(const f
                                                                            float *__restrict__ dX, int B, int H, int W, int C, int nH,
                                                                            int nW, int CB)
 {
+    after_previous_kernel(dV, Vm, dX);
     extern __shared__ __align__(16) float O[];     // [H*W][CB + 2]
     const int b = blockIdx.x, c0 = blockIdx.y * CB;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -685,13 +694,13 @@ int imtrans_fwd(const float *X, float *V, int B, int H, int W, int C, int layout
         if ((C % 4 == 0) && aligned16(X) && aligned16(V) && (!scale || (aligned16(scale) && aligned16(shift)))) {
             const long long total = (long long)B * nH * nW * (C / 4);
             const unsigned g = (unsigned)cdivll(total, 256);
-            if (scale) imtrans_fwd_nhwc_kernel<4, true><<<g, 256, 0, st>>>(X, V, B, H, W, C, nH, nW, relu, scale, shift);
-            else       imtrans_fwd_nhwc_kernel<4, false><<<g, 256, 0, st>>>(X, V, B, H, W, C, nH, nW, relu, scale, shift);
+            if (scale) launch(imtrans_fwd_nhwc_kernel<4, true>, dim3(g), 256, 0, st, X, V, B, H, W, C, nH, nW, relu, scale, shift);
+            else       launch(imtrans_fwd_nhwc_kernel<4, false>, dim3(g), 256, 0, st, X, V, B, H, W, C, nH, nW, relu, scale, shift);
         } else {
             const long long total = (long long)B * nH * nW * C;
             const unsigned g = (unsigned)cdivll(total, 256);
-            if (scale) imtrans_fwd_nhwc_kernel<1, true><<<g, 256, 0, st>>>(X, V, B, H, W, C, nH, nW, relu, scale, shift);
-            else       imtrans_fwd_nhwc_kernel<1, false><<<g, 256, 0, st>>>(X, V, B, H, W, C, nH, nW, relu, scale, shift);
+            if (scale) launch(imtrans_fwd_nhwc_kernel<1, true>, dim3(g), 256, 0, st, X, V, B, H, W, C, nH, nW, relu, scale, shift);
+            else       launch(imtrans_fwd_nhwc_kernel<1, false>, dim3(g), 256, 0, st, X, V, B, H, W, C, nH, nW, relu, scale, shift);
         }
     } else {
         const long long gx = (long long)B * nH * cdiv(nW, kTSEG);
@@ -711,13 +720,8 @@ int imtrans_fwd(const float *X, float *V, int B, int H, int W, int C, int layout
             const int smem = cb * pitch * (int)sizeof(float);
             if ((long long)B * nbands > 0x7fffffffLL || cdiv(C, cb) > 65535) return WG2X2_ERR_UNSUPPORTED;
             const dim3 gb((unsigned)(B * nbands), cdiv(C, cb));
-            auto launch = [&](auto kernel) -> bool {
-                if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return false;
-                kernel<<<gb, 256, smem, st>>>(X, V, B, H, W, C, nH, nW, relu, R, nbands, pitch, scale, shift);
-                return true;
-            };
-            const bool launched = scale ? launch(imtrans_fwd_nchw_vec_kernel<32, true>) : launch(imtrans_fwd_nchw_vec_kernel<32, false>);
-            if (!launched) return WG2X2_ERR_LAUNCH;
+            launch(scale ? imtrans_fwd_nchw_vec_kernel<32, true> : imtrans_fwd_nchw_vec_kernel<32, false>, gb, 256, smem, st, X, V, B, H, W, C,
+                   nH, nW, relu, R, nbands, pitch, scale, shift);
         } else if (W <= 128) {
             int R = (kBandFloats / W - 2) / 2;
             if (R < 1) R = 1;
@@ -731,17 +735,10 @@ int imtrans_fwd(const float *X, float *V, int B, int H, int W, int C, int layout
             const long long gxb = (long long)B * nbands;
             if (gxb > 0x7fffffffLL) return WG2X2_ERR_UNSUPPORTED;
             const dim3 gb((unsigned)gxb, cdiv(C, 32));
-            if (scale) {
-                if (cudaFuncSetAttribute(imtrans_fwd_nchw_band_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-                    return WG2X2_ERR_LAUNCH;
-                imtrans_fwd_nchw_band_kernel<true><<<gb, 256, smem, st>>>(X, V, B, H, W, C, nH, nW, relu, R, nbands, pitch, scale, shift);
-            } else {
-                if (cudaFuncSetAttribute(imtrans_fwd_nchw_band_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-                    return WG2X2_ERR_LAUNCH;
-                imtrans_fwd_nchw_band_kernel<false><<<gb, 256, smem, st>>>(X, V, B, H, W, C, nH, nW, relu, R, nbands, pitch, scale, shift);
-            }
+            launch(scale ? imtrans_fwd_nchw_band_kernel<true> : imtrans_fwd_nchw_band_kernel<false>, gb, 256, smem, st, X, V, B, H, W, C, nH, nW,
+                   relu, R, nbands, pitch, scale, shift);
         } else {
-            imtrans_fwd_nchw_kernel<<<grid, 256, 0, st>>>(X, V, B, H, W, C, nH, nW, relu, scale, shift);
+            launch(imtrans_fwd_nchw_kernel, grid, 256, 0, st, X, V, B, H, W, C, nH, nW, relu, scale, shift);
         }
     }
     return launch_status();
@@ -757,11 +754,11 @@ int imtrans_bwd(const float *dV, const float *Vm, float *dX, int B, int H, int W
         const long long total = (long long)B * nH * nW * (vec ? C / 4 : C);
         const unsigned g = (unsigned)cdivll(total, 256);
         if (vec) {
-            if (Vm) imtrans_bwd_nhwc_kernel<4, true><<<g, 256, 0, st>>>(dV, Vm, dX, B, H, W, C, nH, nW);
-            else    imtrans_bwd_nhwc_kernel<4, false><<<g, 256, 0, st>>>(dV, Vm, dX, B, H, W, C, nH, nW);
+            if (Vm) launch(imtrans_bwd_nhwc_kernel<4, true>, dim3(g), 256, 0, st, dV, Vm, dX, B, H, W, C, nH, nW);
+            else    launch(imtrans_bwd_nhwc_kernel<4, false>, dim3(g), 256, 0, st, dV, Vm, dX, B, H, W, C, nH, nW);
         } else {
-            if (Vm) imtrans_bwd_nhwc_kernel<1, true><<<g, 256, 0, st>>>(dV, Vm, dX, B, H, W, C, nH, nW);
-            else    imtrans_bwd_nhwc_kernel<1, false><<<g, 256, 0, st>>>(dV, Vm, dX, B, H, W, C, nH, nW);
+            if (Vm) launch(imtrans_bwd_nhwc_kernel<1, true>, dim3(g), 256, 0, st, dV, Vm, dX, B, H, W, C, nH, nW);
+            else    launch(imtrans_bwd_nhwc_kernel<1, false>, dim3(g), 256, 0, st, dV, Vm, dX, B, H, W, C, nH, nW);
         }
     } else {
         // small images: one block per image and channel block, every value of dV read once
@@ -772,30 +769,16 @@ int imtrans_bwd(const float *dV, const float *Vm, float *dX, int B, int H, int W
             if ((C & 1) == 0 && aligned8(dV) && (!Vm || aligned8(Vm)) && cdiv(C, CB) <= 65535) {      // two channels per lane
                 const int smem2 = HW * (CB + 2) * (int)sizeof(float);
                 const dim3 grid2((unsigned)B, cdiv(C, CB));
-                if (Vm) {
-                    if (cudaFuncSetAttribute(imtrans_bwd_nchw_image2_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2) != cudaSuccess)
-                        return WG2X2_ERR_LAUNCH;
-                    imtrans_bwd_nchw_image2_kernel<true><<<grid2, 256, smem2, st>>>(dV, Vm, dX, B, H, W, C, nH, nW, CB);
-                } else {
-                    if (cudaFuncSetAttribute(imtrans_bwd_nchw_image2_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2) != cudaSuccess)
-                        return WG2X2_ERR_LAUNCH;
-                    imtrans_bwd_nchw_image2_kernel<false><<<grid2, 256, smem2, st>>>(dV, Vm, dX, B, H, W, C, nH, nW, CB);
-                }
+                launch(Vm ? imtrans_bwd_nchw_image2_kernel<true> : imtrans_bwd_nchw_image2_kernel<false>, grid2, 256, smem2, st, dV, Vm, dX, B, H,
+                       W, C, nH, nW, CB);
                 return launch_status();
             }
             const int pitch = HW | 1;
             const int smem = CB * pitch * (int)sizeof(float);
             if (cdiv(C, CB) <= 65535) {
                 const dim3 grid((unsigned)B, cdiv(C, CB));
-                if (Vm) {
-                    if (cudaFuncSetAttribute(imtrans_bwd_nchw_image_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-                        return WG2X2_ERR_LAUNCH;
-                    imtrans_bwd_nchw_image_kernel<true><<<grid, 256, smem, st>>>(dV, Vm, dX, B, H, W, C, nH, nW, CB, pitch);
-                } else {
-                    if (cudaFuncSetAttribute(imtrans_bwd_nchw_image_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-                        return WG2X2_ERR_LAUNCH;
-                    imtrans_bwd_nchw_image_kernel<false><<<grid, 256, smem, st>>>(dV, Vm, dX, B, H, W, C, nH, nW, CB, pitch);
-                }
+                launch(Vm ? imtrans_bwd_nchw_image_kernel<true> : imtrans_bwd_nchw_image_kernel<false>, grid, 256, smem, st, dV, Vm, dX, B, H, W,
+                       C, nH, nW, CB, pitch);
                 return launch_status();
             }
         }
@@ -817,25 +800,20 @@ int imtrans_bwd(const float *dV, const float *Vm, float *dX, int B, int H, int W
             const long long blocks = (long long)B * cut.nbands * cut.nsegs;
             if (blocks * cdiv(C, cb) > 0x7fffffffLL || cdiv(C, cb) > 65535) return WG2X2_ERR_UNSUPPORTED;
             const dim3 grid = Vm ? dim3((unsigned)blocks, cdiv(C, cb)) : dim3((unsigned)(blocks * cdiv(C, cb)));
-            auto launch = [&](auto kernel) -> bool {
-                if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return false;
-                kernel<<<grid, 256, smem, st>>>(dV, Vm, dX, B, H, W, C, nH, nW, cut.R, cut.nbands, cut.S, cut.nsegs, pitch);
-                return true;
+            auto go = [&](auto kernel) {
+                return launch(kernel, grid, 256, smem, st, dV, Vm, dX, B, H, W, C, nH, nW, cut.R, cut.nbands, cut.S, cut.nsegs, pitch);
             };
             // (the kernels with wider blocks are only taken where those already fill the GPU: they have no segments)
-            const bool launched =
-                wide ? (Vm ? launch(imtrans_bwd_nchw_band_kernel<4, 32, true, false>) : launch(imtrans_bwd_nchw_band_kernel<4, 32, false, false>))
-                : vec ? (Vm ? launch(imtrans_bwd_nchw_band_kernel<4, 16, true, false>) : launch(imtrans_bwd_nchw_band_kernel<4, 16, false, false>))
-                : cut.nsegs == 1 ? (Vm ? launch(imtrans_bwd_nchw_band_kernel<1, 32, true, false>) : launch(imtrans_bwd_nchw_band_kernel<1, 32, false, false>))
-                                 : (Vm ? launch(imtrans_bwd_nchw_band_kernel<1, 32, true, true>) : launch(imtrans_bwd_nchw_band_kernel<1, 32, false, true>));
-            if (!launched) return WG2X2_ERR_LAUNCH;
-            return launch_status();
+            return wide ? (Vm ? go(imtrans_bwd_nchw_band_kernel<4, 32, true, false>) : go(imtrans_bwd_nchw_band_kernel<4, 32, false, false>))
+                : vec ? (Vm ? go(imtrans_bwd_nchw_band_kernel<4, 16, true, false>) : go(imtrans_bwd_nchw_band_kernel<4, 16, false, false>))
+                : cut.nsegs == 1 ? (Vm ? go(imtrans_bwd_nchw_band_kernel<1, 32, true, false>) : go(imtrans_bwd_nchw_band_kernel<1, 32, false, false>))
+                                 : (Vm ? go(imtrans_bwd_nchw_band_kernel<1, 32, true, true>) : go(imtrans_bwd_nchw_band_kernel<1, 32, false, true>));
         }
         const long long gx = (long long)B * nH * cdiv(nW, kTSEG);
         if (gx > 0x7fffffffLL || cdiv(C, kCCH) > 65535) return WG2X2_ERR_UNSUPPORTED;
         dim3 grid((unsigned)gx, cdiv(C, kCCH));
-        if (Vm) imtrans_bwd_nchw_kernel<true><<<grid, 256, 0, st>>>(dV, Vm, dX, B, H, W, C, nH, nW);
-        else    imtrans_bwd_nchw_kernel<false><<<grid, 256, 0, st>>>(dV, Vm, dX, B, H, W, C, nH, nW);
+        if (Vm) launch(imtrans_bwd_nchw_kernel<true>, grid, 256, 0, st, dV, Vm, dX, B, H, W, C, nH, nW);
+        else    launch(imtrans_bwd_nchw_kernel<false>, grid, 256, 0, st, dV, Vm, dX, B, H, W, C, nH, nW);
     }
     return launch_status();
 }

@@ -20,6 +20,7 @@ __global__ void __launch_bounds__(256) maxpool_vec_kernel(const float *__restric
                                                             const float *__restrict__ rs, const float *__restrict__ rb, int C,
                                                             long long planes, int H, int W, int OH, int OW, int ph)
 {
+    after_previous_kernel(X, Y, Yr, rs, rb);
     const int OW4 = OW >> 2;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long total = planes * OH * OW4;
@@ -65,6 +66,7 @@ __global__ void __launch_bounds__(256) maxpool_vec2_kernel(const float *__restri
                                                              const float *__restrict__ rs, const float *__restrict__ rb, int C,
                                                              long long planes, int H, int W, int OH, int OW, int ph)
 {
+    after_previous_kernel(X, Y, Yr, rs, rb);
     const int OW2 = OW >> 1;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= planes * OH * OW2) return;
@@ -99,6 +101,7 @@ __global__ void __launch_bounds__(256) maxpool_any_kernel(const float *__restric
                                                             const float *__restrict__ rs, const float *__restrict__ rb, int C,
                                                             long long planes, int H, int W, int OH, int OW, int ph, int pw)
 {
+    after_previous_kernel(X, Y, Yr, rs, rb);
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= planes * OH * OW) return;
     const int ow = (int)(idx % OW);
@@ -129,6 +132,7 @@ __global__ void __launch_bounds__(256) maxpool_nhwc_in_kernel(const float *__res
                                                                 const float *__restrict__ rs, const float *__restrict__ rb, int C, int H,
                                                                 int W, int OH, int OW, int ph, int pw, int pitch)
 {
+    after_previous_kernel(X, Y, Yr, rs, rb);
     constexpr int CB = 32 * VEC;
     extern __shared__ float S[];                    // [CB channels][pitch]
     const int oh = blockIdx.x % OH, b = blockIdx.x / OH;
@@ -179,7 +183,7 @@ int maxpool3x3s2_same_nhwc_in(const float *X, float *Y, float *Yrelu, const floa
     const size_t smem = (size_t)cb * pitch * sizeof(float);
     if ((long long)B * OH > 0x7fffffffLL || cdiv(C, cb) > 65535 || smem > 48 * 1024) return WG2X2_ERR_UNSUPPORTED;
     const dim3 grid((unsigned)(B * OH), cdiv(C, cb));
-#define WG_POOL_LAUNCH(V, R) maxpool_nhwc_in_kernel<V, R><<<grid, 256, smem, st>>>(X, Y, Yrelu, rs, rb, C, H, W, OH, OW, ph, pw, pitch)
+#define WG_POOL_LAUNCH(V, R) launch(maxpool_nhwc_in_kernel<V, R>, dim3(grid), 256, smem, st, X, Y, Yrelu, rs, rb, C, H, W, OH, OW, ph, pw, pitch)
     if (vec2) { if (Yrelu) WG_POOL_LAUNCH(2, true); else WG_POOL_LAUNCH(2, false); }
     else      { if (Yrelu) WG_POOL_LAUNCH(1, true); else WG_POOL_LAUNCH(1, false); }
 #undef WG_POOL_LAUNCH
@@ -198,19 +202,19 @@ int maxpool3x3s2_same(const float *X, float *Y, float *Yrelu, const float *rs, c
         const long long total = planes * OH * (OW / 4);
         const long long blocks = cdivll(total, 256);
         if (blocks > 0x7fffffffLL) return WG2X2_ERR_UNSUPPORTED;
-        if (Yrelu) maxpool_vec_kernel<true><<<(unsigned)blocks, 256, 0, st>>>(X, Y, Yrelu, rs, rb, C, planes, H, W, OH, OW, ph);
-        else       maxpool_vec_kernel<false><<<(unsigned)blocks, 256, 0, st>>>(X, Y, Yrelu, rs, rb, C, planes, H, W, OH, OW, ph);
+        if (Yrelu) launch(maxpool_vec_kernel<true>, dim3((unsigned)blocks), 256, 0, st, X, Y, Yrelu, rs, rb, C, planes, H, W, OH, OW, ph);
+        else       launch(maxpool_vec_kernel<false>, dim3((unsigned)blocks), 256, 0, st, X, Y, Yrelu, rs, rb, C, planes, H, W, OH, OW, ph);
     } else if ((W % 4) == 0 && al16(X) && al16(Y) && (!Yrelu || al16(Yrelu))) {
         const long long total = planes * OH * (OW / 2);
         const long long blocks = cdivll(total, 256);
         if (blocks > 0x7fffffffLL) return WG2X2_ERR_UNSUPPORTED;
-        if (Yrelu) maxpool_vec2_kernel<true><<<(unsigned)blocks, 256, 0, st>>>(X, Y, Yrelu, rs, rb, C, planes, H, W, OH, OW, ph);
-        else       maxpool_vec2_kernel<false><<<(unsigned)blocks, 256, 0, st>>>(X, Y, Yrelu, rs, rb, C, planes, H, W, OH, OW, ph);
+        if (Yrelu) launch(maxpool_vec2_kernel<true>, dim3((unsigned)blocks), 256, 0, st, X, Y, Yrelu, rs, rb, C, planes, H, W, OH, OW, ph);
+        else       launch(maxpool_vec2_kernel<false>, dim3((unsigned)blocks), 256, 0, st, X, Y, Yrelu, rs, rb, C, planes, H, W, OH, OW, ph);
     } else {
         const long long blocks = cdivll(planes * OH * OW, 256);
         if (blocks > 0x7fffffffLL) return WG2X2_ERR_UNSUPPORTED;
-        if (Yrelu) maxpool_any_kernel<true><<<(unsigned)blocks, 256, 0, st>>>(X, Y, Yrelu, rs, rb, C, planes, H, W, OH, OW, ph, pw);
-        else       maxpool_any_kernel<false><<<(unsigned)blocks, 256, 0, st>>>(X, Y, Yrelu, rs, rb, C, planes, H, W, OH, OW, ph, pw);
+        if (Yrelu) launch(maxpool_any_kernel<true>, dim3((unsigned)blocks), 256, 0, st, X, Y, Yrelu, rs, rb, C, planes, H, W, OH, OW, ph, pw);
+        else       launch(maxpool_any_kernel<false>, dim3((unsigned)blocks), 256, 0, st, X, Y, Yrelu, rs, rb, C, planes, H, W, OH, OW, ph, pw);
     }
     return launch_status();
 }

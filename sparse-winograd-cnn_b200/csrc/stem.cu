@@ -82,6 +82,7 @@ __device__ __forceinline__ void stem_tmem_ld32(uint32_t taddr, float (&r)[8][4])
 // k = 8*(3*ky + c) + kx.
 __global__ void stem_prepare_kernel(const float *__restrict__ W, float *__restrict__ Wp)
 {
+    after_previous_kernel(W, Wp);
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= kStemWt) return;
     const int e = ((idx >> 7) & 3) * 4 + (idx & 3), lane = (idx >> 2) & 31, ks = idx >> 9;
@@ -174,6 +175,7 @@ __global__ void __launch_bounds__(kStemThreads, 2)
 stem_pool_kernel(const float *__restrict__ X, const float *__restrict__ Wp, float *__restrict__ Y, float *__restrict__ Yr,
                  const float *__restrict__ rs, const float *__restrict__ rb, int H, int W, int bands, int band_rows)
 {
+    after_previous_kernel(X, Wp, Y, Yr, rs, rb);
     extern __shared__ __align__(16) unsigned char stem_smem_raw[];
     StemSmem &sm = *reinterpret_cast<StemSmem *>(stem_smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -278,7 +280,7 @@ stem_pool_kernel(const float *__restrict__ X, const float *__restrict__ Wp, floa
 int stem_prepare(const float *W, float *Wp, cudaStream_t st)
 {
     if (!W || !Wp) return WG2X2_ERR_BAD_ARG;
-    stem_prepare_kernel<<<cdiv(kStemWt, 256), 256, 0, st>>>(W, Wp);
+    launch(stem_prepare_kernel, dim3(cdiv(kStemWt, 256)), 256, 0, st, W, Wp);
     return launch_status();
 }
 
@@ -304,18 +306,17 @@ int stem_pool(const float *X, const float *Wp, float *Y, float *Yrelu, const flo
     const long long blocks = (long long)B * bands;
     if (blocks > 0x7fffffffLL) return WG2X2_ERR_UNSUPPORTED;
     const size_t smem = sizeof(StemSmem);
-    if (Yrelu) {
-        if (cudaFuncSetAttribute(stem_pool_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-            cudaFuncSetAttribute(stem_pool_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess)
+    auto *kernel = Yrelu ? stem_pool_kernel<true> : stem_pool_kernel<false>;
+    // the whole shared-memory carve-out, so that two blocks fit an SM; asked for once per thread, kernel and device
+    thread_local int carved[2] = {-1, -1};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return WG2X2_ERR_LAUNCH;
+    if (carved[Yrelu != nullptr] != dev) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess)
             return WG2X2_ERR_LAUNCH;
-        stem_pool_kernel<true><<<(unsigned)blocks, kStemThreads, smem, st>>>(X, Wp, Y, Yrelu, rs, rb, H, W, bands, band_rows);
-    } else {
-        if (cudaFuncSetAttribute(stem_pool_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-            cudaFuncSetAttribute(stem_pool_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess)
-            return WG2X2_ERR_LAUNCH;
-        stem_pool_kernel<false><<<(unsigned)blocks, kStemThreads, smem, st>>>(X, Wp, Y, Yrelu, rs, rb, H, W, bands, band_rows);
+        carved[Yrelu != nullptr] = dev;
     }
-    return launch_status();
+    return launch(kernel, dim3((unsigned)blocks), kStemThreads, smem, st, X, Wp, Y, Yrelu, rs, rb, H, W, bands, band_rows);
 }
 
 }  // namespace wg

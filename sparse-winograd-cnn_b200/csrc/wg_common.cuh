@@ -3,6 +3,9 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <stdlib.h>
+
+#include <initializer_list>
 
 #include "../../include/winograd2x2_b200.h"
 
@@ -108,6 +111,63 @@ inline BandCut cut_bands(int nH, int nW, long long blocks, int max_rows)
 inline int launch_status()
 {
     return cudaGetLastError() == cudaSuccess ? WG2X2_OK : WG2X2_ERR_LAUNCH;
+}
+
+// ---- launches ------------------------------------------------------------------------------
+// Every kernel goes out with programmatic stream serialisation: its CTAs may be scheduled while the kernel before it in the
+// stream still runs its last ones, and wait there (after_previous_kernel) until that kernel has completed and its writes are
+// visible.  A layer is up to seven kernels of a few microseconds; what a boundary between two of them costs otherwise -- launch
+// latency, scheduling, set-up -- is one to two microseconds each.  Not during graph capture; WG2X2_PDL=0 turns it off.
+//
+// When the next kernel may come in: at once where this grid is small (max_ctas), else when its CTAs have ended.  Let in
+// early beside a grid that occupies the SMs, the next one's CTAs pile up on those that have room or finish first, and a
+// kernel of only one wave then runs unbalanced (16.8 against 14.4 us for the 64 x 256 x 14 x 14 input transform).
+__device__ __forceinline__ void wait_for_previous_kernel(unsigned max_ctas)
+{
+    if (gridDim.x * gridDim.y * gridDim.z <= max_ctas) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// First statement of a kernel that touches global memory only through the given pointers.  The pointers pass through the
+// wait, so that no load from them can be moved in front of it.
+template <typename... P>
+__device__ __forceinline__ void after_previous_kernel(P &...p)
+{
+    wait_for_previous_kernel(kNumSMs);
+    (void)std::initializer_list<int>{([](P &q) { asm volatile("" : "+l"(q)::"memory"); }(p), 0)...};
+}
+
+// Dynamic shared memory above 48 KB has to be granted once per kernel and device; remembered per thread.
+inline bool grant_smem(const void *kernel, size_t bytes)
+{
+    struct Entry { const void *kernel; int dev; size_t bytes; };
+    thread_local Entry seen[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    Entry &e = seen[(reinterpret_cast<uintptr_t>(kernel) >> 4) & 63];
+    if (e.kernel == kernel && e.dev == dev && e.bytes >= bytes) return true;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return false;
+    e = Entry{kernel, dev, bytes};
+    return true;
+}
+
+template <typename... KernelArgs, typename... Args>
+int launch(void (*kernel)(KernelArgs...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args &&...args)
+{
+    if (smem > 48 * 1024 && !grant_smem(reinterpret_cast<const void *>(kernel), smem)) return WG2X2_ERR_LAUNCH;
+    static const bool pdl_env = [] { const char *e = getenv("WG2X2_PDL"); return !(e && e[0] == '0'); }();
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) return WG2X2_ERR_LAUNCH;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_env && capturing == cudaStreamCaptureStatusNone ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KernelArgs>(args)...) == cudaSuccess ? launch_status() : WG2X2_ERR_LAUNCH;
 }
 
 }  // namespace wg
