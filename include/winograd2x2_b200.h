@@ -79,8 +79,8 @@ int wg2x2_imtrans_bwd(const float *dV, const float *V_relu, float *dX, int B, in
  * Replaces Winograd2x2ConvComputeLauncher (winograd2x2_conv_op.cc:31,
  * winograd2x2_conv_cuda.cu.cc:65-93): the 16 cublasSgemmBatched products and the
  * Output_transform kernel become one kernel that stores no product tensor -- except for
- * WG2X2_MATH_TF32 with C, K >= 256 and a workspace that has room for it, where the products
- * go through scratch memory (see wg2x2_conv_fwd_prepared_ws).
+ * WG2X2_MATH_TF32 with many channels or few tiles and a workspace that has room for it, where
+ * the products go through scratch memory (see wg2x2_conv_fwd_prepared_ws).
  * workspace: see wg2x2_conv_fwd_workspace_bytes (0 bytes for WG2X2_MATH_FP32).
  */
 int wg2x2_conv_fwd(const float *V, const float *Wt, float *Y, int B, int nH, int nW, int C, int K,
@@ -114,8 +114,8 @@ int wg2x2_conv_fwd_prepared_fused(const float *V, const void *prepared, float *Y
                                   const float *residual, void *stream);
 
 /*
- * wg2x2_conv_fwd_prepared_fused with scratch memory, which lets layers with many channels (C, K >= 256) take
- * the wide path: the 16 products as GEMMs with 256 output channels per unit into `workspace` (16*P*K floats,
+ * wg2x2_conv_fwd_prepared_fused with scratch memory, which lets layers with many channels (C, K >= 256), or with
+ * few tiles, take the wide path: the 16 products as GEMMs with up to 256 output channels per unit into `workspace` (16*P*K floats,
  * wg2x2_conv_fwd_prepared_workspace_bytes; 0 = the shape does not use it), then one pass for A^T m A — the
  * reference's own two-step structure (winograd2x2_conv_cuda.cu.cc:80-89) on tensor cores.  With workspace ==
  * NULL, or for smaller layers, the single-kernel path of wg2x2_conv_fwd_prepared_fused runs.
@@ -187,8 +187,8 @@ int wg2x2_layer_fwd_prepared(const float *X, const void *prepared, float *Y, flo
                              int C, int K, int layout, int relu, const float *out_scale, const float *out_shift,
                              const float *residual, void *stream);
 /*
- * The same with scratch memory for the products, which lets layers with many channels (C, K >= 256) take their
- * fastest form too: input transform into V_scratch, then the wide path of wg2x2_conv_fwd_prepared_ws through
+ * The same with scratch memory for the products, which lets layers with many channels (C, K >= 256) or few tiles take
+ * their fastest form too: input transform into V_scratch, then the wide path of wg2x2_conv_fwd_prepared_ws through
  * `workspace` (wg2x2_layer_fwd_prepared_workspace_bytes; 0 = the shape does not use one).  With workspace == NULL, or
  * for other shapes, this is wg2x2_layer_fwd_prepared.
  */
@@ -197,6 +197,8 @@ int wg2x2_layer_fwd_prepared_ws(const float *X, const void *prepared, float *Y, 
                                 const float *residual, void *workspace, size_t workspace_bytes, void *stream);
 size_t wg2x2_layer_fwd_prepared_workspace_bytes(int B, int H, int W, int C, int K);
 int wg2x2_layer_fwd_fused_supported(int B, int H, int W, int C, int K, int layout);
+/* 1 where wg2x2_layer_fwd_prepared_ws runs the one kernel even if both scratch buffers are given (it then reads neither). */
+int wg2x2_layer_fwd_fused_preferred(int B, int H, int W, int C, int K, int layout);
 /* The one-kernel layer forward on its own (NCHW in and out); WG2X2_ERR_UNSUPPORTED outside the shapes above.
  * residual may be Y itself: the result is then added into Y in place (the TMA unit does the addition);
  * otherwise residual is first copied to Y on the same stream and must not overlap it. */

@@ -28,12 +28,13 @@ size_t prepared_weights_bytes(int C, int K);
 int weights_prepare(const float *Wt, int C, int K, void *prepared, size_t bytes, cudaStream_t st);
 int conv_fwd_tc_prepared(const float *V, const void *prepared, float *Y, int B, int nH, int nW, int C, int K, int outH, int outW,
                          int layout, const float *out_scale, const float *out_shift, const float *residual, cudaStream_t st);
-bool conv_fwd_wide_preferred(int C, int K);
+bool conv_fwd_wide_preferred(long long P, int C, int K);
 size_t conv_fwd_wide_workspace_bytes(long long P, int K);
 int conv_fwd_tc_wide(const float *V, const void *prepared, float *Y, int B, int nH, int nW, int C, int K, int outH, int outW,
                      int layout, const float *out_scale, const float *out_shift, const float *residual, void *ws, size_t ws_bytes,
                      cudaStream_t st);
 bool fused_fwd_supported(int B, int H, int W, int C, int K, int layout);
+bool layer_fused_preferred(int B, int H, int W, int C, int K, int layout);
 int layer_fwd_fused(const float *X, const void *prepared, float *Y, int B, int H, int W, int C, int K, int relu,
                     const float *in_scale, const float *in_shift, const float *out_scale, const float *out_shift,
                     const float *residual, cudaStream_t st);
@@ -187,7 +188,7 @@ int wg2x2_layer_fwd(const float *X, const float *Wt, float *Y, float *V_out, int
 
 size_t wg2x2_conv_fwd_prepared_workspace_bytes(int B, int nH, int nW, int C, int K)
 {
-    if (B <= 0 || nH <= 0 || nW <= 0 || C <= 0 || K <= 0 || !conv_fwd_wide_preferred(C, K)) return 0;
+    if (B <= 0 || nH <= 0 || nW <= 0 || C <= 0 || K <= 0 || !conv_fwd_wide_preferred((long long)B * nH * nW, C, K)) return 0;
     return conv_fwd_wide_workspace_bytes((long long)B * nH * nW, K);
 }
 
@@ -199,7 +200,7 @@ int wg2x2_conv_fwd_prepared_ws(const float *V, const void *prepared, float *Y, i
     if (!layout_ok(layout) || !crop_ok(out_h, nH) || !crop_ok(out_w, nW)) return WG2X2_ERR_BAD_ARG;
     if ((out_scale == nullptr) != (out_shift == nullptr)) return WG2X2_ERR_BAD_ARG;
     cudaStream_t st = (cudaStream_t)stream;
-    if (conv_fwd_wide_preferred(C, K) && workspace)
+    if (workspace && conv_fwd_wide_preferred((long long)B * nH * nW, C, K))
         return conv_fwd_tc_wide(V, prepared, Y, B, nH, nW, C, K, out_h, out_w, layout, out_scale, out_shift, residual, workspace,
                                 workspace_bytes, st);
     return conv_fwd_tc_prepared(V, prepared, Y, B, nH, nW, C, K, out_h, out_w, layout, out_scale, out_shift, residual, st);
@@ -208,6 +209,11 @@ int wg2x2_conv_fwd_prepared_ws(const float *V, const void *prepared, float *Y, i
 int wg2x2_layer_fwd_fused_supported(int B, int H, int W, int C, int K, int layout)
 {
     return (B > 0 && H > 0 && W > 0 && C > 0 && K > 0 && fused_fwd_supported(B, H, W, C, K, layout)) ? 1 : 0;
+}
+
+int wg2x2_layer_fwd_fused_preferred(int B, int H, int W, int C, int K, int layout)
+{
+    return (B > 0 && H > 0 && W > 0 && C > 0 && K > 0 && layer_fused_preferred(B, H, W, C, K, layout)) ? 1 : 0;
 }
 
 int wg2x2_layer_fwd_prepared(const float *X, const void *prepared, float *Y, float *V_scratch, int B, int H, int W, int C, int K,
@@ -234,6 +240,8 @@ int wg2x2_layer_fwd_prepared(const float *X, const void *prepared, float *Y, flo
 size_t wg2x2_layer_fwd_prepared_workspace_bytes(int B, int H, int W, int C, int K)
 {
     if (B <= 0 || H <= 0 || W <= 0 || C <= 0 || K <= 0) return 0;
+    // (the layout is not known here: NHWC callers may ask wg2x2_conv_fwd_prepared_workspace_bytes instead)
+    if (layer_fused_preferred(B, H, W, C, K, WG2X2_NCHW)) return 0;
     return wg2x2_conv_fwd_prepared_workspace_bytes(B, (H + 1) / 2, (W + 1) / 2, C, K);
 }
 
@@ -243,9 +251,12 @@ int wg2x2_layer_fwd_prepared_ws(const float *X, const void *prepared, float *Y, 
 {
     if (!X || !prepared || !Y || B <= 0 || H <= 0 || W <= 0 || C <= 0 || K <= 0) return WG2X2_ERR_BAD_ARG;
     if (!layout_ok(layout)) return WG2X2_ERR_BAD_ARG;
-    // layers with many channels: input transform, then the products as wide GEMMs through the workspace
-    if (conv_fwd_wide_preferred(C, K) && V_scratch && workspace) {
-        const int nH = (H + 1) / 2, nW = (W + 1) / 2;
+    const int nH = (H + 1) / 2, nW = (W + 1) / 2;
+    const bool aligned16 = ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y)) & 15u) == 0;
+    if (aligned16 && layer_fused_preferred(B, H, W, C, K, layout))
+        return layer_fwd_fused(X, prepared, Y, B, H, W, C, K, relu, nullptr, nullptr, out_scale, out_shift, residual, (cudaStream_t)stream);
+    // many channels or few tiles: input transform, then the products as wide GEMMs through the workspace
+    if (V_scratch && workspace && conv_fwd_wide_preferred((long long)B * nH * nW, C, K)) {
         const int s = imtrans_fwd(X, V_scratch, B, H, W, C, layout, relu, nullptr, nullptr, (cudaStream_t)stream);
         if (s != WG2X2_OK) return s;
         return wg2x2_conv_fwd_prepared_ws(V_scratch, prepared, Y, B, nH, nW, C, K, H, W, layout, out_scale, out_shift, residual, workspace,

@@ -493,9 +493,11 @@ PyObject *py_layer_fwd_prepared(WG_ARGS)
         OnDevice on(x);
         if (!Y.defined()) Y = new_float(ys, x);
         Scratch vs, ws;
-        const size_t nws = wg2x2_layer_fwd_prepared_workspace_bytes(d.B, d.H, d.W, d.C, K);
+        const bool fused = wg2x2_layer_fwd_fused_preferred(d.B, d.H, d.W, d.C, K, layout) &&
+                           ((reinterpret_cast<uintptr_t>(x.data_ptr()) | reinterpret_cast<uintptr_t>(Y.data_ptr())) & 15u) == 0;
+        const size_t nws = fused ? 0 : wg2x2_conv_fwd_prepared_workspace_bytes(d.B, (d.H + 1) / 2, (d.W + 1) / 2, d.C, K);
         float *vp = ptr(V);
-        if (!vp && (nws || !wg2x2_layer_fwd_fused_supported(d.B, d.H, d.W, d.C, K, layout))) {
+        if (!vp && !fused && (nws || !wg2x2_layer_fwd_fused_supported(d.B, d.H, d.W, d.C, K, layout))) {
             vs.take(sizeof(float) * 16 * (size_t)d.B * ((d.H + 1) / 2) * ((d.W + 1) / 2) * d.C);
             vp = static_cast<float *>(vs.get());
         }

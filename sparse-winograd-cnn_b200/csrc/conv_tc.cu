@@ -196,38 +196,64 @@ __host__ __device__ constexpr uint32_t make_idesc_tf32(int M, int N)
 // 64-bit map mask[t][kb] whose bit cc is set when the 64x32 block (out-channels kb*64..,
 // in-channels cc*32..) of position t has any non-zero weight.  Layers with more than 64
 // chunks (C > 2048) keep every bit set: nothing is skipped there.
+// A CTA takes 64 out-channels x 256 in-channels of one position: one byte of a map word, which it alone writes (so that the
+// map needs no clearing first), the first CTA along C also the bytes beyond the last one.
 // ---------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) pack_weights_kernel(const float *__restrict__ Wt, float *__restrict__ Wp,
-                                                             unsigned long long *__restrict__ masks, int C, int K, int nKB, int nCC)
+constexpr int kPackC = 256;
+constexpr int kPackThreads = 1024;        // four blocks at a time
+// byte `group` of the map word: bit r = block r of the group; nbytes: bytes of a word that the CTAs along the chunks write
+__device__ __forceinline__ void store_map_byte(unsigned long long *word, int group, int ngroups, int nCC, unsigned bits)
+{
+    unsigned char *b = reinterpret_cast<unsigned char *>(word);
+    if (nCC > 64) {
+        if (group == 0) *word = ~0ull;
+        return;
+    }
+    b[group] = (unsigned char)bits;
+    if (group == 0)
+        for (int g = ngroups; g < 8; ++g) b[g] = 0;
+}
+__global__ void __launch_bounds__(kPackThreads) pack_weights_kernel(const float *__restrict__ Wt, float *__restrict__ Wp,
+                                                                      unsigned long long *__restrict__ masks, int C, int K, int nKB, int nCC)
 {
     after_previous_kernel(Wt, Wp, masks);
-    __shared__ float tile[32][33];
-    __shared__ int any;
-    const int t = blockIdx.z;
-    const int c0 = blockIdx.y * 32, k0 = blockIdx.x * 32;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
-    if (threadIdx.x == 0) any = 0;
+    __shared__ float tile[kPackThreads / 128][32][33];
+    __shared__ int live;
+    if (threadIdx.x == 0) live = 0;
     __syncthreads();
-    int nz = 0;
+    const int t = blockIdx.z, kb = blockIdx.x;
+    const int tx = threadIdx.x & 31, ty = (threadIdx.x >> 5) & 3, part = threadIdx.x >> 7;   // 128 threads turn a 32 x 32 half of a block
+    const int k0 = kb * 64 + 32 * (part & 1);
+#pragma unroll 1
+    for (int r0 = 0; r0 < kPackC / 32; r0 += kPackThreads / 256) {
+        const int r = r0 + (part >> 1), c0 = blockIdx.y * kPackC + r * 32;
+        int nz = 0;
+        float w[8];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const int c = c0 + ty + 8 * r, k = k0 + tx;
-        float w = 0.f;
-        if (c < C && k < K) w = __ldg(Wt + ((long long)t * C + c) * K + k);
-        uint32_t u;
-        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(w));
-        w = __uint_as_float(u);
-        nz |= (w != 0.f);
-        tile[ty + 8 * r][tx] = w;
+        for (int q = 0; q < 8; ++q) {
+            const int c = c0 + ty + 4 * q, k = k0 + tx;
+            w[q] = (c < C && k < K) ? __ldg(Wt + ((long long)t * C + c) * K + k) : 0.f;
+        }
+        if (r0) __syncthreads();           // the turned values of the round before have been read
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            uint32_t u;
+            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(w[q]));
+            w[q] = __uint_as_float(u);
+            nz |= (w[q] != 0.f);
+            tile[part][ty + 4 * q][tx] = w[q];
+        }
+        if (__any_sync(0xffffffffu, nz) && tx == 0) atomicOr(&live, 1 << r);
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int k = k0 + ty + 4 * q, c = c0 + tx;
+            if (c < C && k < K) Wp[((long long)t * K + k) * C + c] = tile[part][tx][ty + 4 * q];
+        }
+        if (blockIdx.y * kPackC + (r0 + kPackThreads / 256) * 32 >= C) break;
     }
-    if (nz) any = 1;
     __syncthreads();
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const int k = k0 + ty + 8 * r, c = c0 + tx;
-        if (c < C && k < K) Wp[((long long)t * K + k) * C + c] = tile[tx][ty + 8 * r];
-    }
-    if (threadIdx.x == 0 && any && nCC <= 64) atomicOr(masks + (long long)t * nKB + (k0 / kBlockN), 1ull << (c0 / kBlockK));
+    if (threadIdx.x == 0) store_map_byte(masks + (long long)t * nKB + kb, blockIdx.y, gridDim.y, nCC, (unsigned)live);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -714,11 +740,7 @@ int weights_prepare(const float *Wt, int C, int K, void *prepared, size_t bytes,
     float *Wp = static_cast<float *>(prepared);
     unsigned long long *masks = reinterpret_cast<unsigned long long *>(static_cast<unsigned char *>(prepared) +
                                                                        align_up((size_t)16 * K * C * sizeof(float), 256));
-    if (cudaMemsetAsync(masks, nCC <= 64 ? 0 : 0xFF, (size_t)16 * nKB * sizeof(unsigned long long), st) != cudaSuccess)
-        return WG2X2_ERR_LAUNCH;
-    dim3 grid(cdiv(K, 32), cdiv(C, 32), 16);
-    launch(pack_weights_kernel, grid, 256, 0, st, Wt, Wp, masks, C, K, nKB, nCC);
-    return launch_status();
+    return launch(pack_weights_kernel, dim3(nKB, cdiv(C, kPackC), 16), kPackThreads, 0, st, Wt, Wp, masks, C, K, nKB, nCC);
 }
 
 // Launcher.  `contr` = contraction length C, `ncols` = output channels K; A is (16, P, contr), Bop is
@@ -778,7 +800,7 @@ int conv_fwd_tc_prepared(const float *V, const void *prepared, float *Y, int B, 
                      out_scale, out_shift, residual, st);
 }
 
-bool conv_fwd_wide_preferred(int C, int K);
+bool conv_fwd_wide_preferred(long long P, int C, int K);
 size_t conv_fwd_wide_workspace_bytes(long long P, int K);
 int conv_fwd_tc_wide(const float *V, const void *prepared, float *Y, int B, int nH, int nW, int C, int K, int outH, int outW,
                      int layout, const float *out_scale, const float *out_shift, const float *residual, void *ws, size_t ws_bytes,
@@ -788,7 +810,7 @@ size_t conv_fwd_tc_workspace_bytes(int B, int nH, int nW, int C, int K)
 {
     if (C <= 0 || K <= 0 || B <= 0 || nH <= 0 || nW <= 0) return 0;
     size_t n = prepared_weights_bytes(C, K);
-    if (conv_fwd_wide_preferred(C, K)) n += conv_fwd_wide_workspace_bytes((long long)B * nH * nW, K);
+    if (conv_fwd_wide_preferred((long long)B * nH * nW, C, K)) n += conv_fwd_wide_workspace_bytes((long long)B * nH * nW, K);
     return n;
 }
 
@@ -800,7 +822,7 @@ int conv_fwd_tc(const float *V, const float *Wt, float *Y, int B, int nH, int nW
     const int s = weights_prepare(Wt, C, K, ws, ws_bytes, st);
     if (s != WG2X2_OK) return s;
     const size_t pb = prepared_weights_bytes(C, K);
-    if (conv_fwd_wide_preferred(C, K) && ws_bytes >= pb + conv_fwd_wide_workspace_bytes((long long)B * nH * nW, K))
+    if (conv_fwd_wide_preferred((long long)B * nH * nW, C, K) && ws_bytes >= pb + conv_fwd_wide_workspace_bytes((long long)B * nH * nW, K))
         return conv_fwd_tc_wide(V, ws, Y, B, nH, nW, C, K, outH, outW, layout, nullptr, nullptr, nullptr,
                                 static_cast<char *>(ws) + pb, ws_bytes - pb, st);
     return conv_fwd_tc_prepared(V, ws, Y, B, nH, nW, C, K, outH, outW, layout, nullptr, nullptr, nullptr, st);

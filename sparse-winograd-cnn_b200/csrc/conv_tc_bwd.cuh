@@ -73,14 +73,15 @@ __global__ void __launch_bounds__(256) conv_dm_nchw_kernel(const float *__restri
     const int w0 = 2 * tw0, SW = SEG ? min(2 * ns, W - w0) : W;      // pixels of a staged row
     const int lo = 2 * th0, hi = min(2 * th0 + 2 * rows_tile, H);
     const int nfill = (hi - lo) * SW;
-    for (int kk = warp; kk < 32; kk += 8) {
-        if (k0 + kk >= K) break;
-        const float *src = dY + (((long long)b * K + k0 + kk) * H + lo) * W + w0;
-        float *dst = S + kk * pitch;
-        if (!SEG) {
+    if (SEG) {       // two rows of a segment
+        stage_channels(dY + (((long long)b * K + k0) * H + lo) * W + w0, (long long)H * W, K - k0, nfill, S, pitch,
+                       [&](int i) { return i >= SW ? W + i - SW : i; });
+    } else {
+        for (int kk = warp; kk < 32; kk += 8) {
+            if (k0 + kk >= K) break;
+            const float *src = dY + (((long long)b * K + k0 + kk) * H + lo) * W;
+            float *dst = S + kk * pitch;
             for (int i = lane; i < nfill; i += 32) dst[i] = __ldg(src + i);
-        } else {                                             // two rows of a segment
-            for (int i = lane; i < nfill; i += 32) dst[i] = __ldg(src + (i >= SW ? W + i - SW : i));
         }
     }
     __syncthreads();
@@ -174,39 +175,52 @@ __global__ void __launch_bounds__(256, 3) conv_dm_nchw_vec_kernel(const float *_
 
 // W (16, C, K) -> W rounded to TF32, plus the zero-block map of the forward's prepared weights: bit cc of
 // map[t][kb] is set when the block (input channels cc*32.., output channels kb*64..) holds a non-zero.
-// One CTA per block: 32 rows of 64 consecutive floats.
-__global__ void __launch_bounds__(256) round_and_map_kernel(const float *__restrict__ Wt, float *__restrict__ Wr,
-                                                              unsigned long long *__restrict__ map, int C, int K, int nKB, int nCC)
+// One CTA per eight blocks along the input channels: one byte of the map, 256 threads per block (see pack_weights_kernel).
+__global__ void __launch_bounds__(kPackThreads) round_and_map_kernel(const float *__restrict__ Wt, float *__restrict__ Wr,
+                                                                       unsigned long long *__restrict__ map, int C, int K, int nKB, int nCC)
 {
     after_previous_kernel(Wt, Wr, map);
-    const int kb = blockIdx.x, cc = blockIdx.y, t = blockIdx.z;
-    int nz = 0;
-    if ((K & 3) == 0 && ((reinterpret_cast<uintptr_t>(Wt) | reinterpret_cast<uintptr_t>(Wr)) & 15u) == 0) {
-        // 16 bytes per access: 32 rows of 16 float4, two per thread
+    __shared__ int live;
+    if (threadIdx.x == 0) live = 0;
+    __syncthreads();
+    const int kb = blockIdx.x, t = blockIdx.z, tid = threadIdx.x & 255;
+    const bool vec = (K & 3) == 0 && ((reinterpret_cast<uintptr_t>(Wt) | reinterpret_cast<uintptr_t>(Wr)) & 15u) == 0;
+    for (int r = threadIdx.x >> 8; r < 8; r += kPackThreads / 256) {
+        const int c0 = (blockIdx.y * 8 + r) * 32;
+        if (c0 >= C) break;
+        int nz = 0;
+        if (vec) {
+            // 16 bytes per access: 32 rows of 16 float4, two per thread
+            float4 w[2];
+            long long o[2];
 #pragma unroll
-        for (int e = threadIdx.x; e < 32 * 16; e += 256) {
-            const int c = cc * 32 + (e >> 4), k = kb * 64 + 4 * (e & 15);
-            if (c < C && k < K) {
-                const long long o = ((long long)t * C + c) * K + k;
-                float4 w = __ldg(reinterpret_cast<const float4 *>(Wt + o));
-                w.x = round_tf32(w.x); w.y = round_tf32(w.y); w.z = round_tf32(w.z); w.w = round_tf32(w.w);
-                *reinterpret_cast<float4 *>(Wr + o) = w;
-                nz |= (w.x != 0.f) | (w.y != 0.f) | (w.z != 0.f) | (w.w != 0.f);
+            for (int q = 0; q < 2; ++q) {
+                const int e = tid + 256 * q, c = c0 + (e >> 4), k = kb * 64 + 4 * (e & 15);
+                o[q] = (c < C && k < K) ? ((long long)t * C + c) * K + k : -1;
+                if (o[q] >= 0) w[q] = __ldg(reinterpret_cast<const float4 *>(Wt + o[q]));
+            }
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+                if (o[q] >= 0) {
+                    w[q].x = round_tf32(w[q].x); w[q].y = round_tf32(w[q].y); w[q].z = round_tf32(w[q].z); w[q].w = round_tf32(w[q].w);
+                    *reinterpret_cast<float4 *>(Wr + o[q]) = w[q];
+                    nz |= (w[q].x != 0.f) | (w[q].y != 0.f) | (w[q].z != 0.f) | (w[q].w != 0.f);
+                }
+        } else {
+            for (int e = tid; e < 32 * 64; e += 256) {
+                const int c = c0 + (e >> 6), k = kb * 64 + (e & 63);
+                if (c < C && k < K) {
+                    const long long o = ((long long)t * C + c) * K + k;
+                    const float w = round_tf32(__ldg(Wt + o));
+                    Wr[o] = w;
+                    nz |= (w != 0.f);
+                }
             }
         }
-    } else {
-        for (int e = threadIdx.x; e < 32 * 64; e += 256) {
-            const int c = cc * 32 + (e >> 6), k = kb * 64 + (e & 63);
-            if (c < C && k < K) {
-                const long long o = ((long long)t * C + c) * K + k;
-                const float w = round_tf32(__ldg(Wt + o));
-                Wr[o] = w;
-                nz |= (w != 0.f);
-            }
-        }
+        if (__any_sync(0xffffffffu, nz) && (threadIdx.x & 31) == 0) atomicOr(&live, 1 << r);
     }
-    nz = __syncthreads_or(nz);
-    if (threadIdx.x == 0 && nz && nCC <= 64) atomicOr(map + (long long)t * nKB + kb, 1ull << cc);
+    __syncthreads();
+    if (threadIdx.x == 0) store_map_byte(map + (long long)t * nKB + kb, blockIdx.y, gridDim.y, nCC, (unsigned)live);
 }
 
 static int launch_dm(const float *dY, float *dM, int B, int H, int W, int K, int layout, cudaStream_t st)
@@ -280,12 +294,12 @@ bool tc_bwd_shape_supported(int C, int K) { return C % 4 == 0 && K % 4 == 0 && C
 // The epilogue turns each 32 x 32 block through shared memory so that stores are whole 128-byte lines, and
 // applies the pruning mask (KIND 0, one split) or the ReLU mask V > 0 (KIND 1) on the way out.
 // ---------------------------------------------------------------------------------------
-constexpr int kGgStages = 4;
+constexpr int kGgMaxStages = 8;                          // 4 / 6 / 8 stages of 48 / 32 / 24 KB for 256 / 128 / 64 columns
 constexpr int kGgBoxBytes = 32 * 32 * 4;                 // [32 rows][32 fp32]
 constexpr int kGgABytes = 4 * kGgBoxBytes;               // 128 rows x 32 contraction steps
 constexpr int kGgBBytesMax = 8 * kGgBoxBytes;            // up to 256 columns
-constexpr int kGgStageBytes = kGgABytes + kGgBBytesMax;  // 48 KB
-constexpr int kGgSmemBytes = kGgStages * kGgStageBytes + 1024 + kCtrlBytes + kEpiWarps * kEpiStageBytes;
+constexpr int kGgRingBytes = 4 * (kGgABytes + kGgBBytesMax);   // 192 KB
+constexpr int kGgSmemBytes = kGgRingBytes + 1024 + kCtrlBytes + kEpiWarps * kEpiStageBytes;
 
 struct GgParams {
     float *out;              // [split][16][rows][cols] (split dimension only when !direct)
@@ -369,20 +383,22 @@ conv_grad_gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t *gen_base = smem_raw + (base - raw);
-    const uint32_t bars = base + kGgStages * kGgStageBytes;
-    uint64_t *bars_gen = reinterpret_cast<uint64_t *>(gen_base + kGgStages * kGgStageBytes);
+    const uint32_t bars = base + kGgRingBytes;
+    uint64_t *bars_gen = reinterpret_cast<uint64_t *>(gen_base + kGgRingBytes);
     auto full_bar = [&](int s) { return bars + 8u * s; };
-    auto empty_bar = [&](int s) { return bars + 8u * (kGgStages + s); };
-    auto accf_bar = [&](int b) { return bars + 8u * (2 * kGgStages + b); };
-    auto acce_bar = [&](int b) { return bars + 8u * (2 * kGgStages + 2 + b); };
-    volatile uint32_t *tmem_ptr_slot = reinterpret_cast<volatile uint32_t *>(bars_gen + 2 * kGgStages + 4);
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(bars_gen + 2 * kGgStages + 5);
-    float *epi_stage_all = reinterpret_cast<float *>(gen_base + kGgStages * kGgStageBytes + kCtrlBytes);
+    auto empty_bar = [&](int s) { return bars + 8u * (kGgMaxStages + s); };
+    auto accf_bar = [&](int b) { return bars + 8u * (2 * kGgMaxStages + b); };
+    auto acce_bar = [&](int b) { return bars + 8u * (2 * kGgMaxStages + 2 + b); };
+    volatile uint32_t *tmem_ptr_slot = reinterpret_cast<volatile uint32_t *>(bars_gen + 2 * kGgMaxStages + 4);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(bars_gen + 2 * kGgMaxStages + 5);
+    float *epi_stage_all = reinterpret_cast<float *>(gen_base + kGgRingBytes + kCtrlBytes);
+    const int nstages = prm.N > 128 ? 4 : (prm.N > 64 ? 6 : 8);
+    const uint32_t stage_bytes = (uint32_t)(kGgABytes + prm.N * 128);
 
     // (broadcast from lane 0: the compiler then treats the warp index, and all that is derived from it, as warp-uniform)
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kGgStages; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
+        for (int s = 0; s < kGgMaxStages; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(accf_bar(b), 1); mbar_init(acce_bar(b), kEpiWarps); }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -422,7 +438,7 @@ conv_grad_gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_
                     if (KIND == 1 && kc < 64 * 32 && !((live >> (kc >> 5)) & 1ull)) continue;   // all-zero weight blocks: nothing to add
                     if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, 0x500u | s)) { ok = false; break; }
                     mbar_expect_tx(full_bar(s), stage_tx);
-                    const uint32_t a_dst = base + s * kGgStageBytes;
+                    const uint32_t a_dst = base + s * stage_bytes;
                     const uint32_t b_dst = a_dst + kGgABytes;
                     if (KIND == 0 && prm.mn4) {      // all 32-channel blocks of an operand in one box each
                         tma_load_4d_gg(a_dst, &mapA, full_bar(s), 0, (int)kc, rb * 4, t);
@@ -437,7 +453,7 @@ conv_grad_gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_
                         tma_load_3d(a_dst, &mapA, full_bar(s), (int)kc, rb * 128, t);
                         tma_load_3d(b_dst, &mapB, full_bar(s), (int)kc, cb * N, t);
                     }
-                    if (++s == kGgStages) { s = 0; ph ^= 1u; }
+                    if (++s == nstages) { s = 0; ph ^= 1u; }
                 }
             }
             if (!ok)
@@ -469,7 +485,7 @@ conv_grad_gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_
                     if (KIND == 1 && kc < 64 * 32 && !((live >> (kc >> 5)) & 1ull)) continue;
                     if (!mbar_wait_warp(full_bar(s), ph, abort_flag, 0x700u | s)) { ok = false; break; }
                     tc_fence_after();
-                    const uint32_t a_addr = base + s * kGgStageBytes;
+                    const uint32_t a_addr = base + s * stage_bytes;
                     const uint64_t adesc = KIND == 0 ? make_desc_mn_sw128(a_addr) : make_desc_k_sw128(a_addr);
                     const uint64_t bdesc = KIND == 0 ? make_desc_mn_sw128(a_addr + kGgABytes) : make_desc_k_sw128(a_addr + kGgABytes);
                     const uint32_t step = KIND == 0 ? 64u : 2u;   // 1024 B / 32 B per 8 contraction steps
@@ -481,7 +497,7 @@ conv_grad_gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_
                     }
                     __syncwarp();
                     first = 0;
-                    if (++s == kGgStages) { s = 0; ph ^= 1u; }
+                    if (++s == nstages) { s = 0; ph ^= 1u; }
                 }
                 if (ok && leader) umma_commit(accf_bar(buf));
                 __syncwarp();
@@ -644,18 +660,41 @@ static bool make_map_gg4(CUtensorMap *map, const float *ptr, long long ch, long 
 
 static int gg_cols(int n) { return n > 128 ? 256 : (n > 64 ? 128 : 64); }
 
-// Splits of the P range for dW: enough units for every SM, at least 8 chunks of 32 tiles per split
+// Columns per unit of a product with `rows` x n results and a contraction of `contr`: the width whose rounds over the SMs
+// take least.  A unit takes about (chunks of 32) x c + e microseconds, measured with c = 0.37 / 0.45 / 0.60 and e = 0.3 / 0.5 / 0.9
+// for 64 / 128 / 256 columns: wide units share the A tile among more columns, narrow ones put more SMs to work (one 14 x 14
+// image of 512 channels: 13.9 us with 256 columns, 10.4 with 64).
+static int gg_pick_cols(long long rows, int n, int contr)
+{
+    const int widest = gg_cols(n);
+    const double ch = cdiv(contr, 32);
+    int best = widest;
+    double t = 1e30;
+    for (int N = widest; N >= 64; N >>= 1) {
+        const long long units = 16 * cdivll(rows, 128) * cdiv(n, N);
+        const double per = N == 64 ? 0.37 * ch + 0.3 : N == 128 ? 0.45 * ch + 0.5 : 0.60 * ch + 0.9;
+        const double u = (double)cdivll(units, kNumSMs) * per;
+        if (u < t) { t = u; best = N; }
+    }
+    return best;
+}
+
+// Splits of the P range for dW: the count that takes least, rounds over the SMs x chunks of 32 tiles per split (at least 8)
+// at 0.37 us each, plus the reduction pass over the partial sums.  (Just covering the SMs is not enough: 16 blocks x 10
+// splits are two rounds where 16 x 9 are one -- 109 against 64 us at 64 x 64 x 56 x 56.)
 int conv_dw_tc_splits(long long P, int C, int K)
 {
     const long long base_units = (long long)16 * cdiv(C, 128) * cdiv(K, gg_cols(K));
     const long long chunks = cdivll(P, 32);
-    // one split when the unsplit units already cover most SMs: a second round plus the reduction pass
-    // would cost more than the idle SMs do
-    long long s = base_units * 3 >= kNumSMs * 2 ? 1 : cdivll(kNumSMs, base_units);
     const long long max_s = chunks / 8 > 0 ? chunks / 8 : 1;
-    if (s > max_s) s = max_s;
-    if (s < 1) s = 1;
-    const long long cps = cdivll(chunks, s);
+    const double pass = 16.0 * C * K * 4 / 4e6;         // microseconds to move dW once
+    long long best = 1;
+    double t = 1e30;
+    for (long long s = 1; s <= max_s && s <= kNumSMs; ++s) {
+        const double u = (double)cdivll(base_units * s, kNumSMs) * cdivll(chunks, s) * 0.37 + (s > 1 ? 2.5 + (2 * s + 1) * pass : 0.0);
+        if (u < t) { t = u; best = s; }
+    }
+    const long long cps = cdivll(chunks, best);
     return (int)cdivll(chunks, cps);
 }
 
@@ -775,12 +814,10 @@ int conv_dv_tc(const float *V, const float *Wt, const float *dM, float *Wr, unsi
     if (P > 0x7fffffffLL - 128) return WG2X2_ERR_UNSUPPORTED;
     const int nKB = cdiv(K, 64), nCC = cdiv(C, 32);
     if (nCC > 65535) return WG2X2_ERR_UNSUPPORTED;
-    if (cudaMemsetAsync(map, nCC <= 64 ? 0 : 0xFF, (size_t)16 * nKB * sizeof(unsigned long long), st) != cudaSuccess) return WG2X2_ERR_LAUNCH;
-    launch(round_and_map_kernel, dim3(nKB, nCC, 16), 256, 0, st, Wt, Wr, map, C, K, nKB, nCC);
-    if (launch_status() != WG2X2_OK) return WG2X2_ERR_LAUNCH;
+    if (launch(round_and_map_kernel, dim3(nKB, cdiv(nCC, 8), 16), kPackThreads, 0, st, Wt, Wr, map, C, K, nKB, nCC) != WG2X2_OK) return WG2X2_ERR_LAUNCH;
     GgParams prm;
     prm.rows = P; prm.cols = C; prm.contr = K;
-    prm.N = gg_cols(C);
+    prm.N = gg_pick_cols(P, C, K);
     prm.nRB = (int)cdivll(P, 128);
     prm.nCB = cdiv(C, prm.N);
     prm.splits = 1;
@@ -886,26 +923,32 @@ __global__ void __launch_bounds__(256) out_transform_nhwc_kernel(const float *__
         }
 }
 
-// NCHW: lane = output channel over a band of R tile rows; the 2R x outW pixels of each channel collect in
-// shared memory and leave as one contiguous run per channel.
+// NCHW: lane = output channel over a band of R tile rows (or, SEG, a segment of one row); the output pixels of each channel
+// collect in shared memory and leave as one contiguous run per channel.
+template <bool SEG>
 __global__ void __launch_bounds__(256) out_transform_nchw_kernel(const float *__restrict__ M, float *__restrict__ Y, long long P,
-                                                                   int nH, int nW, int K, int outH, int outW, int R, int nbands,
-                                                                   int pitch, OutExtras ex)
+                                                                   int nH, int nW, int K, int outH, int outW, int R, int nbands, int S,
+                                                                   int nsegs, int pitch, OutExtras ex)
 {
     after_previous_kernel(M, Y, ex.scale, ex.shift, ex.residual);
     extern __shared__ float O[];
-    const int band = blockIdx.x % nbands;
-    const int b = blockIdx.x / nbands;
+    int bb = blockIdx.x;
+    const int seg = SEG ? bb % nsegs : 0;
+    if (SEG) bb /= nsegs;
+    const int band = bb % nbands;
+    const int b = bb / nbands;
     const int k0 = blockIdx.y * 32;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int th0 = band * R;
     const int rows_blk = min(R, nH - th0);
+    const int tw0 = SEG ? seg * S : 0, ns = SEG ? min(S, nW - tw0) : nW;
+    const int OW = SEG ? min(2 * ns, outW - 2 * tw0) : outW;        // pixels of an output row of the block
     const bool k_ok = k0 + lane < K;
     const float sc = (ex.scale && k_ok) ? __ldg(ex.scale + k0 + lane) : 1.f;
     const float sh = (ex.scale && k_ok) ? __ldg(ex.shift + k0 + lane) : 0.f;
-    for (int q = warp; q < rows_blk * nW; q += 8) {
-        const int br = q / nW, tw = q - br * nW;
-        const long long p = ((long long)b * nH + th0 + br) * nW + tw;
+    for (int q = warp; q < rows_blk * ns; q += 8) {
+        const int br = q / ns, tl = q - br * ns;
+        const long long p = ((long long)b * nH + th0 + br) * nW + tw0 + tl;
         float y[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
         if (k_ok) {
 #pragma unroll
@@ -922,21 +965,40 @@ __global__ void __launch_bounds__(256) out_transform_nchw_kernel(const float *__
         for (int a = 0; a < 2; ++a)
 #pragma unroll
             for (int e = 0; e < 2; ++e)
-                if (2 * tw + e < outW) O[lane * pitch + (2 * br + a) * outW + 2 * tw + e] = fmaf(y[a][e], sc, sh);
+                if (2 * tl + e < OW) O[lane * pitch + (2 * br + a) * OW + 2 * tl + e] = fmaf(y[a][e], sc, sh);
     }
     __syncthreads();
     const int lo = 2 * th0, hi = min(2 * th0 + 2 * rows_blk, outH);
-    const int n = (hi - lo) * outW;
+    const int n = (hi - lo) * OW;
     for (int kk = warp; kk < 32; kk += 8) {
         if (k0 + kk >= K) break;
-        const long long o = (((long long)b * K + k0 + kk) * outH + lo) * outW;
+        const long long o = (((long long)b * K + k0 + kk) * outH + lo) * outW + 2 * tw0;
         const float *src = O + kk * pitch;
-        if (ex.residual) { for (int i = lane; i < n; i += 32) Y[o + i] = src[i] + __ldg(ex.residual + o + i); }
-        else             { for (int i = lane; i < n; i += 32) Y[o + i] = src[i]; }
+        if (!SEG) {
+            if (ex.residual) { for (int i = lane; i < n; i += 32) Y[o + i] = src[i] + __ldg(ex.residual + o + i); }
+            else             { for (int i = lane; i < n; i += 32) Y[o + i] = src[i]; }
+        } else {                                                    // two rows of a segment
+            for (int i = lane; i < n; i += 32) {
+                const long long d = o + (i >= OW ? outW + i - OW : i);
+                Y[d] = ex.residual ? src[i] + __ldg(ex.residual + d) : src[i];
+            }
+        }
     }
 }
 
-bool conv_fwd_wide_preferred(int C, int K) { return C >= 256 && K >= 256 && C % 4 == 0 && K % 4 == 0; }
+// Row-walk kernel or wide path for P tiles?  Microseconds, from timing both over 16 .. 25088 tiles and 32 .. 512 channels: a
+// row-walk unit (128 tiles x 64 channels) is a serial chain of 16 x C / 32 chunks of 0.27 us and few tiles are few units, while
+// the GEMM spreads the 16 positions over the SMs; the wide path in turn moves the products through memory.  3 x 11 x 11 tiles
+// of a 512 -> 96 channel layer: 71 us on two SMs against 11.
+bool conv_fwd_wide_preferred(long long P, int C, int K)
+{
+    if (C % 4 || K % 4) return false;
+    if (C >= 256 && K >= 256) return true;
+    const double rounds = (double)cdivll(cdivll(P, kBlockM) * cdiv(K, kBlockN), kNumSMs);
+    const double row_walk = fmax(7.5 + rounds * 4.3 * cdiv(C, kBlockK), 5.0 + (64.0 * P * C + 16.0 * P * K) / 6e6);
+    const double wide = 6.8 + (64.0 * P * (C + 2.0 * K) + 16.0 * P * K) / 5.5e6;
+    return wide < row_walk;
+}
 size_t conv_fwd_wide_workspace_bytes(long long P, int K) { return align_up((size_t)16 * P * K * sizeof(float), 256); }
 
 int conv_fwd_tc_wide(const float *V, const void *prepared, float *Y, int B, int nH, int nW, int C, int K, int outH, int outW,
@@ -953,7 +1015,7 @@ int conv_fwd_tc_wide(const float *V, const void *prepared, float *Y, int B, int 
     float *M = static_cast<float *>(ws);
     GgParams prm;
     prm.rows = P; prm.cols = K; prm.contr = C;
-    prm.N = gg_cols(K);
+    prm.N = gg_pick_cols(P, K, C);
     prm.nRB = (int)cdivll(P, 128);
     prm.nCB = cdiv(K, prm.N);
     prm.splits = 1;
@@ -976,18 +1038,13 @@ int conv_fwd_tc_wide(const float *V, const void *prepared, float *Y, int B, int 
     if (layout == WG2X2_NHWC) {
         launch(out_transform_nhwc_kernel, dim3((unsigned)cdivll(P * (K / 4), 256)), 256, 0, st, M, Y, P, nH, nW, K, outH, outW, ex);
     } else {
-        int R = 384 / (2 * outW);
-        if (R < 1) R = 1;
-        if (R > nH) R = nH;
-        // a small batch: lower bands, so that the grid still gives every SM a few blocks
-        while (R > 1 && (long long)B * cdiv(nH, R) * cdiv(K, 32) < 3LL * kNumSMs) --R;
-        const int nbands = cdiv(nH, R);
-        R = cdiv(nH, nbands);
-        const int pitch = (2 * R * outW) | 1;
+        const BandCut cut = cut_bands(nH, nW, (long long)B * cdiv(K, 32), 384 / (2 * outW));
+        const int pitch = (2 * cut.R * (cut.nsegs == 1 ? outW : 2 * cut.S)) | 1;
         const int smem = 32 * pitch * (int)sizeof(float);
-        if ((long long)B * nbands > 0x7fffffffLL || smem > 200 * 1024) return WG2X2_ERR_UNSUPPORTED;
-        launch(out_transform_nchw_kernel, dim3((unsigned)(B * nbands), cdiv(K, 32)), 256, smem, st, M, Y, P, nH, nW, K, outH, outW, R,
-                                                                                                 nbands, pitch, ex);
+        const long long blocks = (long long)B * cut.nbands * cut.nsegs;
+        if (blocks > 0x7fffffffLL || smem > 200 * 1024) return WG2X2_ERR_UNSUPPORTED;
+        launch(cut.nsegs == 1 ? out_transform_nchw_kernel<false> : out_transform_nchw_kernel<true>, dim3((unsigned)blocks, cdiv(K, 32)), 256, smem, st,
+               M, Y, P, nH, nW, K, outH, outW, cut.R, cut.nbands, cut.S, cut.nsegs, pitch, ex);
     }
     return launch_status();
 }

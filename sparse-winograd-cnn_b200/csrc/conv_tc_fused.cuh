@@ -908,3 +908,22 @@ int layer_fwd_fused(const float *X, const void *prepared, float *Y, int B, int H
                           : (affine ? layer_fwd_fused_kernel<false, true> : layer_fwd_fused_kernel<false, false>);
     return launch(kernel, dim3((unsigned)grid), kFuThreads, kFuSmemBytes, st, mapX1, mapX2, mapW, mapW2, mapY, p);
 }
+
+// One-kernel layer or input transform + wide path?  Microseconds, from timing both over 1 .. 64 images of 8 .. 56 pixels and
+// 32 .. 256 channels.  A unit of the one-kernel layer is a serial chain over the input channels (4 us per 32 when its SM has
+// nothing else to do, 5.8 in a full grid; a third more where the tiles fill their lanes and the outer pixels need loads of
+// their own), the wide path is three short kernels plus what they move through memory: 64 -> 64 channels at 56 x 56 take
+// 13.9 against 17.6 us for one image, 128 -> 128 at 16 x 16 take 25 against 11.5.
+bool layer_fused_preferred(int B, int H, int W, int C, int K, int layout)
+{
+    if (!fused_fwd_supported(B, H, W, C, K, layout)) return false;
+    FuParams p;
+    p.B = B; p.H = H; p.W = W; p.C = C; p.K = K;
+    if (!fused_geometry(p)) return false;
+    const double P = (double)B * p.nH * p.nW, rounds = cdiv(p.units, kNumSMs);
+    const bool by_lanes = (1 << p.lp_log2) - p.TW >= 2;
+    const double fused = 6.0 + (4.0 + 5.8 * (rounds - 1)) * p.nC32 * (by_lanes ? 1.0 : 1.3);
+    if (K % 4) return true;
+    const double wide = 9.5 + (4.0 * B * H * W * ((double)C + K) + 128.0 * P * ((double)C + K)) / 5.3e6;
+    return fused <= wide;
+}

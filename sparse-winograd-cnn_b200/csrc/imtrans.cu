@@ -207,6 +207,50 @@ __global__ void __launch_bounds__(256) imtrans_fwd_nchw_band_kernel(const float 
     }
 }
 
+// The same for small problems: a segment of S tiles of one tile row per CTA (cut_bands).  (A kernel of its own: as a variant of
+// the one above it cost that one eight registers and 7 % of its speed.)
+template <bool AFFINE>
+__global__ void __launch_bounds__(256) imtrans_fwd_nchw_row_kernel(const float *__restrict__ X, float *__restrict__ V,
+                                                                     int B, int H, int W, int C, int nH, int nW, int relu,
+                                                                     int S_, int nsegs, int pitch,
+                                                                     const float *__restrict__ scale, const float *__restrict__ shift)
+{
+    after_previous_kernel(X, V, scale, shift);
+    extern __shared__ float S[];   // [32 channels][pitch]
+    const int seg = blockIdx.x % nsegs, th = (blockIdx.x / nsegs) % nH, b = blockIdx.x / nsegs / nH;
+    const int c0 = blockIdx.y * 32;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int gy0 = 2 * th - 1, lo = max(gy0, 0), hi = min(gy0 + 4, H);
+    const int tw0 = seg * S_, ns = min(S_, nW - tw0);
+    const int x0 = max(2 * tw0 - 1, 0), SW = min(2 * (tw0 + ns) + 1, W) - x0;     // staged columns: the tiles' and their neighbours
+    stage_channels(X + (((long long)b * C + c0) * H + lo) * W + x0, (long long)H * W, C - c0, (hi - lo) * SW, S + (lo - gy0) * SW, pitch,
+                   [&](int i) { return i + (i / SW) * (W - SW); });
+    __syncthreads();
+    if (c0 + lane >= C) return;
+    const long long plane = (long long)B * nH * nW * C;
+    const float *Sc = S + lane * pitch;
+    const float sc = AFFINE ? __ldg(scale + c0 + lane) : 1.f, sh = AFFINE ? __ldg(shift + c0 + lane) : 0.f;
+    for (int tl = warp; tl < ns; tl += 8) {
+        float d[4][4], v[4][4];
+#pragma unroll
+        for (int y = 0; y < 4; ++y) {
+            const bool row_ok = gy0 + y >= 0 && gy0 + y < H;
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                const int gx = 2 * (tw0 + tl) - 1 + x;
+                const bool in = row_ok && gx >= 0 && gx < W;
+                d[y][x] = in ? (AFFINE ? fmaf(Sc[y * SW + gx - x0], sc, sh) : Sc[y * SW + gx - x0]) : 0.f;
+            }
+        }
+        bt_d_b(d, v);
+        const long long off = (((long long)b * nH + th) * nW + tw0 + tl) * C + c0 + lane;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) V[(long long)(4 * i + j) * plane + off] = relu ? fmaxf(v[i][j], 0.f) : v[i][j];
+    }
+}
+
 // The same with four channels per lane: every plane store is 16 bytes per lane, 512 bytes per warp with LC = 32
 // lanes along the channels (128 per CTA), 256 bytes with LC = 16 (64 per CTA, the two halves of a warp on two tiles
 // at once).  Where the band is the whole image the CTA's channels are one contiguous run of X and are staged as such.
@@ -723,20 +767,18 @@ int imtrans_fwd(const float *X, float *V, int B, int H, int W, int C, int layout
             launch(scale ? imtrans_fwd_nchw_vec_kernel<32, true> : imtrans_fwd_nchw_vec_kernel<32, false>, gb, 256, smem, st, X, V, B, H, W, C,
                    nH, nW, relu, R, nbands, pitch, scale, shift);
         } else if (W <= 128) {
-            int R = (kBandFloats / W - 2) / 2;
-            if (R < 1) R = 1;
-            if (R > nH) R = nH;
-            // a small batch: lower bands, so that the grid still gives every SM a few blocks
-            while (R > 1 && (long long)B * cdiv(nH, R) * cdiv(C, 32) < 3LL * kNumSMs) --R;
-            const int nbands = cdiv(nH, R);
-            R = cdiv(nH, nbands);
-            const int pitch = ((2 * R + 2) * W) | 1;
+            const BandCut cut = cut_bands(nH, nW, (long long)B * cdiv(C, 32), (kBandFloats / W - 2) / 2);
+            const int pitch = ((2 * cut.R + 2) * (cut.nsegs == 1 ? W : 2 * cut.S + 2)) | 1;
             const int smem = 32 * pitch * (int)sizeof(float);
-            const long long gxb = (long long)B * nbands;
+            const long long gxb = (long long)B * cut.nbands * cut.nsegs;
             if (gxb > 0x7fffffffLL) return WG2X2_ERR_UNSUPPORTED;
             const dim3 gb((unsigned)gxb, cdiv(C, 32));
-            launch(scale ? imtrans_fwd_nchw_band_kernel<true> : imtrans_fwd_nchw_band_kernel<false>, gb, 256, smem, st, X, V, B, H, W, C, nH, nW,
-                   relu, R, nbands, pitch, scale, shift);
+            if (cut.nsegs == 1)
+                launch(scale ? imtrans_fwd_nchw_band_kernel<true> : imtrans_fwd_nchw_band_kernel<false>, gb, 256, smem, st, X, V, B, H, W, C, nH,
+                       nW, relu, cut.R, cut.nbands, pitch, scale, shift);
+            else
+                launch(scale ? imtrans_fwd_nchw_row_kernel<true> : imtrans_fwd_nchw_row_kernel<false>, gb, 256, smem, st, X, V, B, H, W, C, nH, nW,
+                       relu, cut.S, cut.nsegs, pitch, scale, shift);
         } else {
             launch(imtrans_fwd_nchw_kernel, grid, 256, 0, st, X, V, B, H, W, C, nH, nW, relu, scale, shift);
         }

@@ -108,6 +108,24 @@ inline BandCut cut_bands(int nH, int nW, long long blocks, int max_rows)
     return c;
 }
 
+// Staging for those kernels: each of eight warps copies four of 32 channel planes (nch of them exist) to rows of shared memory,
+// `n` floats per channel at src(i) / dst[i], four channels at a time so that as many loads are in flight.
+template <typename Src>
+__device__ __forceinline__ void stage_channels(const float *__restrict__ plane0, long long plane, int nch, int n, float *dst0, int pitch, Src src)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const float *p = plane0 + warp * plane;
+    float *d = dst0 + warp * pitch;
+    for (int i = lane; i < n; i += 32) {
+        const int o = src(i);
+        float v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = warp + 8 * q < nch ? __ldg(p + 8 * q * plane + o) : 0.f;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) d[8 * q * pitch + i] = v[q];
+    }
+}
+
 inline int launch_status()
 {
     return cudaGetLastError() == cudaSuccess ? WG2X2_OK : WG2X2_ERR_LAUNCH;

@@ -98,10 +98,9 @@ class _WinogradLayer(torch.nn.Module):
         return self._from_kernel(y, layout)
 
     def onekernel_pays(self, x, layout):
-        """True where the whole layer (both BatchNorms, ReLU, products, shortcut add) runs as the one-kernel path."""
+        """True where the whole layer (both BatchNorms, ReLU, products, shortcut add) is fastest as the one-kernel path."""
         B, C, H, W = x.shape
-        return (layout == "NCHW" and (self.cout <= 128 or (self.cout <= 256 and C <= 64))
-                and wg2x2.fused_supported(B, H, W, C, self.cout, "NCHW"))
+        return wg2x2.fused_preferred(B, H, W, C, self.cout, layout)
 
     def forward_onekernel(self, x, bn_in, bn_out=None, residual=None):
         """BatchNorm -> transform + ReLU -> product [-> BatchNorm + shortcut add] in one kernel (NCHW)."""

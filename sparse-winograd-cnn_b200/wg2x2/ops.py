@@ -85,11 +85,16 @@ def fused_supported(B, H, W, C, K, layout="NCHW"):
     return bool(lib.wg2x2_layer_fwd_fused_supported(B, H, W, C, K, _LAYOUTS[layout]))
 
 
+def fused_preferred(B, H, W, C, K, layout="NCHW"):
+    """True where layer_fwd_prepared runs the whole layer as one kernel."""
+    return bool(lib.wg2x2_layer_fwd_fused_preferred(B, H, W, C, K, _LAYOUTS[layout]))
+
+
 def layer_fwd_prepared(x, prepared, K, relu=True, layout="NHWC", out=None, V_scratch=None, out_scale=None, out_shift=None,
                        residual=None, workspace=None):
-    """Whole layer with prepared weights: one fused kernel where supported (V never stored), else transform +
-    product through V_scratch (allocated here when not given); layers with C, K >= 256 take the wide product path
-    through `workspace` (allocated here when not given; layer_fwd_prepared_workspace_bytes)."""
+    """Whole layer with prepared weights: one fused kernel where supported and faster (V never stored), else transform +
+    product through V_scratch (allocated here when not given); layers with many channels or few tiles take the wide
+    product path through `workspace` (allocated here when not given; layer_fwd_prepared_workspace_bytes)."""
     return _native.layer_fwd_prepared(x, prepared, K, relu, _LAYOUTS[layout], out, V_scratch, out_scale, out_shift, residual, workspace)
 
 

@@ -27,3 +27,35 @@ def test_segmented_rows(oracle, shape):
     assert oracle.max_rel(gV.cpu().numpy(), dVo) <= 5e-3
     assert oracle.max_rel(gW.cpu().numpy(), dWo) <= 5e-3
     assert wg2x2.last_device_status()[0] == 0
+
+
+# few tiles: the wide path with 64, 128 and 256 columns per unit, channel counts that end inside a tile, a chunk and a byte of
+# the zero-block map (the last shape has more than 64 chunks: no map); every third 64 x 32 weight block is empty
+@pytest.mark.parametrize("layout", ["NHWC", "NCHW"])
+@pytest.mark.parametrize("shape", [(1, 1, 1, 4, 4), (3, 11, 11, 512, 96), (1, 14, 14, 300, 68), (2, 27, 26, 128, 132), (4, 14, 15, 64, 516),
+                                   (16, 7, 7, 260, 260), (1, 8, 8, 36, 4), (1, 3, 3, 2080, 64)])
+def test_few_tiles(oracle, shape, layout):
+    import torch
+    import wg2x2
+    B, H, W, C, K = shape
+    rng = np.random.default_rng(sum(shape))
+    X = rng.standard_normal((B, H, W, C)).astype(np.float32)
+    Wt = (rng.standard_normal((16, C, K)) / np.sqrt(C)).astype(np.float32)
+    for t in range(16):
+        for cc in range(0, C, 32):
+            for kb in range(0, K, 64):
+                if (t + cc // 32 + kb // 64) % 3 == 0:
+                    Wt[t, cc:cc + 32, kb:kb + 64] = 0
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    img = lambda a: dev(a if layout == "NHWC" else np.transpose(a, (0, 3, 1, 2)))
+    back = lambda t: t.cpu().numpy() if layout == "NHWC" else np.transpose(t.cpu().numpy(), (0, 2, 3, 1))
+    V = oracle.imtrans_fwd(X, relu=True, dtype=np.float32)
+    want = oracle.conv_fwd(V, Wt, H, W)
+    assert wg2x2._lib.lib.wg2x2_conv_fwd_prepared_workspace_bytes(B, (H + 1) // 2, (W + 1) // 2, C, K) > 0
+    prepared = wg2x2.prepare_weights(dev(Wt))
+    for Y in (wg2x2.conv_fwd(dev(V), dev(Wt), H, W, layout=layout, math="tf32"),
+              wg2x2.conv_fwd_prepared(dev(V), prepared, K, H, W, layout=layout),
+              wg2x2.conv_fwd_prepared(dev(V), prepared, K, H, W, layout=layout, wide=False),
+              wg2x2.layer_fwd_prepared(img(X), prepared, K, relu=True, layout=layout)):
+        assert oracle.max_rel(back(Y), want) <= 5e-3
+    assert wg2x2.last_device_status()[0] == 0
