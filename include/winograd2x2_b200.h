@@ -196,6 +196,20 @@ int wg2x2_layer_fwd_prepared_ws(const float *X, const void *prepared, float *Y, 
                                 int C, int K, int layout, int relu, const float *out_scale, const float *out_shift,
                                 const float *residual, void *workspace, size_t workspace_bytes, void *stream);
 size_t wg2x2_layer_fwd_prepared_workspace_bytes(int B, int H, int W, int C, int K);
+/*
+ * The general form of the two calls above, with the options of a residual block's layers: in_scale / in_shift (C floats each,
+ * or NULL) are the affine map in front of the transform as in wg2x2_layer_fwd_fused_affine; with residual_relu the shortcut
+ * passes through a ReLU before it is added.  Layers of few tiles run as one kernel on clusters of four CTAs in either
+ * layout and at any image size (X, Y, residual, in_scale and in_shift 16-byte aligned) and read neither scratch buffer.
+ * wg2x2_layer_fwd_prepared_scratch: the bytes of V_scratch and workspace with which the call is fastest (0: not used);
+ * `aligned`: whether all of those pointers are on 16-byte boundaries.
+ */
+int wg2x2_layer_fwd_prepared_ex(const float *X, const float *in_scale, const float *in_shift, const void *prepared, float *Y,
+                                float *V_scratch, int B, int H, int W, int C, int K, int layout, int relu,
+                                const float *out_scale, const float *out_shift, const float *residual, int residual_relu,
+                                void *workspace, size_t workspace_bytes, void *stream);
+void wg2x2_layer_fwd_prepared_scratch(int B, int H, int W, int C, int K, int layout, int aligned, size_t *v_bytes,
+                                      size_t *workspace_bytes);
 int wg2x2_layer_fwd_fused_supported(int B, int H, int W, int C, int K, int layout);
 /* 1 where wg2x2_layer_fwd_prepared_ws runs the one kernel even if both scratch buffers are given (it then reads neither). */
 int wg2x2_layer_fwd_fused_preferred(int B, int H, int W, int C, int K, int layout);

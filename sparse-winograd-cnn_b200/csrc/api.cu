@@ -27,17 +27,22 @@ int tc_wait_probe(long long polls, unsigned where, cudaStream_t st);
 size_t prepared_weights_bytes(int C, int K);
 int weights_prepare(const float *Wt, int C, int K, void *prepared, size_t bytes, cudaStream_t st);
 int conv_fwd_tc_prepared(const float *V, const void *prepared, float *Y, int B, int nH, int nW, int C, int K, int outH, int outW,
-                         int layout, const float *out_scale, const float *out_shift, const float *residual, cudaStream_t st);
+                         int layout, const float *out_scale, const float *out_shift, const float *residual, int res_relu, cudaStream_t st);
 bool conv_fwd_wide_preferred(long long P, int C, int K);
 size_t conv_fwd_wide_workspace_bytes(long long P, int K);
 int conv_fwd_tc_wide(const float *V, const void *prepared, float *Y, int B, int nH, int nW, int C, int K, int outH, int outW,
-                     int layout, const float *out_scale, const float *out_shift, const float *residual, void *ws, size_t ws_bytes,
-                     cudaStream_t st);
+                     int layout, const float *out_scale, const float *out_shift, const float *residual, int res_relu, void *ws,
+                     size_t ws_bytes, cudaStream_t st);
 bool fused_fwd_supported(int B, int H, int W, int C, int K, int layout);
 bool layer_fused_preferred(int B, int H, int W, int C, int K, int layout);
+bool layer_cluster_preferred(int B, int H, int W, int C, int K, int layout);
+bool fused_beats_wide(int B, int H, int W, int C, int K, int layout, double *us);
 int layer_fwd_fused(const float *X, const void *prepared, float *Y, int B, int H, int W, int C, int K, int relu,
                     const float *in_scale, const float *in_shift, const float *out_scale, const float *out_shift,
-                    const float *residual, cudaStream_t st);
+                    const float *residual, int res_relu, cudaStream_t st);
+int layer_fwd_cluster(const float *X, const void *prepared, float *Y, int B, int H, int W, int C, int K, int layout, int relu,
+                      const float *in_scale, const float *in_shift, const float *out_scale, const float *out_shift, const float *residual,
+                      int res_relu, cudaStream_t st);
 size_t conv_bwd_tc_workspace_bytes(long long P, int C, int K, int want_dW);
 int conv_bwd_tc(const float *V, const float *Wt, const float *dY, const float *mask, float *dV, float *dW, int B, int H, int W,
                 int C, int K, int layout, int relu, void *ws, size_t ws_bytes, cudaStream_t st);
@@ -115,7 +120,7 @@ int wg2x2_conv_fwd_prepared(const float *V, const void *prepared, float *Y, int 
 {
     if (!V || !prepared || !Y || B <= 0 || nH <= 0 || nW <= 0 || C <= 0 || K <= 0) return WG2X2_ERR_BAD_ARG;
     if (!layout_ok(layout) || !crop_ok(out_h, nH) || !crop_ok(out_w, nW)) return WG2X2_ERR_BAD_ARG;
-    return conv_fwd_tc_prepared(V, prepared, Y, B, nH, nW, C, K, out_h, out_w, layout, nullptr, nullptr, nullptr, (cudaStream_t)stream);
+    return conv_fwd_tc_prepared(V, prepared, Y, B, nH, nW, C, K, out_h, out_w, layout, nullptr, nullptr, nullptr, 0, (cudaStream_t)stream);
 }
 
 int wg2x2_conv_fwd_prepared_fused(const float *V, const void *prepared, float *Y, int B, int nH, int nW, int C, int K, int out_h,
@@ -124,7 +129,7 @@ int wg2x2_conv_fwd_prepared_fused(const float *V, const void *prepared, float *Y
 {
     if (!V || !prepared || !Y || B <= 0 || nH <= 0 || nW <= 0 || C <= 0 || K <= 0) return WG2X2_ERR_BAD_ARG;
     if (!layout_ok(layout) || !crop_ok(out_h, nH) || !crop_ok(out_w, nW)) return WG2X2_ERR_BAD_ARG;
-    return conv_fwd_tc_prepared(V, prepared, Y, B, nH, nW, C, K, out_h, out_w, layout, out_scale, out_shift, residual,
+    return conv_fwd_tc_prepared(V, prepared, Y, B, nH, nW, C, K, out_h, out_w, layout, out_scale, out_shift, residual, 0,
                                 (cudaStream_t)stream);
 }
 
@@ -192,6 +197,17 @@ size_t wg2x2_conv_fwd_prepared_workspace_bytes(int B, int nH, int nW, int C, int
     return conv_fwd_wide_workspace_bytes((long long)B * nH * nW, K);
 }
 
+// the products of a transformed input: wide path where preferred and given its scratch, else the row-walk kernel
+static int products_fwd(const float *V, const void *prepared, float *Y, int B, int nH, int nW, int C, int K, int out_h, int out_w, int layout,
+                        const float *out_scale, const float *out_shift, const float *residual, int res_relu, void *workspace,
+                        size_t workspace_bytes, cudaStream_t st)
+{
+    if (workspace && conv_fwd_wide_preferred((long long)B * nH * nW, C, K))
+        return conv_fwd_tc_wide(V, prepared, Y, B, nH, nW, C, K, out_h, out_w, layout, out_scale, out_shift, residual, res_relu, workspace,
+                                workspace_bytes, st);
+    return conv_fwd_tc_prepared(V, prepared, Y, B, nH, nW, C, K, out_h, out_w, layout, out_scale, out_shift, residual, res_relu, st);
+}
+
 int wg2x2_conv_fwd_prepared_ws(const float *V, const void *prepared, float *Y, int B, int nH, int nW, int C, int K, int out_h,
                                int out_w, int layout, const float *out_scale, const float *out_shift, const float *residual,
                                void *workspace, size_t workspace_bytes, void *stream)
@@ -199,11 +215,8 @@ int wg2x2_conv_fwd_prepared_ws(const float *V, const void *prepared, float *Y, i
     if (!V || !prepared || !Y || B <= 0 || nH <= 0 || nW <= 0 || C <= 0 || K <= 0) return WG2X2_ERR_BAD_ARG;
     if (!layout_ok(layout) || !crop_ok(out_h, nH) || !crop_ok(out_w, nW)) return WG2X2_ERR_BAD_ARG;
     if ((out_scale == nullptr) != (out_shift == nullptr)) return WG2X2_ERR_BAD_ARG;
-    cudaStream_t st = (cudaStream_t)stream;
-    if (workspace && conv_fwd_wide_preferred((long long)B * nH * nW, C, K))
-        return conv_fwd_tc_wide(V, prepared, Y, B, nH, nW, C, K, out_h, out_w, layout, out_scale, out_shift, residual, workspace,
-                                workspace_bytes, st);
-    return conv_fwd_tc_prepared(V, prepared, Y, B, nH, nW, C, K, out_h, out_w, layout, out_scale, out_shift, residual, st);
+    return products_fwd(V, prepared, Y, B, nH, nW, C, K, out_h, out_w, layout, out_scale, out_shift, residual, 0, workspace, workspace_bytes,
+                        (cudaStream_t)stream);
 }
 
 int wg2x2_layer_fwd_fused_supported(int B, int H, int W, int C, int K, int layout)
@@ -216,60 +229,73 @@ int wg2x2_layer_fwd_fused_preferred(int B, int H, int W, int C, int K, int layou
     return (B > 0 && H > 0 && W > 0 && C > 0 && K > 0 && layer_fused_preferred(B, H, W, C, K, layout)) ? 1 : 0;
 }
 
-int wg2x2_layer_fwd_prepared(const float *X, const void *prepared, float *Y, float *V_scratch, int B, int H, int W, int C, int K,
-                             int layout, int relu, const float *out_scale, const float *out_shift, const float *residual,
-                             void *stream)
-{
-    if (!X || !prepared || !Y || B <= 0 || H <= 0 || W <= 0 || C <= 0 || K <= 0) return WG2X2_ERR_BAD_ARG;
-    if (!layout_ok(layout)) return WG2X2_ERR_BAD_ARG;
-    cudaStream_t st = (cudaStream_t)stream;
-    // The one-kernel path redoes the input transform for every block of 64 output channels, so it wins while
-    // there are few of them (measured: K <= 128, or K <= 256 with C <= 64); beyond that the two-kernel path,
-    // whose wide GEMM shares one transformed input among 256 output channels, is faster.
-    const bool fused_pays = K <= 128 || (K <= 256 && C <= 64);
-    const bool aligned16 = ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y)) & 15u) == 0;   // TMA both ways
-    if (fused_fwd_supported(B, H, W, C, K, layout) && aligned16 && (fused_pays || !V_scratch))
-        return layer_fwd_fused(X, prepared, Y, B, H, W, C, K, relu, nullptr, nullptr, out_scale, out_shift, residual, st);
-    if (!V_scratch) return WG2X2_ERR_WORKSPACE;
-    const int nH = (H + 1) / 2, nW = (W + 1) / 2;
-    const int s = imtrans_fwd(X, V_scratch, B, H, W, C, layout, relu, nullptr, nullptr, st);
-    if (s != WG2X2_OK) return s;
-    return conv_fwd_tc_prepared(V_scratch, prepared, Y, B, nH, nW, C, K, H, W, layout, out_scale, out_shift, residual, st);
-}
-
 size_t wg2x2_layer_fwd_prepared_workspace_bytes(int B, int H, int W, int C, int K)
 {
     if (B <= 0 || H <= 0 || W <= 0 || C <= 0 || K <= 0) return 0;
     // (the layout is not known here: NHWC callers may ask wg2x2_conv_fwd_prepared_workspace_bytes instead)
-    if (layer_fused_preferred(B, H, W, C, K, WG2X2_NCHW)) return 0;
+    double us;
+    if (fused_beats_wide(B, H, W, C, K, WG2X2_NCHW, &us)) return 0;
     return wg2x2_conv_fwd_prepared_workspace_bytes(B, (H + 1) / 2, (W + 1) / 2, C, K);
+}
+
+void wg2x2_layer_fwd_prepared_scratch(int B, int H, int W, int C, int K, int layout, int aligned, size_t *v_bytes, size_t *workspace_bytes)
+{
+    *v_bytes = *workspace_bytes = 0;
+    if (B <= 0 || H <= 0 || W <= 0 || C <= 0 || K <= 0 || !layout_ok(layout)) return;
+    if (aligned && (layer_cluster_preferred(B, H, W, C, K, layout) || layer_fused_preferred(B, H, W, C, K, layout))) return;
+    const int nH = (H + 1) / 2, nW = (W + 1) / 2;
+    *workspace_bytes = wg2x2_conv_fwd_prepared_workspace_bytes(B, nH, nW, C, K);
+    if (*workspace_bytes || !aligned || !fused_fwd_supported(B, H, W, C, K, layout)) *v_bytes = sizeof(float) * 16 * (size_t)B * nH * nW * C;
+}
+
+int wg2x2_layer_fwd_prepared_ex(const float *X, const float *in_scale, const float *in_shift, const void *prepared, float *Y,
+                                float *V_scratch, int B, int H, int W, int C, int K, int layout, int relu, const float *out_scale,
+                                const float *out_shift, const float *residual, int residual_relu, void *workspace,
+                                size_t workspace_bytes, void *stream)
+{
+    if (!X || !prepared || !Y || B <= 0 || H <= 0 || W <= 0 || C <= 0 || K <= 0) return WG2X2_ERR_BAD_ARG;
+    if (!layout_ok(layout) || (in_scale == nullptr) != (in_shift == nullptr)) return WG2X2_ERR_BAD_ARG;
+    cudaStream_t st = (cudaStream_t)stream;
+    const int nH = (H + 1) / 2, nW = (W + 1) / 2;
+    auto on16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+    const bool aligned = on16(X) && on16(Y);           // TMA and 16-byte accesses both ways
+    const bool wide = V_scratch && workspace && conv_fwd_wide_preferred((long long)B * nH * nW, C, K);
+    if (aligned && on16(residual) && on16(in_scale) && on16(in_shift) && layer_cluster_preferred(B, H, W, C, K, layout))
+        return layer_fwd_cluster(X, prepared, Y, B, H, W, C, K, layout, relu, in_scale, in_shift, out_scale, out_shift, residual, residual_relu, st);
+    // The one-kernel path redoes the input transform for every block of 64 output channels.  Without scratch for the wide
+    // path it wins while there are few of them (measured: K <= 128, or K <= 256 with C <= 64).
+    if (aligned && fused_fwd_supported(B, H, W, C, K, layout) &&
+        (layer_fused_preferred(B, H, W, C, K, layout) || (!wide && (K <= 128 || (K <= 256 && C <= 64) || !V_scratch))))
+        return layer_fwd_fused(X, prepared, Y, B, H, W, C, K, relu, in_scale, in_shift, out_scale, out_shift, residual, residual_relu, st);
+    if (!V_scratch) return WG2X2_ERR_WORKSPACE;
+    if ((out_scale == nullptr) != (out_shift == nullptr)) return WG2X2_ERR_BAD_ARG;
+    const int s = imtrans_fwd(X, V_scratch, B, H, W, C, layout, relu, in_scale, in_shift, st);
+    if (s != WG2X2_OK) return s;
+    return products_fwd(V_scratch, prepared, Y, B, nH, nW, C, K, H, W, layout, out_scale, out_shift, residual, residual_relu, workspace,
+                        workspace_bytes, st);
+}
+
+int wg2x2_layer_fwd_prepared(const float *X, const void *prepared, float *Y, float *V_scratch, int B, int H, int W, int C, int K,
+                             int layout, int relu, const float *out_scale, const float *out_shift, const float *residual,
+                             void *stream)
+{
+    return wg2x2_layer_fwd_prepared_ex(X, nullptr, nullptr, prepared, Y, V_scratch, B, H, W, C, K, layout, relu, out_scale, out_shift, residual, 0,
+                                       nullptr, 0, stream);
 }
 
 int wg2x2_layer_fwd_prepared_ws(const float *X, const void *prepared, float *Y, float *V_scratch, int B, int H, int W, int C, int K,
                                 int layout, int relu, const float *out_scale, const float *out_shift, const float *residual,
                                 void *workspace, size_t workspace_bytes, void *stream)
 {
-    if (!X || !prepared || !Y || B <= 0 || H <= 0 || W <= 0 || C <= 0 || K <= 0) return WG2X2_ERR_BAD_ARG;
-    if (!layout_ok(layout)) return WG2X2_ERR_BAD_ARG;
-    const int nH = (H + 1) / 2, nW = (W + 1) / 2;
-    const bool aligned16 = ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y)) & 15u) == 0;
-    if (aligned16 && layer_fused_preferred(B, H, W, C, K, layout))
-        return layer_fwd_fused(X, prepared, Y, B, H, W, C, K, relu, nullptr, nullptr, out_scale, out_shift, residual, (cudaStream_t)stream);
-    // many channels or few tiles: input transform, then the products as wide GEMMs through the workspace
-    if (V_scratch && workspace && conv_fwd_wide_preferred((long long)B * nH * nW, C, K)) {
-        const int s = imtrans_fwd(X, V_scratch, B, H, W, C, layout, relu, nullptr, nullptr, (cudaStream_t)stream);
-        if (s != WG2X2_OK) return s;
-        return wg2x2_conv_fwd_prepared_ws(V_scratch, prepared, Y, B, nH, nW, C, K, H, W, layout, out_scale, out_shift, residual, workspace,
-                                          workspace_bytes, stream);
-    }
-    return wg2x2_layer_fwd_prepared(X, prepared, Y, V_scratch, B, H, W, C, K, layout, relu, out_scale, out_shift, residual, stream);
+    return wg2x2_layer_fwd_prepared_ex(X, nullptr, nullptr, prepared, Y, V_scratch, B, H, W, C, K, layout, relu, out_scale, out_shift, residual, 0,
+                                       workspace, workspace_bytes, stream);
 }
 
 int wg2x2_layer_fwd_fused(const float *X, const void *prepared, float *Y, int B, int H, int W, int C, int K, int relu,
                           const float *out_scale, const float *out_shift, const float *residual, void *stream)
 {
     if (!X || !prepared || !Y || B <= 0 || H <= 0 || W <= 0 || C <= 0 || K <= 0) return WG2X2_ERR_BAD_ARG;
-    return layer_fwd_fused(X, prepared, Y, B, H, W, C, K, relu, nullptr, nullptr, out_scale, out_shift, residual, (cudaStream_t)stream);
+    return layer_fwd_fused(X, prepared, Y, B, H, W, C, K, relu, nullptr, nullptr, out_scale, out_shift, residual, 0, (cudaStream_t)stream);
 }
 
 int wg2x2_layer_fwd_fused_affine(const float *X, const void *prepared, float *Y, int B, int H, int W, int C, int K, int relu,
@@ -277,7 +303,7 @@ int wg2x2_layer_fwd_fused_affine(const float *X, const void *prepared, float *Y,
                                  const float *residual, void *stream)
 {
     if (!X || !prepared || !Y || B <= 0 || H <= 0 || W <= 0 || C <= 0 || K <= 0) return WG2X2_ERR_BAD_ARG;
-    return layer_fwd_fused(X, prepared, Y, B, H, W, C, K, relu, in_scale, in_shift, out_scale, out_shift, residual, (cudaStream_t)stream);
+    return layer_fwd_fused(X, prepared, Y, B, H, W, C, K, relu, in_scale, in_shift, out_scale, out_shift, residual, 0, (cudaStream_t)stream);
 }
 
 int wg2x2_last_device_status(void *stream, unsigned int *where)

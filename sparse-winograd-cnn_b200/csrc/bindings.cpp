@@ -472,11 +472,42 @@ PyObject *py_layer_fwd(WG_ARGS)
     END_HANDLE_TH_ERRORS
 }
 
-// x, prepared, K, relu, layout, out, V_scratch, out_scale, out_shift, residual, workspace
+// The scratch buffers of a layer call, taken here where the caller gives none (or too little)
+struct LayerScratch {
+    Scratch vs, ws;
+    float *v = nullptr;
+    void *w = nullptr;
+    size_t wn = 0;
+    LayerScratch(const Img &d, int64_t K, int layout, bool aligned, const Tensor &V, const Tensor &uws)
+    {
+        size_t nv, nw;
+        wg2x2_layer_fwd_prepared_scratch(d.B, d.H, d.W, d.C, K, layout, aligned, &nv, &nw);
+        v = ptr(V);
+        if (!v && nv) { vs.take(nv); v = static_cast<float *>(vs.get()); }
+        if (nw) {
+            if (uws.defined() && (size_t)uws.numel() >= nw) w = uws.data_ptr();
+            else { ws.take(nw); w = ws.get(); }
+            wn = nw;
+        }
+    }
+};
+bool on16(const Tensor &t) { return !t.defined() || (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0; }
+
+void layer_fwd_prepared(const Tensor &x, const Tensor &prep, const Tensor &Y, const Img &d, int64_t K, bool relu, int layout, const Tensor &in_scale,
+                        const Tensor &in_shift, const Tensor &out_scale, const Tensor &out_shift, const Tensor &residual, bool residual_relu,
+                        const Tensor &V, const Tensor &uws, void *stream)
+{
+    const LayerScratch s(d, K, layout, on16(x) && on16(Y) && on16(residual) && on16(in_scale) && on16(in_shift), V, uws);
+    check(wg2x2_layer_fwd_prepared_ex(cptr(x), cptr(in_scale), cptr(in_shift), prep.data_ptr(), ptr(Y), s.v, d.B, d.H, d.W, d.C, K, layout, relu,
+                                      cptr(out_scale), cptr(out_shift), cptr(residual), residual_relu, s.w, s.wn, stream),
+          "wg2x2_layer_fwd_prepared_ex");
+}
+
+// x, prepared, K, relu, layout, out, V_scratch, out_scale, out_shift, residual, workspace, in_scale, in_shift, residual_relu
 PyObject *py_layer_fwd_prepared(WG_ARGS)
 {
     HANDLE_TH_ERRORS
-    want(n, 11);
+    want(n, 14);
     const Tensor x = arg(a[0], "x");
     const int layout = arg_int(a[4]);
     const Img d = img_of(x, layout, "x");
@@ -488,27 +519,13 @@ PyObject *py_layer_fwd_prepared(WG_ARGS)
     const Tensor sc = arg_shaped(a[7], {K}, "out_scale"), sh = arg_shaped(a[8], {K}, "out_shift"), res = arg_shaped(a[9], ys, "residual");
     const Tensor V = arg_shaped(a[6], {16, d.B, (d.H + 1) / 2, (d.W + 1) / 2, d.C}, "V_scratch");
     const Tensor uws = arg_raw(a[10], "workspace");
+    const Tensor isc = arg_shaped(a[11], {d.C}, "in_scale"), ish = arg_shaped(a[12], {d.C}, "in_shift");
+    const bool res_relu = arg_bool(a[13]);
     {
         WG_NOGIL;
         OnDevice on(x);
         if (!Y.defined()) Y = new_float(ys, x);
-        Scratch vs, ws;
-        const bool fused = wg2x2_layer_fwd_fused_preferred(d.B, d.H, d.W, d.C, K, layout) &&
-                           ((reinterpret_cast<uintptr_t>(x.data_ptr()) | reinterpret_cast<uintptr_t>(Y.data_ptr())) & 15u) == 0;
-        const size_t nws = fused ? 0 : wg2x2_conv_fwd_prepared_workspace_bytes(d.B, (d.H + 1) / 2, (d.W + 1) / 2, d.C, K);
-        float *vp = ptr(V);
-        if (!vp && !fused && (nws || !wg2x2_layer_fwd_fused_supported(d.B, d.H, d.W, d.C, K, layout))) {
-            vs.take(sizeof(float) * 16 * (size_t)d.B * ((d.H + 1) / 2) * ((d.W + 1) / 2) * d.C);
-            vp = static_cast<float *>(vs.get());
-        }
-        void *wp = nullptr;
-        if (nws) {
-            if (uws.defined() && (size_t)uws.numel() >= nws) wp = uws.data_ptr();
-            else { ws.take(nws); wp = ws.get(); }
-        }
-        check(wg2x2_layer_fwd_prepared_ws(cptr(x), prep.data_ptr(), ptr(Y), vp, d.B, d.H, d.W, d.C, K, layout, relu, cptr(sc), cptr(sh), cptr(res),
-                                          wp, nws, on.stream),
-              "wg2x2_layer_fwd_prepared_ws");
+        layer_fwd_prepared(x, prep, Y, d, K, relu, layout, isc, ish, sc, sh, res, res_relu, V, uws, on.stream);
     }
     return THPVariable_Wrap(Y);
     END_HANDLE_TH_ERRORS

@@ -263,6 +263,7 @@ struct TcParams {
     float *Y;
     // optional epilogue extras: Y = acc * out_scale[k] + out_shift[k] (+ residual, same shape and layout as Y)
     const float *out_scale, *out_shift, *residual;
+    int res_relu;            // the residual passes through a ReLU first
     const unsigned long long *masks;
     long long P;
     int nH, nW, C, K, outH, outW;
@@ -493,6 +494,7 @@ conv_fwd_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
                                 off[r] = __shfl_sync(0xffffffffu, my_off, 4 * r + (lane >> 3));
                                 rs[r] = make_float4(0.f, 0.f, 0.f, 0.f);
                                 if (EXTRAS && prm.residual && off[r] >= 0) rs[r] = __ldg(reinterpret_cast<const float4 *>(prm.residual + off[r]) + (lane & 7));
+                                if (EXTRAS && prm.res_relu) rs[r] = make_float4(fmaxf(rs[r].x, 0.f), fmaxf(rs[r].y, 0.f), fmaxf(rs[r].z, 0.f), fmaxf(rs[r].w, 0.f));
                             }
 #pragma unroll
                             for (int r = 0; r < 8; ++r) {
@@ -521,7 +523,7 @@ conv_fwd_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
                                 if (kbase + c < prm.K) {
                                     float v = y[2 * a + e][c];
                                     if (EXTRAS && prm.out_scale) v = fmaf(v, __ldg(prm.out_scale + kbase + c), __ldg(prm.out_shift + kbase + c));
-                                    if (EXTRAS && prm.residual) v += __ldg(prm.residual + o + c);
+                                    if (EXTRAS && prm.residual) v += prm.res_relu ? fmaxf(__ldg(prm.residual + o + c), 0.f) : __ldg(prm.residual + o + c);
                                     prm.Y[o + c] = v;
                                 }
                         }
@@ -547,6 +549,7 @@ conv_fwd_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
                                 const float *rp = prm.residual + o0 + (cg + c) * cstride;
                                 if (pair) rs[c] = __ldg(reinterpret_cast<const float2 *>(rp));
                                 else { rs[c].x = __ldg(rp); if (2 * tw + 1 < prm.outW) rs[c].y = __ldg(rp + 1); }
+                                if (prm.res_relu) rs[c] = make_float2(fmaxf(rs[c].x, 0.f), fmaxf(rs[c].y, 0.f));
                             }
                         }
 #pragma unroll
@@ -747,12 +750,12 @@ int weights_prepare(const float *Wt, int C, int K, void *prepared, size_t bytes,
 // (16, ncols, contr), both contraction-contiguous.
 static int tc_launch(int layout, const float *A, const float *Bop, const unsigned long long *masks, float *out, long long P,
                      int nH, int nW, int contr, int ncols, int outH, int outW, const float *out_scale, const float *out_shift,
-                     const float *residual, cudaStream_t st)
+                     const float *residual, int res_relu, cudaStream_t st)
 {
     if (P > 0x7fffffffLL - kBlockM) return WG2X2_ERR_UNSUPPORTED;
     TcParams prm;
     prm.Y = out;
-    prm.out_scale = out_scale; prm.out_shift = out_shift; prm.residual = residual;
+    prm.out_scale = out_scale; prm.out_shift = out_shift; prm.residual = residual; prm.res_relu = res_relu;
     prm.masks = masks;
     prm.P = P; prm.nH = nH; prm.nW = nW; prm.C = contr; prm.K = ncols; prm.outH = outH; prm.outW = outW;
     prm.nKB = cdiv(ncols, kBlockN);
@@ -786,7 +789,7 @@ static int tc_launch(int layout, const float *A, const float *Bop, const unsigne
 }
 
 int conv_fwd_tc_prepared(const float *V, const void *prepared, float *Y, int B, int nH, int nW, int C, int K, int outH, int outW,
-                         int layout, const float *out_scale, const float *out_shift, const float *residual, cudaStream_t st)
+                         int layout, const float *out_scale, const float *out_shift, const float *residual, int res_relu, cudaStream_t st)
 {
     if (!V || !prepared || !Y) return WG2X2_ERR_BAD_ARG;
     if ((out_scale == nullptr) != (out_shift == nullptr)) return WG2X2_ERR_BAD_ARG;
@@ -797,14 +800,14 @@ int conv_fwd_tc_prepared(const float *V, const void *prepared, float *Y, int B, 
     const unsigned long long *masks = reinterpret_cast<const unsigned long long *>(
         static_cast<const unsigned char *>(prepared) + align_up((size_t)16 * K * C * sizeof(float), 256));
     return tc_launch(layout, V, static_cast<const float *>(prepared), masks, Y, (long long)B * nH * nW, nH, nW, C, K, outH, outW,
-                     out_scale, out_shift, residual, st);
+                     out_scale, out_shift, residual, res_relu, st);
 }
 
 bool conv_fwd_wide_preferred(long long P, int C, int K);
 size_t conv_fwd_wide_workspace_bytes(long long P, int K);
 int conv_fwd_tc_wide(const float *V, const void *prepared, float *Y, int B, int nH, int nW, int C, int K, int outH, int outW,
-                     int layout, const float *out_scale, const float *out_shift, const float *residual, void *ws, size_t ws_bytes,
-                     cudaStream_t st);
+                     int layout, const float *out_scale, const float *out_shift, const float *residual, int res_relu, void *ws,
+                     size_t ws_bytes, cudaStream_t st);
 
 size_t conv_fwd_tc_workspace_bytes(int B, int nH, int nW, int C, int K)
 {
@@ -823,14 +826,15 @@ int conv_fwd_tc(const float *V, const float *Wt, float *Y, int B, int nH, int nW
     if (s != WG2X2_OK) return s;
     const size_t pb = prepared_weights_bytes(C, K);
     if (conv_fwd_wide_preferred((long long)B * nH * nW, C, K) && ws_bytes >= pb + conv_fwd_wide_workspace_bytes((long long)B * nH * nW, K))
-        return conv_fwd_tc_wide(V, ws, Y, B, nH, nW, C, K, outH, outW, layout, nullptr, nullptr, nullptr,
+        return conv_fwd_tc_wide(V, ws, Y, B, nH, nW, C, K, outH, outW, layout, nullptr, nullptr, nullptr, 0,
                                 static_cast<char *>(ws) + pb, ws_bytes - pb, st);
-    return conv_fwd_tc_prepared(V, ws, Y, B, nH, nW, C, K, outH, outW, layout, nullptr, nullptr, nullptr, st);
+    return conv_fwd_tc_prepared(V, ws, Y, B, nH, nW, C, K, outH, outW, layout, nullptr, nullptr, nullptr, 0, st);
 }
 
 void dw_reduce_launch(const float *partial, const float *mask, float *dW, long long n, int splits, cudaStream_t st);  // conv_ffma.cu
 
 #include "conv_tc_bwd.cuh"
+#include "conv_tc_cluster.cuh"
 #include "conv_tc_fused.cuh"
 
 #if defined(WG_TC_TRACE) || defined(WG_TC_DIAG)   // development builds only

@@ -878,6 +878,8 @@ int conv_bwd_tc(const float *V, const float *Wt, const float *dY, const float *m
 // ---------------------------------------------------------------------------------------
 struct OutExtras {
     const float *scale, *shift, *residual;
+    int res_relu;            // the residual passes through a ReLU first
+    __device__ __forceinline__ float shortcut(long long o) const { const float r = __ldg(residual + o); return res_relu ? fmaxf(r, 0.f) : r; }
 };
 
 // NHWC: one thread = one tile x 4 output channels
@@ -918,7 +920,9 @@ __global__ void __launch_bounds__(256) out_transform_nhwc_kernel(const float *__
             const long long o = ((((long long)b * outH + h) * outW + w) * K) / 4 + kv;
             float4 v = y[a][e];
             if (ex.scale) { v.x = fmaf(v.x, sc.x, sh.x); v.y = fmaf(v.y, sc.y, sh.y); v.z = fmaf(v.z, sc.z, sh.z); v.w = fmaf(v.w, sc.w, sh.w); }
-            if (ex.residual) { const float4 r = __ldg(reinterpret_cast<const float4 *>(ex.residual) + o); v = v + r; }
+            if (ex.residual) { float4 r = __ldg(reinterpret_cast<const float4 *>(ex.residual) + o);
+                               if (ex.res_relu) r = make_float4(fmaxf(r.x, 0.f), fmaxf(r.y, 0.f), fmaxf(r.z, 0.f), fmaxf(r.w, 0.f));
+                               v = v + r; }
             reinterpret_cast<float4 *>(Y)[o] = v;
         }
 }
@@ -975,12 +979,12 @@ __global__ void __launch_bounds__(256) out_transform_nchw_kernel(const float *__
         const long long o = (((long long)b * K + k0 + kk) * outH + lo) * outW + 2 * tw0;
         const float *src = O + kk * pitch;
         if (!SEG) {
-            if (ex.residual) { for (int i = lane; i < n; i += 32) Y[o + i] = src[i] + __ldg(ex.residual + o + i); }
+            if (ex.residual) { for (int i = lane; i < n; i += 32) Y[o + i] = src[i] + ex.shortcut(o + i); }
             else             { for (int i = lane; i < n; i += 32) Y[o + i] = src[i]; }
         } else {                                                    // two rows of a segment
             for (int i = lane; i < n; i += 32) {
                 const long long d = o + (i >= OW ? outW + i - OW : i);
-                Y[d] = ex.residual ? src[i] + __ldg(ex.residual + d) : src[i];
+                Y[d] = ex.residual ? src[i] + ex.shortcut(d) : src[i];
             }
         }
     }
@@ -1002,8 +1006,8 @@ bool conv_fwd_wide_preferred(long long P, int C, int K)
 size_t conv_fwd_wide_workspace_bytes(long long P, int K) { return align_up((size_t)16 * P * K * sizeof(float), 256); }
 
 int conv_fwd_tc_wide(const float *V, const void *prepared, float *Y, int B, int nH, int nW, int C, int K, int outH, int outW,
-                     int layout, const float *out_scale, const float *out_shift, const float *residual, void *ws, size_t ws_bytes,
-                     cudaStream_t st)
+                     int layout, const float *out_scale, const float *out_shift, const float *residual, int res_relu, void *ws,
+                     size_t ws_bytes, cudaStream_t st)
 {
     const long long P = (long long)B * nH * nW;
     if (P > 0x7fffffffLL - 128) return WG2X2_ERR_UNSUPPORTED;
@@ -1034,7 +1038,7 @@ int conv_fwd_tc_wide(const float *V, const void *prepared, float *Y, int B, int 
         return WG2X2_ERR_LAUNCH;
     int s = gg_launch<1>(mapA, mapB, prm, st, &mapBh);
     if (s != WG2X2_OK) return s;
-    OutExtras ex{out_scale, out_shift, residual};
+    OutExtras ex{out_scale, out_shift, residual, res_relu};
     if (layout == WG2X2_NHWC) {
         launch(out_transform_nhwc_kernel, dim3((unsigned)cdivll(P * (K / 4), 256)), 256, 0, st, M, Y, P, nH, nW, K, outH, outW, ex);
     } else {

@@ -828,9 +828,21 @@ static bool fused_geometry(FuParams &p)
     return true;
 }
 
+// The shortcut, ReLU applied, into the output buffer that the kernel then adds to (in place where they are one)
+__global__ void __launch_bounds__(256) relu_copy_kernel(const float *src, float *dst, long long n4)
+{
+    after_previous_kernel(src, dst);
+    const float4 *s = reinterpret_cast<const float4 *>(src);
+    float4 *d = reinterpret_cast<float4 *>(dst);
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n4; i += (long long)gridDim.x * 256) {
+        const float4 v = s[i];
+        d[i] = make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
+    }
+}
+
 int layer_fwd_fused(const float *X, const void *prepared, float *Y, int B, int H, int W, int C, int K, int relu,
                     const float *in_scale, const float *in_shift, const float *out_scale, const float *out_shift,
-                    const float *residual, cudaStream_t st)
+                    const float *residual, int res_relu, cudaStream_t st)
 {
     if (!X || !prepared || !Y) return WG2X2_ERR_BAD_ARG;
     if ((in_scale == nullptr) != (in_shift == nullptr)) return WG2X2_ERR_BAD_ARG;
@@ -842,9 +854,15 @@ int layer_fwd_fused(const float *X, const void *prepared, float *Y, int B, int H
     // The shortcut is added by the TMA unit: Y receives it first (unless it is Y already), then every box is reduced
     // into Y instead of stored.
     p.accumulate = residual != nullptr;
-    if (residual && residual != Y &&
-        cudaMemcpyAsync(Y, residual, sizeof(float) * (size_t)B * K * H * W, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
+    if (residual && res_relu) {
+        if (misaligned16(residual)) return WG2X2_ERR_BAD_ARG;
+        const long long n4 = (long long)B * K * H * W / 4;         // W % 4 == 0 here
+        const int s = launch(relu_copy_kernel, dim3((unsigned)(n4 < 256LL * 32 * kNumSMs ? cdivll(n4, 256) : 32 * kNumSMs)), 256, 0, st, residual, Y, n4);
+        if (s != WG2X2_OK) return s;
+    } else if (residual && residual != Y &&
+               cudaMemcpyAsync(Y, residual, sizeof(float) * (size_t)B * K * H * W, cudaMemcpyDeviceToDevice, st) != cudaSuccess) {
         return WG2X2_ERR_LAUNCH;
+    }
     p.in_scale = in_scale; p.in_shift = in_shift;
     p.masks = reinterpret_cast<const unsigned long long *>(static_cast<const unsigned char *>(prepared) +
                                                            align_up((size_t)16 * K * C * sizeof(float), 256));
@@ -914,7 +932,7 @@ int layer_fwd_fused(const float *X, const void *prepared, float *Y, int B, int H
 // nothing else to do, 5.8 in a full grid; a third more where the tiles fill their lanes and the outer pixels need loads of
 // their own), the wide path is three short kernels plus what they move through memory: 64 -> 64 channels at 56 x 56 take
 // 13.9 against 17.6 us for one image, 128 -> 128 at 16 x 16 take 25 against 11.5.
-bool layer_fused_preferred(int B, int H, int W, int C, int K, int layout)
+bool fused_beats_wide(int B, int H, int W, int C, int K, int layout, double *us)
 {
     if (!fused_fwd_supported(B, H, W, C, K, layout)) return false;
     FuParams p;
@@ -923,7 +941,36 @@ bool layer_fused_preferred(int B, int H, int W, int C, int K, int layout)
     const double P = (double)B * p.nH * p.nW, rounds = cdiv(p.units, kNumSMs);
     const bool by_lanes = (1 << p.lp_log2) - p.TW >= 2;
     const double fused = 6.0 + (4.0 + 5.8 * (rounds - 1)) * p.nC32 * (by_lanes ? 1.0 : 1.3);
+    *us = fused;
     if (K % 4) return true;
     const double wide = 9.5 + (4.0 * B * H * W * ((double)C + K) + 128.0 * P * ((double)C + K)) / 5.3e6;
     return fused <= wide;
+}
+
+// The layer of few tiles on clusters (conv_tc_cluster.cuh) against the others, all in microseconds: the one-kernel layer above,
+// the wide path, or transform + row-walk kernel (the formulas of the rules that choose among those).  1 x 14 x 14 with 256
+// channels 11.7 -> 9.0 us, 82 x 5 x 5 tiles of 64 channels 16.8 -> 7.6; above about 33 clusters' worth of work the wide path wins.
+bool layer_cluster_preferred(int B, int H, int W, int C, int K, int layout)
+{
+    if (!tc_shape_supported(C, K)) return false;
+    const long long P = (long long)B * ((H + 1) / 2) * ((W + 1) / 2);
+    if (P > 0x7fffffffLL - kBlockM) return false;
+    const double pixels = (double)B * H * W;
+    double other = 0.0;
+    if (!fused_beats_wide(B, H, W, C, K, layout, &other)) {
+        if (conv_fwd_wide_preferred(P, C, K)) {
+            other = 9.5 + (4.0 * pixels * ((double)C + K) + 128.0 * P * ((double)C + K)) / 5.3e6;
+        } else {
+            const double rounds = (double)cdivll(cdivll(P, kBlockM) * cdiv(K, kBlockN), kNumSMs);
+            other = fmax(7.5 + rounds * 4.3 * cdiv(C, kBlockK), 5.0 + (64.0 * P * C + 16.0 * P * K) / 6e6) + 3.0 +
+                    (4.0 * pixels + 64.0 * P) * C / 5e6;
+        }
+    }
+    return cl_cut(P, C, K).us < 0.97 * other;
+}
+
+bool layer_fused_preferred(int B, int H, int W, int C, int K, int layout)
+{
+    double us;
+    return !layer_cluster_preferred(B, H, W, C, K, layout) && fused_beats_wide(B, H, W, C, K, layout, &us);
 }

@@ -91,11 +91,14 @@ def fused_preferred(B, H, W, C, K, layout="NCHW"):
 
 
 def layer_fwd_prepared(x, prepared, K, relu=True, layout="NHWC", out=None, V_scratch=None, out_scale=None, out_shift=None,
-                       residual=None, workspace=None):
-    """Whole layer with prepared weights: one fused kernel where supported and faster (V never stored), else transform +
-    product through V_scratch (allocated here when not given); layers with many channels or few tiles take the wide
-    product path through `workspace` (allocated here when not given; layer_fwd_prepared_workspace_bytes)."""
-    return _native.layer_fwd_prepared(x, prepared, K, relu, _LAYOUTS[layout], out, V_scratch, out_scale, out_shift, residual, workspace)
+                       residual=None, workspace=None, in_scale=None, in_shift=None, residual_relu=False):
+    """Whole layer with prepared weights: one kernel where supported and faster (V never stored: a kernel of its own for few
+    tiles, the NCHW one for few channels), else transform + product through V_scratch (allocated here when not given); layers
+    with many channels take the wide product path through `workspace` (allocated here when not given;
+    layer_fwd_prepared_workspace_bytes).  in_scale / in_shift (C,): affine map of the pixels in front of the transform, the
+    padding stays zero; residual_relu: the shortcut passes through a ReLU first."""
+    return _native.layer_fwd_prepared(x, prepared, K, relu, _LAYOUTS[layout], out, V_scratch, out_scale, out_shift, residual, workspace,
+                                      in_scale, in_shift, residual_relu)
 
 
 def layer_fwd_prepared_workspace_bytes(B, H, W, C, K):
