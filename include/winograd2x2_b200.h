@@ -173,6 +173,12 @@ int wg2x2_layer_fwd(const float *X, const float *Wt, float *Y, float *V_out, int
 size_t wg2x2_layer_fwd_workspace_bytes(int B, int H, int W, int C, int K, int math, int keep_V);
 
 /*
+ * out[p] = mean over the n values of plane p of relu(X): the ReLU and global average pool in front of the classifier
+ * (ResNet-18-var/imagenet-resnet-transWino-prune.py:216-219).  X: planes x n floats.
+ */
+int wg2x2_relu_mean(const float *X, float *out, long long planes, int n, void *stream);
+
+/*
  * Whole layer forward with prepared weights (tensor-core path), the call pair of
  * ResNet-18-var/imagenet-resnet-transWino-prune.py:118-119 in its fastest form for the shape that needs no scratch
  * memory beyond V_scratch (wg2x2_layer_fwd_prepared_ws adds the wide path for C, K >= 256):

@@ -531,6 +531,54 @@ PyObject *py_layer_fwd_prepared(WG_ARGS)
     END_HANDLE_TH_ERRORS
 }
 
+// x, shortcut, K, prepared_a, in_scale_a, in_shift_a, prepared_b, in_scale_b, in_shift_b, out_scale, out_shift, layout: the two
+// layers of a residual block in one call.  The shortcut is added in place where there is one, else it is relu(x).
+PyObject *py_residual_block(WG_ARGS)
+{
+    HANDLE_TH_ERRORS
+    want(n, 12);
+    const Tensor x = arg(a[0], "x");
+    const int layout = arg_int(a[11]);
+    const Img d = img_of(x, layout, "x");
+    const int64_t K = arg_int(a[2]);
+    const auto ys = img_shape(d.B, d.H, d.W, K, layout);
+    const Tensor shortcut = arg_shaped(a[1], ys, "shortcut");
+    if (!shortcut.defined() && d.C != K) value_error("a block that changes the channel count needs a shortcut");
+    const Tensor pa = arg_prepared(a[3], d.C, K), pb = arg_prepared(a[6], K, K);
+    const Tensor sa = arg_shaped(a[4], {d.C}, "in_scale_a"), ta = arg_shaped(a[5], {d.C}, "in_shift_a");
+    const Tensor sb = arg_shaped(a[7], {K}, "in_scale_b"), tb = arg_shaped(a[8], {K}, "in_shift_b");
+    const Tensor so = arg_shaped(a[9], {K}, "out_scale"), to = arg_shaped(a[10], {K}, "out_shift");
+    Tensor y;
+    {
+        WG_NOGIL;
+        OnDevice on(x);
+        const Tensor mid = new_float(ys, x), none;
+        layer_fwd_prepared(x, pa, mid, d, K, true, layout, sa, ta, none, none, none, false, none, none, on.stream);
+        y = shortcut.defined() ? shortcut : new_float(ys, x);
+        layer_fwd_prepared(mid, pb, y, Img{d.B, d.H, d.W, K}, K, true, layout, sb, tb, so, to, shortcut.defined() ? shortcut : x,
+                           !shortcut.defined(), none, none, on.stream);
+    }
+    return THPVariable_Wrap(y);
+    END_HANDLE_TH_ERRORS
+}
+
+// x (B,C,H,W) -> (B,C): mean of relu(x) over the pixels
+PyObject *py_relu_mean(PyObject *, PyObject *o)
+{
+    HANDLE_TH_ERRORS
+    const Tensor x = arg(o, "x");
+    const Img d = img_of(x, WG2X2_NCHW, "x");
+    Tensor y;
+    {
+        WG_NOGIL;
+        OnDevice on(x);
+        y = new_float({d.B, d.C}, x);
+        check(wg2x2_relu_mean(cptr(x), ptr(y), d.B * d.C, (int)(d.H * d.W), on.stream), "wg2x2_relu_mean");
+    }
+    return THPVariable_Wrap(y);
+    END_HANDLE_TH_ERRORS
+}
+
 // x, prepared, K, relu, out, out_scale, out_shift, residual, in_scale, in_shift
 PyObject *py_layer_fwd_fused(WG_ARGS)
 {
@@ -662,6 +710,8 @@ PyMethodDef methods[] = {
     WG_FN("layer_fwd", py_layer_fwd),
     WG_FN("layer_fwd_prepared", py_layer_fwd_prepared),
     WG_FN("layer_fwd_fused", py_layer_fwd_fused),
+    WG_FN("residual_block", py_residual_block),
+    {"relu_mean", py_relu_mean, METH_O, nullptr},
     WG_FN("maxpool", py_maxpool),
     WG_FN("stem_pool", py_stem_pool),
     WG_FN("imtrans_op", py_imtrans_op),

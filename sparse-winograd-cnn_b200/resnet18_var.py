@@ -41,12 +41,10 @@ class _BN(torch.nn.Module):
     def forward(self, x):
         return x * self.scale.view(1, -1, 1, 1) + self.shift.view(1, -1, 1, 1)
 
-
-class _Affine:
-    """A (scale, shift) pair in the shape the layer calls take a BatchNorm."""
-
-    def __init__(self, scale, shift):
-        self.scale, self.shift = scale, shift
+    def pair(self):
+        """(scale, shift) in the form the layer calls take a BatchNorm"""
+        b = self._buffers
+        return b["scale"], b["shift"]
 
 
 class _WinogradLayer(torch.nn.Module):
@@ -63,8 +61,9 @@ class _WinogradLayer(torch.nn.Module):
         self._prepared = None
 
     def prepared(self):
-        if self._prepared is None or self._prepared.device != self.W.device:
-            self._prepared = wg2x2.prepare_weights(self.W)
+        W = self._buffers["W"]
+        if self._prepared is None or self._prepared.device != W.device:
+            self._prepared = wg2x2.prepare_weights(W)
         return self._prepared
 
     @staticmethod
@@ -85,31 +84,6 @@ class _WinogradLayer(torch.nn.Module):
         else:
             y = wg2x2.conv_fwd(v, self.W, H, W, layout=layout, math="fp32")
         return self._from_kernel(y, layout)
-
-    def forward_fused(self, x, bn_in, bn_out=None, residual=None, layout="NCHW"):
-        """BatchNorm -> transform + ReLU -> product [-> BatchNorm + shortcut add] in two kernels: bn_in folds
-        into the transform's load, bn_out and the residual into the product's epilogue (tensor-core path)."""
-        B, C, H, W = x.shape
-        v = wg2x2.imtrans_fwd(self._to_kernel(x, layout), relu=True, layout=layout, in_scale=bn_in.scale, in_shift=bn_in.shift)
-        y = wg2x2.conv_fwd_prepared(v, self.prepared(), self.cout, H, W, layout=layout,
-                                    out_scale=None if bn_out is None else bn_out.scale,
-                                    out_shift=None if bn_out is None else bn_out.shift,
-                                    residual=None if residual is None else self._to_kernel(residual, layout))
-        return self._from_kernel(y, layout)
-
-    def onekernel_pays(self, x, layout):
-        """True where the whole layer (both BatchNorms, ReLU, products, shortcut add) is fastest as the one-kernel path."""
-        B, C, H, W = x.shape
-        return wg2x2.fused_preferred(B, H, W, C, self.cout, layout)
-
-    def forward_onekernel(self, x, bn_in, bn_out=None, residual=None):
-        """BatchNorm -> transform + ReLU -> product [-> BatchNorm + shortcut add] in one kernel (NCHW)."""
-        res = None if residual is None else residual.contiguous()
-        # the shortcut tensor is not used again: the kernel adds into it in place (no copy of it into a new output)
-        return wg2x2.layer_fwd_fused(x.contiguous(), self.prepared(), self.cout, relu=True, out=res,
-                                     in_scale=bn_in.scale, in_shift=bn_in.shift,
-                                     out_scale=None if bn_out is None else bn_out.scale,
-                                     out_shift=None if bn_out is None else bn_out.shift, residual=res)
 
     def forward_reference(self, x):
         """The same layer from the transform matrices with float64 einsums (for tests)."""
@@ -154,19 +128,19 @@ class ResNet18Var(torch.nn.Module):
     def _block(self, blk, l, main, ref, main_bias=None):
         """main [+ main_bias] + bn2c(conv(bn2b(conv(bn2a(l))))) with the Winograd layers as `ref` says.  main_bias is a
         per-channel constant still owed to `main` (the folded BatchNorm shift of the 1x1 shortcut): on the fused path it
-        rides on the last kernel's output shift instead of costing a pass over `main`."""
+        rides on the last kernel's output shift instead of costing a pass over `main`.  main=None: relu(l)."""
         if not ref and self.math == "tf32" and self.fused:
-            wa, wb = blk["w2a"], blk["w2b"]
-            t = (wa.forward_onekernel(l, blk["bn2a"]) if wa.onekernel_pays(l, self.layout)
-                 else wa.forward_fused(l, blk["bn2a"], layout=self.layout))
-            bn_out = blk["bn2c"]
+            # both layers, BatchNorms, ReLUs and the shortcut in one call; a shortcut of None is relu(l)
+            wa, wb, (s_out, t_out) = blk["w2a"], blk["w2b"], blk["bn2c"].pair()
             if main_bias is not None:
-                if getattr(blk, "_out_folded", None) is None or blk._out_folded.shift.device != bn_out.shift.device:
-                    blk._out_folded = _Affine(bn_out.scale, (bn_out.shift + main_bias).detach())
-                bn_out = blk._out_folded
-            if wb.onekernel_pays(t, self.layout):
-                return wb.forward_onekernel(t, blk["bn2b"], bn_out=bn_out, residual=main)
-            return wb.forward_fused(t, blk["bn2b"], bn_out=bn_out, residual=main, layout=self.layout)
+                if getattr(blk, "_out_shift_folded", None) is None or blk._out_shift_folded.device != t_out.device:
+                    blk._out_shift_folded = (t_out + main_bias).detach()
+                t_out = blk._out_shift_folded
+            y = wg2x2.residual_block(wa._to_kernel(l, self.layout), None if main is None else wa._to_kernel(main, self.layout), wa.prepared(),
+                                     blk["bn2a"].pair(), wb.prepared(), blk["bn2b"].pair(), (s_out, t_out), wa.cout, layout=self.layout)
+            return wa._from_kernel(y, self.layout)
+        if main is None:
+            main = torch.relu(l)
         if main_bias is not None:
             main = main + main_bias.view(1, -1, 1, 1)
         conv = (lambda m, t: m.forward_reference(t)) if ref else (lambda m, t: m(t, self.math, self.layout))
@@ -219,14 +193,17 @@ class ResNet18Var(torch.nn.Module):
                     blk_a._short_folded = (blk_a.short * blk_a["bn1"].scale.view(-1, 1, 1, 1)).detach()
                 main = F.conv2d(main, blk_a._short_folded)      # its shift is added by the block's last kernel
             l = self._block(blk_a, l, main, reference, main_bias=None if (reference or not self.fused) else blk_a["bn1"].shift)
-            l = self._block(blk_b, l, torch.relu(l), reference)
+            l = self._block(blk_b, l, None, reference)
             l_relu = None
             if s < 2 or (s == 2 and self.stage5_pool):
                 if own_pool:
                     l, l_relu = wg2x2.maxpool3x3s2_same(l.contiguous(), with_relu=True)
                 else:
                     l = _same_pool(l)
-        l = torch.relu(l).mean(dim=(2, 3))
+        if own_pool and l.is_contiguous():
+            l = wg2x2.relu_mean(l)
+        else:
+            l = torch.relu(l).mean(dim=(2, 3))
         return F.linear(l, self.fc_w, self.fc_b)
 
     def winograd_layers(self):

@@ -112,6 +112,18 @@ def layer_fwd_fused(x, prepared, K, relu=True, out=None, out_scale=None, out_shi
     return _native.layer_fwd_fused(x, prepared, K, relu, out, out_scale, out_shift, residual, in_scale, in_shift)
 
 
+def residual_block(x, shortcut, prepared_a, bn_a, prepared_b, bn_b, bn_out, K, layout="NCHW"):
+    """shortcut + bn_out(layer_b(bn_b(layer_a(bn_a(x))))), both layers with prepared weights and K output channels; bn_*: (scale,
+    shift) pairs.  The result is written over `shortcut`; with None the shortcut is relu(x)."""
+    return _native.residual_block(x, shortcut, K, prepared_a, bn_a[0], bn_a[1], prepared_b, bn_b[0], bn_b[1], bn_out[0], bn_out[1],
+                                  _LAYOUTS[layout])
+
+
+def relu_mean(x):
+    """x (B,C,H,W) -> (B,C): the mean of relu(x) over the pixels."""
+    return _native.relu_mean(x)
+
+
 def maxpool3x3s2_same(x, with_relu=False, relu_scale=None, relu_shift=None):
     """3x3 / stride 2 max-pooling with TensorFlow's SAME padding of a (B,C,H,W) tensor into NCHW outputs; with_relu=True
     returns (pooled, relu(relu_scale[c] * pooled + relu_shift[c])) from the same pass (scale 1, shift 0 when not given).
