@@ -88,6 +88,9 @@ int wg2x2_conv_fwd(const float *V, const float *Wt, float *Y, int B, int nH, int
                    void *stream);
 size_t wg2x2_conv_fwd_workspace_bytes(int B, int nH, int nW, int C, int K, int math);
 
+/* out = Wt * mask, element by element ((16,C,K) floats each): W of a pruned layer (ResNet-18-var/winograd_conv.py:21-26). */
+int wg2x2_weights_mask(const float *Wt, const float *mask, float *out, int C, int K, void *stream);
+
 /*
  * Weights prepared once for the tensor-core path, for callers whose weights do not change
  * between calls (inference, or between optimiser steps): W (16,C,K) is repacked to (16,K,C),

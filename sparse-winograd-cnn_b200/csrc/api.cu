@@ -16,6 +16,7 @@ int conv_dw_splits(long long P, int C, int K);
 size_t conv_dw_scratch_bytes(long long P, int C, int K);
 int conv_dw_ffma(const float *V, const float *dY, const float *mask, float *dW, int B, int H, int W, int C, int K, int layout,
                  float *scratch, int splits, cudaStream_t st);
+int weights_mask(const float *Wt, const float *mask, float *out, int C, int K, cudaStream_t st);
 // conv_tc.cu
 size_t conv_fwd_tc_workspace_bytes(int B, int nH, int nW, int C, int K);
 int conv_fwd_tc(const float *V, const float *Wt, float *Y, int B, int nH, int nW, int C, int K, int outH, int outW, int layout,
@@ -108,6 +109,12 @@ int wg2x2_conv_fwd(const float *V, const float *Wt, float *Y, int B, int nH, int
 size_t wg2x2_prepared_weights_bytes(int C, int K)
 {
     return (C > 0 && K > 0) ? prepared_weights_bytes(C, K) : 0;
+}
+
+int wg2x2_weights_mask(const float *Wt, const float *mask, float *out, int C, int K, void *stream)
+{
+    if (!Wt || !mask || !out || C <= 0 || K <= 0) return WG2X2_ERR_BAD_ARG;
+    return weights_mask(Wt, mask, out, C, K, (cudaStream_t)stream);
 }
 
 int wg2x2_weights_prepare(const float *Wt, int C, int K, void *prepared, size_t prepared_bytes, void *stream)

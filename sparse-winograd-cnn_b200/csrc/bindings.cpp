@@ -258,17 +258,17 @@ struct ImTransBackward : public torch::autograd::Node {
 };
 
 struct ConvBackward : public torch::autograd::Node {
-    SavedVariable I_, W_;
+    SavedVariable I_, W_, mask_;      // W with the mask applied
     int layout = 0, math = 0;
     std::string name() const override { return "Winograd2x2ConvBackward"; }
-    void release_variables() override { I_.reset_data(); W_.reset_data(); }
+    void release_variables() override { I_.reset_data(); W_.reset_data(); mask_.reset_data(); }
     variable_list apply(variable_list &&grads) override
     {
         if (!grads[0].defined()) return {Tensor(), Tensor()};
         const bool dI = task_should_compute_output(0), dW = task_should_compute_output(1);
         const Tensor g = grads[0].contiguous();
         require(g, "dY");
-        auto r = conv_bwd(I_.unpack(), W_.unpack(), g, Tensor(), layout, false, math, dI, dW);
+        auto r = conv_bwd(I_.unpack(), W_.unpack(), g, mask_.unpack(), layout, false, math, dI, dW);
         return {r.first, r.second};
     }
 };
@@ -296,17 +296,29 @@ Tensor imtrans_op(const Tensor &in, bool relu, int layout)
     return V;
 }
 
-Tensor conv_op(const Tensor &in, const Tensor &win, int out_h, int out_w, int layout, int math)
+// With a mask the weights are win * mask.  The product is made here, not by the caller, so that neither it nor its gradient (the
+// mask on dW, which the dW kernels apply anyway) is a node and a kernel of its own: 12 + 10 us of host time in a training step.
+Tensor conv_op(const Tensor &in, const Tensor &win, const Tensor &mask, int out_h, int out_w, int layout, int math)
 {
-    const Tensor I = in.contiguous(), Wt = win.contiguous();
+    const Tensor I = in.contiguous();
+    Tensor Wt = win.contiguous();
     require(I, "V");
     require(Wt, "Wt");
+    const Tensor W0 = Wt;
+    if (mask.defined()) {
+        if (Wt.dim() != 3 || Wt.size(0) != 16 || mask.sizes() != Wt.sizes() || mask.device() != Wt.device())
+            value_error("mask must have the weights' shape (16, C, K) and be on their device");
+        OnDevice on(Wt);
+        Wt = new_float(W0.sizes(), W0);
+        check(wg2x2_weights_mask(cptr(W0), cptr(mask), ptr(Wt), (int)W0.size(1), (int)W0.size(2), on.stream), "wg2x2_weights_mask");
+    }
     Tensor Y = conv_fwd(I, Wt, out_h, out_w, layout, math, Tensor(), Tensor());
-    if (torch::autograd::compute_requires_grad(I, Wt)) {
-        auto n = new_node<ConvBackward>(torch::autograd::collect_next_edges(I, Wt));
+    if (torch::autograd::compute_requires_grad(I, W0)) {
+        auto n = new_node<ConvBackward>(torch::autograd::collect_next_edges(I, W0));
         n->layout = layout; n->math = math;
         n->I_ = SavedVariable(I, false);
         n->W_ = SavedVariable(Wt, false);
+        if (mask.defined()) n->mask_ = SavedVariable(mask, false);
         torch::autograd::set_history(Y, n);
     }
     return Y;
@@ -684,17 +696,18 @@ PyObject *py_imtrans_op(WG_ARGS)
     END_HANDLE_TH_ERRORS
 }
 
-// I, W, out_h, out_w, layout, math: differentiable
+// I, W, out_h, out_w, layout, math, mask: differentiable in I and W
 PyObject *py_conv_op(WG_ARGS)
 {
     HANDLE_TH_ERRORS
-    want(n, 6);
+    want(n, 7);
     if (!THPVariable_Check(a[0])) not_a_tensor("V");
     if (!THPVariable_Check(a[1])) not_a_tensor("Wt");
     const Tensor I = THPVariable_Unpack(a[0]), Wt = THPVariable_Unpack(a[1]);
     const int oh = arg_int_or(a[2], -1), ow = arg_int_or(a[3], -1), layout = arg_int(a[4]), math = arg_int(a[5]);
     Tensor Y;
-    { WG_NOGIL; Y = conv_op(I, Wt, oh, ow, layout, math); }
+    const Tensor mask = arg(a[6], "mask", true);
+    { WG_NOGIL; Y = conv_op(I, Wt, mask, oh, ow, layout, math); }
     return THPVariable_Wrap(Y);
     END_HANDLE_TH_ERRORS
 }

@@ -641,6 +641,30 @@ __global__ void __launch_bounds__(256) conv_dw_reduce_kernel(const float *__rest
     }
 }
 
+// W with the pruning mask applied, four values at a time where both are on 16-byte boundaries
+template <int VEC>
+__global__ void __launch_bounds__(256) mask_weights_kernel(const float *__restrict__ Wt, const float *__restrict__ mask, float *__restrict__ out,
+                                                             long long n)
+{
+    after_previous_kernel(Wt, mask, out);
+    for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * VEC; i < n; i += (long long)gridDim.x * blockDim.x * VEC) {
+        if (VEC == 4) {
+            const float4 w = __ldg(reinterpret_cast<const float4 *>(Wt + i)), m = __ldg(reinterpret_cast<const float4 *>(mask + i));
+            *reinterpret_cast<float4 *>(out + i) = make_float4(w.x * m.x, w.y * m.y, w.z * m.z, w.w * m.w);
+        } else {
+            out[i] = __ldg(Wt + i) * __ldg(mask + i);
+        }
+    }
+}
+
+int weights_mask(const float *Wt, const float *mask, float *out, int C, int K, cudaStream_t st)
+{
+    const long long n = 16LL * C * K;         // a multiple of 4
+    const bool vec = ((reinterpret_cast<uintptr_t>(Wt) | reinterpret_cast<uintptr_t>(mask) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
+    const int blocks = (int)min((long long)kNumSMs * 16, cdivll(n, vec ? 1024 : 256));
+    return launch(vec ? mask_weights_kernel<4> : mask_weights_kernel<1>, dim3((unsigned)blocks), 256, 0, st, Wt, mask, out, n);
+}
+
 void dw_reduce_launch(const float *partial, const float *mask, float *dW, long long n, int splits, cudaStream_t st)
 {
     const int blocks = (int)min((long long)kNumSMs * 8, cdivll(n, 256));

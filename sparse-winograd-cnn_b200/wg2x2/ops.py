@@ -47,9 +47,9 @@ def conv_fwd(V, Wt, out_h=None, out_w=None, layout="NHWC", math="fp32", out=None
     return _native.conv_fwd(V, Wt, out_h, out_w, _LAYOUTS[layout], _MATHS[math], out, workspace)
 
 
-def conv_op(V, Wt, out_h=None, out_w=None, layout="NHWC", math="fp32"):
-    """conv_fwd for autograd: differentiable in V and Wt (any strides)."""
-    return _native.conv_op(V, Wt, out_h, out_w, _LAYOUTS[layout], _MATHS[math])
+def conv_op(V, Wt, out_h=None, out_w=None, layout="NHWC", math="fp32", mask=None):
+    """conv_fwd for autograd: differentiable in V and Wt (any strides).  mask (16,C,K), constant: the weights are Wt * mask."""
+    return _native.conv_op(V, Wt, out_h, out_w, _LAYOUTS[layout], _MATHS[math], mask)
 
 
 def prepare_weights(Wt):

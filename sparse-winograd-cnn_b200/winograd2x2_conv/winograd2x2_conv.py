@@ -10,9 +10,10 @@ winograd2x2_conv.py:13-36): same function names and tensor shapes, on torch CUDA
 from wg2x2 import ops as _ops
 
 
-def winograd2x2_conv(I, W, out_hw=None, data_format="NHWC", math="fp32"):
+def winograd2x2_conv(I, W, out_hw=None, data_format="NHWC", math="fp32", mask=None):
+    """mask: a constant pruning mask of W's shape; the product is that of I and W * mask."""
     oh, ow = out_hw if out_hw is not None else (None, None)
-    return _ops.conv_op(I, W, oh, ow, data_format, math)
+    return _ops.conv_op(I, W, oh, ow, data_format, math, mask)
 
 
 def winograd2x2_conv_grad(i1, i2, grad, data_format="NHWC", math="fp32"):

@@ -36,8 +36,10 @@ class WinogradConvLayer(torch.nn.Module):
             self.mask = None
 
     def forward(self, x, out_hw=None, data_format="NHWC", math="fp32"):
-        W = self.W if self.mask is None else self.W * self.mask
-        return winograd2x2_conv(x, W, out_hw=out_hw, data_format=data_format, math=math)
+        W, mask = self.W, self.mask
+        if mask is not None and (mask.requires_grad or mask.shape != W.shape or mask.dtype != W.dtype or not mask.is_contiguous()):
+            W, mask = W * mask, None          # a mask of its own kind: as torch multiplies it
+        return winograd2x2_conv(x, W, out_hw=out_hw, data_format=data_format, math=math, mask=mask)
 
 
 _layers = {}

@@ -59,3 +59,24 @@ def test_few_tiles(oracle, shape, layout):
               wg2x2.layer_fwd_prepared(img(X), prepared, K, relu=True, layout=layout)):
         assert oracle.max_rel(back(Y), want) <= 5e-3
     assert wg2x2.last_device_status()[0] == 0
+
+
+# the pruning mask folded into the product op against W * mask as torch's autograd has it
+@pytest.mark.parametrize("math", ["fp32", "tf32"])
+@pytest.mark.parametrize("layout", ["NHWC", "NCHW"])
+@pytest.mark.parametrize("C,K", [(4, 4), (36, 20), (96, 72)])
+def test_masked_layer(C, K, layout, math):
+    import torch
+    import wg2x2
+    from winograd_conv import WinogradConvLayer
+    g = torch.Generator(device="cuda").manual_seed(C + K)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    V, W = rnd(16, 2, 4, 5, C).requires_grad_(True), rnd(16, C, K)
+    mask = (torch.rand((16, C, K), generator=g, device="cuda") < 0.4).float()
+    dY = rnd(2, 7, 10, K) if layout == "NHWC" else rnd(2, K, 7, 10)
+    layer = WinogradConvLayer(C, K, mask=mask, W_init=lambda s: W, device="cuda")
+    y = layer(V, out_hw=(7, 10), data_format=layout, math=math)
+    y2 = wg2x2.ops.conv_op(V, layer.W * layer.mask, 7, 10, layout, math)
+    assert torch.equal(y, y2)
+    for a, b in zip(torch.autograd.grad(y, (V, layer.W), dY), torch.autograd.grad(y2, (V, layer.W), dY)):
+        assert torch.equal(a, b)
