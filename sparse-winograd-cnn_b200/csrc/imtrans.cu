@@ -251,85 +251,122 @@ __global__ void __launch_bounds__(256) imtrans_fwd_nchw_row_kernel(const float *
     }
 }
 
-// The same with four channels per lane: every plane store is 16 bytes per lane, 512 bytes per warp with LC = 32
-// lanes along the channels (128 per CTA), 256 bytes with LC = 16 (64 per CTA, the two halves of a warp on two tiles
-// at once).  Where the band is the whole image the CTA's channels are one contiguous run of X and are staged as such.
-template <int LC, bool AFFINE>
-__global__ void __launch_bounds__(256, 3) imtrans_fwd_nchw_vec_kernel(const float *__restrict__ X, float *__restrict__ V,
-                                                                        int B, int H, int W, int C, int nH, int nW, int relu,
-                                                                        int R, int nbands, int pitch,
-                                                                        const float *__restrict__ scale, const float *__restrict__ shift)
+// ------------------------------------------------------------------------------------------
+// Forward, NCHW, short rows and enough tiles to fill the GPU: two channels per lane (64 per CTA), image kept in shared memory as
+// [pixel][channel] with its zero padding, so that a warp reads it without predicates, and walks consecutive tiles of a row, of
+// which it loads only the two new columns and keeps the row-transformed two old ones.  Per tile of 64 channels 8 eight-byte
+// loads, 16 + 32 additions, 16 stores of 256 bytes off uniform plane addresses, against 32 loads, 128 additions and predicates
+// and 32 stores with one channel per lane.
+// ------------------------------------------------------------------------------------------
+constexpr int kPairCB = 64, kPairPitch = kPairCB + 2;   // channels per CTA; floats of a pixel in shared memory
+
+// Stage rows gy0 .. gy0 + rows - 1 of 64 channels: slot (row, x) receives pixel (gy0 + row, x - 1), PW slots a row, zeros outside
+// the image.  Asynchronous copies, all in flight at once: staged through registers, the few loads that a warp had open at a
+// time were what the kernel waited for (34 against 29 us at 128 x 256 x 14 x 14).  inv = ceil(2^20 / PW).
+__device__ __forceinline__ void stage_pairs(const float *__restrict__ X, float *S, int b, int c0, int C, int H, int W, int gy0, int rows, int PW,
+                                            unsigned inv)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nch = min(kPairCB, C - c0) - warp;          // channels warp, warp + 8, ... of the block: (nch + 7) / 8 of them exist
+    const long long HW8 = 8LL * H * W;
+    const float *plane = X + ((long long)b * C + c0 + warp) * H * W;
+    for (int i = lane; i < rows * PW; i += 32) {
+        const int r = (int)(((unsigned)i * inv) >> 20), x = i - r * PW - 1, y = gy0 + r;
+        const bool in = y >= 0 && y < H && x >= 0 && x < W;
+        const float *src = plane + (in ? (long long)y * W + x : 0);
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(S + i * kPairPitch + warp);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const bool ok = in && 8 * q < nch;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + 32u * q), "l"(ok ? src + q * HW8 : X), "r"(ok ? 4 : 0) : "memory");
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+template <bool AFFINE, bool RELU>
+__global__ void __launch_bounds__(256, 4) imtrans_fwd_nchw_pair_kernel(const float *__restrict__ X, float *__restrict__ V, int H, int W, int C,
+                                                                         int nH, int nW, int R, int nbands, unsigned inv, unsigned plane_bytes,
+                                                                         const float *__restrict__ scale, const float *__restrict__ shift)
 {
     after_previous_kernel(X, V, scale, shift);
-    constexpr int CB = 4 * LC, QW = 32 / LC;
-    extern __shared__ float S[];   // [CB channels][pitch]
-    const int band = blockIdx.x % nbands;
-    const int b = blockIdx.x / nbands;
-    const int c0 = blockIdx.y * CB;
+    extern __shared__ __align__(16) float S[];
+    const int band = blockIdx.x % nbands, b = blockIdx.x / nbands, c0 = blockIdx.y * kPairCB;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int lc = lane % LC, lq = lane / LC;
-    const int th0 = band * R;
-    const int rows_tile = min(R, nH - th0);
-    const int gy0 = 2 * th0 - 1;                                  // first input row of the band (may be -1)
-    const int lo = max(gy0, 0), hi = min(gy0 + 2 * rows_tile + 2, H);
-    const int nfill = (hi - lo) * W;
-    const int nch = min(CB, C - c0);
-    if (nfill == H * W) {
-        const float *src = X + ((long long)b * C + c0) * nfill;
-        float *dst = S + (lo - gy0) * W;
-        for (int k = threadIdx.x; k < nch * nfill; k += 256) {
-            const int cc = k / nfill;
-            dst[((cc & 3) * LC + (cc >> 2)) * pitch + (k - cc * nfill)] = __ldg(src + k);
-        }
-    } else {
-        for (int cc = warp; cc < nch; cc += 8) {
-            const float *src = X + (((long long)b * C + c0 + cc) * H + lo) * W;
-            float *dst = S + ((cc & 3) * LC + (cc >> 2)) * pitch + (lo - gy0) * W;
-            for (int i = lane; i < nfill; i += 32) dst[i] = __ldg(src + i);
-        }
-    }
+    const int th0 = band * R, rows_tile = min(R, nH - th0), PW = 2 * nW + 2, gy0 = 2 * th0 - 1;
+    stage_pairs(X, S, b, c0, C, H, W, gy0, 2 * rows_tile + 2, PW, inv);
     __syncthreads();
-    if (c0 + 4 * lc >= C) return;
-
-    const long long plane = (long long)B * nH * nW * C;
-    // channel 4 * lc + ch sits in row ch * LC + lc: for a given ch the lanes read rows one odd pitch apart (no bank conflicts)
-    const float *Sc = S + lc * pitch;
-    float4 sc = make_float4(1.f, 1.f, 1.f, 1.f), sh = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (AFFINE) {
-        sc = __ldg(reinterpret_cast<const float4 *>(scale + c0) + lc);
-        sh = __ldg(reinterpret_cast<const float4 *>(shift + c0) + lc);
-    }
-    const float scv[4] = {sc.x, sc.y, sc.z, sc.w}, shv[4] = {sh.x, sh.y, sh.z, sh.w};
-#pragma unroll 1
-    for (int q = warp * QW + lq; q < rows_tile * nW; q += 8 * QW) {
-        const int tr = q / nW, tw = q - tr * nW;
-        float v[4][4][4];          // [channel][i][j]
+    if (c0 + 2 * lane >= C) return;
+    // the warp's share of the band's tiles, in row order
+    const int ntiles = rows_tile * nW, each = cdiv(ntiles, 8);
+    const int q0 = warp * each, q1 = min(q0 + each, ntiles);
+    if (q0 >= q1) return;
+    int tr = q0 / nW, tw = q0 - tr * nW;
+    unsigned off = (unsigned)((((long long)b * nH + th0) * nW + q0) * C + c0 + 2 * lane) * 4u;
+    const float2 *P = reinterpret_cast<const float2 *>(S + (2 * tr * PW + 2 * tw) * kPairPitch) + lane;
+    char *const Vb = reinterpret_cast<char *>(V);
+    float2 sc = make_float2(1.f, 1.f), sh = make_float2(0.f, 0.f);
+    if (AFFINE) { sc = __ldg(reinterpret_cast<const float2 *>(scale + c0) + lane); sh = __ldg(reinterpret_cast<const float2 *>(shift + c0) + lane); }
+    float2 r[4][4];
+    auto column = [&](int x) {            // column x of the window, transformed along the rows
+        float2 d[4];
 #pragma unroll
-        for (int ch = 0; ch < 4; ++ch) {
-            float d[4][4];
-#pragma unroll
-            for (int y = 0; y < 4; ++y) {
-                const int gy = gy0 + 2 * tr + y;
-                const bool row_ok = (gy >= 0) && (gy < H);
-#pragma unroll
-                for (int x = 0; x < 4; ++x) {
-                    const int gx = 2 * tw - 1 + x;
-                    const bool in = row_ok && gx >= 0 && gx < W;
-                    const float raw = in ? Sc[ch * LC * pitch + (2 * tr + y) * W + gx] : 0.f;
-                    d[y][x] = in ? (AFFINE ? fmaf(raw, scv[ch], shv[ch]) : raw) : 0.f;
-                }
-            }
-            bt_d_b(d, v[ch]);
+        for (int y = 0; y < 4; ++y) {
+            d[y] = P[(y * PW + x) * (kPairPitch / 2)];
+            if (AFFINE && gy0 + 2 * tr + y >= 0 && gy0 + 2 * tr + y < H && 2 * tw + x >= 1 && 2 * tw + x <= W)
+                d[y] = make_float2(fmaf(d[y].x, sc.x, sh.x), fmaf(d[y].y, sc.y, sh.y));
         }
-        const long long off = (((long long)b * nH + th0 + tr) * nW + tw) * C + c0 + 4 * lc;
-        const float lo_v = relu ? 0.f : -__int_as_float(0x7f800000);
+        r[0][x] = make_float2(d[0].x - d[2].x, d[0].y - d[2].y);
+        r[1][x] = make_float2(d[1].x + d[2].x, d[1].y + d[2].y);
+        r[2][x] = make_float2(d[2].x - d[1].x, d[2].y - d[1].y);
+        r[3][x] = make_float2(d[1].x - d[3].x, d[1].y - d[3].y);
+    };
+    column(0);
+    column(1);
+#pragma unroll 1
+    for (int q = q0;;) {
+        column(2);
+        column(3);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                *reinterpret_cast<float4 *>(V + (long long)(4 * i + j) * plane + off) =
-                    make_float4(fmaxf(v[0][i][j], lo_v), fmaxf(v[1][i][j], lo_v), fmaxf(v[2][i][j], lo_v), fmaxf(v[3][i][j], lo_v));
+            for (int j = 0; j < 4; ++j) {
+                const int a = j == 0 ? 0 : j == 2 ? 2 : 1, c = j == 2 ? 1 : j == 3 ? 3 : 2;      // r0 - r2, r1 + r2, r2 - r1, r1 - r3
+                float2 v = j == 1 ? make_float2(r[i][a].x + r[i][c].x, r[i][a].y + r[i][c].y) : make_float2(r[i][a].x - r[i][c].x, r[i][a].y - r[i][c].y);
+                if (RELU) v = make_float2(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f));
+                *reinterpret_cast<float2 *>(Vb + (size_t)plane_bytes * (4 * i + j) + off) = v;
+            }
+        if (++q >= q1) break;
+        off += (unsigned)C * 4u;
+        P += kPairPitch;                  // two slots, in units of two floats
+        if (++tw == nW) {                 // a new row: over the last two slots of this one and one more row
+            tw = 0;
+            ++tr;
+            P += (PW + 2) * (kPairPitch / 2);
+            column(0);
+            column(1);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { r[i][0] = r[i][2]; r[i][1] = r[i][3]; }
+        }
     }
+}
+
+// The band height of that kernel: least work of the busiest SM (a tile is 146 issue slots, a staged pixel 10 per 64 channels, and
+// a CTA costs something of its own), shared memory for three CTAs per SM.  0: too few CTAs to fill the GPU.
+inline int pair_rows(int B, int C, int nH, int nW, int W)
+{
+    const long long per_band = (long long)B * cdiv(C, kPairCB);
+    int best = 0;
+    double t = 1e300;
+    for (int R = 1; R <= nH; ++R) {
+        if (R > 1 && (2 * R + 2) * (2 * nW + 2) * kPairPitch * 4 > 72 * 1024) break;
+        const long long ctas = per_band * cdiv(nH, R);
+        if (ctas < 2LL * kNumSMs) continue;
+        const double u = (double)cdivll(ctas, kNumSMs) * ((2.0 * R + 2) * W * 10 + (double)R * nW * 146 + 1500);
+        if (u < t) { t = u; best = R; }
+    }
+    return best ? cdiv(nH, cdiv(nH, best)) : 0;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -750,22 +787,19 @@ int imtrans_fwd(const float *X, float *V, int B, int H, int W, int C, int layout
         const long long gx = (long long)B * nH * cdiv(nW, kTSEG);
         if (gx > 0x7fffffffLL || cdiv(C, kCCH) > 65535) return WG2X2_ERR_UNSUPPORTED;
         dim3 grid((unsigned)gx, cdiv(C, kCCH));
-        // Four channels per lane, 128 per CTA, where the whole image is one small band (7 x 7: 39.8 against 43.5 us on
-        // 256 x 512 channels) and the CTAs still fill the GPU.  With several bands per image, or 64 channels per CTA
-        // and a 14 x 14 image, the one-channel-per-lane kernel below measured faster (33 against 39-52 us).
-        const int rows_all = 2 * nH + 2;
-        const bool wide = (C % 4 == 0) && C >= 128 && aligned16(V) && (!scale || (aligned16(scale) && aligned16(shift))) &&
-                          rows_all * W <= 96 && (long long)B * cdiv(C, 128) >= 4LL * kNumSMs;
-        const bool vec = wide;
-        if (vec) {
-            const int cb = 128;
-            const int R = nH, nbands = 1;
-            const int pitch = ((2 * R + 2) * W) | 1;
-            const int smem = cb * pitch * (int)sizeof(float);
-            if ((long long)B * nbands > 0x7fffffffLL || cdiv(C, cb) > 65535) return WG2X2_ERR_UNSUPPORTED;
-            const dim3 gb((unsigned)(B * nbands), cdiv(C, cb));
-            launch(scale ? imtrans_fwd_nchw_vec_kernel<32, true> : imtrans_fwd_nchw_vec_kernel<32, false>, gb, 256, smem, st, X, V, B, H, W, C,
-                   nH, nW, relu, R, nbands, pitch, scale, shift);
+        // Two channels per lane where a row of tiles is short (the one-channel kernel's predicates and divisions weigh more there:
+        // 256 x 512 x 7 x 7 39 -> 34 us, 256 x 256 x 14 x 14 59 -> 53, 32 x 256 x 28 x 28 32 -> 31, but 54 -> 58 at 56 x 56),
+        // blocks of 64 channels are full, the bands fill the GPU, and a plane is within 32-bit reach.
+        const bool pair_ok = C % kPairCB == 0 && W <= 28 && ((reinterpret_cast<uintptr_t>(V) | reinterpret_cast<uintptr_t>(scale) |
+                             reinterpret_cast<uintptr_t>(shift)) & 7u) == 0 && (long long)B * nH * nW * C < (1LL << 30) && C / kPairCB <= 65535;
+        const int R = pair_ok ? pair_rows(B, C, nH, nW, W) : 0;
+        if (R) {
+            const int nbands = cdiv(nH, R), smem = (2 * R + 2) * (2 * nW + 2) * kPairPitch * (int)sizeof(float);
+            if ((long long)B * nbands > 0x7fffffffLL) return WG2X2_ERR_UNSUPPORTED;
+            auto *kernel = scale ? (relu ? imtrans_fwd_nchw_pair_kernel<true, true> : imtrans_fwd_nchw_pair_kernel<true, false>)
+                                 : (relu ? imtrans_fwd_nchw_pair_kernel<false, true> : imtrans_fwd_nchw_pair_kernel<false, false>);
+            launch(kernel, dim3((unsigned)(B * nbands), C / kPairCB), 256, smem, st, X, V, H, W, C, nH, nW, R, nbands,
+                   (unsigned)cdiv(1 << 20, 2 * nW + 2), (unsigned)((long long)B * nH * nW * C * 4), scale, shift);
         } else if (W <= 128) {
             const BandCut cut = cut_bands(nH, nW, (long long)B * cdiv(C, 32), (kBandFloats / W - 2) / 2);
             const int pitch = ((2 * cut.R + 2) * (cut.nsegs == 1 ? W : 2 * cut.S + 2)) | 1;
