@@ -74,6 +74,15 @@ int wg2x2_imtrans_bwd(const float *dV, const float *V_relu, float *dX, int B, in
                       int layout, void *stream);
 
 /*
+ * The transform with ReLU for a training step, and its gradient with the mask as bits: the forward call also writes 16 bits per
+ * tile and channel ([B*nH*nW][C] 16-bit words, bit t = position t of V is positive; wg2x2_relu_bits_bytes, 16-byte aligned),
+ * which the gradient reads in place of V (1/32 of its bytes).
+ */
+int wg2x2_imtrans_fwd_relu_bits(const float *X, float *V, void *bits, int B, int H, int W, int C, int layout, void *stream);
+int wg2x2_imtrans_bwd_relu_bits(const float *dV, const void *bits, float *dX, int B, int H, int W, int C, int layout, void *stream);
+size_t wg2x2_relu_bits_bytes(int B, int H, int W, int C);
+
+/*
  * Winograd-domain product and output transform: Y = A^T (V_t . W_t) A, cropped to
  * out_h x out_w (2nH-1 <= out_h <= 2nH, same for w).
  * Replaces Winograd2x2ConvComputeLauncher (winograd2x2_conv_op.cc:31,

@@ -4,9 +4,9 @@
 
 namespace wg {
 // imtrans.cu
-int imtrans_fwd(const float *X, float *V, int B, int H, int W, int C, int layout, int relu, const float *scale, const float *shift,
+int imtrans_fwd(const float *X, float *V, void *signs, int B, int H, int W, int C, int layout, int relu, const float *scale, const float *shift,
                 cudaStream_t st);
-int imtrans_bwd(const float *dV, const float *Vm, float *dX, int B, int H, int W, int C, int layout, cudaStream_t st);
+int imtrans_bwd(const float *dV, const void *Vm, int mask_bits, float *dX, int B, int H, int W, int C, int layout, cudaStream_t st);
 // conv_ffma.cu
 int conv_fwd_ffma(const float *V, const float *Wt, float *Y, int B, int nH, int nW, int C, int K, int outH, int outW,
                   int layout, cudaStream_t st);
@@ -75,19 +75,36 @@ int wg2x2_abi_version(void) { return 1; }
 
 int wg2x2_imtrans_fwd(const float *X, float *V, int B, int H, int W, int C, int layout, int relu, void *stream)
 {
-    return imtrans_fwd(X, V, B, H, W, C, layout, relu, nullptr, nullptr, (cudaStream_t)stream);
+    return imtrans_fwd(X, V, nullptr, B, H, W, C, layout, relu, nullptr, nullptr, (cudaStream_t)stream);
 }
 
 int wg2x2_imtrans_fwd_affine(const float *X, const float *in_scale, const float *in_shift, float *V, int B, int H, int W, int C,
                              int layout, int relu, void *stream)
 {
     if (!in_scale || !in_shift) return WG2X2_ERR_BAD_ARG;
-    return imtrans_fwd(X, V, B, H, W, C, layout, relu, in_scale, in_shift, (cudaStream_t)stream);
+    return imtrans_fwd(X, V, nullptr, B, H, W, C, layout, relu, in_scale, in_shift, (cudaStream_t)stream);
 }
 
 int wg2x2_imtrans_bwd(const float *dV, const float *V_relu, float *dX, int B, int H, int W, int C, int layout, void *stream)
 {
-    return imtrans_bwd(dV, V_relu, dX, B, H, W, C, layout, (cudaStream_t)stream);
+    return imtrans_bwd(dV, V_relu, 0, dX, B, H, W, C, layout, (cudaStream_t)stream);
+}
+
+size_t wg2x2_relu_bits_bytes(int B, int H, int W, int C)
+{
+    return B > 0 && H > 0 && W > 0 && C > 0 ? sizeof(unsigned short) * (size_t)B * ((H + 1) / 2) * ((W + 1) / 2) * C : 0;
+}
+
+int wg2x2_imtrans_fwd_relu_bits(const float *X, float *V, void *bits, int B, int H, int W, int C, int layout, void *stream)
+{
+    if (!bits) return WG2X2_ERR_BAD_ARG;
+    return imtrans_fwd(X, V, bits, B, H, W, C, layout, 1, nullptr, nullptr, (cudaStream_t)stream);
+}
+
+int wg2x2_imtrans_bwd_relu_bits(const float *dV, const void *bits, float *dX, int B, int H, int W, int C, int layout, void *stream)
+{
+    if (!bits) return WG2X2_ERR_BAD_ARG;
+    return imtrans_bwd(dV, bits, 1, dX, B, H, W, C, layout, (cudaStream_t)stream);
 }
 
 size_t wg2x2_conv_fwd_workspace_bytes(int B, int nH, int nW, int C, int K, int math)
@@ -276,7 +293,7 @@ int wg2x2_layer_fwd_prepared_ex(const float *X, const float *in_scale, const flo
         return layer_fwd_fused(X, prepared, Y, B, H, W, C, K, relu, in_scale, in_shift, out_scale, out_shift, residual, residual_relu, st);
     if (!V_scratch) return WG2X2_ERR_WORKSPACE;
     if ((out_scale == nullptr) != (out_shift == nullptr)) return WG2X2_ERR_BAD_ARG;
-    const int s = imtrans_fwd(X, V_scratch, B, H, W, C, layout, relu, in_scale, in_shift, st);
+    const int s = imtrans_fwd(X, V_scratch, nullptr, B, H, W, C, layout, relu, in_scale, in_shift, st);
     if (s != WG2X2_OK) return s;
     return products_fwd(V_scratch, prepared, Y, B, nH, nW, C, K, H, W, layout, out_scale, out_shift, residual, residual_relu, workspace,
                         workspace_bytes, st);

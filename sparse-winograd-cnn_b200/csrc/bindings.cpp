@@ -241,19 +241,24 @@ std::pair<Tensor, Tensor> conv_bwd(const Tensor &V, const Tensor &Wt, const Tens
 // winograd2x2_imTrans.py:29-33, winograd2x2_conv.py:32-36)
 // ---------------------------------------------------------------------------------------
 struct ImTransBackward : public torch::autograd::Node {
-    SavedVariable V_;          // post-ReLU output, kept only where the ReLU was applied
+    Tensor bits;               // where the output is positive, kept only where the ReLU was applied
     int64_t H = 0, W = 0;
     int layout = 0;
     bool relu = false;
     std::string name() const override { return "Winograd2x2ImTransBackward"; }
-    void release_variables() override { V_.reset_data(); }
+    void release_variables() override { bits.reset(); }
     variable_list apply(variable_list &&grads) override
     {
         if (!grads[0].defined()) return {Tensor()};
-        Tensor V = relu ? V_.unpack(shared_from_this()) : Tensor();
+        TORCH_CHECK(!relu || bits.defined(), torch::autograd::ERR_BACKWARD_TWICE);
         const Tensor g = grads[0].contiguous();
         require(g, "dV");
-        return {imtrans_bwd(g, H, W, V, layout)};
+        if (!relu) return {imtrans_bwd(g, H, W, Tensor(), layout)};
+        OnDevice on(g);
+        const int64_t B = g.size(1), C = g.size(4);
+        Tensor dX = new_float(img_shape(B, H, W, C, layout), g);
+        check(wg2x2_imtrans_bwd_relu_bits(cptr(g), bits.data_ptr(), ptr(dX), B, H, W, C, layout, on.stream), "wg2x2_imtrans_bwd_relu_bits");
+        return {dX};
     }
 };
 
@@ -285,13 +290,23 @@ Tensor imtrans_op(const Tensor &in, bool relu, int layout)
 {
     const Tensor I = in.contiguous();
     require(I, "x");
-    Tensor V = imtrans_fwd(I, relu, layout, Tensor(), Tensor(), Tensor());
-    if (torch::autograd::compute_requires_grad(I)) {
+    const bool grad = torch::autograd::compute_requires_grad(I);
+    Tensor V, bits;
+    if (grad && relu) {
+        const Img d = img_of(I, layout, "x");
+        OnDevice on(I);
+        V = new_float({16, d.B, (d.H + 1) / 2, (d.W + 1) / 2, d.C}, I);
+        bits = Tensor(at::detail::empty_cuda({d.B, (d.H + 1) / 2, (d.W + 1) / 2, d.C}, at::kShort, I.device(), std::nullopt));
+        check(wg2x2_imtrans_fwd_relu_bits(cptr(I), ptr(V), bits.data_ptr(), d.B, d.H, d.W, d.C, layout, on.stream), "wg2x2_imtrans_fwd_relu_bits");
+    } else {
+        V = imtrans_fwd(I, relu, layout, Tensor(), Tensor(), Tensor());
+    }
+    if (grad) {
         auto n = new_node<ImTransBackward>(torch::autograd::collect_next_edges(I));
         const Img d = img_of(I, layout, "x");
         n->H = d.H; n->W = d.W; n->layout = layout; n->relu = relu;
+        n->bits = bits;
         torch::autograd::set_history(V, n);
-        if (relu) n->V_ = SavedVariable(V, true);
     }
     return V;
 }

@@ -25,16 +25,41 @@ __device__ __forceinline__ void put_lanes(float *p, int, float v) { p[0] = v; }
 __device__ __forceinline__ float4 keep_where_pos(float4 g, float4 m) { return make_float4(m.x > 0.f ? g.x : 0.f, m.y > 0.f ? g.y : 0.f, m.z > 0.f ? g.z : 0.f, m.w > 0.f ? g.w : 0.f); }
 __device__ __forceinline__ float keep_where_pos(float g, float m) { return m > 0.f ? g : 0.f; }
 
+// The ReLU mask as bits: 16 per tile and channel, bit t set where position t of V is positive.  [P][C] of them, 1/32 of V, is what
+// the backward pass reads instead of V itself (64 x 64 x 56 x 56: 6.4 MB for 205).
+typedef unsigned short signs_t;
+__device__ __forceinline__ signs_t signs_of(const float (&v)[4][4])
+{
+    unsigned m = 0;
+#pragma unroll
+    for (int t = 0; t < 16; ++t) m |= v[t >> 2][t & 3] > 0.f ? 1u << t : 0u;
+    return (signs_t)m;
+}
+__device__ __forceinline__ void put_signs(signs_t *s, const float4 (&v)[4][4])
+{
+    unsigned m[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int t = 0; t < 16; ++t) {
+        const float4 x = v[t >> 2][t & 3];
+        m[0] |= x.x > 0.f ? 1u << t : 0u;
+        m[1] |= x.y > 0.f ? 1u << t : 0u;
+        m[2] |= x.z > 0.f ? 1u << t : 0u;
+        m[3] |= x.w > 0.f ? 1u << t : 0u;
+    }
+    *reinterpret_cast<uint2 *>(s) = make_uint2(m[0] | (m[1] << 16), m[2] | (m[3] << 16));
+}
+__device__ __forceinline__ void put_signs(signs_t *s, const float (&v)[4][4]) { *s = signs_of(v); }
+
 // ------------------------------------------------------------------------------------------
 // Forward, NHWC.  One thread = one tile x VEC channels; consecutive threads walk the channel
 // axis first, so each of the 16 plane stores of a warp is one contiguous run.
 // ------------------------------------------------------------------------------------------
-template <int VEC, bool AFFINE>
-__global__ void __launch_bounds__(256) imtrans_fwd_nhwc_kernel(const float *__restrict__ X, float *__restrict__ V,
+template <int VEC, bool AFFINE, bool SIGNS>
+__global__ void __launch_bounds__(256) imtrans_fwd_nhwc_kernel(const float *__restrict__ X, float *__restrict__ V, signs_t *__restrict__ signs,
                                                                  int B, int H, int W, int C, int nH, int nW, int relu,
                                                                  const float *__restrict__ scale, const float *__restrict__ shift)
 {
-    after_previous_kernel(X, V, scale, shift);
+    after_previous_kernel(X, V, signs, scale, shift);
     using T = typename Vec<VEC>::type;
     const int CV = C / VEC;
     const long long total = (long long)B * nH * nW * CV;
@@ -69,6 +94,7 @@ __global__ void __launch_bounds__(256) imtrans_fwd_nhwc_kernel(const float *__re
     T *Vv = reinterpret_cast<T *>(V);
     const long long plane = (long long)B * nH * nW * CV;
     const long long off = p * CV + cv;
+    if (SIGNS) put_signs(signs + off * VEC, v);
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -87,11 +113,11 @@ constexpr int kTSEG = 32;                      // tiles along W per CTA
 constexpr int kRowPitch = 2 * kTSEG + 2;       // 66 pixels feed 32 tiles
 constexpr int kChanPitch = 4 * kRowPitch + 1;  // odd, so 32 channels hit 32 different banks
 
-__global__ void __launch_bounds__(256) imtrans_fwd_nchw_kernel(const float *__restrict__ X, float *__restrict__ V,
+__global__ void __launch_bounds__(256) imtrans_fwd_nchw_kernel(const float *__restrict__ X, float *__restrict__ V, signs_t *__restrict__ signs,
                                                                  int B, int H, int W, int C, int nH, int nW, int relu,
                                                                  const float *__restrict__ scale, const float *__restrict__ shift)
 {
-    after_previous_kernel(X, V, scale, shift);
+    after_previous_kernel(X, V, signs, scale, shift);
     __shared__ float S[kCCH * kChanPitch];
     const int nseg = cdiv(nW, kTSEG);
     int bx = blockIdx.x;
@@ -130,6 +156,7 @@ __global__ void __launch_bounds__(256) imtrans_fwd_nchw_kernel(const float *__re
             for (int x = 0; x < 4; ++x) d[y][x] = S[c * kChanPitch + y * kRowPitch + 2 * twl + x];
         bt_d_b(d, v);
         const long long off = (((long long)b * nH + th) * nW + tw) * C + c0 + c;
+        if (signs) signs[off] = signs_of(v);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -149,13 +176,13 @@ __global__ void __launch_bounds__(256) imtrans_fwd_nchw_kernel(const float *__re
 // ------------------------------------------------------------------------------------------
 constexpr int kBandFloats = 384;   // at most this many input floats per channel in shared memory
 
-template <bool AFFINE>
-__global__ void __launch_bounds__(256) imtrans_fwd_nchw_band_kernel(const float *__restrict__ X, float *__restrict__ V,
+template <bool AFFINE, bool SIGNS>
+__global__ void __launch_bounds__(256) imtrans_fwd_nchw_band_kernel(const float *__restrict__ X, float *__restrict__ V, signs_t *__restrict__ signs,
                                                                       int B, int H, int W, int C, int nH, int nW, int relu,
                                                                       int R, int nbands, int pitch,
                                                                       const float *__restrict__ scale, const float *__restrict__ shift)
 {
-    after_previous_kernel(X, V, scale, shift);
+    after_previous_kernel(X, V, signs, scale, shift);
     extern __shared__ float S[];   // [32 channels][pitch]
     const int band = blockIdx.x % nbands;
     const int b = blockIdx.x / nbands;
@@ -198,6 +225,7 @@ __global__ void __launch_bounds__(256) imtrans_fwd_nchw_band_kernel(const float 
         bt_d_b(d, v);
         if (c_ok) {
             const long long off = (((long long)b * nH + th0 + tr) * nW + tw) * C + c0 + lane;
+            if (SIGNS) signs[off] = signs_of(v);
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -209,13 +237,13 @@ __global__ void __launch_bounds__(256) imtrans_fwd_nchw_band_kernel(const float 
 
 // The same for small problems: a segment of S tiles of one tile row per CTA (cut_bands).  (A kernel of its own: as a variant of
 // the one above it cost that one eight registers and 7 % of its speed.)
-template <bool AFFINE>
-__global__ void __launch_bounds__(256) imtrans_fwd_nchw_row_kernel(const float *__restrict__ X, float *__restrict__ V,
+template <bool AFFINE, bool SIGNS>
+__global__ void __launch_bounds__(256) imtrans_fwd_nchw_row_kernel(const float *__restrict__ X, float *__restrict__ V, signs_t *__restrict__ signs,
                                                                      int B, int H, int W, int C, int nH, int nW, int relu,
                                                                      int S_, int nsegs, int pitch,
                                                                      const float *__restrict__ scale, const float *__restrict__ shift)
 {
-    after_previous_kernel(X, V, scale, shift);
+    after_previous_kernel(X, V, signs, scale, shift);
     extern __shared__ float S[];   // [32 channels][pitch]
     const int seg = blockIdx.x % nsegs, th = (blockIdx.x / nsegs) % nH, b = blockIdx.x / nsegs / nH;
     const int c0 = blockIdx.y * 32;
@@ -244,6 +272,7 @@ __global__ void __launch_bounds__(256) imtrans_fwd_nchw_row_kernel(const float *
         }
         bt_d_b(d, v);
         const long long off = (((long long)b * nH + th) * nW + tw0 + tl) * C + c0 + lane;
+        if (SIGNS) signs[off] = signs_of(v);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -284,12 +313,13 @@ __device__ __forceinline__ void stage_pairs(const float *__restrict__ X, float *
     asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-template <bool AFFINE, bool RELU>
-__global__ void __launch_bounds__(256, 4) imtrans_fwd_nchw_pair_kernel(const float *__restrict__ X, float *__restrict__ V, int H, int W, int C,
+template <bool AFFINE, bool RELU, bool SIGNS>
+__global__ void __launch_bounds__(256, 4) imtrans_fwd_nchw_pair_kernel(const float *__restrict__ X, float *__restrict__ V,
+                                                                         signs_t *__restrict__ signs, int H, int W, int C,
                                                                          int nH, int nW, int R, int nbands, unsigned inv, unsigned plane_bytes,
                                                                          const float *__restrict__ scale, const float *__restrict__ shift)
 {
-    after_previous_kernel(X, V, scale, shift);
+    after_previous_kernel(X, V, signs, scale, shift);
     extern __shared__ __align__(16) float S[];
     const int band = blockIdx.x % nbands, b = blockIdx.x / nbands, c0 = blockIdx.y * kPairCB;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -327,6 +357,7 @@ __global__ void __launch_bounds__(256, 4) imtrans_fwd_nchw_pair_kernel(const flo
     for (int q = q0;;) {
         column(2);
         column(3);
+        unsigned m = 0, m2 = 0;
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -334,8 +365,10 @@ __global__ void __launch_bounds__(256, 4) imtrans_fwd_nchw_pair_kernel(const flo
                 const int a = j == 0 ? 0 : j == 2 ? 2 : 1, c = j == 2 ? 1 : j == 3 ? 3 : 2;      // r0 - r2, r1 + r2, r2 - r1, r1 - r3
                 float2 v = j == 1 ? make_float2(r[i][a].x + r[i][c].x, r[i][a].y + r[i][c].y) : make_float2(r[i][a].x - r[i][c].x, r[i][a].y - r[i][c].y);
                 if (RELU) v = make_float2(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f));
+                if (SIGNS) { m |= v.x > 0.f ? 1u << (4 * i + j) : 0u; m2 |= v.y > 0.f ? 1u << (4 * i + j) : 0u; }
                 *reinterpret_cast<float2 *>(Vb + (size_t)plane_bytes * (4 * i + j) + off) = v;
             }
+        if (SIGNS) *reinterpret_cast<unsigned *>(reinterpret_cast<char *>(signs) + (off >> 1)) = m | (m2 << 16);
         if (++q >= q1) break;
         off += (unsigned)C * 4u;
         P += kPairPitch;                  // two slots, in units of two floats
@@ -382,8 +415,99 @@ __host__ __device__ constexpr bool row_needed(int dt, int i)
     return dt == 0 ? true : (dt < 0 ? i == 3 : i == 0);
 }
 
-template <typename T, bool MASK>
-__device__ __forceinline__ void imtrans_bwd_block(const T *__restrict__ dV, const T *__restrict__ Vm, long long plane,
+// MASK: the ReLU mask of a gradient, none, V > 0, or bits (signs_t)
+enum { kNoMask = 0, kMaskV = 1, kMaskBits = 2 };
+__device__ __forceinline__ float keep_bits(float g, unsigned m, int t) { return (m >> t) & 1u ? g : 0.f; }
+__device__ __forceinline__ float2 keep_bits(float2 g, unsigned m, int t)
+{
+    return make_float2((m >> t) & 1u ? g.x : 0.f, (m >> (16 + t)) & 1u ? g.y : 0.f);
+}
+__device__ __forceinline__ float4 keep_bits(float4 g, uint2 m, int t)
+{
+    return make_float4((m.x >> t) & 1u ? g.x : 0.f, (m.x >> (16 + t)) & 1u ? g.y : 0.f, (m.y >> t) & 1u ? g.z : 0.f, (m.y >> (16 + t)) & 1u ? g.w : 0.f);
+}
+__device__ __forceinline__ float2 ldg(const float2 *p) { return __ldg(p); }
+__device__ __forceinline__ float2 zero_of(float2) { return make_float2(0.f, 0.f); }
+__device__ __forceinline__ float2 operator+(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ float2 operator-(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+template <> struct Vec<2> { using type = float2; };
+// the bits of the channels a lane holds at element `at` of [P][C / VEC]
+template <typename T> struct SignBits;
+template <> struct SignBits<float>  { unsigned m; __device__ __forceinline__ void load(const void *s, long long at) { m = __ldg(static_cast<const signs_t *>(s) + at); } };
+template <> struct SignBits<float2> { unsigned m; __device__ __forceinline__ void load(const void *s, long long at) { m = __ldg(static_cast<const unsigned *>(s) + at); } };
+template <> struct SignBits<float4> { uint2 m;    __device__ __forceinline__ void load(const void *s, long long at) { m = __ldg(static_cast<const uint2 *>(s) + at); } };
+
+// ------------------------------------------------------------------------------------------
+// Backward gather along a row of tiles (without a mask or with bits).  The sums over the tile rows come first, per tile column
+// and Winograd column j
+//   h0[j] = g1j - g2j + g3j - g3j(tile above),  h1[j] = g1j + g2j - g0j + g0j(tile below)
+// and the two pixels of a tile in output row a are  h[1] - h[2] + h[3] - h[3](tile left)  and  h[1] + h[2] - h[0] + h[0](tile
+// right), so that a walk along the row loads 24 values per tile (16, 4 above, 4 below) where a gather on its own loads 36,
+// and keeps the neighbours' sums in registers.  put(a, x, value): pixel x of output row a.  (For NHWC the gather per tile
+// stays: 54 against 59 us at 64 x 64 x 56 x 56, its 36 independent loads hide more latency.)
+// ------------------------------------------------------------------------------------------
+template <typename T, int MASK, typename Put>
+__device__ __forceinline__ void imtrans_bwd_walk(const T *__restrict__ dV, const void *__restrict__ Vm, long long plane, int b, int th, int tw0,
+                                                 int tw1, int nH, int nW, int CV, int cv, Put put)
+{
+    const long long row = (((long long)b * nH + th) * nW) * CV + cv, up = (long long)nW * CV;
+    const bool above = th > 0, below = th + 1 < nH;
+    auto get = [&](int t, long long at, const SignBits<T> &bits) {
+        const T g = ldg(dV + (long long)t * plane + at);
+        return MASK == kMaskBits ? keep_bits(g, bits.m, t) : g;
+    };
+    auto sums = [&](int tw, int j0, int j1, T (&h0)[4], T (&h1)[4]) {
+        const long long at = row + (long long)tw * CV;
+        SignBits<T> bc = {}, ba = {}, bb = {};
+        if (MASK == kMaskBits) {
+            bc.load(Vm, at);
+            if (above) ba.load(Vm, at - up);
+            if (below) bb.load(Vm, at + up);
+        }
+        T ga[4], gb[4], g[4][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (j < j0 || j >= j1) continue;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) g[i][j] = get(4 * i + j, at, bc);
+            ga[j] = above ? get(12 + j, at - up, ba) : zero_of(T());
+            gb[j] = below ? get(j, at + up, bb) : zero_of(T());
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (j < j0 || j >= j1) continue;
+            h0[j] = g[1][j] - g[2][j] + g[3][j] - ga[j];
+            h1[j] = g[1][j] + g[2][j] - g[0][j] + gb[j];
+        }
+    };
+    T h[2][4], left[2] = {zero_of(T()), zero_of(T())}, odd[2];
+    if (tw0 > 0) {
+        sums(tw0 - 1, 3, 4, h[0], h[1]);
+        left[0] = h[0][3]; left[1] = h[1][3];
+    }
+#pragma unroll 1
+    for (int tw = tw0; tw < tw1; ++tw) {
+        sums(tw, 0, 4, h[0], h[1]);
+#pragma unroll
+        for (int a = 0; a < 2; ++a) {
+            if (tw > tw0) put(a, 2 * tw - 1, odd[a] + h[a][0]);
+            put(a, 2 * tw, h[a][1] - h[a][2] + h[a][3] - left[a]);
+            odd[a] = h[a][1] + h[a][2] - h[a][0];
+            left[a] = h[a][3];
+        }
+    }
+    if (tw1 < nW) {
+        sums(tw1, 0, 1, h[0], h[1]);
+        put(0, 2 * tw1 - 1, odd[0] + h[0][0]);
+        put(1, 2 * tw1 - 1, odd[1] + h[1][0]);
+    } else {
+        put(0, 2 * tw1 - 1, odd[0]);
+        put(1, 2 * tw1 - 1, odd[1]);
+    }
+}
+
+template <typename T, int MASK>
+__device__ __forceinline__ void imtrans_bwd_block(const T *__restrict__ dV, const void *__restrict__ Vm, long long plane,
                                                   int b, int bh, int bw, int nH, int nW, int CV, int cv, T (&out)[2][2])
 {
 #pragma unroll
@@ -399,13 +523,16 @@ __device__ __forceinline__ void imtrans_bwd_block(const T *__restrict__ dV, cons
             const int tw = bw + dtw;
             if (tw < 0 || tw >= nW) continue;
             const long long base = (((long long)b * nH + th) * nW + tw) * CV + cv;
+            SignBits<T> bits = {};
+            if (MASK == kMaskBits) bits.load(Vm, base);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     if (!row_needed(dth, i) || !row_needed(dtw, j)) continue;
                     T g = ldg(dV + (long long)(4 * i + j) * plane + base);
-                    if (MASK) g = keep_where_pos(g, ldg(Vm + (long long)(4 * i + j) * plane + base));
+                    if (MASK == kMaskV) g = keep_where_pos(g, ldg(static_cast<const T *>(Vm) + (long long)(4 * i + j) * plane + base));
+                    if (MASK == kMaskBits) g = keep_bits(g, bits.m, 4 * i + j);
 #pragma unroll
                     for (int a = 0; a < 2; ++a) {
 #pragma unroll
@@ -423,8 +550,8 @@ __device__ __forceinline__ void imtrans_bwd_block(const T *__restrict__ dV, cons
     }
 }
 
-template <int VEC, bool MASK>
-__global__ void __launch_bounds__(256) imtrans_bwd_nhwc_kernel(const float *__restrict__ dV, const float *__restrict__ Vm,
+template <int VEC, int MASK>
+__global__ void __launch_bounds__(256) imtrans_bwd_nhwc_kernel(const float *__restrict__ dV, const void *__restrict__ Vm,
                                                                  float *__restrict__ dX, int B, int H, int W, int C, int nH, int nW)
 {
     after_previous_kernel(dV, Vm, dX);
@@ -439,7 +566,7 @@ __global__ void __launch_bounds__(256) imtrans_bwd_nhwc_kernel(const float *__re
     const int bh = (int)((p / nW) % nH);
     const int b = (int)(p / ((long long)nW * nH));
     T out[2][2];
-    imtrans_bwd_block<T, MASK>(reinterpret_cast<const T *>(dV), reinterpret_cast<const T *>(Vm),
+    imtrans_bwd_block<T, MASK>(reinterpret_cast<const T *>(dV), Vm,
                                (long long)B * nH * nW * CV, b, bh, bw, nH, nW, CV, cv, out);
     T *dXv = reinterpret_cast<T *>(dX);
 #pragma unroll
@@ -451,10 +578,48 @@ __global__ void __launch_bounds__(256) imtrans_bwd_nhwc_kernel(const float *__re
         }
 }
 
+// NCHW, enough tiles to fill the GPU: the walk with lane = VEC channels over a band of R tile rows, each cut into segments of S
+// tiles for the eight warps; the pixels collect in shared memory as [pixel][channel] and leave as one contiguous run per channel.
+// 64 x 64 x 56 x 56 without a mask 84 us as gathers, 62 so (257 MB: 40 at the copy rate); 128 x 96 x 20 x 22 51 -> 30; with the ReLU
+// mask 108 (V) -> 74 (bits).
+template <int VEC, int MASK>
+__global__ void __launch_bounds__(256, 3) imtrans_bwd_nchw_walk_kernel(const float *__restrict__ dV, const void *__restrict__ Vm,
+                                                                         float *__restrict__ dX, int B, int H, int W, int C, int nH, int nW,
+                                                                         int R, int nbands, int S, int nseg)
+{
+    after_previous_kernel(dV, Vm, dX);
+    using T = typename Vec<VEC>::type;
+    constexpr int CB = 32 * VEC, CBP = CB + (VEC == 1 ? 1 : 2);
+    extern __shared__ __align__(16) float O[];          // [2R rows x W pixels][CBP]
+    const int c0 = blockIdx.y * CB;
+    const int band = blockIdx.x % nbands, b = blockIdx.x / nbands;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int th0 = band * R, rows = min(R, nH - th0);
+    const int CV = C / VEC;
+    if (c0 + VEC * lane < C) {
+#pragma unroll 1
+        for (int q = warp; q < rows * nseg; q += 8) {
+            const int tr = q / nseg, seg = q - tr * nseg, tw0 = seg * S;
+            if (tw0 >= nW) continue;
+            float *const o = O + 2 * tr * W * CBP + VEC * lane;
+            imtrans_bwd_walk<T, MASK>(reinterpret_cast<const T *>(dV), Vm, (long long)B * nH * nW * CV, b, th0 + tr, tw0, min(tw0 + S, nW), nH, nW,
+                                      CV, c0 / VEC + lane, [&](int a, int x, T v) {
+                                          if (x < W) *reinterpret_cast<T *>(o + (a * W + x) * CBP) = v;
+                                      });
+        }
+    }
+    __syncthreads();
+    const int n = (min(2 * (th0 + rows), H) - 2 * th0) * W, nch = min(CB, C - c0);
+    for (int c = warp; c < nch; c += 8) {
+        float *d = dX + (((long long)b * C + c0 + c) * H + 2 * th0) * W;
+        for (int i = lane; i < n; i += 32) d[i] = O[i * CBP + c];
+    }
+}
+
 // NCHW: the same gather with the channel index fastest across a warp (coalesced dV reads), then a
 // shared-memory turn so that dX rows are written contiguously along W.
-template <bool MASK>
-__global__ void __launch_bounds__(256) imtrans_bwd_nchw_kernel(const float *__restrict__ dV, const float *__restrict__ Vm,
+template <int MASK>
+__global__ void __launch_bounds__(256) imtrans_bwd_nchw_kernel(const float *__restrict__ dV, const void *__restrict__ Vm,
                                                                  float *__restrict__ dX, int B, int H, int W, int C, int nH, int nW)
 {
     after_previous_kernel(dV, Vm, dX);
@@ -493,14 +658,14 @@ __global__ void __launch_bounds__(256) imtrans_bwd_nchw_kernel(const float *__re
     }
 }
 
-// NCHW, image rows up to 192 pixels: the same gather with lane = VEC consecutive channels over a band of R tile
+// NCHW, image rows up to 192 pixels, with V as the mask or too few tiles for the walk above to fill the GPU: the same gather with lane = VEC consecutive channels over a band of R tile
 // rows; the 2R x W output pixels of each channel collect in shared memory (odd pitch between channels) and
 // leave as one contiguous run per channel -- or, where the band is the whole image, as one contiguous run for
 // all the block's channels.  VEC = 4 reads dV (and the ReLU mask) with 16-byte loads: LC = 32 lanes along the
 // channels (128 per block, 512 bytes per request) where such a band fits four blocks per SM, else LC = 16 (64
 // channels per block, the two halves of a warp on two tiles at once).
-template <int VEC, int LC, bool MASK, bool SEG>
-__global__ void __launch_bounds__(256, 4) imtrans_bwd_nchw_band_kernel(const float *__restrict__ dV, const float *__restrict__ Vm,
+template <int VEC, int LC, int MASK, bool SEG>
+__global__ void __launch_bounds__(256, 4) imtrans_bwd_nchw_band_kernel(const float *__restrict__ dV, const void *__restrict__ Vm,
                                                                          float *__restrict__ dX, int B, int H, int W, int C, int nH,
                                                                          int nW, int R, int nbands, int S, int nsegs, int pitch)
 {
@@ -510,11 +675,11 @@ __global__ void __launch_bounds__(256, 4) imtrans_bwd_nchw_band_kernel(const flo
     constexpr int QW = 32 / LC;              // tiles a warp works on at once
     extern __shared__ float O[];             // [CB channels][pitch]
     // Block order.  One input stream: a one-dimensional grid with the channel blocks fastest, so that neighbouring
-    // blocks read neighbouring segments of every dV row.  With the mask (32 streams of rows open at once) that
+    // blocks read neighbouring segments of every dV row.  With V as the mask (32 streams of rows open at once) that
     // order measured slower than images fastest, which is the two-dimensional grid (66 vs 78 us on
     // 256 x 512 x 7 x 7; without the mask 50 vs 58 us the other way).
     int c0, bb;
-    if (MASK) {
+    if (MASK == kMaskV) {
         c0 = blockIdx.y * CB;
         bb = blockIdx.x;
     } else {
@@ -544,7 +709,7 @@ __global__ void __launch_bounds__(256, 4) imtrans_bwd_nchw_band_kernel(const flo
 #pragma unroll
             for (int e = 0; e < 2; ++e) out[a][e] = zero_of(T());
         if (c_ok)
-            imtrans_bwd_block<T, MASK>(reinterpret_cast<const T *>(dV), reinterpret_cast<const T *>(Vm), plane, b, th0 + br, bw, nH,
+            imtrans_bwd_block<T, MASK>(reinterpret_cast<const T *>(dV), Vm, plane, b, th0 + br, bw, nH,
                                        nW, CV, c0 / VEC + lc, out);
 #pragma unroll
         for (int a = 0; a < 2; ++a)
@@ -587,8 +752,8 @@ __global__ void __launch_bounds__(256, 4) imtrans_bwd_nchw_band_kernel(const flo
 // passes by the parity of (tile row, tile column) with a barrier between passes, and plain read-modify-writes suffice
 // (no atomics: the result does not depend on the order of the warps).  The image is kept as [channel][pixel] with an
 // odd pitch (lanes hit distinct banks) and leaves as one contiguous run: CB channels x H*W pixels are adjacent in dX.
-template <bool MASK>
-__global__ void __launch_bounds__(256) imtrans_bwd_nchw_image_kernel(const float *__restrict__ dV, const float *__restrict__ Vm,
+template <int MASK>
+__global__ void __launch_bounds__(256) imtrans_bwd_nchw_image_kernel(const float *__restrict__ dV, const void *__restrict__ Vm,
                                                                        float *__restrict__ dX, int B, int H, int W, int C, int nH, int nW,
                                                                        int CB, int pitch)
 {
@@ -629,14 +794,20 @@ __global__ void __launch_bounds__(256) imtrans_bwd_nchw_image_kernel(const float
             const int cl = gr * 32 + lane;
             if (cl < nch) {
                 const float *gp = dV + ((((long long)b * nH + th) * nW + tw) * C + c0 + cl);
-                const float *vp = MASK ? Vm + ((((long long)b * nH + th) * nW + tw) * C + c0 + cl) : nullptr;
+                const long long at = (((long long)b * nH + th) * nW + tw) * C + c0 + cl;
                 float g[4][4];
 #pragma unroll
                 for (int t = 0; t < 16; ++t) g[t >> 2][t & 3] = __ldg(gp + (long long)t * plane);
-                if (MASK) {
+                if (MASK == kMaskBits) {
+                    SignBits<float> bits;
+                    bits.load(Vm, at);
+#pragma unroll
+                    for (int t = 0; t < 16; ++t) g[t >> 2][t & 3] = keep_bits(g[t >> 2][t & 3], bits.m, t);
+                }
+                if (MASK == kMaskV) {
                     float v[16];
 #pragma unroll
-                    for (int t = 0; t < 16; ++t) v[t] = __ldg(vp + (long long)t * plane);
+                    for (int t = 0; t < 16; ++t) v[t] = __ldg(static_cast<const float *>(Vm) + at + (long long)t * plane);
 #pragma unroll
                     for (int t = 0; t < 16; ++t)
                         if (!(v[t] > 0.f)) g[t >> 2][t & 3] = 0.f;
@@ -687,8 +858,8 @@ __device__ __forceinline__ float2 f2add(float2 a, float2 b) { return make_float2
 __device__ __forceinline__ float2 f2sub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ float2 f2neg(float2 a) { return make_float2(-a.x, -a.y); }
 
-template <bool MASK>
-__global__ void __launch_bounds__(256, 4) imtrans_bwd_nchw_image2_kernel(const float *__restrict__ dV, const float *__restrict__ Vm,
+template <int MASK>
+__global__ void __launch_bounds__(256, 4) imtrans_bwd_nchw_image2_kernel(const float *__restrict__ dV, const void *__restrict__ Vm,
                                                                            float *__restrict__ dX, int B, int H, int W, int C, int nH,
                                                                            int nW, int CB)
 {
@@ -717,10 +888,16 @@ __global__ void __launch_bounds__(256, 4) imtrans_bwd_nchw_image2_kernel(const f
                 float2 g[4][4];
 #pragma unroll
                 for (int t = 0; t < 16; ++t) g[t >> 2][t & 3] = __ldg(reinterpret_cast<const float2 *>(dV + base + (long long)t * plane));
-                if (MASK) {
+                if (MASK == kMaskBits) {
+                    SignBits<float2> bits;
+                    bits.load(Vm, base >> 1);
+#pragma unroll
+                    for (int t = 0; t < 16; ++t) g[t >> 2][t & 3] = keep_bits(g[t >> 2][t & 3], bits.m, t);
+                }
+                if (MASK == kMaskV) {
 #pragma unroll
                     for (int t = 0; t < 16; ++t) {
-                        const float2 v = __ldg(reinterpret_cast<const float2 *>(Vm + base + (long long)t * plane));
+                        const float2 v = __ldg(reinterpret_cast<const float2 *>(static_cast<const float *>(Vm) + base + (long long)t * plane));
                         if (!(v.x > 0.f)) g[t >> 2][t & 3].x = 0.f;
                         if (!(v.y > 0.f)) g[t >> 2][t & 3].y = 0.f;
                     }
@@ -764,24 +941,26 @@ __global__ void __launch_bounds__(256, 4) imtrans_bwd_nchw_image2_kernel(const f
 // ------------------------------------------------------------------------------------------
 static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-int imtrans_fwd(const float *X, float *V, int B, int H, int W, int C, int layout, int relu, const float *scale, const float *shift,
-                cudaStream_t st)
+int imtrans_fwd(const float *X, float *V, void *signs_out, int B, int H, int W, int C, int layout, int relu, const float *scale,
+                const float *shift, cudaStream_t st)
 {
     if (!X || !V || B <= 0 || H <= 0 || W <= 0 || C <= 0) return WG2X2_ERR_BAD_ARG;
     if ((scale == nullptr) != (shift == nullptr)) return WG2X2_ERR_BAD_ARG;
+    signs_t *signs = static_cast<signs_t *>(signs_out);
+    if (signs && (scale || !aligned16(signs))) return WG2X2_ERR_BAD_ARG;
     if (layout != WG2X2_NHWC && layout != WG2X2_NCHW) return WG2X2_ERR_BAD_ARG;
     const int nH = (H + 1) / 2, nW = (W + 1) / 2;
     if (layout == WG2X2_NHWC) {
         if ((C % 4 == 0) && aligned16(X) && aligned16(V) && (!scale || (aligned16(scale) && aligned16(shift)))) {
             const long long total = (long long)B * nH * nW * (C / 4);
             const unsigned g = (unsigned)cdivll(total, 256);
-            if (scale) launch(imtrans_fwd_nhwc_kernel<4, true>, dim3(g), 256, 0, st, X, V, B, H, W, C, nH, nW, relu, scale, shift);
-            else       launch(imtrans_fwd_nhwc_kernel<4, false>, dim3(g), 256, 0, st, X, V, B, H, W, C, nH, nW, relu, scale, shift);
+            launch(scale ? imtrans_fwd_nhwc_kernel<4, true, false> : signs ? imtrans_fwd_nhwc_kernel<4, false, true> : imtrans_fwd_nhwc_kernel<4, false, false>,
+                   dim3(g), 256, 0, st, X, V, signs, B, H, W, C, nH, nW, relu, scale, shift);
         } else {
             const long long total = (long long)B * nH * nW * C;
             const unsigned g = (unsigned)cdivll(total, 256);
-            if (scale) launch(imtrans_fwd_nhwc_kernel<1, true>, dim3(g), 256, 0, st, X, V, B, H, W, C, nH, nW, relu, scale, shift);
-            else       launch(imtrans_fwd_nhwc_kernel<1, false>, dim3(g), 256, 0, st, X, V, B, H, W, C, nH, nW, relu, scale, shift);
+            launch(scale ? imtrans_fwd_nhwc_kernel<1, true, false> : signs ? imtrans_fwd_nhwc_kernel<1, false, true> : imtrans_fwd_nhwc_kernel<1, false, false>,
+                   dim3(g), 256, 0, st, X, V, signs, B, H, W, C, nH, nW, relu, scale, shift);
         }
     } else {
         const long long gx = (long long)B * nH * cdiv(nW, kTSEG);
@@ -796,9 +975,10 @@ int imtrans_fwd(const float *X, float *V, int B, int H, int W, int C, int layout
         if (R) {
             const int nbands = cdiv(nH, R), smem = (2 * R + 2) * (2 * nW + 2) * kPairPitch * (int)sizeof(float);
             if ((long long)B * nbands > 0x7fffffffLL) return WG2X2_ERR_UNSUPPORTED;
-            auto *kernel = scale ? (relu ? imtrans_fwd_nchw_pair_kernel<true, true> : imtrans_fwd_nchw_pair_kernel<true, false>)
-                                 : (relu ? imtrans_fwd_nchw_pair_kernel<false, true> : imtrans_fwd_nchw_pair_kernel<false, false>);
-            launch(kernel, dim3((unsigned)(B * nbands), C / kPairCB), 256, smem, st, X, V, H, W, C, nH, nW, R, nbands,
+            auto *kernel = scale ? (relu ? imtrans_fwd_nchw_pair_kernel<true, true, false> : imtrans_fwd_nchw_pair_kernel<true, false, false>)
+                         : signs ? (relu ? imtrans_fwd_nchw_pair_kernel<false, true, true> : imtrans_fwd_nchw_pair_kernel<false, false, true>)
+                                 : (relu ? imtrans_fwd_nchw_pair_kernel<false, true, false> : imtrans_fwd_nchw_pair_kernel<false, false, false>);
+            launch(kernel, dim3((unsigned)(B * nbands), C / kPairCB), 256, smem, st, X, V, signs, H, W, C, nH, nW, R, nbands,
                    (unsigned)cdiv(1 << 20, 2 * nW + 2), (unsigned)((long long)B * nH * nW * C * 4), scale, shift);
         } else if (W <= 128) {
             const BandCut cut = cut_bands(nH, nW, (long long)B * cdiv(C, 32), (kBandFloats / W - 2) / 2);
@@ -808,89 +988,110 @@ int imtrans_fwd(const float *X, float *V, int B, int H, int W, int C, int layout
             if (gxb > 0x7fffffffLL) return WG2X2_ERR_UNSUPPORTED;
             const dim3 gb((unsigned)gxb, cdiv(C, 32));
             if (cut.nsegs == 1)
-                launch(scale ? imtrans_fwd_nchw_band_kernel<true> : imtrans_fwd_nchw_band_kernel<false>, gb, 256, smem, st, X, V, B, H, W, C, nH,
+                launch(scale ? imtrans_fwd_nchw_band_kernel<true, false> : signs ? imtrans_fwd_nchw_band_kernel<false, true> : imtrans_fwd_nchw_band_kernel<false, false>,
+                       gb, 256, smem, st, X, V, signs, B, H, W, C, nH,
                        nW, relu, cut.R, cut.nbands, pitch, scale, shift);
             else
-                launch(scale ? imtrans_fwd_nchw_row_kernel<true> : imtrans_fwd_nchw_row_kernel<false>, gb, 256, smem, st, X, V, B, H, W, C, nH, nW,
+                launch(scale ? imtrans_fwd_nchw_row_kernel<true, false> : signs ? imtrans_fwd_nchw_row_kernel<false, true> : imtrans_fwd_nchw_row_kernel<false, false>,
+                       gb, 256, smem, st, X, V, signs, B, H, W, C, nH, nW,
                        relu, cut.S, cut.nsegs, pitch, scale, shift);
         } else {
-            launch(imtrans_fwd_nchw_kernel, grid, 256, 0, st, X, V, B, H, W, C, nH, nW, relu, scale, shift);
+            launch(imtrans_fwd_nchw_kernel, grid, 256, 0, st, X, V, signs, B, H, W, C, nH, nW, relu, scale, shift);
         }
     }
     return launch_status();
 }
 
-int imtrans_bwd(const float *dV, const float *Vm, float *dX, int B, int H, int W, int C, int layout, cudaStream_t st)
+// The kernel of a family for the kind of mask
+#define WG_BY_MASK(...) (mask == kNoMask ? WG_INST(kNoMask, __VA_ARGS__) : mask == kMaskV ? WG_INST(kMaskV, __VA_ARGS__) : WG_INST(kMaskBits, __VA_ARGS__))
+
+// Vm: the mask, V itself (mask_bits == 0) or its bits as imtrans_fwd wrote them; NULL: none
+int imtrans_bwd(const float *dV, const void *Vm, int mask_bits, float *dX, int B, int H, int W, int C, int layout, cudaStream_t st)
 {
     if (!dV || !dX || B <= 0 || H <= 0 || W <= 0 || C <= 0) return WG2X2_ERR_BAD_ARG;
     if (layout != WG2X2_NHWC && layout != WG2X2_NCHW) return WG2X2_ERR_BAD_ARG;
     const int nH = (H + 1) / 2, nW = (W + 1) / 2;
+    const int mask = !Vm ? kNoMask : mask_bits ? kMaskBits : kMaskV;
+    // n-byte accesses to dV and to the mask (`n` bytes of V are n / 2 bytes of bits)
+    const auto on = [&](uintptr_t n) {
+        return (reinterpret_cast<uintptr_t>(dV) & (n - 1)) == 0 && (reinterpret_cast<uintptr_t>(Vm) & ((mask == kMaskBits ? n / 2 : n) - 1)) == 0;
+    };
     if (layout == WG2X2_NHWC) {
-        const bool vec = (C % 4 == 0) && aligned16(dV) && aligned16(dX) && (!Vm || aligned16(Vm));
-        const long long total = (long long)B * nH * nW * (vec ? C / 4 : C);
-        const unsigned g = (unsigned)cdivll(total, 256);
-        if (vec) {
-            if (Vm) launch(imtrans_bwd_nhwc_kernel<4, true>, dim3(g), 256, 0, st, dV, Vm, dX, B, H, W, C, nH, nW);
-            else    launch(imtrans_bwd_nhwc_kernel<4, false>, dim3(g), 256, 0, st, dV, Vm, dX, B, H, W, C, nH, nW);
-        } else {
-            if (Vm) launch(imtrans_bwd_nhwc_kernel<1, true>, dim3(g), 256, 0, st, dV, Vm, dX, B, H, W, C, nH, nW);
-            else    launch(imtrans_bwd_nhwc_kernel<1, false>, dim3(g), 256, 0, st, dV, Vm, dX, B, H, W, C, nH, nW);
-        }
-    } else {
-        // small images: one block per image and channel block, every value of dV read once
-        const int HW = H * W;
-        if (HW <= 200 && (long long)B * cdiv(C, HW <= 64 ? 128 : 64) >= 2LL * kNumSMs && B <= 0x7fffffff) {
-            const int CB = HW <= 64 ? 128 : 64;
-            const auto aligned8 = [](const void *q) { return (reinterpret_cast<uintptr_t>(q) & 7u) == 0; };
-            if ((C & 1) == 0 && aligned8(dV) && (!Vm || aligned8(Vm)) && cdiv(C, CB) <= 65535) {      // two channels per lane
-                const int smem2 = HW * (CB + 2) * (int)sizeof(float);
-                const dim3 grid2((unsigned)B, cdiv(C, CB));
-                launch(Vm ? imtrans_bwd_nchw_image2_kernel<true> : imtrans_bwd_nchw_image2_kernel<false>, grid2, 256, smem2, st, dV, Vm, dX, B, H,
-                       W, C, nH, nW, CB);
-                return launch_status();
-            }
-            const int pitch = HW | 1;
-            const int smem = CB * pitch * (int)sizeof(float);
-            if (cdiv(C, CB) <= 65535) {
-                const dim3 grid((unsigned)B, cdiv(C, CB));
-                launch(Vm ? imtrans_bwd_nchw_image_kernel<true> : imtrans_bwd_nchw_image_kernel<false>, grid, 256, smem, st, dV, Vm, dX, B, H, W,
-                       C, nH, nW, CB, pitch);
-                return launch_status();
-            }
-        }
-        if (W <= 192) {
-            // four channels per lane (16-byte loads) where the channels allow it and a band of 128 channels stays small
-            // four channels per lane (16-byte loads) where the channels allow it; 128 channels per block where a band of
-            // them stays below 50 KB (four blocks per SM), else 64
-            // -- and where that still leaves four CTAs for every SM (a small batch keeps the narrower blocks)
-            auto ctas = [&](int cbk, int band_floats) { return (long long)B * cdiv(nH, max(1, min(nH, band_floats / (2 * W)))) * cdiv(C, cbk); };
-            const long long fill = 4LL * kNumSMs;
-            const bool vec_ok = (C % 4 == 0) && C >= 64 && aligned16(dV) && (!Vm || aligned16(Vm)) && 2 * W <= kBandFloats / 2;
-            const bool wide = vec_ok && C >= 128 && 2 * W <= kBandFloats / 4 && ctas(128, kBandFloats / 4) >= fill;
-            const bool vec = wide || (vec_ok && ctas(64, kBandFloats / 2) >= fill);
-            const int cb = wide ? 128 : (vec ? 64 : 32);
-            const int max_rows = (wide ? kBandFloats / 4 : (vec ? kBandFloats / 2 : kBandFloats)) / (2 * W);
-            const BandCut cut = cut_bands(nH, nW, (long long)B * cdiv(C, cb), max_rows);
-            const int pitch = (2 * cut.R * (cut.nsegs == 1 ? W : 2 * cut.S)) | 1;
-            const int smem = cb * pitch * (int)sizeof(float);
-            const long long blocks = (long long)B * cut.nbands * cut.nsegs;
-            if (blocks * cdiv(C, cb) > 0x7fffffffLL || cdiv(C, cb) > 65535) return WG2X2_ERR_UNSUPPORTED;
-            const dim3 grid = Vm ? dim3((unsigned)blocks, cdiv(C, cb)) : dim3((unsigned)(blocks * cdiv(C, cb)));
-            auto go = [&](auto kernel) {
-                return launch(kernel, grid, 256, smem, st, dV, Vm, dX, B, H, W, C, nH, nW, cut.R, cut.nbands, cut.S, cut.nsegs, pitch);
-            };
-            // (the kernels with wider blocks are only taken where those already fill the GPU: they have no segments)
-            return wide ? (Vm ? go(imtrans_bwd_nchw_band_kernel<4, 32, true, false>) : go(imtrans_bwd_nchw_band_kernel<4, 32, false, false>))
-                : vec ? (Vm ? go(imtrans_bwd_nchw_band_kernel<4, 16, true, false>) : go(imtrans_bwd_nchw_band_kernel<4, 16, false, false>))
-                : cut.nsegs == 1 ? (Vm ? go(imtrans_bwd_nchw_band_kernel<1, 32, true, false>) : go(imtrans_bwd_nchw_band_kernel<1, 32, false, false>))
-                                 : (Vm ? go(imtrans_bwd_nchw_band_kernel<1, 32, true, true>) : go(imtrans_bwd_nchw_band_kernel<1, 32, false, true>));
-        }
-        const long long gx = (long long)B * nH * cdiv(nW, kTSEG);
-        if (gx > 0x7fffffffLL || cdiv(C, kCCH) > 65535) return WG2X2_ERR_UNSUPPORTED;
-        dim3 grid((unsigned)gx, cdiv(C, kCCH));
-        if (Vm) launch(imtrans_bwd_nchw_kernel<true>, grid, 256, 0, st, dV, Vm, dX, B, H, W, C, nH, nW);
-        else    launch(imtrans_bwd_nchw_kernel<false>, grid, 256, 0, st, dV, Vm, dX, B, H, W, C, nH, nW);
+        const bool vec = C % 4 == 0 && on(16) && aligned16(dX);
+        const long long grid = cdivll((long long)B * nH * nW * (vec ? C / 4 : C), 256);
+        if (grid > 0x7fffffffLL) return WG2X2_ERR_UNSUPPORTED;
+#define WG_INST(M, V) imtrans_bwd_nhwc_kernel<V, M>
+        launch(vec ? WG_BY_MASK(4) : WG_BY_MASK(1), dim3((unsigned)grid), 256, 0, st, dV, Vm, dX, B, H, W, C, nH, nW);
+#undef WG_INST
+        return launch_status();
     }
+    // small images: one block per image and channel block, every value of dV read once
+    const int HW = H * W;
+    if (HW <= 200 && (long long)B * cdiv(C, HW <= 64 ? 128 : 64) >= 2LL * kNumSMs && cdiv(C, HW <= 64 ? 128 : 64) <= 65535) {
+        const int CB = HW <= 64 ? 128 : 64;
+        const dim3 grid((unsigned)B, cdiv(C, CB));
+        if ((C & 1) == 0 && on(8)) {      // two channels per lane
+#define WG_INST(M, V) imtrans_bwd_nchw_image2_kernel<M>
+            launch(WG_BY_MASK(0), grid, 256, HW * (CB + 2) * sizeof(float), st, dV, Vm, dX, B, H, W, C, nH, nW, CB);
+#undef WG_INST
+        } else {
+            const int pitch = HW | 1;
+#define WG_INST(M, V) imtrans_bwd_nchw_image_kernel<M>
+            launch(WG_BY_MASK(0), grid, 256, CB * pitch * sizeof(float), st, dV, Vm, dX, B, H, W, C, nH, nW, CB, pitch);
+#undef WG_INST
+        }
+        return launch_status();
+    }
+    if (W <= 192) {
+        // The walk, except with V as the mask (it holds too much then: 141 against 108 us at 64 x 64 x 56 x 56).  Two channels per lane
+        // where the last block of 64 is more than half full and there is no mask (with bits 81 against 74 us); bands as high as
+        // leave the busiest SM least to do, below 64 KB of shared memory.
+        const bool two = mask == kNoMask && (C & 1) == 0 && on(8) && (C % 64 == 0 || C % 64 > 32);
+        const int cb = two ? 64 : 32, px = (two ? cb + 2 : cb + 1) * (int)sizeof(float);
+        int R = 0;
+        double t = 1e300;
+        for (int r = 1; mask != kMaskV && r <= nH && (r == 1 || 2 * r * W * px <= 64 * 1024); ++r) {
+            const long long ctas = (long long)B * cdiv(nH, r) * cdiv(C, cb);
+            if (ctas < 3LL * kNumSMs) break;
+            const double u = (double)cdivll(ctas, 3 * kNumSMs) * (r * nW + 8.0);
+            if (u < t) { t = u; R = r; }
+        }
+        if (R && cdiv(C, cb) <= 65535 && (long long)B * cdiv(nH, R) <= 0x7fffffffLL) {
+            R = cdiv(nH, cdiv(nH, R));
+            const int nbands = cdiv(nH, R), S = cdiv(nW, R >= 8 ? 1 : cdiv(8, R)), nseg = cdiv(nW, S);
+            launch(two ? imtrans_bwd_nchw_walk_kernel<2, kNoMask> : mask == kNoMask ? imtrans_bwd_nchw_walk_kernel<1, kNoMask>
+                                                                 : imtrans_bwd_nchw_walk_kernel<1, kMaskBits>,
+                   dim3((unsigned)(B * nbands), cdiv(C, cb)), 256, 2 * R * W * px, st, dV, Vm, dX, B, H, W, C, nH, nW, R, nbands, S, nseg);
+            return launch_status();
+        }
+        // four channels per lane (16-byte loads) where the channels allow it; 128 channels per block where a band of
+        // them stays below 50 KB (four blocks per SM), else 64
+        // -- and where that still leaves four CTAs for every SM (a small batch keeps the narrower blocks)
+        auto ctas = [&](int cbk, int band_floats) { return (long long)B * cdiv(nH, max(1, min(nH, band_floats / (2 * W)))) * cdiv(C, cbk); };
+        const long long fill = 4LL * kNumSMs;
+        const bool vec_ok = mask == kMaskV && (C % 4 == 0) && C >= 64 && on(16) && 2 * W <= kBandFloats / 2;
+        const bool wide = vec_ok && C >= 128 && 2 * W <= kBandFloats / 4 && ctas(128, kBandFloats / 4) >= fill;
+        const bool vec = wide || (vec_ok && ctas(64, kBandFloats / 2) >= fill);
+        const int bcb = wide ? 128 : (vec ? 64 : 32);
+        const int max_rows = (wide ? kBandFloats / 4 : (vec ? kBandFloats / 2 : kBandFloats)) / (2 * W);
+        const BandCut cut = cut_bands(nH, nW, (long long)B * cdiv(C, bcb), max_rows);
+        const int pitch = (2 * cut.R * (cut.nsegs == 1 ? W : 2 * cut.S)) | 1;
+        const long long blocks = (long long)B * cut.nbands * cut.nsegs;
+        if (blocks * cdiv(C, bcb) > 0x7fffffffLL || cdiv(C, bcb) > 65535) return WG2X2_ERR_UNSUPPORTED;
+        const dim3 grid = mask == kMaskV ? dim3((unsigned)blocks, cdiv(C, bcb)) : dim3((unsigned)(blocks * cdiv(C, bcb)));
+        // (the kernels with wider blocks are only taken where those already fill the GPU: they have no segments)
+#define WG_INST(M, S) imtrans_bwd_nchw_band_kernel<1, 32, M, S>
+        launch(wide ? imtrans_bwd_nchw_band_kernel<4, 32, kMaskV, false> : vec ? imtrans_bwd_nchw_band_kernel<4, 16, kMaskV, false>
+                    : cut.nsegs == 1 ? WG_BY_MASK(false) : WG_BY_MASK(true),
+               grid, 256, bcb * pitch * sizeof(float), st, dV, Vm, dX, B, H, W, C, nH, nW, cut.R, cut.nbands, cut.S, cut.nsegs, pitch);
+#undef WG_INST
+        return launch_status();
+    }
+    const long long gx = (long long)B * nH * cdiv(nW, kTSEG);
+    if (gx > 0x7fffffffLL || cdiv(C, kCCH) > 65535) return WG2X2_ERR_UNSUPPORTED;
+#define WG_INST(M, V) imtrans_bwd_nchw_kernel<M>
+    launch(WG_BY_MASK(0), dim3((unsigned)gx, cdiv(C, kCCH)), 256, 0, st, dV, Vm, dX, B, H, W, C, nH, nW);
+#undef WG_INST
     return launch_status();
 }
 

@@ -35,6 +35,9 @@ _SIGS = {
     "wg2x2_imtrans_fwd": (_i, [_p, _p, _i, _i, _i, _i, _i, _i, _p]),
     "wg2x2_imtrans_fwd_affine": (_i, [_p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _p]),
     "wg2x2_imtrans_bwd": (_i, [_p, _p, _p, _i, _i, _i, _i, _i, _p]),
+    "wg2x2_imtrans_fwd_relu_bits": (_i, [_p, _p, _p, _i, _i, _i, _i, _i, _p]),
+    "wg2x2_imtrans_bwd_relu_bits": (_i, [_p, _p, _p, _i, _i, _i, _i, _i, _p]),
+    "wg2x2_relu_bits_bytes": (_z, [_i, _i, _i, _i]),
     "wg2x2_conv_fwd": (_i, [_p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _i, _p, _z, _p]),
     "wg2x2_conv_fwd_workspace_bytes": (_z, [_i, _i, _i, _i, _i, _i]),
     "wg2x2_prepared_weights_bytes": (_z, [_i, _i]),

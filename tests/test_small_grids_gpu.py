@@ -80,3 +80,27 @@ def test_masked_layer(C, K, layout, math):
     assert torch.equal(y, y2)
     for a, b in zip(torch.autograd.grad(y, (V, layer.W), dY), torch.autograd.grad(y2, (V, layer.W), dY)):
         assert torch.equal(a, b)
+
+
+# the ReLU mask as bits, forward and gradient, through every kernel that writes or reads them: vector and scalar channels, rows cut
+# into segments, bands, walks along a row with one and two channels per lane, whole small images, rows wider than a band
+@pytest.mark.parametrize("layout", ["NHWC", "NCHW"])
+@pytest.mark.parametrize("shape", [(2, 9, 13, 32), (3, 6, 7, 5), (1, 64, 64, 16), (2, 28, 28, 36), (32, 28, 30, 32), (40, 21, 27, 64), (75, 14, 14, 256),
+                                   (300, 7, 7, 33), (1, 3, 200, 8), (20, 45, 44, 68)])
+def test_relu_bits(oracle, shape, layout):
+    import torch
+    import wg2x2
+    B, H, W, C = shape
+    rng = np.random.default_rng(sum(shape))
+    X = rng.standard_normal((B, H, W, C)).astype(np.float32)
+    G = rng.standard_normal((16, B, (H + 1) // 2, (W + 1) // 2, C)).astype(np.float32)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    img = lambda a: dev(a if layout == "NHWC" else np.transpose(a, (0, 3, 1, 2)))
+    back = lambda t: t.cpu().numpy() if layout == "NHWC" else np.transpose(t.cpu().numpy(), (0, 2, 3, 1))
+    for relu in (True, False):
+        x = img(X).requires_grad_(True)
+        v = wg2x2.ops.imtrans_op(x, relu, layout)
+        assert torch.equal(v, wg2x2.imtrans_fwd(x.detach(), relu=relu, layout=layout))
+        V = v.detach().cpu().numpy()
+        dx, = torch.autograd.grad(v, x, dev(G))
+        assert oracle.max_rel(back(dx), oracle.imtrans_bwd(G, H, W, Vmask=V if relu else None)) <= 1e-5
