@@ -10,7 +10,7 @@ import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
-SOURCES = ["imtrans.cu", "conv_ffma.cu", "conv_tc.cu", "api.cu", "ref_launchers.cu", "noalloc.cu", "pool.cu", "stem.cu"]
+SOURCES = ["imtrans.cu", "conv_ffma.cu", "conv_tc.cu", "api.cu", "ref_launchers.cu", "noalloc.cu", "pool.cu"]
 LIB = os.path.join(HERE, "libwinograd2x2_b200.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 NATIVE = os.path.join(HERE, "wg2x2", "_native.so")

@@ -836,6 +836,7 @@ void dw_reduce_launch(const float *partial, const float *mask, float *dW, long l
 #include "conv_tc_bwd.cuh"
 #include "conv_tc_cluster.cuh"
 #include "conv_tc_fused.cuh"
+#include "stem_tc.cuh"
 
 #if defined(WG_TC_TRACE) || defined(WG_TC_DIAG)   // development builds only
 extern "C" int wg2x2_debug_read_diag(unsigned int *host)
@@ -867,3 +868,13 @@ int tc_last_device_status(cudaStream_t st, unsigned int *where)
 }
 
 }  // namespace wg
+
+extern "C" int wg2x2_stem_prepared_floats(void) { return wg::kStWtFloats; }
+
+extern "C" int wg2x2_stem_prepare(const float *W, float *Wp, void *stream) { return wg::stem_prepare(W, Wp, (cudaStream_t)stream); }
+
+extern "C" int wg2x2_stem7x7s2_pool(const float *X, const float *Wp, float *Y, float *Y_relu, const float *relu_scale,
+                                    const float *relu_shift, int B, int H, int W, void *stream)
+{
+    return wg::stem_pool(X, Wp, Y, Y_relu, relu_scale, relu_shift, B, H, W, (cudaStream_t)stream);
+}
