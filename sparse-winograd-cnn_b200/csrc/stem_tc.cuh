@@ -16,7 +16,7 @@
 //   warps 0-3   image rows: global -> shared memory (cp.async, eight rows ahead) -> TF32 (nearest) -> tensor memory
 //   warp 4      MMAs
 //   warps 5-12  two per lane quarter, 32 channels each: vertical maximum of the pool window in registers from convolution row to
-//               convolution row, horizontal maximum by two shuffles, both outputs stored
+//               convolution row, horizontal maximum through shared memory, both outputs stored
 // Bound: 21 MMAs of 32 clocks per convolution row, 68 us for 256 images of 224 x 224 on 148 SMs; the image and both outputs are
 // 257 MB, 40 us.  The warp-level tensor path (mma.sync), whose fragments re-read the staged image for every convolution row,
 // took 490 us.
@@ -32,8 +32,9 @@ constexpr int kStPitch = 240;                   // a staged row of one channel: 
 constexpr int kStWtBytes = 7 * 64 * 128;        // per ky 64 output channels x 32 (24 of them taps), 128-byte swizzle
 constexpr int kStWtFloats = 7 * 64 * kStCols;   // as prepared: [ky][out channel][8 c + kx]
 constexpr int kStImgBytes = kStStages * 3 * kStPitch * 4;
-constexpr int kStSmemBytes = 120 * 1024;        // (asked for in full: one CTA per SM, it takes all of tensor memory)
-static_assert(1024 + kStWtBytes + kStImgBytes + 1024 + 512 <= kStSmemBytes && kStAccCol + 128 <= 512, "carve-up");
+constexpr int kStEPitch = 120;                  // pixels of a channel in a pool buffer: up to 112, then minus infinity
+constexpr int kStSmemBytes = 1024 + kStWtBytes + kStImgBytes + 1024 + 2 * 64 * kStEPitch * 4;   // one CTA per SM, it takes all of tensor memory
+static_assert(kStSmemBytes > 116 * 1024 && kStSmemBytes <= 232448 && kStAccCol + 128 <= 512, "carve-up");
 
 struct StParams {
     const float *X, *Wp;
@@ -79,6 +80,7 @@ __global__ void __launch_bounds__(kStThreads, 1) stem_pool_kernel(const StParams
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t *gen_base = smem_raw + (base - raw);
     float *img_s = reinterpret_cast<float *>(gen_base + kStWtBytes);
+    float *pool_s = reinterpret_cast<float *>(gen_base + kStWtBytes + kStImgBytes + 1024);
     float2 *affine = reinterpret_cast<float2 *>(gen_base + kStWtBytes + kStImgBytes + 512);     // scale and shift of the ReLU output
     const uint32_t bars = base + kStWtBytes + kStImgBytes;
     static_assert((kStWtBytes + kStImgBytes) % 8 == 0, "barriers");
@@ -101,6 +103,7 @@ __global__ void __launch_bounds__(kStThreads, 1) stem_pool_kernel(const StParams
         tmem_relinquish();
     }
     for (int i = tid; i < kStImgBytes / 4; i += kStThreads) img_s[i] = 0.f;       // (the padding columns stay zero)
+    for (int i = tid; i < 2 * 64 * kStEPitch; i += kStThreads) pool_s[i] = -__int_as_float(0x7f800000);   // (columns beyond the row never win)
     wait_for_previous_kernel(kNumSMs);
     for (int i = tid; i < kStWtFloats / 4; i += kStThreads) {       // a row is six 16-byte pieces (the last two of its 128 bytes are not read)
         const int row = i / 6, piece = i - 6 * row;
@@ -240,18 +243,25 @@ __global__ void __launch_bounds__(kStThreads, 1) stem_pool_kernel(const StParams
         }
     } else {
         // ---------------- pool and store ----------------
-        const int quarter = warp & 3, half = (warp - 5) >> 2;
-        const int x = 14 * quarter + (lane >> 1);
-        const bool mine = !(lane & 1) && lane < 28 && x < PW, right = 2 * x + 2 < OW;
+        // The vertical maxima of a pooled row meet in shared memory (two buffers); there every thread takes the horizontal maxima of
+        // four outputs and stores them as 16 bytes of both results.  (Shuffles and stores straight from the lanes, 56 bytes
+        // each, kept the load/store unit busy for 2500 clocks a pooled row: 235 us at 256 images.)
+        const int quarter = warp & 3, half = (warp - 5) >> 2, et = tid - 160;
+        const int px = 28 * quarter + lane;
+        const bool mine = lane < 28 && px < OW;
+        const int nq = (PW + 3) >> 2, items = 64 * nq;
+        const bool vec = (PW & 3) == 0 && ((reinterpret_cast<uintptr_t>(prm.Y) | reinterpret_cast<uintptr_t>(prm.Yr)) & 15u) == 0;
+        const int ch0 = et / nq, xq0 = et - ch0 * nq, dch = 256 / nq, dxq = 256 - dch * nq;     // item et, and the step to item et + 256
         const long long plane = (long long)PH * PW;
         bool ok = true;
-        int r = 0;
-        for (int u = blockIdx.x; u < prm.units && ok; u += gridDim.x) {
+        int r = 0, eb = 0;
+        for (int u = blockIdx.x; u < prm.units; u += gridDim.x) {
             const StUnit t(prm, u);
             float m[32];
             for (int k = 0; k < t.convs; ++k, ++r) {
                 const int buf = r & 1;
-                if (!mbar_wait_warp(accf_bar(buf), (r >> 1) & 1, abort_flag, 0x1900u | buf, prm.spin_limit)) { ok = false; break; }
+                // (a warp that gave up keeps walking: the others count on it at the barrier)
+                if (ok) ok = mbar_wait_warp(accf_bar(buf), (r >> 1) & 1, abort_flag, 0x1900u | buf, prm.spin_limit);
                 tc_fence_after();
                 float v[32];
                 const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(kStAccCol + 64 * buf + 32 * half);
@@ -264,37 +274,53 @@ __global__ void __launch_bounds__(kStThreads, 1) stem_pool_kernel(const StParams
                 // convolution row 2 i + 2 ends pooled row i = pr0 + k / 2 - 1 and begins the next; where it does not exist, row
                 // 2 i + 1 ends it
                 const bool last = k + 1 == t.convs && (k & 1);
-                if (k == 0) {
+                if (k > 0) {
 #pragma unroll
-                    for (int c = 0; c < 32; ++c) m[c] = v[c];
-                    continue;
+                    for (int c = 0; c < 32; ++c) m[c] = fmaxf(m[c], v[c]);
                 }
+                if (k > 0 && (!(k & 1) || last)) {
+                    const int i = t.pr0 + (last ? k >> 1 : (k >> 1) - 1);
+                    float *E = pool_s + eb * (64 * kStEPitch);
+                    eb ^= 1;
+                    if (mine) {
 #pragma unroll
-                for (int c = 0; c < 32; ++c) m[c] = fmaxf(m[c], v[c]);
-                if ((k & 1) && !last) continue;
-                const int i = t.pr0 + (last ? k >> 1 : (k >> 1) - 1);
-                // (all shuffles first, then all stores: a load or a branch per channel between them put the latencies in a row)
+                        for (int c = 0; c < 32; ++c) E[(32 * half + c) * kStEPitch + px] = m[c];
+                    }
+                    asm volatile("bar.sync 2, 256;" ::: "memory");
+                    int ch = ch0, xq = xq0;
+#pragma unroll 1
+                    for (int e = et; e < items; e += 256) {
+                        const float *p = E + ch * kStEPitch + 8 * xq;
+                        const float4 a = *reinterpret_cast<const float4 *>(p), b = *reinterpret_cast<const float4 *>(p + 4);
+                        const float z = p[8];
+                        const float4 o = make_float4(fmaxf(fmaxf(a.x, a.y), a.z), fmaxf(fmaxf(a.z, a.w), b.x), fmaxf(fmaxf(b.x, b.y), b.z),
+                                                     fmaxf(fmaxf(b.z, b.w), z));
+                        const long long at = ((long long)t.b * 64 + ch) * plane + (long long)i * PW + 4 * xq;
+                        const float2 af = affine[ch];
+                        const float4 q = make_float4(fmaxf(fmaf(o.x, af.x, af.y), 0.f), fmaxf(fmaf(o.y, af.x, af.y), 0.f),
+                                                     fmaxf(fmaf(o.z, af.x, af.y), 0.f), fmaxf(fmaf(o.w, af.x, af.y), 0.f));
+                        if (vec) {
+                            *reinterpret_cast<float4 *>(prm.Y + at) = o;
+                            if (prm.Yr) *reinterpret_cast<float4 *>(prm.Yr + at) = q;
+                        } else {
+                            const int nx = PW - 4 * xq;
+                            const float ov[4] = {o.x, o.y, o.z, o.w}, qv[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-                for (int c = 0; c < 32; ++c) {
-                    const float n1 = __shfl_down_sync(0xffffffffu, m[c], 1), n2 = __shfl_down_sync(0xffffffffu, m[c], 2);
-                    m[c] = fmaxf(fmaxf(m[c], n1), right ? n2 : n1);
-                }
-                if (mine) {
-                    float *y = prm.Y + ((long long)t.b * 64 + 32 * half) * plane + (long long)i * PW + x;
-#pragma unroll
-                    for (int c = 0; c < 32; ++c, y += plane) *y = m[c];
-                    if (prm.Yr) {
-                        float *yr = prm.Yr + ((long long)t.b * 64 + 32 * half) * plane + (long long)i * PW + x;
-#pragma unroll
-                        for (int c = 0; c < 32; ++c, yr += plane) {
-                            const float2 af = affine[32 * half + c];
-                            *yr = fmaxf(fmaf(m[c], af.x, af.y), 0.f);
+                            for (int x = 0; x < 4; ++x)
+                                if (x < nx) {
+                                    prm.Y[at + x] = ov[x];
+                                    if (prm.Yr) prm.Yr[at + x] = qv[x];
+                                }
                         }
+                        ch += dch;
+                        xq += dxq;
+                        if (xq >= nq) { xq -= nq; ++ch; }
                     }
                 }
-                __syncwarp();
+                if (!(k & 1)) {
 #pragma unroll
-                for (int c = 0; c < 32; ++c) m[c] = v[c];
+                    for (int c = 0; c < 32; ++c) m[c] = v[c];
+                }
             }
         }
     }
