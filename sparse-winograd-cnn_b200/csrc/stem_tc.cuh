@@ -17,9 +17,11 @@
 //   warp 4      MMAs
 //   warps 5-12  two per lane quarter, 32 channels each: vertical maximum of the pool window in registers from convolution row to
 //               convolution row, horizontal maximum through shared memory, both outputs stored
-// Bound: 21 MMAs of 32 clocks per convolution row, 68 us for 256 images of 224 x 224 on 148 SMs; the image and both outputs are
-// 257 MB, 40 us.  The warp-level tensor path (mma.sync), whose fragments re-read the staged image for every convolution row,
-// took 490 us.
+// Bound: 21 MMAs of 32 clocks per convolution row would be 68 us for 256 images of 224 x 224 on 148 SMs, the image and both outputs
+// (257 MB) 40 us; measured 230 us, with the tensor pipe at 0.31, issue slots at 0.40 and shared memory at 0.45 of active
+// cycles: 7000 instructions per pooled row over thirteen warps, each a chain of barrier, shared memory, tensor memory and barrier.  (A
+// second set of image-row warps, at 96 registers a thread, took 572 us.)  The warp-level tensor path (mma.sync), whose fragments
+// re-read the staged image for every convolution row, took 490 us.
 #pragma once
 
 constexpr int kStThreads = 32 * 13;
