@@ -990,6 +990,88 @@ __global__ void __launch_bounds__(256) out_transform_nchw_kernel(const float *__
     }
 }
 
+// NCHW, enough tiles to fill the GPU and whole blocks of 64 channels: two channels per lane, a tile's sixteen 8-byte loads all in
+// flight before the first is used (the kernel above, short of registers, has four), pixels in shared memory as [pixel][channel].
+// The shortcut arrives there first, by asynchronous copies beside the other CTAs' work; loaded in the copy-out it cost 20 us more.
+// Products + output transform: 128 x 256 x 14 x 14 68.5 -> 64 us, 256 x 256 x 14 x 14 with a shortcut 147 -> 130, 12 x 256 x 56 x 56 with
+// one 141 -> 98.
+constexpr int kOutCB = 64, kOutPitch = kOutCB + 2;
+__global__ void __launch_bounds__(256, 3) out_transform_nchw_pair_kernel(const float *__restrict__ M, float *__restrict__ Y, long long P, int nH,
+                                                                           int nW, int K, int outH, int outW, int R, int nbands, OutExtras ex)
+{
+    after_previous_kernel(M, Y, ex.scale, ex.shift, ex.residual);
+    extern __shared__ __align__(16) float O[];          // [2R rows x outW pixels][kOutPitch]
+    const int band = blockIdx.x % nbands, b = blockIdx.x / nbands, k0 = blockIdx.y * kOutCB;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int th0 = band * R, rows = min(R, nH - th0);
+    const int KV = K >> 1;
+    const long long plane = P * KV;
+    const float2 *const Mv = reinterpret_cast<const float2 *>(M) + (k0 >> 1) + lane;
+    float2 sc = make_float2(1.f, 1.f), sh = make_float2(0.f, 0.f);
+    if (ex.scale) { sc = __ldg(reinterpret_cast<const float2 *>(ex.scale + k0) + lane); sh = __ldg(reinterpret_cast<const float2 *>(ex.shift + k0) + lane); }
+    const int n = (min(2 * (th0 + rows), outH) - 2 * th0) * outW;
+    const long long o0 = (((long long)b * K + k0 + warp) * outH + 2 * th0) * outW, hw8 = 8LL * outH * outW;     // channels warp, warp + 8, ...
+    if (ex.residual) {
+        for (int i = lane; i < n; i += 32) {
+            const uint32_t dst = smem_u32(O + i * kOutPitch + warp);
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + 32u * c), "l"(ex.residual + o0 + c * hw8 + i) : "memory");
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+    }
+#pragma unroll 1
+    for (int q = warp; q < rows * nW; q += 8) {
+        const int br = q / nW, tw = q - br * nW;
+        const float2 *p = Mv + (((long long)b * nH + th0 + br) * nW + tw) * KV;
+        float2 m[16];
+#pragma unroll
+        for (int t = 0; t < 16; ++t) m[t] = __ldg(p + t * plane);
+        float y0[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, y1[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float z0, z1;
+            at_cols(m[4 * i].x, m[4 * i + 1].x, m[4 * i + 2].x, m[4 * i + 3].x, z0, z1);
+            at_rows_accum(i, z0, z1, y0);
+            at_cols(m[4 * i].y, m[4 * i + 1].y, m[4 * i + 2].y, m[4 * i + 3].y, z0, z1);
+            at_rows_accum(i, z0, z1, y1);
+        }
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+                if (2 * tw + e < outW && 2 * (th0 + br) + a < outH) {
+                    float2 *o = reinterpret_cast<float2 *>(O + ((2 * br + a) * outW + 2 * tw + e) * kOutPitch) + lane;
+                    float2 v = make_float2(fmaf(y0[a][e], sc.x, sh.x), fmaf(y1[a][e], sc.y, sh.y));
+                    if (ex.residual) {
+                        const float2 r = *o;
+                        v = ex.res_relu ? make_float2(v.x + fmaxf(r.x, 0.f), v.y + fmaxf(r.y, 0.f)) : make_float2(v.x + r.x, v.y + r.y);
+                    }
+                    *o = v;
+                }
+    }
+    __syncthreads();
+    for (int c = 0; c < 8; ++c) {
+        float *dst = Y + o0 + c * hw8;
+        const float *src = O + warp + 8 * c;
+        for (int i = lane; i < n; i += 32) dst[i] = src[i * kOutPitch];
+    }
+}
+// its band height: least rounds of three CTAs per SM x tiles, 72 KB of shared memory at most; 0: too few CTAs to fill the GPU
+static int out_pair_rows(int B, int K, int nH, int nW, int outW)
+{
+    int best = 0;
+    double t = 1e300;
+    for (int R = 1; R <= nH && (R == 1 || 2 * R * outW * kOutPitch * 4 <= 72 * 1024); ++R) {
+        const long long ctas = (long long)B * cdiv(nH, R) * (K / kOutCB);
+        if (ctas < 3LL * kNumSMs) break;
+        const double u = (double)cdivll(ctas, 3 * kNumSMs) * (R * nW + 8.0);
+        if (u < t) { t = u; best = R; }
+    }
+    return best ? cdiv(nH, cdiv(nH, best)) : 0;
+}
+
 // Row-walk kernel or wide path for P tiles?  Microseconds, from timing both over 16 .. 25088 tiles and 32 .. 512 channels: a
 // row-walk unit (128 tiles x 64 channels) is a serial chain of 16 x C / 32 chunks of 0.27 us and few tiles are few units, while
 // the GEMM spreads the 16 positions over the SMs; the wide path in turn moves the products through memory.  3 x 11 x 11 tiles
@@ -1041,6 +1123,11 @@ int conv_fwd_tc_wide(const float *V, const void *prepared, float *Y, int B, int 
     OutExtras ex{out_scale, out_shift, residual, res_relu};
     if (layout == WG2X2_NHWC) {
         launch(out_transform_nhwc_kernel, dim3((unsigned)cdivll(P * (K / 4), 256)), 256, 0, st, M, Y, P, nH, nW, K, outH, outW, ex);
+    } else if (const int R = K % kOutCB == 0 && K / kOutCB <= 65535 && outW <= 128 ? out_pair_rows(B, K, nH, nW, outW) : 0) {
+        const int nbands = cdiv(nH, R);
+        if ((long long)B * nbands > 0x7fffffffLL) return WG2X2_ERR_UNSUPPORTED;
+        launch(out_transform_nchw_pair_kernel, dim3((unsigned)(B * nbands), K / kOutCB), 256, 2 * R * outW * kOutPitch * sizeof(float), st, M, Y, P, nH, nW,
+               K, outH, outW, R, nbands, ex);
     } else {
         const BandCut cut = cut_bands(nH, nW, (long long)B * cdiv(K, 32), 384 / (2 * outW));
         const int pitch = (2 * cut.R * (cut.nsegs == 1 ? outW : 2 * cut.S)) | 1;

@@ -37,7 +37,7 @@ def test_layer_of_few_tiles(oracle, shape, layout):
 
 # residual_relu where the other paths run: one-kernel NCHW layer, wide path, transform + row-walk kernel
 @pytest.mark.parametrize("shape,layout", [((16, 56, 56, 64, 64), "NCHW"), ((48, 14, 14, 256, 256), "NCHW"), ((48, 14, 14, 256, 256), "NHWC"),
-                                          ((24, 48, 48, 64, 64), "NHWC"), ((40, 49, 49, 32, 64), "NCHW")])
+                                          ((24, 48, 48, 64, 64), "NHWC"), ((40, 49, 49, 32, 64), "NCHW"), ((40, 13, 15, 256, 256), "NCHW")])
 def test_residual_relu_of_the_other_paths(shape, layout):
     import torch
     import wg2x2
@@ -50,3 +50,21 @@ def test_residual_relu_of_the_other_paths(shape, layout):
     kw = dict(relu=True, layout=layout, out_scale=sc, out_shift=sh)
     got = wg2x2.layer_fwd_prepared(x, prepared, K, residual=r, residual_relu=True, **kw)
     assert torch.equal(got, wg2x2.layer_fwd_prepared(x, prepared, K, residual=torch.relu(r), **kw))
+
+
+# the output transform of the wide path, NCHW against NHWC (the same sums in the same order), odd sizes and one band or several
+@pytest.mark.parametrize("shape", [(64, 13, 15, 256, 256), (40, 27, 26, 256, 320), (500, 7, 7, 256, 256), (9, 57, 56, 256, 256)])
+def test_output_transform_layouts_agree(shape):
+    import torch
+    import wg2x2
+    B, H, W, C, K = shape
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    v, prepared = rnd(16, B, (H + 1) // 2, (W + 1) // 2, C), wg2x2.prepare_weights(rnd(16, C, K) / C ** 0.5)
+    sc, sh, r = 1 + 0.2 * rnd(K), 0.3 * rnd(K), rnd(B, H, W, K)
+    for kw in ({}, dict(out_scale=sc, out_shift=sh, residual=r)):
+        a = wg2x2.conv_fwd_prepared(v, prepared, K, H, W, layout="NHWC", **kw)
+        if kw:
+            kw["residual"] = r.permute(0, 3, 1, 2).contiguous()
+        b = wg2x2.conv_fwd_prepared(v, prepared, K, H, W, layout="NCHW", **kw)
+        assert torch.equal(a.permute(0, 3, 1, 2), b)
