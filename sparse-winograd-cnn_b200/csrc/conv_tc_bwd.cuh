@@ -108,68 +108,35 @@ __global__ void __launch_bounds__(256) conv_dm_nchw_kernel(const float *__restri
     }
 }
 
-// The same with four channels per lane: 16-byte plane stores, 512 bytes per warp and store with LC = 32 lanes along
-// the channels (128 per CTA; LC = 16 would be 64 per CTA, the two halves of a warp on two tiles at once -- not used:
-// it measured slower than one channel per lane).  Where the band is the whole image, the CTA's channels are one
-// contiguous run of dY and are staged as such.
-template <int LC>
-__global__ void __launch_bounds__(256, 3) conv_dm_nchw_vec_kernel(const float *__restrict__ dY, float *__restrict__ dM, long long P, int nH,
-                                                                    int nW, int H, int W, int K, int R, int nbands, int pitch)
+// The same for whole blocks of 64 channels and enough tiles to fill the GPU: two channels per lane off an asynchronously staged
+// image, 256 bytes per store off uniform plane addresses.  dM is only ever read by the tensor core, which keeps the upper 19
+// bits: adding half a unit of the last kept place rounds to nearest as cvt.rna.tf32 does, for one integer add.  256 x 512 x 7 x 7 36 ->
+// 28 us (160 MB: 25 at the copy rate), dM and dW of 256 x 256 x 14 x 14 136 -> 128, of 64 x 64 x 56 x 56 128 -> 120.
+__global__ void __launch_bounds__(256, 4) conv_dm_nchw_pair_kernel(const float *__restrict__ dY, float *__restrict__ dM, int nH, int nW, int H,
+                                                                     int W, int K, int R, int nbands, unsigned inv, unsigned plane_bytes)
 {
     after_previous_kernel(dY, dM);
-    constexpr int CB = 4 * LC, QW = 32 / LC;
-    extern __shared__ float S[];
-    const int band = blockIdx.x % nbands;
-    const int b = blockIdx.x / nbands;
-    const int k0 = blockIdx.y * CB;
+    extern __shared__ __align__(16) float S[];
+    const int band = blockIdx.x % nbands, b = blockIdx.x / nbands, k0 = blockIdx.y * kPairCB;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int lc = lane % LC, lq = lane / LC;
-    const int th0 = band * R;
-    const int rows_tile = min(R, nH - th0);
-    const int lo = 2 * th0, hi = min(2 * th0 + 2 * rows_tile, H);
-    const int nfill = (hi - lo) * W;
-    const int nch = min(CB, K - k0);
-    if (nfill == H * W) {
-        const float *src = dY + ((long long)b * K + k0) * nfill;
-        for (int k = threadIdx.x; k < nch * nfill; k += 256) {
-            const int kk = k / nfill;
-            S[kk * pitch + (k - kk * nfill)] = __ldg(src + k);
-        }
-    } else {
-        for (int kk = warp; kk < nch; kk += 8) {
-            const float *src = dY + (((long long)b * K + k0 + kk) * H + lo) * W;
-            float *dst = S + kk * pitch;
-            for (int i = lane; i < nfill; i += 32) dst[i] = __ldg(src + i);
-        }
-    }
+    const int th0 = band * R, rows = min(R, nH - th0), PW = 2 * nW;
+    stage_pairs(dY, S, b, k0, K, H, W, 2 * th0, 0, 2 * rows, PW, inv);
     __syncthreads();
-    if (k0 + 4 * lc >= K) return;
-    const float *Sk = S + 4 * lc * pitch;
-#pragma unroll 1
-    for (int q = warp * QW + lq; q < rows_tile * nW; q += 8 * QW) {
+    char *const Mb = reinterpret_cast<char *>(dM);
+    const int n = rows * nW;
+#pragma unroll 2
+    for (int q = warp; q < n; q += 8) {
         const int tr = q / nW, tw = q - tr * nW;
-        float g[4][2][2];
+        const float2 *p = reinterpret_cast<const float2 *>(S + (2 * tr * PW + 2 * tw) * kPairPitch) + lane;
+        const float2 g00 = p[0], g01 = p[kPairPitch / 2], g10 = p[PW * (kPairPitch / 2)], g11 = p[(PW + 1) * (kPairPitch / 2)];
+        float m0[4][4], m1[4][4];
+        a_g_at(g00.x, g01.x, g10.x, g11.x, m0);
+        a_g_at(g00.y, g01.y, g10.y, g11.y, m1);
+        const unsigned off = (unsigned)((((long long)b * nH + th0) * nW + q) * K + k0 + 2 * lane) * 4u;
 #pragma unroll
-        for (int v = 0; v < 4; ++v)
-#pragma unroll
-            for (int a = 0; a < 2; ++a)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int h = lo + 2 * tr + a, w = 2 * tw + e;
-                    g[v][a][e] = (h < H && w < W) ? Sk[v * pitch + (2 * tr + a) * W + w] : 0.f;
-                }
-        float m0[4][4], m1[4][4], m2[4][4], m3[4][4];
-        a_g_at(g[0][0][0], g[0][0][1], g[0][1][0], g[0][1][1], m0);
-        a_g_at(g[1][0][0], g[1][0][1], g[1][1][0], g[1][1][1], m1);
-        a_g_at(g[2][0][0], g[2][0][1], g[2][1][0], g[2][1][1], m2);
-        a_g_at(g[3][0][0], g[3][0][1], g[3][1][0], g[3][1][1], m3);
-        const long long p = ((long long)b * nH + th0 + tr) * nW + tw;
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                *reinterpret_cast<float4 *>(dM + ((long long)(4 * i + j) * P + p) * K + k0 + 4 * lc) =
-                    make_float4(round_tf32(m0[i][j]), round_tf32(m1[i][j]), round_tf32(m2[i][j]), round_tf32(m3[i][j]));
+        for (int t = 0; t < 16; ++t)
+            *reinterpret_cast<uint2 *>(Mb + (size_t)plane_bytes * t + off) =
+                make_uint2(__float_as_uint(m0[t >> 2][t & 3]) + 0x1000u, __float_as_uint(m1[t >> 2][t & 3]) + 0x1000u);
     }
 }
 
@@ -229,17 +196,12 @@ static int launch_dm(const float *dY, float *dM, int B, int H, int W, int K, int
     const long long P = (long long)B * nH * nW;
     if (layout == WG2X2_NHWC) {
         launch(conv_dm_nhwc_kernel, dim3((unsigned)cdivll(P * (K / 4), 256)), 256, 0, st, dY, dM, P, nH, nW, H, W, K);
-    } else if (K % 4 == 0 && K >= 128 && 2 * nH * W <= 96 && (reinterpret_cast<uintptr_t>(dM) & 15u) == 0 &&
-               (long long)B * cdiv(K, 128) >= 4LL * kNumSMs) {
-        // Four channels per lane, 128 per CTA, where the whole image is one small band and the CTAs fill the GPU
-        // (256 x 512 x 7 x 7: the backward step 193 against 197 us).  With several bands per image, or 64 channels
-        // per CTA, the one-channel-per-lane kernel below measured faster (144 against 161 us at 14 x 14).
-        const int R = nH, nbands = 1;
-        const int pitch = (2 * R * W) | 1;
-        const int smem = 128 * pitch * (int)sizeof(float);
-        if ((long long)B > 0x7fffffffLL || cdiv(K, 128) > 65535) return WG2X2_ERR_UNSUPPORTED;
-        const dim3 grid((unsigned)B, cdiv(K, 128));
-        launch(conv_dm_nchw_vec_kernel<32>, dim3(grid), 256, smem, st, dY, dM, P, nH, nW, H, W, K, R, nbands, pitch);
+    } else if (const int R = K % kPairCB == 0 && K / kPairCB <= 65535 && 2 * nW * 2 * kPairPitch * 4 <= 72 * 1024 && P * K < (1LL << 30) &&
+                                     (reinterpret_cast<uintptr_t>(dM) & 7u) == 0 ? pair_rows(B, K, nH, nW, W, 0) : 0) {
+        const int nbands = cdiv(nH, R);
+        if ((long long)B * nbands > 0x7fffffffLL) return WG2X2_ERR_UNSUPPORTED;
+        launch(conv_dm_nchw_pair_kernel, dim3((unsigned)(B * nbands), K / kPairCB), 256, 2 * R * 2 * nW * kPairPitch * sizeof(float), st, dY, dM, nH, nW, H, W,
+               K, R, nbands, (unsigned)cdiv(1 << 20, 2 * nW), (unsigned)(P * K * 4));
     } else {
         const BandCut cut = cut_bands(nH, nW, (long long)B * cdiv(K, 32), 384 / (2 * W));
         const int pitch = (2 * cut.R * (cut.nsegs == 1 ? W : 2 * cut.S)) | 1;

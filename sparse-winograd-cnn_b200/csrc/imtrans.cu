@@ -287,32 +287,6 @@ __global__ void __launch_bounds__(256) imtrans_fwd_nchw_row_kernel(const float *
 // loads, 16 + 32 additions, 16 stores of 256 bytes off uniform plane addresses, against 32 loads, 128 additions and predicates
 // and 32 stores with one channel per lane.
 // ------------------------------------------------------------------------------------------
-constexpr int kPairCB = 64, kPairPitch = kPairCB + 2;   // channels per CTA; floats of a pixel in shared memory
-
-// Stage rows gy0 .. gy0 + rows - 1 of 64 channels: slot (row, x) receives pixel (gy0 + row, x - 1), PW slots a row, zeros outside
-// the image.  Asynchronous copies, all in flight at once: staged through registers, the few loads that a warp had open at a
-// time were what the kernel waited for (34 against 29 us at 128 x 256 x 14 x 14).  inv = ceil(2^20 / PW).
-__device__ __forceinline__ void stage_pairs(const float *__restrict__ X, float *S, int b, int c0, int C, int H, int W, int gy0, int rows, int PW,
-                                            unsigned inv)
-{
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nch = min(kPairCB, C - c0) - warp;          // channels warp, warp + 8, ... of the block: (nch + 7) / 8 of them exist
-    const long long HW8 = 8LL * H * W;
-    const float *plane = X + ((long long)b * C + c0 + warp) * H * W;
-    for (int i = lane; i < rows * PW; i += 32) {
-        const int r = (int)(((unsigned)i * inv) >> 20), x = i - r * PW - 1, y = gy0 + r;
-        const bool in = y >= 0 && y < H && x >= 0 && x < W;
-        const float *src = plane + (in ? (long long)y * W + x : 0);
-        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(S + i * kPairPitch + warp);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const bool ok = in && 8 * q < nch;
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + 32u * q), "l"(ok ? src + q * HW8 : X), "r"(ok ? 4 : 0) : "memory");
-        }
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-}
-
 template <bool AFFINE, bool RELU, bool SIGNS>
 __global__ void __launch_bounds__(256, 4) imtrans_fwd_nchw_pair_kernel(const float *__restrict__ X, float *__restrict__ V,
                                                                          signs_t *__restrict__ signs, int H, int W, int C,
@@ -324,7 +298,7 @@ __global__ void __launch_bounds__(256, 4) imtrans_fwd_nchw_pair_kernel(const flo
     const int band = blockIdx.x % nbands, b = blockIdx.x / nbands, c0 = blockIdx.y * kPairCB;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int th0 = band * R, rows_tile = min(R, nH - th0), PW = 2 * nW + 2, gy0 = 2 * th0 - 1;
-    stage_pairs(X, S, b, c0, C, H, W, gy0, 2 * rows_tile + 2, PW, inv);
+    stage_pairs(X, S, b, c0, C, H, W, gy0, 1, 2 * rows_tile + 2, PW, inv);
     __syncthreads();
     if (c0 + 2 * lane >= C) return;
     // the warp's share of the band's tiles, in row order
@@ -385,22 +359,6 @@ __global__ void __launch_bounds__(256, 4) imtrans_fwd_nchw_pair_kernel(const flo
     }
 }
 
-// The band height of that kernel: least work of the busiest SM (a tile is 146 issue slots, a staged pixel 10 per 64 channels, and
-// a CTA costs something of its own), shared memory for three CTAs per SM.  0: too few CTAs to fill the GPU.
-inline int pair_rows(int B, int C, int nH, int nW, int W)
-{
-    const long long per_band = (long long)B * cdiv(C, kPairCB);
-    int best = 0;
-    double t = 1e300;
-    for (int R = 1; R <= nH; ++R) {
-        if (R > 1 && (2 * R + 2) * (2 * nW + 2) * kPairPitch * 4 > 72 * 1024) break;
-        const long long ctas = per_band * cdiv(nH, R);
-        if (ctas < 2LL * kNumSMs) continue;
-        const double u = (double)cdivll(ctas, kNumSMs) * ((2.0 * R + 2) * W * 10 + (double)R * nW * 146 + 1500);
-        if (u < t) { t = u; best = R; }
-    }
-    return best ? cdiv(nH, cdiv(nH, best)) : 0;
-}
 
 // ------------------------------------------------------------------------------------------
 // Backward gather for one 2x2 output block (bh,bw) and VEC channels.
@@ -971,7 +929,7 @@ int imtrans_fwd(const float *X, float *V, void *signs_out, int B, int H, int W, 
         // blocks of 64 channels are full, the bands fill the GPU, and a plane is within 32-bit reach.
         const bool pair_ok = C % kPairCB == 0 && W <= 28 && ((reinterpret_cast<uintptr_t>(V) | reinterpret_cast<uintptr_t>(scale) |
                              reinterpret_cast<uintptr_t>(shift)) & 7u) == 0 && (long long)B * nH * nW * C < (1LL << 30) && C / kPairCB <= 65535;
-        const int R = pair_ok ? pair_rows(B, C, nH, nW, W) : 0;
+        const int R = pair_ok ? pair_rows(B, C, nH, nW, W, 2) : 0;
         if (R) {
             const int nbands = cdiv(nH, R), smem = (2 * R + 2) * (2 * nW + 2) * kPairPitch * (int)sizeof(float);
             if ((long long)B * nbands > 0x7fffffffLL) return WG2X2_ERR_UNSUPPORTED;

@@ -126,6 +126,50 @@ __device__ __forceinline__ void stage_channels(const float *__restrict__ plane0,
     }
 }
 
+// ---- 64 channels of an NCHW image in shared memory as [pixel][channel], for kernels with two channels per lane ----
+constexpr int kPairCB = 64, kPairPitch = kPairCB + 2;   // channels per CTA; floats of a pixel in shared memory
+
+// Stage rows gy0 .. gy0 + rows - 1 of 64 channels: slot (row, x) receives pixel (gy0 + row, x - gx0), PW slots a row, zeros outside
+// the image.  Asynchronous copies, all in flight at once: staged through registers, the few loads that a warp had open at a
+// time were what the kernel waited for (34 against 29 us at 128 x 256 x 14 x 14).  inv = ceil(2^20 / PW).
+__device__ __forceinline__ void stage_pairs(const float *__restrict__ X, float *S, int b, int c0, int C, int H, int W, int gy0, int gx0, int rows, int PW,
+                                            unsigned inv)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nch = min(kPairCB, C - c0) - warp;          // channels warp, warp + 8, ... of the block: (nch + 7) / 8 of them exist
+    const long long HW8 = 8LL * H * W;
+    const float *plane = X + ((long long)b * C + c0 + warp) * H * W;
+    for (int i = lane; i < rows * PW; i += 32) {
+        const int r = (int)(((unsigned)i * inv) >> 20), x = i - r * PW - gx0, y = gy0 + r;
+        const bool in = y >= 0 && y < H && x >= 0 && x < W;
+        const float *src = plane + (in ? (long long)y * W + x : 0);
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(S + i * kPairPitch + warp);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const bool ok = in && 8 * q < nch;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + 32u * q), "l"(ok ? src + q * HW8 : X), "r"(ok ? 4 : 0) : "memory");
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
+// The band height of the kernels that stage so (bands of 2 R + extra rows): least work of the busiest SM (a tile is 146 issue slots, a staged pixel 10 per 64 channels, and
+// a CTA costs something of its own), shared memory for three CTAs per SM.  0: too few CTAs to fill the GPU.
+inline int pair_rows(int B, int C, int nH, int nW, int W, int extra)
+{
+    const long long per_band = (long long)B * cdiv(C, kPairCB);
+    int best = 0;
+    double t = 1e300;
+    for (int R = 1; R <= nH; ++R) {
+        if (R > 1 && (2 * R + extra) * (2 * nW + extra) * kPairPitch * 4 > 72 * 1024) break;
+        const long long ctas = per_band * cdiv(nH, R);
+        if (ctas < 2LL * kNumSMs) continue;
+        const double u = (double)cdivll(ctas, kNumSMs) * ((2.0 * R + extra) * W * 10 + (double)R * nW * 146 + 1500);
+        if (u < t) { t = u; best = R; }
+    }
+    return best ? cdiv(nH, cdiv(nH, best)) : 0;
+}
+
 inline int launch_status()
 {
     return cudaGetLastError() == cudaSuccess ? WG2X2_OK : WG2X2_ERR_LAUNCH;
