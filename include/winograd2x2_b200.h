@@ -185,6 +185,14 @@ int wg2x2_layer_fwd(const float *X, const float *Wt, float *Y, float *V_out, int
 size_t wg2x2_layer_fwd_workspace_bytes(int B, int H, int W, int C, int K, int math, int keep_V);
 
 /*
+ * 1 x 1 convolution, NCHW: Y[b][k][p] = sum_c W[k][c] X[b][c][p], p < HW, on the tensor cores (TF32; W (K,C), 16-byte aligned, is
+ * expected rounded to TF32).  C a multiple of 4, at most 256, else WG2X2_ERR_UNSUPPORTED.  Made for few pixels:
+ * wg2x2_conv1x1_preferred says where it is worth taking.
+ */
+int wg2x2_conv1x1(const float *X, const float *W, float *Y, int B, int C, int K, int HW, void *stream);
+int wg2x2_conv1x1_preferred(int B, int C, int K, int HW);
+
+/*
  * out[p] = mean over the n values of plane p of relu(X): the ReLU and global average pool in front of the classifier
  * (ResNet-18-var/imagenet-resnet-transWino-prune.py:216-219).  X: planes x n floats.
  */

@@ -589,6 +589,26 @@ PyObject *py_residual_block(WG_ARGS)
     END_HANDLE_TH_ERRORS
 }
 
+// x (B,C,H,W), w (K,C) rounded to TF32 -> (B,K,H,W), or None where the kernel is not worth taking
+PyObject *py_conv1x1(WG_ARGS)
+{
+    HANDLE_TH_ERRORS
+    want(n, 2);
+    const Tensor x = arg(a[0], "x"), w = arg(a[1], "w");
+    const Img d = img_of(x, WG2X2_NCHW, "x");
+    if (w.dim() < 2 || w.numel() != w.size(0) * d.C || w.size(1) != d.C) value_error("w must be (K, C)");
+    if (!wg2x2_conv1x1_preferred(d.B, d.C, w.size(0), (int)(d.H * d.W)) || (reinterpret_cast<uintptr_t>(w.data_ptr()) & 15u)) Py_RETURN_NONE;
+    Tensor y;
+    {
+        WG_NOGIL;
+        OnDevice on(x);
+        y = new_float({d.B, w.size(0), d.H, d.W}, x);
+        check(wg2x2_conv1x1(cptr(x), cptr(w), ptr(y), d.B, d.C, w.size(0), (int)(d.H * d.W), on.stream), "wg2x2_conv1x1");
+    }
+    return THPVariable_Wrap(y);
+    END_HANDLE_TH_ERRORS
+}
+
 // x (B,C,H,W) -> (B,C): mean of relu(x) over the pixels
 PyObject *py_relu_mean(PyObject *, PyObject *o)
 {
@@ -739,6 +759,7 @@ PyMethodDef methods[] = {
     WG_FN("layer_fwd_prepared", py_layer_fwd_prepared),
     WG_FN("layer_fwd_fused", py_layer_fwd_fused),
     WG_FN("residual_block", py_residual_block),
+    WG_FN("conv1x1", py_conv1x1),
     {"relu_mean", py_relu_mean, METH_O, nullptr},
     WG_FN("maxpool", py_maxpool),
     WG_FN("stem_pool", py_stem_pool),

@@ -837,6 +837,7 @@ void dw_reduce_launch(const float *partial, const float *mask, float *dW, long l
 #include "conv_tc_cluster.cuh"
 #include "conv_tc_fused.cuh"
 #include "stem_tc.cuh"
+#include "conv1x1_tc.cuh"
 
 #if defined(WG_TC_TRACE) || defined(WG_TC_DIAG)   // development builds only
 extern "C" int wg2x2_debug_read_diag(unsigned int *host)
@@ -868,6 +869,15 @@ int tc_last_device_status(cudaStream_t st, unsigned int *where)
 }
 
 }  // namespace wg
+
+extern "C" int wg2x2_conv1x1_preferred(int B, int C, int K, int HW)
+{
+    return (B > 0 && C > 0 && K > 0 && HW > 0 && wg::conv1x1_preferred(B, C, K, HW)) ? 1 : 0;
+}
+extern "C" int wg2x2_conv1x1(const float *X, const float *W, float *Y, int B, int C, int K, int HW, void *stream)
+{
+    return wg::conv1x1(X, W, Y, B, C, K, HW, (cudaStream_t)stream);
+}
 
 extern "C" int wg2x2_stem_prepared_floats(void) { return wg::kStWtFloats; }
 

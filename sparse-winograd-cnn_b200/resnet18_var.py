@@ -191,7 +191,10 @@ class ResNet18Var(torch.nn.Module):
             else:   # the BatchNorm after the 1x1 shortcut folds into its weights (once) and bias
                 if getattr(blk_a, "_short_folded", None) is None or blk_a._short_folded.device != blk_a.short.device:
                     blk_a._short_folded = (blk_a.short * blk_a["bn1"].scale.view(-1, 1, 1, 1)).detach()
-                main = F.conv2d(main, blk_a._short_folded)      # its shift is added by the block's last kernel
+                    blk_a._short_tf32 = wg2x2.round_tf32(blk_a._short_folded)
+                # (its shift is added by the block's last kernel)
+                y = wg2x2.conv1x1(main, blk_a._short_tf32) if own_pool and self.math == "tf32" and main.is_contiguous() else None
+                main = F.conv2d(main, blk_a._short_folded) if y is None else y
             l = self._block(blk_a, l, main, reference, main_bias=None if (reference or not self.fused) else blk_a["bn1"].shift)
             l = self._block(blk_b, l, None, reference)
             l_relu = None

@@ -58,6 +58,8 @@ _SIGS = {
     "wg2x2_layer_fwd_prepared_workspace_bytes": (_z, [_i, _i, _i, _i, _i]),
     "wg2x2_layer_fwd_prepared_ex": (_i, [_p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _p, _p, _p, _i, _p, _z, _p]),
     "wg2x2_layer_fwd_prepared_scratch": (None, [_i, _i, _i, _i, _i, _i, _i, ctypes.POINTER(_z), ctypes.POINTER(_z)]),
+    "wg2x2_conv1x1": (_i, [_p, _p, _p, _i, _i, _i, _i, _p]),
+    "wg2x2_conv1x1_preferred": (_i, [_i, _i, _i, _i]),
     "wg2x2_relu_mean": (_i, [_p, _p, ctypes.c_longlong, _i, _p]),
     "wg2x2_layer_fwd_fused": (_i, [_p, _p, _p, _i, _i, _i, _i, _i, _i, _p, _p, _p, _p]),
     "wg2x2_layer_fwd_fused_affine": (_i, [_p, _p, _p, _i, _i, _i, _i, _i, _i, _p, _p, _p, _p, _p, _p]),

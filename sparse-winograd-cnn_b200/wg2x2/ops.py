@@ -119,6 +119,17 @@ def residual_block(x, shortcut, prepared_a, bn_a, prepared_b, bn_b, bn_out, K, l
                                   _LAYOUTS[layout])
 
 
+def conv1x1(x, w):
+    """1x1 convolution of x (B,C,H,W) with w (K,C,1,1), whose values have to be rounded to TF32 (round_tf32): (B,K,H,W), or None
+    where the library's convolution is the better choice (many pixels; more than 256 channels)."""
+    return _native.conv1x1(x, w)
+
+
+def round_tf32(t):
+    """t rounded to TF32, nearest with ties away from zero."""
+    return ((t.contiguous().view(torch.int32) + 0x1000) & ~0x1FFF).view(torch.float32)
+
+
 def relu_mean(x):
     """x (B,C,H,W) -> (B,C): the mean of relu(x) over the pixels."""
     return _native.relu_mean(x)

@@ -132,3 +132,18 @@ def test_stem_kernel_rejects_other_sizes():
     x = torch.zeros((1, 3, 30, 32), device="cuda")
     with pytest.raises(ValueError):
         wg2x2.stem7x7s2_pool(x, wg2x2.stem_prepare(torch.zeros((64, 3, 7, 7), device="cuda")))
+
+
+@pytest.mark.parametrize("shape", [(1, 4, 1, 1, 1), (1, 64, 64, 56, 56), (3, 36, 70, 7, 7), (1, 256, 512, 7, 7), (2, 128, 256, 14, 14), (5, 100, 64, 9, 13)])
+def test_conv1x1_kernel(shape):
+    """The shortcut's 1x1 convolution against float64 of the TF32-rounded operands: only the FP32 accumulation order differs."""
+    import wg2x2
+    B, C, K, H, W = shape
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    x = torch.randn((B, C, H, W), device="cuda", generator=g)
+    w = wg2x2.round_tf32(torch.randn((K, C, 1, 1), device="cuda", generator=g))
+    want = torch.einsum("kc,bchw->bkhw", w.view(K, C).double(), _tf32(x).double())
+    got = wg2x2.conv1x1(x, w)
+    assert got.shape == want.shape and float((got - want).abs().max()) <= 2e-5 * float(want.abs().max())
+    assert wg2x2.conv1x1(torch.zeros((64, 64, 56, 56), device="cuda"), torch.zeros((64, 64, 1, 1), device="cuda")) is None
+    assert wg2x2.last_device_status()[0] == 0
