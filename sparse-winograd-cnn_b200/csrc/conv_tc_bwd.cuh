@@ -18,6 +18,9 @@ __device__ __forceinline__ float round_tf32(float x)
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(x));
     return __uint_as_float(u);
 }
+// The bits of x for an operand that only the tensor core reads, which keeps the upper 19: half a unit of the last kept place added
+// rounds to nearest as the conversion does, for an integer add.  NaN is set apart: CUDA's own, 0x7fffffff, would wrap to -0.
+__device__ __forceinline__ uint32_t tf32_operand(float x) { return x == x ? __float_as_uint(x) + 0x1000u : 0x7fffffffu; }
 
 // NHWC: one thread = one tile x 4 output channels
 __global__ void __launch_bounds__(256) conv_dm_nhwc_kernel(const float *__restrict__ dY, float *__restrict__ dM, long long P, int nH,
@@ -109,9 +112,8 @@ __global__ void __launch_bounds__(256) conv_dm_nchw_kernel(const float *__restri
 }
 
 // The same for whole blocks of 64 channels and enough tiles to fill the GPU: two channels per lane off an asynchronously staged
-// image, 256 bytes per store off uniform plane addresses.  dM is only ever read by the tensor core, which keeps the upper 19
-// bits: adding half a unit of the last kept place rounds to nearest as cvt.rna.tf32 does, for one integer add.  256 x 512 x 7 x 7 36 ->
-// 28 us (160 MB: 25 at the copy rate), dM and dW of 256 x 256 x 14 x 14 136 -> 128, of 64 x 64 x 56 x 56 128 -> 120.
+// image, 256 bytes per store off uniform plane addresses.  dM is only ever read by the tensor core: tf32_operand.  256 x 512 x 7 x 7
+// 36 -> 28 us (160 MB: 25 at the copy rate), dM and dW of 256 x 256 x 14 x 14 136 -> 128, of 64 x 64 x 56 x 56 128 -> 120.
 __global__ void __launch_bounds__(256, 4) conv_dm_nchw_pair_kernel(const float *__restrict__ dY, float *__restrict__ dM, int nH, int nW, int H,
                                                                      int W, int K, int R, int nbands, unsigned inv, unsigned plane_bytes)
 {
@@ -136,7 +138,7 @@ __global__ void __launch_bounds__(256, 4) conv_dm_nchw_pair_kernel(const float *
 #pragma unroll
         for (int t = 0; t < 16; ++t)
             *reinterpret_cast<uint2 *>(Mb + (size_t)plane_bytes * t + off) =
-                make_uint2(__float_as_uint(m0[t >> 2][t & 3]) + 0x1000u, __float_as_uint(m1[t >> 2][t & 3]) + 0x1000u);
+                make_uint2(tf32_operand(m0[t >> 2][t & 3]), tf32_operand(m1[t >> 2][t & 3]));
     }
 }
 

@@ -1,0 +1,44 @@
+"""NaN and infinity through the kernels that round operands to TF32 themselves: where an operand is not finite the result is not, as
+with cvt.rna.tf32, which the other kernels of the same step use."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+NANS = [0x7FFFFFFF, -1, 0x7FC00000, 0xFFC00000 - (1 << 32), 0x7F800001]     # CUDA's, all ones, the x86 pair, a payload in the low bits only
+
+
+def _put(t, at, bits):
+    t.view(torch.int32)[at] = bits
+
+
+def _dm(dY):
+    """A dY A^T in float64 by the additions of the kernels (a zero coefficient is no operand): (16, B, nH, nW, K) of dY (B, K, H, W)."""
+    B, K, H, W = dY.shape
+    g = F.pad(dY.double(), (0, W % 2, 0, H % 2)).reshape(B, K, (H + 1) // 2, 2, (W + 1) // 2, 2)
+    ends = lambda a, b: [a, a + b, a - b, -b]
+    return torch.stack([m for u0, u1 in zip(ends(g[:, :, :, 0, :, 0], g[:, :, :, 1, :, 0]), ends(g[:, :, :, 0, :, 1], g[:, :, :, 1, :, 1]))
+                        for m in ends(u0, u1)]).permute(0, 1, 3, 4, 2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("layout", ["NCHW", "NHWC"])
+@pytest.mark.parametrize("shape", [(44, 32, 64, 14, 14), (90, 32, 128, 7, 7), (2, 32, 64, 14, 14)])      # two channels per lane twice, segments
+def test_dy_reaches_the_gradients(shape, layout):
+    import wg2x2
+    B, C, K, H, W = shape
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    v, w, clean = rnd(16, B, (H + 1) // 2, (W + 1) // 2, C), rnd(16, C, K), rnd(B, K, H, W)
+    cases = [{(1, 3 + i, 5, 6 - i): n} for i, n in enumerate(NANS)]
+    cases.append({(0, 2, 2, 4): 0x7F800000, (0, 2, 3, 4): 0x7F800000})              # inf - inf inside a tile
+    cases.append({(1, 5, H - 1, W - 1): 0xFF800000 - (1 << 32)})
+    for case in cases:
+        dy = clean.clone()
+        for at, bits in case.items():
+            _put(dy, at, bits)
+        dm = _dm(dy)
+        dv, dw = wg2x2.conv_bwd(v, w, dy if layout == "NCHW" else dy.permute(0, 2, 3, 1).contiguous(), layout=layout, math="tf32")
+        assert not dm.isfinite().all()
+        assert torch.equal(~dv.isfinite(), (~dm.isfinite()).any(-1, keepdim=True).expand_as(dv))
+        assert torch.equal(~dw.isfinite(), (~dm.isfinite()).any(3).any(2).any(1)[:, None, :].expand_as(dw))
+        assert dv[dm.isnan().any(-1)].isnan().all() and dw.transpose(1, 2)[dm.isnan().any(3).any(2).any(1)].isnan().all()
