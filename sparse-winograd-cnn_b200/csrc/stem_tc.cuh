@@ -18,10 +18,10 @@
 //   warps 5-12  two per lane quarter, 32 channels each: vertical maximum of the pool window in registers from convolution row to
 //               convolution row, horizontal maximum through shared memory, both outputs stored
 // Bound: 21 MMAs of 32 clocks per convolution row would be 68 us for 256 images of 224 x 224 on 148 SMs, the image and both outputs
-// (257 MB) 40 us; measured 230 us, with the tensor pipe at 0.31, issue slots at 0.40 and shared memory at 0.45 of active
+// (257 MB) 40 us; measured 234 us, with the tensor pipe at 0.31, issue slots at 0.40 and shared memory at 0.45 of active
 // cycles: 7000 instructions per pooled row over thirteen warps, each a chain of barrier, shared memory, tensor memory and barrier.  (A
 // second set of image-row warps, at 96 registers a thread, took 572 us.)  The warp-level tensor path (mma.sync), whose fragments
-// re-read the staged image for every convolution row, took 490 us.
+// re-read the staged image for every convolution row, took 490 us.  (6 of the 234 us are the comparisons that set NaN apart.)
 #pragma once
 
 constexpr int kStThreads = 32 * 13;
@@ -34,7 +34,7 @@ constexpr int kStPitch = 240;                   // a staged row of one channel: 
 constexpr int kStWtBytes = 7 * 64 * 128;        // per ky 64 output channels x 32 (24 of them taps), 128-byte swizzle
 constexpr int kStWtFloats = 7 * 64 * kStCols;   // as prepared: [ky][out channel][8 c + kx]
 constexpr int kStImgBytes = kStStages * 3 * kStPitch * 4;
-constexpr int kStEPitch = 120;                  // pixels of a channel in a pool buffer: up to 112, then minus infinity
+constexpr int kStEPitch = 120;                  // pixels of a channel in a pool buffer: up to 112, then NaN
 constexpr int kStSmemBytes = 1024 + kStWtBytes + kStImgBytes + 1024 + 2 * 64 * kStEPitch * 4;   // one CTA per SM, it takes all of tensor memory
 static_assert(kStSmemBytes > 116 * 1024 && kStSmemBytes <= 232448 && kStAccCol + 128 <= 512, "carve-up");
 
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(kStThreads, 1) stem_pool_kernel(const StParams
         tmem_relinquish();
     }
     for (int i = tid; i < kStImgBytes / 4; i += kStThreads) img_s[i] = 0.f;       // (the padding columns stay zero)
-    for (int i = tid; i < 2 * 64 * kStEPitch; i += kStThreads) pool_s[i] = -__int_as_float(0x7f800000);   // (columns beyond the row never win)
+    for (int i = tid; i < 2 * 64 * kStEPitch; i += kStThreads) pool_s[i] = __int_as_float(0x7fffffff);   // (columns beyond the row: fmaxf takes the other value)
     wait_for_previous_kernel(kNumSMs);
     for (int i = tid; i < kStWtFloats / 4; i += kStThreads) {       // a row is six 16-byte pieces (the last two of its 128 bytes are not read)
         const int row = i / 6, piece = i - 6 * row;
@@ -185,8 +185,8 @@ __global__ void __launch_bounds__(kStThreads, 1) stem_pool_kernel(const StParams
 #pragma unroll
                         for (int h = 0; h < 4; ++h) {
                             const float2 f = in ? *reinterpret_cast<const float2 *>(p + c * kStPitch + 2 * h) : make_float2(0.f, 0.f);
-                            v[e][c][2 * h] = __float_as_uint(f.x) + 0x1000u;       // half a unit of the last place that the MMA keeps:
-                            v[e][c][2 * h + 1] = __float_as_uint(f.y) + 0x1000u;   // rounds to nearest, as cvt.rna.tf32 does
+                            v[e][c][2 * h] = tf32_operand(f.x);
+                            v[e][c][2 * h + 1] = tf32_operand(f.y);
                         }
                 }
                 // (a warp that gave up keeps walking: the others count on it at the barrier)

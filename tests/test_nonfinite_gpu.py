@@ -42,3 +42,30 @@ def test_dy_reaches_the_gradients(shape, layout):
         assert torch.equal(~dv.isfinite(), (~dm.isfinite()).any(-1, keepdim=True).expand_as(dv))
         assert torch.equal(~dw.isfinite(), (~dm.isfinite()).any(3).any(2).any(1)[:, None, :].expand_as(dw))
         assert dv[dm.isnan().any(-1)].isnan().all() and dw.transpose(1, 2)[dm.isnan().any(3).any(2).any(1)].isnan().all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(1, 64, 48), (3, 224, 224)])
+def test_image_reaches_the_stem(shape):
+    """The kernel's eighth tap has weight zero, so a NaN reaches the outputs of 7 x 8 taps; the pool drops NaN beside a number."""
+    import wg2x2
+    from resnet18_var import _same_pool
+    B, H, W = shape
+    g = torch.Generator(device="cuda").manual_seed(B + H + W)
+    x, w = torch.randn((B, 3, H, W), device="cuda", generator=g), torch.randn((64, 3, 7, 7), device="cuda", generator=g) * 0.1
+    prep = wg2x2.stem_prepare(w)
+    for i, bits in enumerate(NANS):
+        bad = x.clone()
+        for c, y, z in ((i % 3, 10 + i, 11), (1, 0, 0), (2, H - 1, W - 1 - i)):
+            bad[B - 1, c, y, z] = 0.0
+        zero = bad.clone()
+        for c, y, z in ((i % 3, 10 + i, 11), (1, 0, 0), (2, H - 1, W - 1 - i)):
+            _put(bad, (B - 1, c, y, z), bits)
+        nan = F.conv2d(F.pad(bad.isnan().float(), (2, 4, 2, 3)), torch.ones((1, 3, 7, 8), device="cuda"), stride=2) > 0.5
+        conv = F.conv2d(F.pad(wg2x2.round_tf32(zero).double(), (2, 3, 2, 3)), wg2x2.round_tf32(w).double(), stride=2).float()
+        want = _same_pool(conv.masked_fill(nan, float("-inf")))
+        lost = torch.isneginf(want)
+        assert lost.any()
+        got = wg2x2.stem7x7s2_pool(bad, prep)
+        assert torch.equal(got.isnan(), lost)
+        assert float((got - want)[~lost].abs().max()) <= 2e-5 * float(want[~lost].abs().max())       # FP32 sums in another order
