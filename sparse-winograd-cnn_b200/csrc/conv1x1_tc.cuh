@@ -70,8 +70,8 @@ __global__ void __launch_bounds__(kC1Threads) conv1x1_tc_kernel(const __grid_con
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
                 const uint32_t dst = base + cc * kC1StageBytes + row * 128 + (((2 * g + half) ^ (row & 7)) << 4);
-                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(__float_as_uint(v[g][0]) + 0x1000u), "r"(__float_as_uint(v[g][1]) + 0x1000u),
-                             "r"(__float_as_uint(v[g][2]) + 0x1000u), "r"(__float_as_uint(v[g][3]) + 0x1000u) : "memory");
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(tf32_operand(v[g][0])), "r"(tf32_operand(v[g][1])),
+                             "r"(tf32_operand(v[g][2])), "r"(tf32_operand(v[g][3])) : "memory");
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();

@@ -126,8 +126,9 @@ def conv1x1(x, w):
 
 
 def round_tf32(t):
-    """t rounded to TF32, nearest with ties away from zero."""
-    return ((t.contiguous().view(torch.int32) + 0x1000) & ~0x1FFF).view(torch.float32)
+    """t rounded to TF32, nearest with ties away from zero; NaN stays NaN."""
+    t = t.contiguous()
+    return torch.where(t.isnan(), t.new_tensor(float("nan")), ((t.view(torch.int32) + 0x1000) & ~0x1FFF).view(torch.float32))
 
 
 def relu_mean(x):

@@ -69,3 +69,31 @@ def test_image_reaches_the_stem(shape):
         got = wg2x2.stem7x7s2_pool(bad, prep)
         assert torch.equal(got.isnan(), lost)
         assert float((got - want)[~lost].abs().max()) <= 2e-5 * float(want[~lost].abs().max())       # FP32 sums in another order
+
+
+@pytest.mark.gpu
+def test_image_and_weights_reach_the_1x1_convolution():
+    import wg2x2
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x, w = torch.randn((2, 100, 9, 13), device="cuda", generator=g), torch.randn((70, 100, 1, 1), device="cuda", generator=g)
+    for bits in NANS + [0x7F800000, 0xFF800000 - (1 << 32)]:
+        bad, wbad = x.clone(), w.clone()
+        _put(bad, (1, 37, 4, 5), bits)
+        _put(wbad, (69, 2, 0, 0), bits)
+        y, clean = wg2x2.conv1x1(bad, wg2x2.round_tf32(w)), wg2x2.conv1x1(x, wg2x2.round_tf32(w))
+        hit = torch.zeros_like(y, dtype=torch.bool)
+        hit[1, :, 4, 5] = True
+        assert torch.equal(~y.isfinite(), hit) and torch.equal(y[~hit], clean[~hit])
+        y = wg2x2.conv1x1(x, wg2x2.round_tf32(wbad))
+        assert not y[:, 69].isfinite().any() and torch.equal(y[:, :69], clean[:, :69])
+
+
+def test_round_tf32_values():
+    """Nearest, ties away from zero, on any device; infinities stay, NaN stays NaN, what rounds beyond the largest value is infinite."""
+    import wg2x2
+    f = lambda *bits: torch.tensor([b - (1 << 32) if b >= 1 << 31 else b for b in bits], dtype=torch.int64).to(torch.int32).view(torch.float32)
+    x = f(0x3F800FFF, 0x3F801000, 0xBF801000, 0x3F803000, 0x7F7FFFFF, 0x7F800000, 0xFF800000, 0x00000000, 0x80000000, 0x00001000)
+    want = f(0x3F800000, 0x3F802000, 0xBF802000, 0x3F804000, 0x7F800000, 0x7F800000, 0xFF800000, 0x00000000, 0x80000000, 0x00002000)
+    assert torch.equal(wg2x2.round_tf32(x).view(torch.int32), want.view(torch.int32))
+    nans = f(*(n & 0xFFFFFFFF for n in NANS))
+    assert wg2x2.round_tf32(nans).isnan().all()
