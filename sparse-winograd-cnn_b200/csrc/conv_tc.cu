@@ -494,7 +494,7 @@ conv_fwd_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
                                 off[r] = __shfl_sync(0xffffffffu, my_off, 4 * r + (lane >> 3));
                                 rs[r] = make_float4(0.f, 0.f, 0.f, 0.f);
                                 if (EXTRAS && prm.residual && off[r] >= 0) rs[r] = __ldg(reinterpret_cast<const float4 *>(prm.residual + off[r]) + (lane & 7));
-                                if (EXTRAS && prm.res_relu) rs[r] = make_float4(fmaxf(rs[r].x, 0.f), fmaxf(rs[r].y, 0.f), fmaxf(rs[r].z, 0.f), fmaxf(rs[r].w, 0.f));
+                                if (EXTRAS && prm.res_relu) rs[r] = relu_nan(rs[r]);
                             }
 #pragma unroll
                             for (int r = 0; r < 8; ++r) {
@@ -523,7 +523,7 @@ conv_fwd_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
                                 if (kbase + c < prm.K) {
                                     float v = y[2 * a + e][c];
                                     if (EXTRAS && prm.out_scale) v = fmaf(v, __ldg(prm.out_scale + kbase + c), __ldg(prm.out_shift + kbase + c));
-                                    if (EXTRAS && prm.residual) v += prm.res_relu ? fmaxf(__ldg(prm.residual + o + c), 0.f) : __ldg(prm.residual + o + c);
+                                    if (EXTRAS && prm.residual) v += prm.res_relu ? relu_nan(__ldg(prm.residual + o + c)) : __ldg(prm.residual + o + c);
                                     prm.Y[o + c] = v;
                                 }
                         }
@@ -549,7 +549,7 @@ conv_fwd_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_consta
                                 const float *rp = prm.residual + o0 + (cg + c) * cstride;
                                 if (pair) rs[c] = __ldg(reinterpret_cast<const float2 *>(rp));
                                 else { rs[c].x = __ldg(rp); if (2 * tw + 1 < prm.outW) rs[c].y = __ldg(rp + 1); }
-                                if (prm.res_relu) rs[c] = make_float2(fmaxf(rs[c].x, 0.f), fmaxf(rs[c].y, 0.f));
+                                if (prm.res_relu) rs[c] = make_float2(relu_nan(rs[c].x), relu_nan(rs[c].y));
                             }
                         }
 #pragma unroll

@@ -843,7 +843,7 @@ int conv_bwd_tc(const float *V, const float *Wt, const float *dY, const float *m
 struct OutExtras {
     const float *scale, *shift, *residual;
     int res_relu;            // the residual passes through a ReLU first
-    __device__ __forceinline__ float shortcut(long long o) const { const float r = __ldg(residual + o); return res_relu ? fmaxf(r, 0.f) : r; }
+    __device__ __forceinline__ float shortcut(long long o) const { const float r = __ldg(residual + o); return res_relu ? relu_nan(r) : r; }
 };
 
 // NHWC: one thread = one tile x 4 output channels
@@ -885,7 +885,7 @@ __global__ void __launch_bounds__(256) out_transform_nhwc_kernel(const float *__
             float4 v = y[a][e];
             if (ex.scale) { v.x = fmaf(v.x, sc.x, sh.x); v.y = fmaf(v.y, sc.y, sh.y); v.z = fmaf(v.z, sc.z, sh.z); v.w = fmaf(v.w, sc.w, sh.w); }
             if (ex.residual) { float4 r = __ldg(reinterpret_cast<const float4 *>(ex.residual) + o);
-                               if (ex.res_relu) r = make_float4(fmaxf(r.x, 0.f), fmaxf(r.y, 0.f), fmaxf(r.z, 0.f), fmaxf(r.w, 0.f));
+                               if (ex.res_relu) r = relu_nan(r);
                                v = v + r; }
             reinterpret_cast<float4 *>(Y)[o] = v;
         }
@@ -1010,7 +1010,7 @@ __global__ void __launch_bounds__(256, 3) out_transform_nchw_pair_kernel(const f
                     float2 v = make_float2(fmaf(y0[a][e], sc.x, sh.x), fmaf(y1[a][e], sc.y, sh.y));
                     if (ex.residual) {
                         const float2 r = *o;
-                        v = ex.res_relu ? make_float2(v.x + fmaxf(r.x, 0.f), v.y + fmaxf(r.y, 0.f)) : make_float2(v.x + r.x, v.y + r.y);
+                        v = ex.res_relu ? make_float2(v.x + relu_nan(r.x), v.y + relu_nan(r.y)) : make_float2(v.x + r.x, v.y + r.y);
                     }
                     *o = v;
                 }

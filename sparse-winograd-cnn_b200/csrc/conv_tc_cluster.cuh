@@ -374,7 +374,7 @@ layer_fwd_cluster_kernel(const __grid_constant__ CUtensorMap mapW, const ClParam
                         for (int x = 0; x < 4; ++x) if (x < nk) rs[x] = __ldg(prm.residual + o + x);
                     }
 #pragma unroll
-                    for (int x = 0; x < 4; ++x) w[x] += prm.res_relu ? fmaxf(rs[x], 0.f) : rs[x];
+                    for (int x = 0; x < 4; ++x) w[x] += prm.res_relu ? relu_nan(rs[x]) : rs[x];
                 }
                 if (vec) {
                     *reinterpret_cast<float4 *>(prm.Y + o) = make_float4(w[0], w[1], w[2], w[3]);
@@ -400,8 +400,8 @@ layer_fwd_cluster_kernel(const __grid_constant__ CUtensorMap mapW, const ClParam
                     float2 rs = make_float2(0.f, 0.f);
                     if (MODE == kClNchwEven) rs = __ldg(reinterpret_cast<const float2 *>(prm.residual + o));
                     else { rs.x = __ldg(prm.residual + o); if (two) rs.y = __ldg(prm.residual + o + 1); }
-                    w0 += prm.res_relu ? fmaxf(rs.x, 0.f) : rs.x;
-                    w1 += prm.res_relu ? fmaxf(rs.y, 0.f) : rs.y;
+                    w0 += prm.res_relu ? relu_nan(rs.x) : rs.x;
+                    w1 += prm.res_relu ? relu_nan(rs.y) : rs.y;
                 }
                 if (MODE == kClNchwEven) *reinterpret_cast<float2 *>(prm.Y + o) = make_float2(w0, w1);
                 else { prm.Y[o] = w0; if (two) prm.Y[o + 1] = w1; }

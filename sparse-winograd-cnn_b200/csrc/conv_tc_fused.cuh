@@ -834,10 +834,7 @@ __global__ void __launch_bounds__(256) relu_copy_kernel(const float *src, float 
     after_previous_kernel(src, dst);
     const float4 *s = reinterpret_cast<const float4 *>(src);
     float4 *d = reinterpret_cast<float4 *>(dst);
-    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n4; i += (long long)gridDim.x * 256) {
-        const float4 v = s[i];
-        d[i] = make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
-    }
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n4; i += (long long)gridDim.x * 256) d[i] = relu_nan(s[i]);
 }
 
 int layer_fwd_fused(const float *X, const void *prepared, float *Y, int B, int H, int W, int C, int K, int relu,

@@ -19,6 +19,15 @@ __host__ __device__ inline long long cdivll(long long a, long long b) { return (
 __device__ __forceinline__ float4 operator+(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 __device__ __forceinline__ float4 operator-(float4 a, float4 b) { return make_float4(a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w); }
 
+// max(x, 0) that keeps NaN, as torch.relu does (fmaxf gives the other value), for the ReLUs that stand in for one of the network's
+__device__ __forceinline__ float relu_nan(float x)
+{
+    float y;
+    asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float4 relu_nan(float4 a) { return make_float4(relu_nan(a.x), relu_nan(a.y), relu_nan(a.z), relu_nan(a.w)); }
+
 // ---- B^T d B, separable: 16 adds for the rows, 16 for the columns -----------------------
 // B^T = [[1,0,-1,0],[0,1,1,0],[0,-1,1,0],[0,1,0,-1]]
 template <typename T>

@@ -1,5 +1,5 @@
-"""NaN and infinity through the kernels that round operands to TF32 themselves: where an operand is not finite the result is not, as
-with cvt.rna.tf32, which the other kernels of the same step use."""
+"""NaN and infinity through the kernels that round operands to TF32 themselves or apply a ReLU of the network: where an operand is not
+finite the result is not, as with cvt.rna.tf32, which the other kernels of the same step use, and torch.relu, which keeps NaN."""
 import pytest
 import torch
 import torch.nn.functional as F
@@ -97,3 +97,27 @@ def test_round_tf32_values():
     assert torch.equal(wg2x2.round_tf32(x).view(torch.int32), want.view(torch.int32))
     nans = f(*(n & 0xFFFFFFFF for n in NANS))
     assert wg2x2.round_tf32(nans).isnan().all()
+
+
+# every kernel that adds relu(shortcut): few tiles (NCHW of even and odd width, NHWC with and without whole groups of four channels), the
+# one-kernel layer, the wide path's output transforms, the row-walk kernel (NHWC in whole blocks and not, NCHW)
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,layout", [
+    ((1, 56, 56, 64, 64), "NCHW"), ((2, 9, 13, 32, 36), "NCHW"), ((2, 9, 13, 32, 36), "NHWC"), ((7, 7, 7, 128, 130), "NHWC"),
+    ((16, 56, 56, 64, 64), "NCHW"), ((48, 14, 14, 256, 256), "NCHW"), ((48, 14, 14, 256, 256), "NHWC"), ((12, 13, 15, 256, 264), "NCHW"),
+    ((24, 48, 48, 64, 64), "NHWC"), ((24, 48, 48, 64, 66), "NHWC"), ((40, 49, 49, 32, 64), "NCHW")])
+def test_shortcut_reaches_the_output(shape, layout):
+    import wg2x2
+    B, H, W, C, K = shape
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    x, r = (rnd(B, H, W, c) if layout == "NHWC" else rnd(B, c, H, W) for c in (C, K))
+    flat = r.view(-1)
+    for i, bits in enumerate(NANS + [0x7F800000, 0xFF800000 - (1 << 32)]):
+        _put(flat, (flat.numel() // 9 * (i + 1) + i,), bits)
+    prepared = wg2x2.prepare_weights(rnd(16, C, K) / C ** 0.5)
+    kw = dict(relu=True, layout=layout, out_scale=1 + 0.2 * rnd(K), out_shift=0.3 * rnd(K))
+    got = wg2x2.layer_fwd_prepared(x, prepared, K, residual=r, residual_relu=True, **kw)
+    want = wg2x2.layer_fwd_prepared(x, prepared, K, residual=torch.relu(r), **kw)
+    assert int(want.isnan().sum()) == len(NANS) and torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(torch.nan_to_num(got, 0.0), torch.nan_to_num(want, 0.0))
