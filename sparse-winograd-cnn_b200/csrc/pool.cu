@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(256) maxpool_nhwc_in_kernel(const float *__res
     }
 }
 
-// Mean of relu(x) over each plane: four planes per warp at a time, so that their loads are in flight together.  Bound by the
+// Mean of relu(x) over each plane, NaN kept: four planes per warp at a time, so that their loads are in flight together.  Bound by the
 // planes' bytes (256 x 512 x 7 x 7: 36 us as torch's relu and mean before), by the launch for one image.
 __global__ void __launch_bounds__(256) relu_mean_kernel(const float *__restrict__ X, float *__restrict__ out, long long planes, int n)
 {
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(256) relu_mean_kernel(const float *__restrict_
     for (int i = lane; i < n; i += 32)
 #pragma unroll
         for (int q = 0; q < 4; ++q)
-            if (p0 + q < planes) s[q] += fmaxf(__ldg(X + (p0 + q) * n + i), 0.f);
+            if (p0 + q < planes) s[q] += relu_nan(__ldg(X + (p0 + q) * n + i));
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
 #pragma unroll

@@ -121,3 +121,19 @@ def test_shortcut_reaches_the_output(shape, layout):
     want = wg2x2.layer_fwd_prepared(x, prepared, K, residual=torch.relu(r), **kw)
     assert int(want.isnan().sum()) == len(NANS) and torch.equal(got.isnan(), want.isnan())
     assert torch.equal(torch.nan_to_num(got, 0.0), torch.nan_to_num(want, 0.0))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 49, 196])
+def test_relu_mean(n):
+    import wg2x2
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn((3, 37, n, 1), device="cuda", generator=g)       # 111 planes: 28 warps of four, the last with three
+    want = torch.relu(x.double()).mean(dim=(2, 3))
+    assert float((wg2x2.relu_mean(x) - want).abs().max()) <= (n + 1) * 2.0 ** -24 * float(x.abs().max())       # n additions and a division
+    for i, bits in enumerate(NANS + [0x7F800000, 0xFF800000 - (1 << 32)]):
+        bad = x.clone()
+        _put(bad, (2, 36 - i, n - 1, 0), bits)
+        want = torch.relu(bad).mean(dim=(2, 3))
+        got = wg2x2.relu_mean(bad)
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
