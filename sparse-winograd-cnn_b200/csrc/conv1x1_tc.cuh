@@ -5,9 +5,9 @@
 // 32 channels), so nothing is recycled: TMA brings every weight tile at the start, eight warps turn the pixels (lane = pixel,
 // 4 channels at a time) into K-major operand tiles, one warp issues the MMAs chunk by chunk, and the eight warps store the
 // accumulator, 32 consecutive pixels per instruction.  Image values and weights are rounded to TF32 (nearest; the weights by
-// the caller).  Why: for one image the library's call costs 20 us of host time for 4 - 8 us of kernel, four times per network; this one
-// takes 5 - 12 us and 4 of host (ResNet-18-var on one image 223 -> 209 us).  (Four chunks of pixels in flight per thread
-// instead of one measured slower, 16 against 12 us at 256 channels.)
+// the caller).  Why: the library's call costs 10 us of host time, this one 4, and the network makes four of them; on the GPU this one
+// takes 4.4 us for 64 channels and 9 for 256 against 3.1 and 7.7 as long as a CTA per SM holds all pixels.  (Four chunks of pixels in
+// flight per thread instead of one measured slower.)
 #pragma once
 
 constexpr int kC1MaxChunks = 8;
@@ -122,8 +122,11 @@ __global__ void __launch_bounds__(kC1Threads) conv1x1_tc_kernel(const __grid_con
     }
 }
 
-// Where this kernel beats the library's call, host time included: few pixels (its CTAs transform their pixels for every 64 output
-// channels again and start from nothing).
+// Where the network is faster with this kernel than with the library's call: up to two rounds of CTAs, each of which transforms its
+// pixels for 64 output channels only and starts from nothing.  ResNet-18-var, microseconds with every call in these bounds here / with
+// none: 1 image 194 / 215, 2 images 216 / 219, 4: 260 / 263, 8: 352 / 360, 16: 457 / 460, 32: 616 / 625, 48: 878 / 884.  Beyond, the
+// library's kernel is the faster one by more than host time can hide (256 channels of 48 x 14 x 14 in two rounds 8.7 against 7.2 us, in
+// four 15.4 against 10.0).
 bool conv1x1_preferred(int B, int C, int K, int HW)
 {
     return C % 4 == 0 && C <= kC1MaxChunks * kBlockK && cdivll((long long)B * HW, kBlockM) * cdiv(K, kBlockN) <= 2 * kNumSMs;
