@@ -6,6 +6,7 @@
 #include <stdlib.h>
 
 #include <initializer_list>
+#include <mutex>
 
 #include "../../include/winograd2x2_b200.h"
 
@@ -207,7 +208,9 @@ __device__ __forceinline__ void after_previous_kernel(P &...p)
     (void)std::initializer_list<int>{([](P &q) { asm volatile("" : "+l"(q)::"memory"); }(p), 0)...};
 }
 
-// Dynamic shared memory above 48 KB has to be granted once per kernel and device; remembered per thread.
+// Dynamic shared memory above 48 KB has to be granted to a kernel, per device and for the whole process.  A kernel may be launched
+// with other sizes by several threads at once, so a grant is only ever raised: one thread at a time looks at it and sets it.  What a
+// thread has seen granted it need not ask for again.
 inline bool grant_smem(const void *kernel, size_t bytes)
 {
     struct Entry { const void *kernel; int dev; size_t bytes; };
@@ -216,8 +219,16 @@ inline bool grant_smem(const void *kernel, size_t bytes)
     if (cudaGetDevice(&dev) != cudaSuccess) return false;
     Entry &e = seen[(reinterpret_cast<uintptr_t>(kernel) >> 4) & 63];
     if (e.kernel == kernel && e.dev == dev && e.bytes >= bytes) return true;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return false;
-    e = Entry{kernel, dev, bytes};
+    static std::mutex one_at_a_time;
+    const std::lock_guard<std::mutex> lock(one_at_a_time);
+    cudaFuncAttributes now;
+    if (cudaFuncGetAttributes(&now, kernel) != cudaSuccess) return false;
+    size_t granted = now.maxDynamicSharedSizeBytes < 0 ? 0 : (size_t)now.maxDynamicSharedSizeBytes;
+    if (granted < bytes) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return false;
+        granted = bytes;
+    }
+    e = Entry{kernel, dev, granted};
     return true;
 }
 
