@@ -229,6 +229,8 @@ size_t wg2x2_layer_fwd_prepared_workspace_bytes(int B, int H, int W, int C, int 
  * layout and at any image size (X, Y, residual, in_scale and in_shift 16-byte aligned) and read neither scratch buffer.
  * wg2x2_layer_fwd_prepared_scratch: the bytes of V_scratch and workspace with which the call is fastest (0: not used);
  * `aligned`: whether all of those pointers are on 16-byte boundaries.
+ * out_scale, out_shift and residual may be at any alignment where the one-kernel layer is supported (X and Y aligned) and C < 256 or
+ * K < 256; that layer is then taken and needs no scratch.
  */
 int wg2x2_layer_fwd_prepared_ex(const float *X, const float *in_scale, const float *in_shift, const void *prepared, float *Y,
                                 float *V_scratch, int B, int H, int W, int C, int K, int layout, int relu,

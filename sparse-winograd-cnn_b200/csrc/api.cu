@@ -286,10 +286,14 @@ int wg2x2_layer_fwd_prepared_ex(const float *X, const float *in_scale, const flo
     const bool wide = V_scratch && workspace && conv_fwd_wide_preferred((long long)B * nH * nW, C, K);
     if (aligned && on16(residual) && on16(in_scale) && on16(in_shift) && layer_cluster_preferred(B, H, W, C, K, layout))
         return layer_fwd_cluster(X, prepared, Y, B, H, W, C, K, layout, relu, in_scale, in_shift, out_scale, out_shift, residual, residual_relu, st);
-    // The one-kernel path redoes the input transform for every block of 64 output channels.  Without scratch for the wide
-    // path it wins while there are few of them (measured: K <= 128, or K <= 256 with C <= 64).
+    // The one-kernel layer: where it is the fastest; without scratch for the wide path, where there are few blocks of 64 output channels
+    // (each redoes the input transform; measured: K <= 128, or K <= 256 with C <= 64), or always without any scratch; and where out_scale,
+    // out_shift or residual is off a 16-byte boundary, which it alone reads so (but not for C, K >= 256 with scratch: such a call has
+    // always been the wide path's, which refuses it).
+    const bool extras_on16 = on16(out_scale) && on16(out_shift) && on16(residual);
     if (aligned && fused_fwd_supported(B, H, W, C, K, layout) &&
-        (layer_fused_preferred(B, H, W, C, K, layout) || (!wide && (K <= 128 || (K <= 256 && C <= 64) || !V_scratch))))
+        (layer_fused_preferred(B, H, W, C, K, layout) || (!wide && (K <= 128 || (K <= 256 && C <= 64) || !V_scratch)) ||
+         (!extras_on16 && (C < 256 || K < 256))))
         return layer_fwd_fused(X, prepared, Y, B, H, W, C, K, relu, in_scale, in_shift, out_scale, out_shift, residual, residual_relu, st);
     if (!V_scratch) return WG2X2_ERR_WORKSPACE;
     if ((out_scale == nullptr) != (out_shift == nullptr)) return WG2X2_ERR_BAD_ARG;

@@ -505,10 +505,10 @@ struct LayerScratch {
     float *v = nullptr;
     void *w = nullptr;
     size_t wn = 0;
-    LayerScratch(const Img &d, int64_t K, int layout, bool aligned, const Tensor &V, const Tensor &uws)
+    LayerScratch(const Img &d, int64_t K, int layout, bool aligned, bool none, const Tensor &V, const Tensor &uws)
     {
-        size_t nv, nw;
-        wg2x2_layer_fwd_prepared_scratch(d.B, d.H, d.W, d.C, K, layout, aligned, &nv, &nw);
+        size_t nv = 0, nw = 0;
+        if (!none) wg2x2_layer_fwd_prepared_scratch(d.B, d.H, d.W, d.C, K, layout, aligned, &nv, &nw);
         v = ptr(V);
         if (!v && nv) { vs.take(nv); v = static_cast<float *>(vs.get()); }
         if (nw) {
@@ -524,7 +524,10 @@ void layer_fwd_prepared(const Tensor &x, const Tensor &prep, const Tensor &Y, co
                         const Tensor &in_shift, const Tensor &out_scale, const Tensor &out_shift, const Tensor &residual, bool residual_relu,
                         const Tensor &V, const Tensor &uws, void *stream)
 {
-    const LayerScratch s(d, K, layout, on16(x) && on16(Y) && on16(residual) && on16(in_scale) && on16(in_shift), V, uws);
+    const bool xy = on16(x) && on16(Y), extras = on16(out_scale) && on16(out_shift) && on16(residual);
+    // (extras off 16 bytes are the one-kernel layer's, or the cluster kernel's; neither reads scratch)
+    const bool one_kernel = xy && !extras && (d.C < 256 || K < 256) && wg2x2_layer_fwd_fused_supported(d.B, d.H, d.W, d.C, K, layout);
+    const LayerScratch s(d, K, layout, xy && on16(residual) && on16(in_scale) && on16(in_shift), one_kernel, V, uws);
     check(wg2x2_layer_fwd_prepared_ex(cptr(x), cptr(in_scale), cptr(in_shift), prep.data_ptr(), ptr(Y), s.v, d.B, d.H, d.W, d.C, K, layout, relu,
                                       cptr(out_scale), cptr(out_shift), cptr(residual), residual_relu, s.w, s.wn, stream),
           "wg2x2_layer_fwd_prepared_ex");

@@ -828,13 +828,15 @@ static bool fused_geometry(FuParams &p)
     return true;
 }
 
-// The shortcut, ReLU applied, into the output buffer that the kernel then adds to (in place where they are one)
+// The shortcut, ReLU applied, into the output buffer that the kernel then adds to (in place where they are one).  dst is on a
+// 16-byte boundary, src need not be.
 __global__ void __launch_bounds__(256) relu_copy_kernel(const float *src, float *dst, long long n4)
 {
     after_previous_kernel(src, dst);
-    const float4 *s = reinterpret_cast<const float4 *>(src);
+    const bool vec = (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
     float4 *d = reinterpret_cast<float4 *>(dst);
-    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n4; i += (long long)gridDim.x * 256) d[i] = relu_nan(s[i]);
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n4; i += (long long)gridDim.x * 256)
+        d[i] = relu_nan(vec ? reinterpret_cast<const float4 *>(src)[i] : make_float4(src[4 * i], src[4 * i + 1], src[4 * i + 2], src[4 * i + 3]));
 }
 
 int layer_fwd_fused(const float *X, const void *prepared, float *Y, int B, int H, int W, int C, int K, int relu,
@@ -852,7 +854,6 @@ int layer_fwd_fused(const float *X, const void *prepared, float *Y, int B, int H
     // into Y instead of stored.
     p.accumulate = residual != nullptr;
     if (residual && res_relu) {
-        if (misaligned16(residual)) return WG2X2_ERR_BAD_ARG;
         const long long n4 = (long long)B * K * H * W / 4;         // W % 4 == 0 here
         const int s = launch(relu_copy_kernel, dim3((unsigned)(n4 < 256LL * 32 * kNumSMs ? cdivll(n4, 256) : 32 * kNumSMs)), 256, 0, st, residual, Y, n4);
         if (s != WG2X2_OK) return s;

@@ -1,8 +1,15 @@
-"""The calls themselves, where several threads make them."""
+"""The calls themselves: made by several threads, with operands off 16-byte boundaries."""
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
+
+
+def _off(t):
+    """The same values one float off a 16-byte boundary."""
+    o = torch.empty(t.numel() + 1, device=t.device)[1:].view(t.shape)
+    assert o.data_ptr() % 16 == 4
+    return o.copy_(t)
 
 
 def _on_new_thread():
@@ -23,3 +30,35 @@ def test_two_threads_with_different_sizes_of_one_kernel():
     first = a(big)
     b(small)
     assert torch.equal(a(big), first) and torch.equal(b(big), first)
+
+
+# NCHW layers whose rows are whole 16-byte pieces have read out_scale, out_shift and residual at any alignment since the one-kernel layer
+# was their only path; the sizes here are now computed on clusters, by the wide path and by the one kernel
+@pytest.mark.parametrize("shape", [(48, 512, 128, 16, 16), (3, 512, 64, 28, 28), (1, 64, 64, 56, 56), (5, 48, 80, 28, 28), (16, 64, 64, 56, 56), (2, 128, 320, 8, 8)])
+def test_extras_at_any_alignment(shape):
+    import wg2x2
+    B, C, K, H, W = shape
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    x, r, prepared = rnd(B, C, H, W), rnd(B, K, H, W), wg2x2.prepare_weights(rnd(16, C, K) / C ** 0.5)
+    sc, sh, isc, ish = 1 + 0.2 * rnd(K), 0.3 * rnd(K), 1 + 0.2 * rnd(C), 0.3 * rnd(C)
+    kw = dict(relu=True, layout="NCHW", in_scale=isc, in_shift=ish)
+    for relu in (False, True):
+        want = wg2x2.layer_fwd_prepared(x, prepared, K, out_scale=sc, out_shift=sh, residual=r, residual_relu=relu, **kw)
+        scale = float(want.abs().max())
+        for s, t, q in ((_off(sc), sh, r), (sc, _off(sh), r), (sc, sh, _off(r)), (_off(sc), _off(sh), _off(r))):
+            got = wg2x2.layer_fwd_prepared(x, prepared, K, out_scale=s, out_shift=t, residual=q, residual_relu=relu, **kw)
+            # another path at worst: V rounded to 11 bits where the other cuts it, 2^-11 of each of C x 16 terms of random sign
+            assert float((got - want).abs().max()) <= 2e-3 * scale
+        got = wg2x2.layer_fwd_prepared(x, prepared, K, out_scale=sc, out_shift=sh, residual=r, residual_relu=relu, relu=True, layout="NCHW",
+                                       in_scale=_off(isc), in_shift=_off(ish))
+        assert float((got - want).abs().max()) <= 2e-3 * scale
+
+
+def test_extras_off_16_bytes_stay_refused_where_only_the_wide_path_runs():
+    import wg2x2
+    x, prepared = torch.zeros((48, 256, 16, 16), device="cuda"), wg2x2.prepare_weights(torch.zeros((16, 256, 256), device="cuda"))
+    s = torch.ones(256, device="cuda")
+    with pytest.raises(wg2x2.Wg2x2Error) as e:
+        wg2x2.layer_fwd_prepared(x, prepared, 256, layout="NCHW", out_scale=_off(s), out_shift=s)
+    assert e.value.status == -1
