@@ -156,6 +156,8 @@ class ResNet18Var(torch.nn.Module):
         # the next stage's shortcut branch starts from), torch's elsewhere
         own_pool = not reference and self.layout == "NCHW" and image.is_cuda
         own_stem = own_pool and self.math == "tf32" and wg2x2.stem_supported(image.shape[2], image.shape[3])
+        # (torch's convolution of the same tensors, which it stands in for, is in 32 bits where the caller asks torch for that)
+        own_1x1 = own_pool and self.math == "tf32" and torch.backends.cudnn.conv.fp32_precision == "tf32"
         pre = self.blocks[0][0]["pre"]
         l_relu = None
         if own_stem:      # conv1 + pool1 (+ the first shortcut's BNReLU) as one tensor-core kernel
@@ -193,7 +195,7 @@ class ResNet18Var(torch.nn.Module):
                     blk_a._short_folded = (blk_a.short * blk_a["bn1"].scale.view(-1, 1, 1, 1)).detach()
                     blk_a._short_tf32 = wg2x2.round_tf32(blk_a._short_folded)
                 # (its shift is added by the block's last kernel)
-                y = wg2x2.conv1x1(main, blk_a._short_tf32) if own_pool and self.math == "tf32" and main.is_contiguous() else None
+                y = wg2x2.conv1x1(main, blk_a._short_tf32) if own_1x1 and main.is_contiguous() else None
                 main = F.conv2d(main, blk_a._short_folded) if y is None else y
             l = self._block(blk_a, l, main, reference, main_bias=None if (reference or not self.fused) else blk_a["bn1"].shift)
             l = self._block(blk_b, l, None, reference)

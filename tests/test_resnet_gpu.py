@@ -147,3 +147,23 @@ def test_conv1x1_kernel(shape):
     assert got.shape == want.shape and float((got - want).abs().max()) <= 2e-5 * float(want.abs().max())
     assert wg2x2.conv1x1(torch.zeros((64, 64, 56, 56), device="cuda"), torch.zeros((64, 64, 1, 1), device="cuda")) is None
     assert wg2x2.last_device_status()[0] == 0
+
+
+def test_shortcuts_in_32_bits_where_torch_is_asked_for_them(monkeypatch):
+    """torch.backends.cudnn.allow_tf32 = False: no 1x1 convolution with TF32 operands, as torch's own would not."""
+    import wg2x2
+    from resnet18_var import ResNet18Var
+    model = ResNet18Var(seed=3).cuda().eval()
+    x = torch.randn((1, 3, 64, 64), device="cuda")
+    calls, conv1x1 = [], wg2x2.conv1x1
+    monkeypatch.setattr(wg2x2, "conv1x1", lambda x, w: calls.append(1) or conv1x1(x, w))
+    keep = torch.backends.cudnn.allow_tf32
+    try:
+        for allow in (True, False):
+            torch.backends.cudnn.allow_tf32 = allow
+            calls.clear()
+            with torch.no_grad():
+                model(x)
+            assert len(calls) == (4 if allow else 0)
+    finally:
+        torch.backends.cudnn.allow_tf32 = keep
