@@ -14,6 +14,8 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
 
+#include <mutex>
+
 #include "../../include/winograd2x2_b200.h"
 
 namespace {
@@ -238,7 +240,8 @@ std::pair<Tensor, Tensor> conv_bwd(const Tensor &V, const Tensor &Wt, const Tens
 
 // ---------------------------------------------------------------------------------------
 // Autograd nodes of the two ops (the reference pairs each op with its gradient op by RegisterGradient:
-// winograd2x2_imTrans.py:29-33, winograd2x2_conv.py:32-36)
+// winograd2x2_imTrans.py:29-33, winograd2x2_conv.py:32-36).  Several threads may run backward over one graph: what a node saved is read
+// and released under its lock.
 // ---------------------------------------------------------------------------------------
 struct ImTransBackward : public torch::autograd::Node {
     Tensor bits;               // where the output is positive, kept only where the ReLU was applied
@@ -246,18 +249,27 @@ struct ImTransBackward : public torch::autograd::Node {
     int layout = 0;
     bool relu = false;
     std::string name() const override { return "Winograd2x2ImTransBackward"; }
-    void release_variables() override { bits.reset(); }
+    void release_variables() override
+    {
+        const std::lock_guard<std::mutex> lock(mutex_);
+        bits.reset();
+    }
     variable_list apply(variable_list &&grads) override
     {
         if (!grads[0].defined()) return {Tensor()};
-        TORCH_CHECK(!relu || bits.defined(), torch::autograd::ERR_BACKWARD_TWICE);
+        Tensor saved;
+        {
+            const std::lock_guard<std::mutex> lock(mutex_);
+            saved = bits;
+        }
+        TORCH_CHECK(!relu || saved.defined(), torch::autograd::ERR_BACKWARD_TWICE);
         const Tensor g = grads[0].contiguous();
         require(g, "dV");
         if (!relu) return {imtrans_bwd(g, H, W, Tensor(), layout)};
         OnDevice on(g);
         const int64_t B = g.size(1), C = g.size(4);
         Tensor dX = new_float(img_shape(B, H, W, C, layout), g);
-        check(wg2x2_imtrans_bwd_relu_bits(cptr(g), bits.data_ptr(), ptr(dX), B, H, W, C, layout, on.stream), "wg2x2_imtrans_bwd_relu_bits");
+        check(wg2x2_imtrans_bwd_relu_bits(cptr(g), saved.data_ptr(), ptr(dX), B, H, W, C, layout, on.stream), "wg2x2_imtrans_bwd_relu_bits");
         return {dX};
     }
 };
@@ -266,14 +278,27 @@ struct ConvBackward : public torch::autograd::Node {
     SavedVariable I_, W_, mask_;      // W with the mask applied
     int layout = 0, math = 0;
     std::string name() const override { return "Winograd2x2ConvBackward"; }
-    void release_variables() override { I_.reset_data(); W_.reset_data(); mask_.reset_data(); }
+    void release_variables() override
+    {
+        const std::lock_guard<std::mutex> lock(mutex_);
+        I_.reset_data();
+        W_.reset_data();
+        mask_.reset_data();
+    }
     variable_list apply(variable_list &&grads) override
     {
         if (!grads[0].defined()) return {Tensor(), Tensor()};
         const bool dI = task_should_compute_output(0), dW = task_should_compute_output(1);
         const Tensor g = grads[0].contiguous();
         require(g, "dY");
-        auto r = conv_bwd(I_.unpack(), W_.unpack(), g, mask_.unpack(), layout, false, math, dI, dW);
+        Tensor I, Wt, mask;
+        {
+            const std::lock_guard<std::mutex> lock(mutex_);
+            I = I_.unpack();
+            Wt = W_.unpack();
+            mask = mask_.unpack();
+        }
+        auto r = conv_bwd(I, Wt, g, mask, layout, false, math, dI, dW);
         return {r.first, r.second};
     }
 };

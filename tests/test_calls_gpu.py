@@ -1,4 +1,6 @@
 """The calls themselves: made by several threads, with operands off 16-byte boundaries."""
+import threading
+
 import pytest
 import torch
 
@@ -62,3 +64,38 @@ def test_extras_off_16_bytes_stay_refused_where_only_the_wide_path_runs():
     with pytest.raises(wg2x2.Wg2x2Error) as e:
         wg2x2.layer_fwd_prepared(x, prepared, 256, layout="NCHW", out_scale=_off(s), out_shift=s)
     assert e.value.status == -1
+
+
+def _layer(g, C=16, K=8):
+    import winograd_conv
+    import winograd_imtrans
+    layer = winograd_conv.WinogradConvLayer(C, K, device="cuda", W_init=lambda s: torch.randn(s, generator=g, device="cuda"))
+    return layer, lambda x: layer(winograd_imtrans.WinogradImTrans(x, nl=torch.relu, data_format="NHWC"), out_hw=x.shape[1:3])
+
+
+def test_backward_of_one_graph_on_several_threads():
+    """Each thread has the gradients, or is told that the graph is gone."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    layer, f = _layer(g)
+    x = torch.randn((3, 9, 8, 16), generator=g, device="cuda", requires_grad=True)
+    y = f(x)
+    dy = torch.randn(y.shape, generator=g, device="cuda")
+    want = torch.autograd.grad(y, (x, layer.W), dy, retain_graph=True)
+    bad = []
+
+    def run(retain, lost_is_fine, y):
+        try:
+            got = torch.autograd.grad(y, (x, layer.W), dy, retain_graph=retain)
+            if not all(torch.equal(p, q) for p, q in zip(got, want)):
+                bad.append("other values")
+        except RuntimeError as e:
+            if not lost_is_fine or "second time" not in str(e):
+                bad.append(e)
+
+    for retain in (True, False):
+        for _ in range(20):
+            yy = y if retain else f(x)
+            ts = [threading.Thread(target=run, args=(retain, not retain, yy)) for _ in range(4)]
+            [t.start() for t in ts]
+            [t.join() for t in ts]
+    assert not bad, bad[0]
