@@ -244,7 +244,7 @@ std::pair<Tensor, Tensor> conv_bwd(const Tensor &V, const Tensor &Wt, const Tens
 // and released under its lock.
 // ---------------------------------------------------------------------------------------
 struct ImTransBackward : public torch::autograd::Node {
-    Tensor bits;               // where the output is positive, kept only where the ReLU was applied
+    SavedVariable bits_;       // where the output is positive, kept only where the ReLU was applied
     int64_t H = 0, W = 0;
     int layout = 0;
     bool relu = false;
@@ -252,24 +252,23 @@ struct ImTransBackward : public torch::autograd::Node {
     void release_variables() override
     {
         const std::lock_guard<std::mutex> lock(mutex_);
-        bits.reset();
+        bits_.reset_data();
     }
     variable_list apply(variable_list &&grads) override
     {
         if (!grads[0].defined()) return {Tensor()};
-        Tensor saved;
-        {
+        Tensor bits;
+        if (relu) {
             const std::lock_guard<std::mutex> lock(mutex_);
-            saved = bits;
+            bits = bits_.unpack();
         }
-        TORCH_CHECK(!relu || saved.defined(), torch::autograd::ERR_BACKWARD_TWICE);
         const Tensor g = grads[0].contiguous();
         require(g, "dV");
         if (!relu) return {imtrans_bwd(g, H, W, Tensor(), layout)};
         OnDevice on(g);
         const int64_t B = g.size(1), C = g.size(4);
         Tensor dX = new_float(img_shape(B, H, W, C, layout), g);
-        check(wg2x2_imtrans_bwd_relu_bits(cptr(g), saved.data_ptr(), ptr(dX), B, H, W, C, layout, on.stream), "wg2x2_imtrans_bwd_relu_bits");
+        check(wg2x2_imtrans_bwd_relu_bits(cptr(g), bits.data_ptr(), ptr(dX), B, H, W, C, layout, on.stream), "wg2x2_imtrans_bwd_relu_bits");
         return {dX};
     }
 };
@@ -330,7 +329,7 @@ Tensor imtrans_op(const Tensor &in, bool relu, int layout)
         auto n = new_node<ImTransBackward>(torch::autograd::collect_next_edges(I));
         const Img d = img_of(I, layout, "x");
         n->H = d.H; n->W = d.W; n->layout = layout; n->relu = relu;
-        n->bits = bits;
+        if (relu) n->bits_ = SavedVariable(bits, false);
         torch::autograd::set_history(V, n);
     }
     return V;

@@ -99,3 +99,18 @@ def test_backward_of_one_graph_on_several_threads():
             [t.start() for t in ts]
             [t.join() for t in ts]
     assert not bad, bad[0]
+
+
+def test_saved_tensor_hooks_see_everything_that_is_saved():
+    """The transform's ReLU mask, and the product's two operands, pass through the hooks (offloading, checkpointing) in both directions."""
+    g = torch.Generator(device="cuda").manual_seed(6)
+    layer, f = _layer(g)
+    x = torch.randn((3, 9, 8, 16), generator=g, device="cuda", requires_grad=True)
+    y = f(x)
+    dy = torch.randn(y.shape, generator=g, device="cuda")
+    want = torch.autograd.grad(y, (x, layer.W), dy)
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: (packed.append(t.shape), t.cpu())[1], lambda t: t.cuda()):
+        y = f(x)
+    assert len(packed) == 3
+    assert all(torch.equal(p, q) for p, q in zip(torch.autograd.grad(y, (x, layer.W), dy), want))
