@@ -310,8 +310,15 @@ std::shared_ptr<N> new_node(torch::autograd::edge_list edges)
     return n;
 }
 
+// There is no forward-mode rule: a tangent is refused, as torch.autograd.Function refuses it, not dropped.
+void no_tangent(const Tensor &t)
+{
+    TORCH_CHECK_NOT_IMPLEMENTED(!t.defined() || !t._fw_grad(0).defined(), "forward-mode automatic differentiation is not implemented for the Winograd ops");
+}
+
 Tensor imtrans_op(const Tensor &in, bool relu, int layout)
 {
+    no_tangent(in);
     const Tensor I = in.contiguous();
     require(I, "x");
     const bool grad = torch::autograd::compute_requires_grad(I);
@@ -339,6 +346,9 @@ Tensor imtrans_op(const Tensor &in, bool relu, int layout)
 // mask on dW, which the dW kernels apply anyway) is a node and a kernel of its own: 12 + 10 us of host time in a training step.
 Tensor conv_op(const Tensor &in, const Tensor &win, const Tensor &mask, int out_h, int out_w, int layout, int math)
 {
+    no_tangent(in);
+    no_tangent(win);
+    no_tangent(mask);
     const Tensor I = in.contiguous();
     Tensor Wt = win.contiguous();
     require(I, "V");

@@ -114,3 +114,18 @@ def test_saved_tensor_hooks_see_everything_that_is_saved():
         y = f(x)
     assert len(packed) == 3
     assert all(torch.equal(p, q) for p, q in zip(torch.autograd.grad(y, (x, layer.W), dy), want))
+
+
+def test_forward_mode_is_refused():
+    import torch.autograd.forward_ad as fw
+    import wg2x2
+    g = torch.Generator(device="cuda").manual_seed(7)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    x, v, w, m = rnd(2, 8, 8, 16), rnd(16, 2, 4, 4, 16), rnd(16, 16, 8), torch.ones((16, 16, 8), device="cuda")
+    with fw.dual_level():
+        dual = lambda t: fw.make_dual(t, torch.ones_like(t))
+        for call in (lambda: wg2x2.ops.imtrans_op(dual(x), True), lambda: wg2x2.ops.conv_op(dual(v), w), lambda: wg2x2.ops.conv_op(v, dual(w)),
+                     lambda: wg2x2.ops.conv_op(v, w, mask=dual(m))):
+            with pytest.raises(NotImplementedError):
+                call()
+        wg2x2.ops.conv_op(wg2x2.ops.imtrans_op(x, True), w, mask=m)
