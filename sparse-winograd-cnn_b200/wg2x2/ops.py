@@ -9,6 +9,8 @@ from . import _native
 
 _native.set_error(Wg2x2Error)
 
+_tracing = torch._C._get_tracing_state       # None outside torch.jit.trace
+
 _LAYOUTS = {"NHWC": NHWC, "NCHW": NCHW, NHWC: NHWC, NCHW: NCHW}
 _MATHS = {"fp32": MATH_FP32, "tf32": MATH_TF32, MATH_FP32: MATH_FP32, MATH_TF32: MATH_TF32}
 
@@ -37,8 +39,49 @@ def imtrans_bwd(dV, H, W, V_relu=None, layout="NHWC"):
     return _native.imtrans_bwd(dV, H, W, V_relu, _LAYOUTS[layout])
 
 
+class _ImTransTraced(torch.autograd.Function):
+    """imtrans_op in the form that torch.jit.trace records, a Python operator; the native calls it does not see.  (The outputs come
+    from torch: the tracer wants to know where a tensor with gradients is from.)"""
+
+    @staticmethod
+    def forward(ctx, x, relu, layout):
+        B, H, W, C = (int(n) for n in (x.shape if layout == NHWC else (x.shape[0], x.shape[2], x.shape[3], x.shape[1])))
+        V = imtrans_fwd(x.contiguous(), relu, layout, out=x.new_empty((16, B, (H + 1) // 2, (W + 1) // 2, C)))
+        ctx.hw = H, W
+        ctx.layout, ctx.relu = layout, relu
+        if relu:
+            ctx.save_for_backward(V)
+        return V
+
+    @staticmethod
+    def backward(ctx, g):
+        V = ctx.saved_tensors[0] if ctx.relu else None
+        return imtrans_bwd(g.contiguous(), ctx.hw[0], ctx.hw[1], V, ctx.layout), None, None
+
+
+class _ConvTraced(torch.autograd.Function):
+    """conv_op likewise, without the mask."""
+
+    @staticmethod
+    def forward(ctx, V, Wt, out_h, out_w, layout, math):
+        V, Wt = V.contiguous(), Wt.contiguous()
+        ctx.save_for_backward(V, Wt)
+        ctx.layout, ctx.math = layout, math
+        B, nH, nW, K = (int(n) for n in (*V.shape[1:4], Wt.shape[2]))
+        H, W = 2 * nH if out_h is None else out_h, 2 * nW if out_w is None else out_w
+        return conv_fwd(V, Wt, H, W, layout, math, out=V.new_empty((B, H, W, K) if layout == NHWC else (B, K, H, W)))
+
+    @staticmethod
+    def backward(ctx, g):
+        V, Wt = ctx.saved_tensors
+        dV, dW = conv_bwd(V, Wt, g.contiguous(), layout=ctx.layout, math=ctx.math, need_dV=ctx.needs_input_grad[0], need_dW=ctx.needs_input_grad[1])
+        return dV, dW, None, None, None, None
+
+
 def imtrans_op(x, relu=False, layout="NHWC"):
     """imtrans_fwd for autograd: differentiable in x (any strides), the ReLU mask applied inside the gradient's gather."""
+    if _tracing() is not None:
+        return _ImTransTraced.apply(x, bool(relu), _LAYOUTS[layout])
     return _native.imtrans_op(x, relu, _LAYOUTS[layout])
 
 
@@ -49,6 +92,8 @@ def conv_fwd(V, Wt, out_h=None, out_w=None, layout="NHWC", math="fp32", out=None
 
 def conv_op(V, Wt, out_h=None, out_w=None, layout="NHWC", math="fp32", mask=None):
     """conv_fwd for autograd: differentiable in V and Wt (any strides).  mask (16,C,K), constant: the weights are Wt * mask."""
+    if _tracing() is not None:
+        return _ConvTraced.apply(V, Wt if mask is None else Wt * mask, *(None if n is None else int(n) for n in (out_h, out_w)), _LAYOUTS[layout], _MATHS[math])
     return _native.conv_op(V, Wt, out_h, out_w, _LAYOUTS[layout], _MATHS[math], mask)
 
 

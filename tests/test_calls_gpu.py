@@ -1,4 +1,4 @@
-"""The calls themselves: made by several threads, with operands off 16-byte boundaries."""
+"""The calls themselves: made by several threads, with operands off 16-byte boundaries, and what autograd and its tools ask of them."""
 import threading
 
 import pytest
@@ -129,3 +129,33 @@ def test_forward_mode_is_refused():
             with pytest.raises(NotImplementedError):
                 call()
         wg2x2.ops.conv_op(wg2x2.ops.imtrans_op(x, True), w, mask=m)
+
+
+@pytest.mark.parametrize("layout,masked", [("NHWC", False), ("NHWC", True), ("NCHW", True)])
+def test_traced_module(layout, masked):
+    """torch.jit.trace records both ops: other inputs give other outputs and gradients, with gradients off too."""
+    import winograd_conv
+    import winograd_imtrans
+    g = torch.Generator(device="cuda").manual_seed(8)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+
+    class Net(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.layer = winograd_conv.WinogradConvLayer(16, 8, device="cuda", W_init=lambda s: rnd(*s), mask=(rnd(16, 16, 8) > 0).float() if masked else None)
+
+        def forward(self, x):
+            v = winograd_imtrans.WinogradImTrans(2 * x, nl=torch.relu, data_format=layout)
+            return torch.tanh(self.layer(v, out_hw=x.shape[1:3] if layout == "NHWC" else x.shape[2:], data_format=layout))
+
+    net, shape = Net(), (2, 9, 8, 16) if layout == "NHWC" else (2, 16, 9, 8)
+    for grad in (True, False):
+        with torch.set_grad_enabled(grad):
+            traced = torch.jit.trace(net, (rnd(*shape),))
+        x = rnd(*shape).requires_grad_(True)
+        y, z = net(x), traced(x)
+        assert torch.equal(y, z)
+        if grad:
+            dy = torch.randn_like(y)
+            want = torch.autograd.grad(y, (x, net.layer.W), dy)
+            assert all(torch.equal(p, q) for p, q in zip(torch.autograd.grad(z, (x, net.layer.W), dy), want))
