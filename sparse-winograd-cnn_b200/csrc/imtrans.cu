@@ -616,12 +616,12 @@ __global__ void __launch_bounds__(256) imtrans_bwd_nchw_kernel(const float *__re
     }
 }
 
-// NCHW, image rows up to 192 pixels, with V as the mask or too few tiles for the walk above to fill the GPU: the same gather with lane = VEC consecutive channels over a band of R tile
-// rows; the 2R x W output pixels of each channel collect in shared memory (odd pitch between channels) and
-// leave as one contiguous run per channel -- or, where the band is the whole image, as one contiguous run for
-// all the block's channels.  VEC = 4 reads dV (and the ReLU mask) with 16-byte loads: LC = 32 lanes along the
-// channels (128 per block, 512 bytes per request) where such a band fits four blocks per SM, else LC = 16 (64
-// channels per block, the two halves of a warp on two tiles at once).
+// NCHW, image rows up to 192 pixels, with V as the mask or too few tiles for the walk above to fill the GPU: the same gather with
+// lane = VEC consecutive channels over a band of R tile rows; the 2R x W output pixels of each channel collect in shared memory (odd
+// pitch between channels) and leave as one contiguous run per channel -- or, where the band is the whole image, as one contiguous run
+// for all the block's channels.  VEC = 4 reads dV (and the ReLU mask) with 16-byte loads: LC = 32 lanes along the channels (128 per
+// block, 512 bytes per request) where such a band fits four blocks per SM, else LC = 16 (64 channels per block, the two halves of a
+// warp on two tiles at once).
 template <int VEC, int LC, int MASK, bool SEG>
 __global__ void __launch_bounds__(256, 4) imtrans_bwd_nchw_band_kernel(const float *__restrict__ dV, const void *__restrict__ Vm,
                                                                          float *__restrict__ dX, int B, int H, int W, int C, int nH,
@@ -812,10 +812,6 @@ __global__ void __launch_bounds__(256) imtrans_bwd_nchw_image_kernel(const float
 // which is what this kernel is short of.  The image is kept as [pixel][channel] (channels innermost, so that the lanes'
 // 8-byte read-modify-writes are conflict-free) with a pitch of CB + 2 floats, and leaves per channel through strided
 // reads (two-way bank conflicts on the smaller side of the traffic).  Needs an even C and 8-byte aligned tensors.
-__device__ __forceinline__ float2 f2add(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 f2sub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ float2 f2neg(float2 a) { return make_float2(-a.x, -a.y); }
-
 template <int MASK>
 __global__ void __launch_bounds__(256, 4) imtrans_bwd_nchw_image2_kernel(const float *__restrict__ dV, const void *__restrict__ Vm,
                                                                            float *__restrict__ dX, int B, int H, int W, int C, int nH,
@@ -864,23 +860,23 @@ __global__ void __launch_bounds__(256, 4) imtrans_bwd_nchw_image2_kernel(const f
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const float2 u1 = g[1][j], u2 = g[2][j];
-                    g[1][j] = f2add(f2sub(u1, u2), g[3][j]);
-                    g[2][j] = f2sub(f2add(u1, u2), g[0][j]);
-                    g[3][j] = f2neg(g[3][j]);
+                    g[1][j] = u1 - u2 + g[3][j];
+                    g[2][j] = u1 + u2 - g[0][j];
+                    g[3][j] = make_float2(-g[3][j].x, -g[3][j].y);
                 }
                 float *o = O + cl;
 #pragma unroll
                 for (int y = 0; y < 4; ++y) {
                     const int h = 2 * th - 1 + y;
                     if (h < 0 || h >= H) continue;
-                    const float2 d0 = g[y][0], d1 = f2add(f2sub(g[y][1], g[y][2]), g[y][3]), d2 = f2sub(f2add(g[y][1], g[y][2]), g[y][0]),
-                                 d3 = f2neg(g[y][3]);
+                    const float2 d0 = g[y][0], d1 = g[y][1] - g[y][2] + g[y][3], d2 = g[y][1] + g[y][2] - g[y][0],
+                                 d3 = make_float2(-g[y][3].x, -g[y][3].y);
                     const int w0 = 2 * tw - 1;
                     float *row = o + (h * W + w0) * CBP;
-                    if (w0 >= 0) { float2 *q = reinterpret_cast<float2 *>(row); *q = f2add(*q, d0); }
-                    { float2 *q = reinterpret_cast<float2 *>(row + CBP); *q = f2add(*q, d1); }
-                    if (w0 + 2 < W) { float2 *q = reinterpret_cast<float2 *>(row + 2 * CBP); *q = f2add(*q, d2); }
-                    if (w0 + 3 < W) { float2 *q = reinterpret_cast<float2 *>(row + 3 * CBP); *q = f2add(*q, d3); }
+                    if (w0 >= 0) { float2 *q = reinterpret_cast<float2 *>(row); *q = *q + d0; }
+                    { float2 *q = reinterpret_cast<float2 *>(row + CBP); *q = *q + d1; }
+                    if (w0 + 2 < W) { float2 *q = reinterpret_cast<float2 *>(row + 2 * CBP); *q = *q + d2; }
+                    if (w0 + 3 < W) { float2 *q = reinterpret_cast<float2 *>(row + 3 * CBP); *q = *q + d3; }
                 }
             }
         }
@@ -905,7 +901,7 @@ int imtrans_fwd(const float *X, float *V, void *signs_out, int B, int H, int W, 
     if (!X || !V || B <= 0 || H <= 0 || W <= 0 || C <= 0) return WG2X2_ERR_BAD_ARG;
     if ((scale == nullptr) != (shift == nullptr)) return WG2X2_ERR_BAD_ARG;
     signs_t *signs = static_cast<signs_t *>(signs_out);
-    if (signs && (scale || !aligned16(signs))) return WG2X2_ERR_BAD_ARG;
+    if (signs && (scale || !relu || !aligned16(signs))) return WG2X2_ERR_BAD_ARG;      // the ReLU's mask of a layer without an affine map
     if (layout != WG2X2_NHWC && layout != WG2X2_NCHW) return WG2X2_ERR_BAD_ARG;
     const int nH = (H + 1) / 2, nW = (W + 1) / 2;
     if (layout == WG2X2_NHWC) {
@@ -934,7 +930,7 @@ int imtrans_fwd(const float *X, float *V, void *signs_out, int B, int H, int W, 
             const int nbands = cdiv(nH, R), smem = (2 * R + 2) * (2 * nW + 2) * kPairPitch * (int)sizeof(float);
             if ((long long)B * nbands > 0x7fffffffLL) return WG2X2_ERR_UNSUPPORTED;
             auto *kernel = scale ? (relu ? imtrans_fwd_nchw_pair_kernel<true, true, false> : imtrans_fwd_nchw_pair_kernel<true, false, false>)
-                         : signs ? (relu ? imtrans_fwd_nchw_pair_kernel<false, true, true> : imtrans_fwd_nchw_pair_kernel<false, false, true>)
+                         : signs ? imtrans_fwd_nchw_pair_kernel<false, true, true>
                                  : (relu ? imtrans_fwd_nchw_pair_kernel<false, true, false> : imtrans_fwd_nchw_pair_kernel<false, false, false>);
             launch(kernel, dim3((unsigned)(B * nbands), C / kPairCB), 256, smem, st, X, V, signs, H, W, C, nH, nW, R, nbands,
                    (unsigned)cdiv(1 << 20, 2 * nW + 2), (unsigned)((long long)B * nH * nW * C * 4), scale, shift);

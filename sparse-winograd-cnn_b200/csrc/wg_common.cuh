@@ -163,8 +163,9 @@ __device__ __forceinline__ void stage_pairs(const float *__restrict__ X, float *
     asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-// The band height of the kernels that stage so (bands of 2 R + extra rows): least work of the busiest SM (a tile is 146 issue slots, a staged pixel 10 per 64 channels, and
-// a CTA costs something of its own), shared memory for three CTAs per SM.  0: too few CTAs to fill the GPU.
+// The band height of the kernels that stage so (bands of 2 R + extra rows): least work of the busiest SM (a tile is 146 issue slots, a
+// staged pixel 10 per 64 channels, and a CTA costs something of its own), shared memory for three CTAs per SM.  0: too few CTAs to
+// fill the GPU.
 inline int pair_rows(int B, int C, int nH, int nW, int W, int extra)
 {
     const long long per_band = (long long)B * cdiv(C, kPairCB);
