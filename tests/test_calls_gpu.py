@@ -66,6 +66,36 @@ def test_extras_off_16_bytes_stay_refused_where_only_the_wide_path_runs():
     assert e.value.status == -1
 
 
+@pytest.mark.parametrize("layout", ["NCHW", "NHWC"])
+@pytest.mark.parametrize("shape", [(1, 64, 64, 56, 56), (2, 32, 96, 9, 13), (16, 64, 64, 56, 56), (24, 256, 256, 14, 14), (24, 64, 64, 28, 28)])
+def test_residual_block(shape, layout):
+    """Both layers one by one, with the ReLUs and the addition by torch: the same kernels where the shortcut is a tensor (written in place),
+    and relu(x) where there is none."""
+    import wg2x2
+    B, C, K, H, W = shape
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    img = lambda c: rnd(B, c, H, W) if layout == "NCHW" else rnd(B, H, W, c)
+    x, short = img(C), img(K)
+    pa, pb = wg2x2.prepare_weights(rnd(16, C, K) / C ** 0.5), wg2x2.prepare_weights(rnd(16, K, K) / K ** 0.5)
+    bn = lambda c: (1 + 0.2 * rnd(c), 0.3 * rnd(c))
+    a, b, o = bn(C), bn(K), bn(K)
+    mid = wg2x2.layer_fwd_prepared(x, pa, K, relu=True, layout=layout, in_scale=a[0], in_shift=a[1])
+    main = wg2x2.layer_fwd_prepared(mid, pb, K, relu=True, layout=layout, in_scale=b[0], in_shift=b[1], out_scale=o[0], out_shift=o[1])
+    tol = 4 * 2.0 ** -24 * float(main.abs().max() + short.abs().max() + x.abs().max())         # the affine map and the addition, rounded once or twice
+    keep, x0 = short.clone(), x.clone()
+    y = wg2x2.residual_block(x, short, pa, a, pb, b, o, K, layout=layout)
+    assert y.data_ptr() == short.data_ptr() and torch.equal(x, x0)
+    assert float((y - (main + keep)).abs().max()) <= tol
+    if C == K:
+        y = wg2x2.residual_block(x, None, pa, a, pb, b, o, K, layout=layout)
+        assert y.data_ptr() != x.data_ptr() and torch.equal(x, x0)
+        assert float((y - (main + torch.relu(x))).abs().max()) <= tol
+    else:
+        with pytest.raises(ValueError):
+            wg2x2.residual_block(x, None, pa, a, pb, b, o, K, layout=layout)
+
+
 def _layer(g, C=16, K=8):
     import winograd_conv
     import winograd_imtrans
