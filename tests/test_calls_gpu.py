@@ -34,6 +34,15 @@ def test_two_threads_with_different_sizes_of_one_kernel():
     assert torch.equal(a(big), first) and torch.equal(b(big), first)
 
 
+# few tiles (clusters), many (the one kernel), many channels (wide path), a layout the one kernel does not take
+@pytest.mark.parametrize("shape,layout,one_kernel", [((1, 64, 64, 56, 56), "NCHW", False), ((64, 64, 64, 56, 56), "NCHW", True),
+                                                     ((128, 256, 256, 14, 14), "NCHW", False), ((64, 64, 64, 56, 56), "NHWC", False)])
+def test_fused_preferred(shape, layout, one_kernel):
+    import wg2x2
+    B, C, K, H, W = shape
+    assert wg2x2.fused_preferred(B, H, W, C, K, layout) == one_kernel
+
+
 # NCHW layers whose rows are whole 16-byte pieces have read out_scale, out_shift and residual at any alignment since the one-kernel layer
 # was their only path; the sizes here are now computed on clusters, by the wide path and by the one kernel
 @pytest.mark.parametrize("shape", [(48, 512, 128, 16, 16), (3, 512, 64, 28, 28), (1, 64, 64, 56, 56), (5, 48, 80, 28, 28), (16, 64, 64, 56, 56), (2, 128, 320, 8, 8)])
