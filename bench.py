@@ -317,7 +317,7 @@ class LayerFwd:
         cws_n = lib.wg2x2_conv_fwd_prepared_workspace_bytes(B, nH, nW, C, K) if self.prepared is not None else 0
         self.cws = torch.empty(cws_n, dtype=torch.uint8, device=ctx.dev) if cws_n else None   # products of the wide path (C, K >= 256)
         fused_ok = self.prepared is not None and layout == "NCHW" and wg2x2.fused_supported(B, H, W, C, K, "NCHW")
-        fused_pays = K <= 128 or (K <= 256 and C <= 64)          # the library's own rule (wg2x2_layer_fwd_prepared)
+        fused_pays = K <= 128 or (K <= 256 and C <= 64)          # the rule of wg2x2_layer_fwd_prepared for a layer of many tiles
         self.use_fused = fused_ok and (path == "fused" or (path == "auto" and fused_pays))
         self.bytesX, self.bytesV, self.bytesY, self.bytesW = 4 * B * C * H * W, 64 * self.P * C, 4 * B * K * H * W, 64 * C * K
         self.flops = 2.0 * 16 * self.P * C * K
@@ -702,7 +702,7 @@ def run_layer(args, ctx):
                    "l2": "%d rotating input buffers (%.0f MB); %.0f MB moved per step" % (L.nbuf, L.nbuf * L.bytesX / 1e6, L.layer_bytes() / 1e6),
                    "weights": "prepared once outside the timed region (wg2x2_weights_prepare)",
                    "timing": "two CUDA events around the steps; per-kernel durations from a separate pass afterwards",
-                   "path": "one fused kernel (wg2x2_layer_fwd_prepared's choice for this shape)" if L.use_fused else "two kernels, V through HBM"},
+                   "path": "one fused kernel (wg2x2_layer_fwd_fused)" if L.use_fused else "two kernels, V through HBM"},
         "layer_gbs": L.layer_bytes() * ctx.world / (ms_step * 1e-3) / 1e9,
         "layer_tflops": L.flops * ctx.world / (ms_step * 1e-3) / 1e12,
         "roofline": roof, "clocks": clocks, "gpu_launches": args.steps * (1 if L.use_fused else 2),
@@ -839,8 +839,8 @@ def main():
     ap.add_argument("--batch", type=int, default=0, help="override the per-GPU batch of the workload (profiling on a small case)")
     ap.add_argument("--e2e-chunks", type=int, default=2, help="chunks of the host-buffer pipeline")
     ap.add_argument("--path", default="auto", choices=["auto", "fused", "two-kernel"],
-                    help="layer forward: the one-kernel path (X -> Y, V never stored), the two kernels, or (auto) whichever "
-                         "wg2x2_layer_fwd_prepared picks for the shape")
+                    help="layer forward: the one-kernel path (X -> Y, V never stored), the two kernels, or (auto) the one "
+                         "kernel for K <= 128, or K <= 256 with C <= 64")
     ap.add_argument("--fused", action="store_true", help="same as --path fused")
     ap.add_argument("--net-layout", default="NCHW", choices=["NHWC", "NCHW"],
                     help="cfg4: physical layout of the activations (NCHW: the 56x56 and 28x28 layers run as one kernel each)")

@@ -201,9 +201,10 @@ int wg2x2_relu_mean(const float *X, float *out, long long planes, int n, void *s
 /*
  * Whole layer forward with prepared weights (tensor-core path), the call pair of
  * ResNet-18-var/imagenet-resnet-transWino-prune.py:118-119 in its fastest form for the shape that needs no scratch
- * memory beyond V_scratch (wg2x2_layer_fwd_prepared_ws adds the wide path for C, K >= 256):
+ * memory beyond V_scratch (wg2x2_layer_fwd_prepared_ws adds the wide path):
+ *  - one kernel on clusters of four CTAs where there are few tiles (either layout, any image size);
  *  - one kernel (wg2x2_layer_fwd_fused) where that is supported (NCHW, W % 4 == 0, C % 16 == 0, X and Y
- *    16-byte aligned) and either it is the faster one (K <= 128, or K <= 256 with C <= 64) or no V_scratch
+ *    16-byte aligned) and either K <= 128, or K <= 256 with C <= 64, or a cost model prefers it, or no V_scratch
  *    was given: both transforms and the ReLU happen on the SM, neither the transformed input nor the
  *    products are written to memory;
  *  - otherwise the two kernels with V_scratch (16*B*nH*nW*C floats) in between; WG2X2_ERR_WORKSPACE if NULL.
@@ -213,10 +214,10 @@ int wg2x2_layer_fwd_prepared(const float *X, const void *prepared, float *Y, flo
                              int C, int K, int layout, int relu, const float *out_scale, const float *out_shift,
                              const float *residual, void *stream);
 /*
- * The same with scratch memory for the products, which lets layers with many channels (C, K >= 256) or few tiles take
- * their fastest form too: input transform into V_scratch, then the wide path of wg2x2_conv_fwd_prepared_ws through
- * `workspace` (wg2x2_layer_fwd_prepared_workspace_bytes; 0 = the shape does not use one).  With workspace == NULL, or
- * for other shapes, this is wg2x2_layer_fwd_prepared.
+ * The same with scratch memory for the products, which lets layers with many channels (C, K >= 256), and others where the cost model
+ * says so, take the wide path of wg2x2_conv_fwd_prepared_ws through `workspace` (wg2x2_layer_fwd_prepared_workspace_bytes; 0 = the
+ * shape does not use one) behind the input transform into V_scratch.  With workspace == NULL, or for other shapes, this is
+ * wg2x2_layer_fwd_prepared.
  */
 int wg2x2_layer_fwd_prepared_ws(const float *X, const void *prepared, float *Y, float *V_scratch, int B, int H, int W,
                                 int C, int K, int layout, int relu, const float *out_scale, const float *out_shift,
@@ -239,7 +240,8 @@ int wg2x2_layer_fwd_prepared_ex(const float *X, const float *in_scale, const flo
 void wg2x2_layer_fwd_prepared_scratch(int B, int H, int W, int C, int K, int layout, int aligned, size_t *v_bytes,
                                       size_t *workspace_bytes);
 int wg2x2_layer_fwd_fused_supported(int B, int H, int W, int C, int K, int layout);
-/* 1 where wg2x2_layer_fwd_prepared_ws runs the one kernel even if both scratch buffers are given (it then reads neither). */
+/* 1 where wg2x2_layer_fwd_prepared_ws runs the one-kernel NCHW layer even if both scratch buffers are given (it then reads neither);
+ * 0 where it runs the whole layer on clusters. */
 int wg2x2_layer_fwd_fused_preferred(int B, int H, int W, int C, int K, int layout);
 /* The one-kernel layer forward on its own (NCHW in and out); WG2X2_ERR_UNSUPPORTED outside the shapes above.
  * residual may be Y itself: the result is then added into Y in place (the TMA unit does the addition);

@@ -834,8 +834,8 @@ int conv_bwd_tc(const float *V, const float *Wt, const float *dY, const float *m
 }
 
 // ---------------------------------------------------------------------------------------
-// Wide forward path for layers with many channels (C, K >= 256): the 16 products as plain GEMMs with
-// N = 256 output channels per unit (conv_grad_gemm_tc_kernel<1>: same operands' major-ness as dV), the
+// Wide forward path, for layers with many channels (C, K >= 256) and wherever conv_fwd_wide_preferred says: the 16 products as plain
+// GEMMs with up to N = 256 output channels per unit (conv_grad_gemm_tc_kernel<1>: same operands' major-ness as dV), the
 // products M (16, P, K) written once to scratch memory, then one HBM-bound pass for A^T m A.  With N = 64
 // (the row-walk kernel, which needs four accumulators live per unit) every A tile is re-read from L2 and
 // from shared memory four times as often, and that, not HBM, is what bounds these shapes.

@@ -7,10 +7,10 @@ the `a` blocks carry a 1x1 shortcut convolution + BatchNorm, the `b` blocks an i
 after a ReLU.  The reference has `pool4` commented out (:191), so its stage 5 runs at 14x14;
 `stage5_pool=True` restores the pool (7x7), which is the shape the benchmark configuration names.
 
-The Winograd layers and (for NCHW activations) the max-pools run on this repository's kernels; the stem, 1x1
-shortcuts and the classifier are stock torch ops.  With layout="NCHW" the layers of the two high-resolution stages (56x56 and 28x28) run
-as one kernel each, BatchNorms and shortcut add included.  Weights are random (seeded): there is
-no checkpoint to load here.
+The Winograd layers and, for NCHW activations, the stem, the pools and the 1x1 shortcuts of few pixels run on this repository's
+kernels; the other 1x1 shortcuts and the classifier are stock torch ops.  With layout="NCHW" the layers of the two high-resolution
+stages (56x56 and 28x28) run as one kernel each, BatchNorms and shortcut add included (a shortcut that goes through a ReLU first gets
+it in a pass of its own there, and inside the last kernel elsewhere).  Weights are random (seeded): there is no checkpoint to load here.
 """
 import numpy as np
 import torch

@@ -131,7 +131,8 @@ def fused_supported(B, H, W, C, K, layout="NCHW"):
 
 
 def fused_preferred(B, H, W, C, K, layout="NCHW"):
-    """True where layer_fwd_prepared runs the whole layer as one kernel."""
+    """True where layer_fwd_prepared runs the one-kernel NCHW layer (layer_fwd_fused) by choice; False where it runs the whole layer on
+    clusters, as for few tiles, or transform and product as kernels of their own."""
     return bool(lib.wg2x2_layer_fwd_fused_preferred(B, H, W, C, K, _LAYOUTS[layout]))
 
 
