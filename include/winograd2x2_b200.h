@@ -231,7 +231,8 @@ size_t wg2x2_layer_fwd_prepared_workspace_bytes(int B, int H, int W, int C, int 
  * wg2x2_layer_fwd_prepared_scratch: the bytes of V_scratch and workspace with which the call is fastest (0: not used);
  * `aligned`: whether all of those pointers are on 16-byte boundaries.
  * out_scale, out_shift and residual may be at any alignment where the one-kernel layer is supported (X and Y aligned) and C < 256 or
- * K < 256; that layer is then taken and needs no scratch.
+ * K < 256; that layer is then taken and needs no scratch.  Y may lie over X where V_scratch is given: the transform is then always a
+ * kernel of its own.  (wg2x2_layer_fwd_prepared_scratch: `aligned` = 0 for such a call.)
  */
 int wg2x2_layer_fwd_prepared_ex(const float *X, const float *in_scale, const float *in_shift, const void *prepared, float *Y,
                                 float *V_scratch, int B, int H, int W, int C, int K, int layout, int relu,

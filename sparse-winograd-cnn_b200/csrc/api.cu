@@ -284,14 +284,18 @@ int wg2x2_layer_fwd_prepared_ex(const float *X, const float *in_scale, const flo
     auto on16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     const bool aligned = on16(X) && on16(Y);           // TMA and 16-byte accesses both ways
     const bool wide = V_scratch && workspace && conv_fwd_wide_preferred((long long)B * nH * nW, C, K);
-    if (aligned && on16(residual) && on16(in_scale) && on16(in_shift) && layer_cluster_preferred(B, H, W, C, K, layout))
+    // Y over X: only with V in between is all of X read before any of Y is written
+    const uintptr_t x0 = reinterpret_cast<uintptr_t>(X), y0 = reinterpret_cast<uintptr_t>(Y);
+    const uintptr_t pixels = sizeof(float) * (uintptr_t)B * H * W;
+    const bool apart = x0 + pixels * C <= y0 || y0 + pixels * K <= x0 || !V_scratch;
+    if (aligned && apart && on16(residual) && on16(in_scale) && on16(in_shift) && layer_cluster_preferred(B, H, W, C, K, layout))
         return layer_fwd_cluster(X, prepared, Y, B, H, W, C, K, layout, relu, in_scale, in_shift, out_scale, out_shift, residual, residual_relu, st);
     // The one-kernel layer: where it is the fastest; without scratch for the wide path, where there are few blocks of 64 output channels
     // (each redoes the input transform; measured: K <= 128, or K <= 256 with C <= 64), or always without any scratch; and where out_scale,
     // out_shift or residual is off a 16-byte boundary, which it alone reads so (but not for C, K >= 256 with scratch: such a call has
     // always been the wide path's, which refuses it).
     const bool extras_on16 = on16(out_scale) && on16(out_shift) && on16(residual);
-    if (aligned && fused_fwd_supported(B, H, W, C, K, layout) &&
+    if (aligned && apart && fused_fwd_supported(B, H, W, C, K, layout) &&
         (layer_fused_preferred(B, H, W, C, K, layout) || (!wide && (K <= 128 || (K <= 256 && C <= 64) || !V_scratch)) ||
          (!extras_on16 && (C < 256 || K < 256))))
         return layer_fwd_fused(X, prepared, Y, B, H, W, C, K, relu, in_scale, in_shift, out_scale, out_shift, residual, residual_relu, st);

@@ -558,8 +558,9 @@ void layer_fwd_prepared(const Tensor &x, const Tensor &prep, const Tensor &Y, co
                         const Tensor &in_shift, const Tensor &out_scale, const Tensor &out_shift, const Tensor &residual, bool residual_relu,
                         const Tensor &V, const Tensor &uws, void *stream)
 {
-    const bool xy = on16(x) && on16(Y), extras = on16(out_scale) && on16(out_shift) && on16(residual);
-    // (extras off 16 bytes are the one-kernel layer's, or the cluster kernel's; neither reads scratch)
+    const bool apart = x.const_data_ptr<float>() + x.numel() <= Y.const_data_ptr<float>() || Y.const_data_ptr<float>() + Y.numel() <= x.const_data_ptr<float>();
+    const bool xy = on16(x) && on16(Y) && apart, extras = on16(out_scale) && on16(out_shift) && on16(residual);
+    // (Y over X needs V in between; extras off 16 bytes are the one-kernel layer's, or the cluster kernel's; neither reads scratch)
     const bool one_kernel = xy && !extras && (d.C < 256 || K < 256) && wg2x2_layer_fwd_fused_supported(d.B, d.H, d.W, d.C, K, layout);
     const LayerScratch s(d, K, layout, xy && on16(residual) && on16(in_scale) && on16(in_shift), one_kernel, V, uws);
     check(wg2x2_layer_fwd_prepared_ex(cptr(x), cptr(in_scale), cptr(in_shift), prep.data_ptr(), ptr(Y), s.v, d.B, d.H, d.W, d.C, K, layout, relu,

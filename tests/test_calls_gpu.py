@@ -66,6 +66,23 @@ def test_extras_at_any_alignment(shape):
         assert float((got - want).abs().max()) <= 2e-3 * scale
 
 
+# few tiles, the one kernel's sizes, many channels: where the layer could run as one kernel, a CTA would read pixels that another has written over
+@pytest.mark.parametrize("layout", ["NCHW", "NHWC"])
+@pytest.mark.parametrize("shape", [(2, 32, 9, 13), (1, 64, 56, 56), (16, 64, 56, 56), (4, 256, 14, 14), (2, 256, 8, 8)])
+def test_output_over_the_input(shape, layout):
+    import wg2x2
+    B, C, H, W = shape
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    x, prepared = rnd(B, C, H, W) if layout == "NCHW" else rnd(B, H, W, C), wg2x2.prepare_weights(rnd(16, C, C) / C ** 0.5)
+    for residual in (None, x.clone()):
+        want = wg2x2.layer_fwd_prepared(x, prepared, C, layout=layout, residual=residual)
+        y = x.clone()
+        got = wg2x2.layer_fwd_prepared(y, prepared, C, layout=layout, out=y, residual=None if residual is None else y)
+        assert got.data_ptr() == y.data_ptr()
+        assert float((got - want).abs().max()) <= 2e-3 * float(want.abs().max())        # another path at worst, as above
+
+
 def test_extras_off_16_bytes_stay_refused_where_only_the_wide_path_runs():
     import wg2x2
     x, prepared = torch.zeros((48, 256, 16, 16), device="cuda"), wg2x2.prepare_weights(torch.zeros((16, 256, 256), device="cuda"))
