@@ -20,6 +20,7 @@ struct C1Params {
     long long pixels;        // B * HW
     int C, K, HW, chunks;
     uint32_t spin_limit;
+    int drop_load;           // test hook: CTA 0 stops in front of this weight load, so that the wait for it runs out
 };
 
 __global__ void __launch_bounds__(kC1Threads) conv1x1_tc_kernel(const __grid_constant__ CUtensorMap mapW, const C1Params prm)
@@ -81,6 +82,7 @@ __global__ void __launch_bounds__(kC1Threads) conv1x1_tc_kernel(const __grid_con
         const bool leader = elect_one();
         if (leader)
             for (int cc = 0; cc < prm.chunks; ++cc) {
+                if (cc == prm.drop_load && blockIdx.x == 0 && blockIdx.y == 0) break;
                 mbar_expect_tx(full0 + 8u * cc, kBBytes);
                 tma_load_3d(base + cc * kC1StageBytes + kABytes, &mapW, full0 + 8u * cc, cc * kBlockK, k0, 0);
             }
@@ -117,6 +119,7 @@ __global__ void __launch_bounds__(kC1Threads) conv1x1_tc_kernel(const __grid_con
     tc_fence_before();
     __syncthreads();
     if (warp == 8) {
+        if (!done) let_them_land();
         tc_fence_after();
         tmem_dealloc(tmem_base, 64);
     }
@@ -140,6 +143,7 @@ int conv1x1(const float *X, const float *W, float *Y, int B, int C, int K, int H
     C1Params p;
     p.X = X; p.Y = Y; p.pixels = (long long)B * HW; p.C = C; p.K = K; p.HW = HW; p.chunks = cdiv(C, kBlockK);
     p.spin_limit = wait_limit();
+    p.drop_load = take_drop_load();
     const long long blocks = cdivll(p.pixels, kBlockM);
     if (blocks > 0x7fffffffLL || cdiv(K, kBlockN) > 65535) return WG2X2_ERR_UNSUPPORTED;
     EncodeTiledFn fn = encode_fn();

@@ -93,7 +93,8 @@ static __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.comm
 static __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 // TMA boxes of a (16, rows, columns) matrix, and the warp's wait for one.  The wait is bounded as everywhere in this library;
-// one that runs out leaves a note in the status word and the warp goes on (its results are then incomplete).
+// one that runs out leaves a note in the status word and gives the copy a last millisecond, and the warp goes on (its results are then
+// incomplete).
 static __device__ __forceinline__ uint32_t ff_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 static __device__ __forceinline__ void ff_tma(float *dst, const CUtensorMap *map, uint32_t bar, int c0, int c1, int c2)
 {
@@ -114,6 +115,7 @@ static __device__ __forceinline__ void ff_wait(uint32_t bar, uint32_t parity, un
     }
     status[1] = 0x1E00u;
     status[0] = 1;
+    for (int it = 0; it < 1000; ++it) __nanosleep(1000);
 }
 struct FfWait {
     unsigned int *status;      // the library's status word

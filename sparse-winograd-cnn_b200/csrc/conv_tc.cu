@@ -102,6 +102,12 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
     return __all_sync(0xffffffffu, ok);
 }
 
+// After a wait that gave up: copies and MMAs already in flight get about a millisecond to end before the CTA hands back its memories
+__device__ __forceinline__ void let_them_land()
+{
+    for (int it = 0; it < 1000; ++it) __nanosleep(1000);
+}
+
 // true in exactly one lane of the (converged) warp
 __device__ __forceinline__ bool elect_one()
 {

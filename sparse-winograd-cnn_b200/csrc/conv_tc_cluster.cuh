@@ -329,6 +329,7 @@ layer_fwd_cluster_kernel(const __grid_constant__ CUtensorMap mapW, const ClParam
     tc_fence_before();
     cluster_sync_all();              // all four rows have arrived; nobody writes here any more
     if (warp == kClWarps) {
+        if (!done) let_them_land();
         tc_fence_after();
         tmem_dealloc(tmem_base, 4 * kClMaxN);
     }

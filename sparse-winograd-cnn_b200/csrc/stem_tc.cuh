@@ -329,6 +329,7 @@ __global__ void __launch_bounds__(kStThreads, 1) stem_pool_kernel(const StParams
     tc_fence_before();
     __syncthreads();
     if (warp == 4) {
+        if (*abort_flag) let_them_land();
         tc_fence_after();
         tmem_dealloc(tmem_base, kTmemCols);
     }

@@ -92,3 +92,20 @@ def test_fused_layer_kernel_times_out_and_recovers(wg, oracle, nth):
     Xn = np.ascontiguousarray(np.transpose(X, (0, 2, 3, 1)))
     want = oracle.conv_fwd(oracle.imtrans_fwd(Xn, relu=True, dtype=np.float32), Wt, H, W)
     assert oracle.max_rel(np.transpose(Y, (0, 2, 3, 1)), want) <= TOL_TF32
+
+
+@pytest.mark.parametrize("nth", [0, 3])
+def test_conv1x1_kernel_times_out_and_recovers(wg, nth):
+    from wg2x2._lib import lib
+    g = torch.Generator(device="cuda").manual_seed(4)
+    x, w = torch.randn((1, 256, 7, 7), generator=g, device="cuda"), wg.round_tf32(torch.randn((512, 256, 1, 1), generator=g, device="cuda"))
+    want = wg.conv1x1(x, w)
+    lib.wg2x2_set_wait_limit(20000)
+    lib.wg2x2_test_drop_load(nth)
+    wg.conv1x1(x, w)
+    st, where = wg.last_device_status()
+    assert st == TIMEOUT
+    # the MMA issuer waiting for the chunk that never came (0x1A), or the warps that wait for the accumulator all along (0x1B)
+    assert where in (0x1A00 | nth, 0x1B00), "0x%x" % where
+    lib.wg2x2_set_wait_limit(0)
+    assert torch.equal(wg.conv1x1(x, w), want) and wg.last_device_status()[0] == 0
