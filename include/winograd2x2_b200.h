@@ -306,7 +306,7 @@ int wg2x2_last_device_status(void *stream, unsigned int *where);
 int wg2x2_set_wait_limit(long long polls);
 /*
  * Test hooks for the time-out path (they fault and hang nothing).  wg2x2_test_drop_load(n): in the next
- * launch of conv_fwd (row-walk) or layer_fwd_fused, CTA 0's weight producer stops before its n-th load, so the
+ * launch of conv_fwd (row-walk), layer_fwd_fused or conv1x1, CTA 0's weight producer stops before its n-th load, so the
  * MMA issuer's wait for that stage runs out; one-shot, n < 0 disarms.  wg2x2_test_wait_probe: a one-thread
  * kernel that waits `polls` polls on a barrier nobody arrives on and records `where`.
  */
