@@ -13,6 +13,7 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 
 #include <mutex>
 
@@ -754,11 +755,12 @@ PyObject *py_stem_pool(WG_ARGS)
     END_HANDLE_TH_ERRORS
 }
 
-// I, relu, layout: differentiable
+// I, relu, layout: differentiable; NotImplemented while torch.jit.trace is on, which does not see native calls
 PyObject *py_imtrans_op(WG_ARGS)
 {
     HANDLE_TH_ERRORS
     want(n, 3);
+    if (torch::jit::tracer::isTracing()) Py_RETURN_NOTIMPLEMENTED;
     if (!THPVariable_Check(a[0])) not_a_tensor("x");
     const Tensor I = THPVariable_Unpack(a[0]);
     const bool relu = arg_bool(a[1]);
@@ -769,11 +771,12 @@ PyObject *py_imtrans_op(WG_ARGS)
     END_HANDLE_TH_ERRORS
 }
 
-// I, W, out_h, out_w, layout, math, mask: differentiable in I and W
+// I, W, out_h, out_w, layout, math, mask: differentiable in I and W; NotImplemented as above
 PyObject *py_conv_op(WG_ARGS)
 {
     HANDLE_TH_ERRORS
     want(n, 7);
+    if (torch::jit::tracer::isTracing()) Py_RETURN_NOTIMPLEMENTED;
     if (!THPVariable_Check(a[0])) not_a_tensor("V");
     if (!THPVariable_Check(a[1])) not_a_tensor("Wt");
     const Tensor I = THPVariable_Unpack(a[0]), Wt = THPVariable_Unpack(a[1]);

@@ -9,8 +9,6 @@ from . import _native
 
 _native.set_error(Wg2x2Error)
 
-_tracing = torch._C._get_tracing_state       # None outside torch.jit.trace
-
 _LAYOUTS = {"NHWC": NHWC, "NCHW": NCHW, NHWC: NHWC, NCHW: NCHW}
 _MATHS = {"fp32": MATH_FP32, "tf32": MATH_TF32, MATH_FP32: MATH_FP32, MATH_TF32: MATH_TF32}
 
@@ -80,9 +78,8 @@ class _ConvTraced(torch.autograd.Function):
 
 def imtrans_op(x, relu=False, layout="NHWC"):
     """imtrans_fwd for autograd: differentiable in x (any strides), the ReLU mask applied inside the gradient's gather."""
-    if _tracing() is not None:
-        return _ImTransTraced.apply(x, bool(relu), _LAYOUTS[layout])
-    return _native.imtrans_op(x, relu, _LAYOUTS[layout])
+    V = _native.imtrans_op(x, relu, _LAYOUTS[layout])
+    return V if V is not NotImplemented else _ImTransTraced.apply(x, bool(relu), _LAYOUTS[layout])
 
 
 def conv_fwd(V, Wt, out_h=None, out_w=None, layout="NHWC", math="fp32", out=None, workspace=None):
@@ -92,9 +89,11 @@ def conv_fwd(V, Wt, out_h=None, out_w=None, layout="NHWC", math="fp32", out=None
 
 def conv_op(V, Wt, out_h=None, out_w=None, layout="NHWC", math="fp32", mask=None):
     """conv_fwd for autograd: differentiable in V and Wt (any strides).  mask (16,C,K), constant: the weights are Wt * mask."""
-    if _tracing() is not None:
-        return _ConvTraced.apply(V, Wt if mask is None else Wt * mask, *(None if n is None else int(n) for n in (out_h, out_w)), _LAYOUTS[layout], _MATHS[math])
-    return _native.conv_op(V, Wt, out_h, out_w, _LAYOUTS[layout], _MATHS[math], mask)
+    Y = _native.conv_op(V, Wt, out_h, out_w, _LAYOUTS[layout], _MATHS[math], mask)
+    if Y is NotImplemented:
+        out_hw = (None if n is None else int(n) for n in (out_h, out_w))
+        Y = _ConvTraced.apply(V, Wt if mask is None else Wt * mask, *out_hw, _LAYOUTS[layout], _MATHS[math])
+    return Y
 
 
 def prepare_weights(Wt):
