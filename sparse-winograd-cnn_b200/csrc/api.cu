@@ -37,6 +37,10 @@ int conv_fwd_tc_wide(const float *V, const void *prepared, float *Y, int B, int 
 bool fused_fwd_supported(int B, int H, int W, int C, int K, int layout);
 bool layer_fused_preferred(int B, int H, int W, int C, int K, int layout);
 bool layer_cluster_preferred(int B, int H, int W, int C, int K, int layout);
+bool layer_pair_preferred(int B, int H, int W, int C, int K, int layout);
+int layer_fwd_pair(const float *X, const void *prepared, float *Y, int B, int H, int W, int C, int K, int relu,
+                   const float *in_scale, const float *in_shift, const float *out_scale, const float *out_shift,
+                   const float *residual, int res_relu, cudaStream_t st);
 bool fused_beats_wide(int B, int H, int W, int C, int K, int layout, double *us);
 int layer_fwd_fused(const float *X, const void *prepared, float *Y, int B, int H, int W, int C, int K, int relu,
                     const float *in_scale, const float *in_shift, const float *out_scale, const float *out_shift,
@@ -253,6 +257,11 @@ int wg2x2_layer_fwd_fused_preferred(int B, int H, int W, int C, int K, int layou
     return (B > 0 && H > 0 && W > 0 && C > 0 && K > 0 && layer_fused_preferred(B, H, W, C, K, layout)) ? 1 : 0;
 }
 
+int wg2x2_layer_fwd_pair_preferred(int B, int H, int W, int C, int K, int layout)
+{
+    return (B > 0 && H > 0 && W > 0 && C > 0 && K > 0 && layer_pair_preferred(B, H, W, C, K, layout)) ? 1 : 0;
+}
+
 size_t wg2x2_layer_fwd_prepared_workspace_bytes(int B, int H, int W, int C, int K)
 {
     if (B <= 0 || H <= 0 || W <= 0 || C <= 0 || K <= 0) return 0;
@@ -266,7 +275,8 @@ void wg2x2_layer_fwd_prepared_scratch(int B, int H, int W, int C, int K, int lay
 {
     *v_bytes = *workspace_bytes = 0;
     if (B <= 0 || H <= 0 || W <= 0 || C <= 0 || K <= 0 || !layout_ok(layout)) return;
-    if (aligned && (layer_cluster_preferred(B, H, W, C, K, layout) || layer_fused_preferred(B, H, W, C, K, layout))) return;
+    if (aligned && (layer_pair_preferred(B, H, W, C, K, layout) || layer_cluster_preferred(B, H, W, C, K, layout) || layer_fused_preferred(B, H, W, C, K, layout)))
+        return;
     const int nH = (H + 1) / 2, nW = (W + 1) / 2;
     *workspace_bytes = wg2x2_conv_fwd_prepared_workspace_bytes(B, nH, nW, C, K);
     if (*workspace_bytes || !aligned || !fused_fwd_supported(B, H, W, C, K, layout)) *v_bytes = sizeof(float) * 16 * (size_t)B * nH * nW * C;
@@ -288,13 +298,15 @@ int wg2x2_layer_fwd_prepared_ex(const float *X, const float *in_scale, const flo
     const uintptr_t x0 = reinterpret_cast<uintptr_t>(X), y0 = reinterpret_cast<uintptr_t>(Y);
     const uintptr_t pixels = sizeof(float) * (uintptr_t)B * H * W;
     const bool apart = x0 + pixels * C <= y0 || y0 + pixels * K <= x0 || !V_scratch;
+    const bool extras_on16 = on16(out_scale) && on16(out_shift) && on16(residual);
+    if (aligned && apart && extras_on16 && layer_pair_preferred(B, H, W, C, K, layout))
+        return layer_fwd_pair(X, prepared, Y, B, H, W, C, K, relu, in_scale, in_shift, out_scale, out_shift, residual, residual_relu, st);
     if (aligned && apart && on16(residual) && on16(in_scale) && on16(in_shift) && layer_cluster_preferred(B, H, W, C, K, layout))
         return layer_fwd_cluster(X, prepared, Y, B, H, W, C, K, layout, relu, in_scale, in_shift, out_scale, out_shift, residual, residual_relu, st);
     // The one-kernel layer: where it is the fastest; without scratch for the wide path, where there are few blocks of 64 output channels
     // (each redoes the input transform; measured: K <= 128, or K <= 256 with C <= 64), or always without any scratch; and where out_scale,
     // out_shift or residual is off a 16-byte boundary, which it alone reads so (but not for C, K >= 256 with scratch: such a call has
     // always been the wide path's, which refuses it).
-    const bool extras_on16 = on16(out_scale) && on16(out_shift) && on16(residual);
     if (aligned && apart && fused_fwd_supported(B, H, W, C, K, layout) &&
         (layer_fused_preferred(B, H, W, C, K, layout) || (!wide && (K <= 128 || (K <= 256 && C <= 64) || !V_scratch)) ||
          (!extras_on16 && (C < 256 || K < 256))))

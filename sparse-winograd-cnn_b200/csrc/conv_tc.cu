@@ -16,6 +16,7 @@
 // and returns (status readable through wg2x2_last_device_status).
 #include <cuda.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstring>
 
@@ -842,6 +843,7 @@ void dw_reduce_launch(const float *partial, const float *mask, float *dW, long l
 #include "conv_tc_bwd.cuh"
 #include "conv_tc_cluster.cuh"
 #include "conv_tc_fused.cuh"
+#include "conv_tc_pair.cuh"
 #include "stem_tc.cuh"
 #include "conv1x1_tc.cuh"
 

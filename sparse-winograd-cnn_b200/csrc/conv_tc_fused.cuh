@@ -830,11 +830,13 @@ static bool fused_geometry(FuParams &p)
 
 // The shortcut, ReLU applied, into the output buffer that the kernel then adds to (in place where they are one).  dst is on a
 // 16-byte boundary, src need not be.
-__global__ void __launch_bounds__(256) relu_copy_kernel(const float *src, float *dst, long long n4)
+__global__ void __launch_bounds__(256) relu_copy_kernel(const float *src, float *dst, long long n)
 {
     after_previous_kernel(src, dst);
     const bool vec = (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
     float4 *d = reinterpret_cast<float4 *>(dst);
+    const long long n4 = n / 4;
+    if (blockIdx.x == 0 && threadIdx.x < (n & 3)) dst[4 * n4 + threadIdx.x] = relu_nan(src[4 * n4 + threadIdx.x]);
     for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n4; i += (long long)gridDim.x * 256)
         d[i] = relu_nan(vec ? reinterpret_cast<const float4 *>(src)[i] : make_float4(src[4 * i], src[4 * i + 1], src[4 * i + 2], src[4 * i + 3]));
 }
@@ -855,7 +857,7 @@ int layer_fwd_fused(const float *X, const void *prepared, float *Y, int B, int H
     p.accumulate = residual != nullptr;
     if (residual && res_relu) {
         const long long n4 = (long long)B * K * H * W / 4;         // W % 4 == 0 here
-        const int s = launch(relu_copy_kernel, dim3((unsigned)(n4 < 256LL * 32 * kNumSMs ? cdivll(n4, 256) : 32 * kNumSMs)), 256, 0, st, residual, Y, n4);
+        const int s = launch(relu_copy_kernel, dim3((unsigned)(n4 < 256LL * 32 * kNumSMs ? cdivll(n4, 256) : 32 * kNumSMs)), 256, 0, st, residual, Y, 4 * n4);
         if (s != WG2X2_OK) return s;
     } else if (residual && residual != Y &&
                cudaMemcpyAsync(Y, residual, sizeof(float) * (size_t)B * K * H * W, cudaMemcpyDeviceToDevice, st) != cudaSuccess) {
@@ -945,26 +947,26 @@ bool fused_beats_wide(int B, int H, int W, int C, int K, int layout, double *us)
     return fused <= wide;
 }
 
-// The layer of few tiles on clusters (conv_tc_cluster.cuh) against the others, all in microseconds: the one-kernel layer above,
-// the wide path, or transform + row-walk kernel (the formulas of the rules that choose among those).  1 x 14 x 14 with 256
-// channels 11.7 -> 9.0 us, 82 x 5 x 5 tiles of 64 channels 16.8 -> 7.6; above about 33 clusters' worth of work the wide path wins.
+// The one-kernel layer above, the wide path, or transform + row-walk kernel, whichever the rules that choose among those take: microseconds
+static double unpaired_us(int B, int H, int W, int C, int K, int layout)
+{
+    const long long P = (long long)B * ((H + 1) / 2) * ((W + 1) / 2);
+    const double pixels = (double)B * H * W;
+    double us = 0.0;
+    if (fused_beats_wide(B, H, W, C, K, layout, &us)) return us;
+    if (conv_fwd_wide_preferred(P, C, K)) return 9.5 + (4.0 * pixels * ((double)C + K) + 128.0 * P * ((double)C + K)) / 5.3e6;
+    const double rounds = (double)cdivll(cdivll(P, kBlockM) * cdiv(K, kBlockN), kNumSMs);
+    return fmax(7.5 + rounds * 4.3 * cdiv(C, kBlockK), 5.0 + (64.0 * P * C + 16.0 * P * K) / 6e6) + 3.0 + (4.0 * pixels + 64.0 * P) * C / 5e6;
+}
+
+// The layer of few tiles on clusters (conv_tc_cluster.cuh) against those.  1 x 14 x 14 with 256 channels 11.7 -> 9.0 us, 82 x 5 x 5
+// tiles of 64 channels 16.8 -> 7.6; above about 33 clusters' worth of work the wide path wins.
 bool layer_cluster_preferred(int B, int H, int W, int C, int K, int layout)
 {
     if (!tc_shape_supported(C, K)) return false;
     const long long P = (long long)B * ((H + 1) / 2) * ((W + 1) / 2);
     if (P > 0x7fffffffLL - kBlockM) return false;
-    const double pixels = (double)B * H * W;
-    double other = 0.0;
-    if (!fused_beats_wide(B, H, W, C, K, layout, &other)) {
-        if (conv_fwd_wide_preferred(P, C, K)) {
-            other = 9.5 + (4.0 * pixels * ((double)C + K) + 128.0 * P * ((double)C + K)) / 5.3e6;
-        } else {
-            const double rounds = (double)cdivll(cdivll(P, kBlockM) * cdiv(K, kBlockN), kNumSMs);
-            other = fmax(7.5 + rounds * 4.3 * cdiv(C, kBlockK), 5.0 + (64.0 * P * C + 16.0 * P * K) / 6e6) + 3.0 +
-                    (4.0 * pixels + 64.0 * P) * C / 5e6;
-        }
-    }
-    return cl_cut(P, C, K).us < 0.97 * other;
+    return cl_cut(P, C, K).us < 0.97 * unpaired_us(B, H, W, C, K, layout);
 }
 
 bool layer_fused_preferred(int B, int H, int W, int C, int K, int layout)

@@ -130,15 +130,15 @@ def fused_supported(B, H, W, C, K, layout="NCHW"):
 
 
 def fused_preferred(B, H, W, C, K, layout="NCHW"):
-    """True where layer_fwd_prepared runs the one-kernel NCHW layer (layer_fwd_fused) by choice; False where it runs the whole layer on
-    clusters, as for few tiles, or transform and product as kernels of their own."""
+    """True where the one-kernel NCHW layer (layer_fwd_fused) is preferred to transform and product as kernels of their own and to the
+    layer on clusters, as for few tiles.  (Many tiles go to the layer on pairs of SMs before that is asked.)"""
     return bool(lib.wg2x2_layer_fwd_fused_preferred(B, H, W, C, K, _LAYOUTS[layout]))
 
 
 def layer_fwd_prepared(x, prepared, K, relu=True, layout="NHWC", out=None, V_scratch=None, out_scale=None, out_shift=None,
                        residual=None, workspace=None, in_scale=None, in_shift=None, residual_relu=False):
     """Whole layer with prepared weights: one kernel where supported and faster (V never stored: a kernel of its own for few
-    tiles, the NCHW one for few channels), else transform + product through V_scratch (allocated here when not given); layers
+    tiles, NCHW ones for many tiles and for few channels), else transform + product through V_scratch (allocated here when not given); layers
     with many channels take the wide product path through `workspace` (allocated here when not given;
     layer_fwd_prepared_workspace_bytes).  in_scale / in_shift (C,): affine map of the pixels in front of the transform, the
     padding stays zero; residual_relu: the shortcut passes through a ReLU first."""

@@ -1,0 +1,126 @@
+"""The layer on pairs of SMs (csrc/conv_tc_pair.cuh) through layer_fwd_prepared, at sizes where its cuts can go wrong: row lengths of
+each alignment, quads that cross rows and images, images copied whole, channel counts that end inside a slot, a weight stage or a block
+of outputs, weights that stay in shared memory and weights that stream, a last unit with one CTA's quads only."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+TOL_TF32 = 5e-3
+
+
+# B, C, K, H, W
+SHAPES = [
+    (96, 64, 64, 40, 56),      # whole 16-byte pieces, weights resident
+    (40, 100, 80, 40, 20),     # a slot of four channels at the end, 16 outputs in the last block
+    (65, 96, 96, 27, 27),      # odd rows: copies from any 4-byte boundary
+    (130, 44, 72, 14, 14),     # rows of 8-byte pieces, quads beyond the image on two sides
+    (513, 64, 128, 11, 12),    # nine quads an image: images copied whole
+    (1100, 48, 136, 9, 10),
+    (600, 72, 64, 10, 11),     # the same with odd rows
+    (17, 256, 256, 28, 31),    # weights stream through their ring
+    (24, 64, 64, 65, 64),      # wide rows
+]
+
+
+def _inputs(shape):
+    import torch
+    B, C, K, H, W = shape
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    return rnd, rnd(B, C, H, W), rnd(16, C, K) * (1.0 / (16 * C)) ** 0.5
+
+
+def _images(B):
+    return sorted({0, B // 2, B - 1})      # the oracle computes these
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_against_the_oracle(oracle, shape):
+    import torch
+    import wg2x2
+    from wg2x2._lib import lib
+    B, C, K, H, W = shape
+    assert lib.wg2x2_layer_fwd_pair_preferred(B, H, W, C, K, 1)
+    rnd, x, w = _inputs(shape)
+    prepared = wg2x2.prepare_weights(w)
+    si, ti, so, to, r = 1 + 0.2 * rnd(C), 0.3 * rnd(C), 1 + 0.2 * rnd(K), 0.3 * rnd(K), rnd(B, K, H, W)
+    pick = _images(B)
+    nhwc = lambda t: np.ascontiguousarray(t[pick].permute(0, 2, 3, 1).cpu().numpy())
+
+    def want(a, relu):
+        v = oracle.imtrans_fwd(a, relu=relu)
+        return oracle.conv_fwd(v, w.cpu().numpy(), H, W)
+
+    for relu in (True, False):
+        y = wg2x2.layer_fwd_prepared(x, prepared, K, relu=relu, layout="NCHW")
+        assert wg2x2.last_device_status()[0] == 0
+        assert oracle.max_rel(nhwc(y), want(nhwc(x), relu)) <= TOL_TF32
+    main = want(nhwc(x * si.view(1, -1, 1, 1) + ti.view(1, -1, 1, 1)), True) * so.cpu().numpy() + to.cpu().numpy()
+    kw = dict(relu=True, layout="NCHW", in_scale=si, in_shift=ti, out_scale=so, out_shift=to)
+    # no shortcut, one of its own, one that Y lies over
+    assert oracle.max_rel(nhwc(wg2x2.layer_fwd_prepared(x, prepared, K, **kw)), main) <= TOL_TF32
+    for res_relu in (False, True):
+        short = torch.relu(r) if res_relu else r
+        keep = r.clone()
+        y = wg2x2.layer_fwd_prepared(x, prepared, K, residual=r, residual_relu=res_relu, **kw)
+        assert oracle.max_rel(nhwc(y), main + nhwc(short)) <= TOL_TF32 and torch.equal(r, keep)
+        again = wg2x2.layer_fwd_prepared(x, prepared, K, residual=keep, residual_relu=res_relu, out=keep, **kw)
+        # the affine map and the addition, in either order of rounding
+        assert again.data_ptr() == keep.data_ptr() and float((again - y).abs().max()) <= 4 * 2.0 ** -24 * float(y.abs().max() + r.abs().max())
+    assert torch.equal(wg2x2.layer_fwd_prepared(x, prepared, K, residual=r, residual_relu=True, **kw), y)       # the same bits every time
+    assert wg2x2.last_device_status()[0] == 0
+
+
+def test_output_is_written_exactly():
+    """Nothing beyond Y is touched, and all of Y is."""
+    import torch
+    import wg2x2
+    for shape in SHAPES:
+        B, C, K, H, W = shape
+        rnd, x, w = _inputs(shape)
+        n = B * K * H * W
+        room = torch.full((n + 64,), 12345.0, device="cuda")
+        y = room[32:32 + n].view(B, K, H, W)
+        y.fill_(float("nan"))
+        wg2x2.layer_fwd_prepared(x, wg2x2.prepare_weights(w), K, layout="NCHW", out=y)
+        assert bool(torch.isfinite(y).all()) and bool((room[:32] == 12345.0).all()) and bool((room[32 + n:] == 12345.0).all())
+
+
+def test_zero_blocks_are_skipped_right(oracle):
+    import wg2x2
+    shape = (64, 160, 128, 28, 28)
+    B, C, K, H, W = shape
+    rnd, x, w = _inputs(shape)
+    for t in range(16):          # every block of 64 outputs x 32 inputs but a few; all of position 5
+        for kb in range(2):
+            for cc in range(5):
+                if t == 5 or (t + kb + cc) % 3:
+                    w[t, 32 * cc:32 * cc + 32, 64 * kb:64 * kb + 64] = 0
+    y = wg2x2.layer_fwd_prepared(x, wg2x2.prepare_weights(w), K, layout="NCHW")
+    nhwc = lambda t: np.ascontiguousarray(t[_images(B)].permute(0, 2, 3, 1).cpu().numpy())
+    assert oracle.max_rel(nhwc(y), oracle.conv_fwd(oracle.imtrans_fwd(nhwc(x), relu=True), w.cpu().numpy(), H, W)) <= TOL_TF32
+
+
+@pytest.mark.parametrize("nth", [0, 3])
+def test_times_out_and_recovers(nth):
+    """CTA 0's weight producer stops before one load, with nothing in flight, under a limit of a few thousand polls."""
+    import torch
+    import wg2x2
+    from wg2x2._lib import lib
+    shape = SHAPES[0]
+    rnd, x, w = _inputs(shape)
+    prepared, K = wg2x2.prepare_weights(w), shape[2]
+    want = wg2x2.layer_fwd_prepared(x, prepared, K, layout="NCHW")
+    torch.cuda.synchronize()
+    try:
+        lib.wg2x2_set_wait_limit(20000)
+        lib.wg2x2_test_drop_load(nth)
+        wg2x2.layer_fwd_prepared(x, prepared, K, layout="NCHW")
+        st, where = wg2x2.last_device_status()
+        assert st == -4
+        # whichever role ran out first: an issuer (0x10 .. 0x13), a transform team (0x0B, 0x0C), a producer (0x09, 0x0A) or the epilogue (0x04)
+        assert (where >> 8) in (0x10, 0x11, 0x12, 0x13, 0x0C, 0x0B, 0x0A, 0x09, 0x04), "0x%x" % where
+    finally:
+        lib.wg2x2_test_drop_load(-1)
+        lib.wg2x2_set_wait_limit(0)
+    assert torch.equal(wg2x2.layer_fwd_prepared(x, prepared, K, layout="NCHW"), want) and wg2x2.last_device_status()[0] == 0
