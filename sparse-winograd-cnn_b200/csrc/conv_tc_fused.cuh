@@ -830,13 +830,11 @@ static bool fused_geometry(FuParams &p)
 
 // The shortcut, ReLU applied, into the output buffer that the kernel then adds to (in place where they are one).  dst is on a
 // 16-byte boundary, src need not be.
-__global__ void __launch_bounds__(256) relu_copy_kernel(const float *src, float *dst, long long n)
+__global__ void __launch_bounds__(256) relu_copy_kernel(const float *src, float *dst, long long n4)
 {
     after_previous_kernel(src, dst);
     const bool vec = (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
     float4 *d = reinterpret_cast<float4 *>(dst);
-    const long long n4 = n / 4;
-    if (blockIdx.x == 0 && threadIdx.x < (n & 3)) dst[4 * n4 + threadIdx.x] = relu_nan(src[4 * n4 + threadIdx.x]);
     for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n4; i += (long long)gridDim.x * 256)
         d[i] = relu_nan(vec ? reinterpret_cast<const float4 *>(src)[i] : make_float4(src[4 * i], src[4 * i + 1], src[4 * i + 2], src[4 * i + 3]));
 }
@@ -857,7 +855,7 @@ int layer_fwd_fused(const float *X, const void *prepared, float *Y, int B, int H
     p.accumulate = residual != nullptr;
     if (residual && res_relu) {
         const long long n4 = (long long)B * K * H * W / 4;         // W % 4 == 0 here
-        const int s = launch(relu_copy_kernel, dim3((unsigned)(n4 < 256LL * 32 * kNumSMs ? cdivll(n4, 256) : 32 * kNumSMs)), 256, 0, st, residual, Y, 4 * n4);
+        const int s = launch(relu_copy_kernel, dim3((unsigned)(n4 < 256LL * 32 * kNumSMs ? cdivll(n4, 256) : 32 * kNumSMs)), 256, 0, st, residual, Y, n4);
         if (s != WG2X2_OK) return s;
     } else if (residual && residual != Y &&
                cudaMemcpyAsync(Y, residual, sizeof(float) * (size_t)B * K * H * W, cudaMemcpyDeviceToDevice, st) != cudaSuccess) {

@@ -47,7 +47,7 @@ struct PrParams {
     int nW, nX, xbytes;                    // stages of weights and pixels, bytes of a pixel stage
     int xpitch, xpart, whole;              // floats of a channel and of a whole image in a pixel stage; whole images are copied (pr_geometry)
     int nKB, nS, units;                    // blocks of N output channels, slots of 8 channels, units of 64 quads x N channels
-    int relu, res_relu, in_place;          // in_place: Y holds the shortcut (its ReLU applied) and is added to
+    int relu, res_relu, in_place;          // in_place: Y holds the shortcut, its ReLU applied, and 16-byte pieces are added to it
     uint32_t spin_limit;                   // polls before a wait gives up (wg2x2_set_wait_limit)
     int drop_load;                         // >= 0: the W producer of CTA 0 leaves out its drop_load-th stage (wg2x2_test_drop_load), else -1
 };
@@ -139,16 +139,16 @@ __device__ __forceinline__ void pr_ldg(float (&d)[4], const float *p, int cols, 
 {
     if (VEC == 4) {
         asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;\n\t"
-                     "@p ld.global.nc.v4.f32 {%0,%1,%2,%3}, [%4];\n\t}" : "=&f"(d[0]), "=&f"(d[1]), "=&f"(d[2]), "=&f"(d[3]) : "l"(p), "r"((int)ok));
+                     "@p ld.global.v4.f32 {%0,%1,%2,%3}, [%4];\n\t}" : "=&f"(d[0]), "=&f"(d[1]), "=&f"(d[2]), "=&f"(d[3]) : "l"(p), "r"((int)ok));
     } else if (VEC == 2) {
 #pragma unroll
         for (int h = 0; h < 2; ++h)
-            asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %3, 0;\n\tmov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\t@p ld.global.nc.v2.f32 {%0,%1}, [%2];\n\t}"
+            asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %3, 0;\n\tmov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\t@p ld.global.v2.f32 {%0,%1}, [%2];\n\t}"
                          : "=&f"(d[2 * h]), "=&f"(d[2 * h + 1]) : "l"(p + 2 * h), "r"((int)(ok && 2 * h < cols)));
     } else {
 #pragma unroll
         for (int x = 0; x < 4; ++x)
-            asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\tmov.b32 %0, 0;\n\t@p ld.global.nc.f32 %0, [%1];\n\t}" : "=&f"(d[x]) : "l"(p + x), "r"((int)(ok && x < cols)));
+            asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\tmov.b32 %0, 0;\n\t@p ld.global.f32 %0, [%1];\n\t}" : "=&f"(d[x]) : "l"(p + x), "r"((int)(ok && x < cols)));
     }
 }
 template <int VEC>
@@ -166,21 +166,10 @@ __device__ __forceinline__ void pr_stg(float *p, float o0, float o1, float o2, f
             asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.global.f32 [%0], %1;\n\t}" ::"l"(p + x), "f"(o[x]), "r"((int)(ok && x < cols)) : "memory");
     }
 }
-// as pr_stg, added to what is there
-template <int VEC>
-__device__ __forceinline__ void pr_red(float *p, float o0, float o1, float o2, float o3, int cols, bool ok)
+// 16 bytes added to what is there
+__device__ __forceinline__ void pr_red4(float *p, float o0, float o1, float o2, float o3, bool ok)
 {
-    if (VEC == 4) {
-        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t@p red.global.add.v4.f32 [%0], {%1,%2,%3,%4};\n\t}" ::"l"(p), "f"(o0), "f"(o1), "f"(o2), "f"(o3), "r"((int)ok) : "memory");
-    } else if (VEC == 2) {
-        asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 q, %6, 0;\n\t@p red.global.add.v2.f32 [%0], {%1,%2};\n\t@q red.global.add.v2.f32 [%0+8], {%3,%4};\n\t}"
-                     ::"l"(p), "f"(o0), "f"(o1), "f"(o2), "f"(o3), "r"((int)ok), "r"((int)(ok && cols > 2)) : "memory");
-    } else {
-        const float o[4] = {o0, o1, o2, o3};
-#pragma unroll
-        for (int x = 0; x < 4; ++x)
-            asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p red.global.add.f32 [%0], %1;\n\t}" ::"l"(p + x), "f"(o[x]), "r"((int)(ok && x < cols)) : "memory");
-    }
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t@p red.global.add.v4.f32 [%0], {%1,%2,%3,%4};\n\t}" ::"l"(p), "f"(o0), "f"(o1), "f"(o2), "f"(o3), "r"((int)ok) : "memory");
 }
 // One channel of a quad's window: the own columns of its six rows, and in lanes at a warp's end the pixel beyond
 template <int VEC>
@@ -565,7 +554,7 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, PrParams prm)
                 float *yp = prm.Y + w.off + (long long)y * prm.W;
 #pragma unroll
                 for (int c = 0; c < N / 8; ++c, yp += 4 * plane)
-                    pr_red<VEC>(yp, v[0][2 * c], v[1][2 * c], v[0][2 * c + 1], v[1][2 * c + 1], w.cols, y < w.rows && w.k0 + 4 * c < prm.K);
+                    pr_red4(yp, v[0][2 * c], v[1][2 * c], v[0][2 * c + 1], v[1][2 * c + 1], y < w.rows && w.k0 + 4 * c < prm.K);
             };
             const uint32_t t_half = tmem_base + ((uint32_t)(sub * 32) << 16) + (uint32_t)(half * (N / 2));
             // v[e] of rows dy of output row a
@@ -591,7 +580,7 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, PrParams prm)
             bool ok = true;
             if constexpr (EXTRAS && VEC < 4) {
                 // The shortcut in narrow pieces: added in front of the stores (8- and 4-byte reductions behind them take longer than its
-                // latency: 103 against 90 us for 128 x 256 x 14 x 14).  A row's loads go out when the row before has been added, the first row's
+                // latency: 103 against 90 us for 128 x 256 x 14 x 14), also where Y lies over it.  A row's loads go out when the row before has been added, the first row's
                 // of a unit while that unit is still being multiplied, and the others into L2 by then.
                 float r[2][N / 4], scale = 1.f, shift = 0.f;
                 Where w = my_units > 0 ? place(0) : Where{};
@@ -641,7 +630,7 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, PrParams prm)
                             if (i < 3) shortcut(w, 2 * ((i + 1) & 1) + ((i + 1) >> 1), r);
                             else if (iu + 1 < my_units) ahead();
                         }
-                        if (prm.in_place) add(here, 2 * dy + a, v); else store(here, 2 * dy + a, v);
+                        store(here, 2 * dy + a, v);
                     }
                 }
             } else {
@@ -779,11 +768,13 @@ int layer_fwd_pair(const float *X, const void *prepared, float *Y, int B, int H,
     p.X = X; p.Y = Y;
     p.in_scale = in_scale; p.in_shift = in_shift; p.out_scale = out_scale; p.out_shift = out_shift; p.residual = residual;
     p.masks = reinterpret_cast<const unsigned long long *>(static_cast<const unsigned char *>(prepared) + align_up((size_t)16 * K * C * sizeof(float), 256));
-    p.relu = relu; p.res_relu = res_relu; p.in_place = residual == Y;      // (a NULL Y was refused)
+    p.relu = relu; p.res_relu = res_relu;
+    // Y over the shortcut: a thread adds its elements to those there
+    p.in_place = W % 4 == 0 && residual == Y;      // (a NULL Y was refused)
     if (p.in_place) {
         if (res_relu) {
-            const long long n = (long long)B * K * H * W;
-            const int s = launch(relu_copy_kernel, dim3((unsigned)std::min(cdivll(n, 1024), 32LL * kNumSMs)), 256, 0, st, residual, Y, n);
+            const long long n4 = (long long)B * K * H * W / 4;
+            const int s = launch(relu_copy_kernel, dim3((unsigned)std::min(cdivll(n4, 256), 32LL * kNumSMs)), 256, 0, st, residual, Y, n4);
             if (s != WG2X2_OK) return s;
         }
         p.residual = nullptr;
