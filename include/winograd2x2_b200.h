@@ -244,8 +244,9 @@ int wg2x2_layer_fwd_fused_supported(int B, int H, int W, int C, int K, int layou
 /* 1 where the one-kernel NCHW layer is preferred to transform, products and output transform through both scratch buffers (it reads
  * neither); 0 where those are, or the whole layer on clusters. */
 int wg2x2_layer_fwd_fused_preferred(int B, int H, int W, int C, int K, int layout);
-/* 1 where wg2x2_layer_fwd_prepared[_ws|_ex] runs the NCHW layer on pairs of SMs, also in one kernel and without scratch (X, Y, residual,
- * out_scale and out_shift 16-byte aligned, Y not over X), before it looks at any of the others. */
+/* 1 where wg2x2_layer_fwd_prepared[_ws|_ex] runs the layer on pairs of SMs, also in one kernel and without scratch (X, Y, residual,
+ * out_scale and out_shift 16-byte aligned, Y not over X), before it looks at any of the others: many tiles, NCHW at any image size,
+ * NHWC with W and K multiples of 4. */
 int wg2x2_layer_fwd_pair_preferred(int B, int H, int W, int C, int K, int layout);
 /* The one-kernel layer forward on its own (NCHW in and out); WG2X2_ERR_UNSUPPORTED outside the shapes above.
  * residual may be Y itself: the result is then added into Y in place (the TMA unit does the addition);

@@ -38,7 +38,7 @@ bool fused_fwd_supported(int B, int H, int W, int C, int K, int layout);
 bool layer_fused_preferred(int B, int H, int W, int C, int K, int layout);
 bool layer_cluster_preferred(int B, int H, int W, int C, int K, int layout);
 bool layer_pair_preferred(int B, int H, int W, int C, int K, int layout);
-int layer_fwd_pair(const float *X, const void *prepared, float *Y, int B, int H, int W, int C, int K, int relu,
+int layer_fwd_pair(const float *X, const void *prepared, float *Y, int B, int H, int W, int C, int K, int layout, int relu,
                    const float *in_scale, const float *in_shift, const float *out_scale, const float *out_shift,
                    const float *residual, int res_relu, cudaStream_t st);
 bool fused_beats_wide(int B, int H, int W, int C, int K, int layout, double *us);
@@ -300,7 +300,7 @@ int wg2x2_layer_fwd_prepared_ex(const float *X, const float *in_scale, const flo
     const bool apart = x0 + pixels * C <= y0 || y0 + pixels * K <= x0 || !V_scratch;
     const bool extras_on16 = on16(out_scale) && on16(out_shift) && on16(residual);
     if (aligned && apart && extras_on16 && layer_pair_preferred(B, H, W, C, K, layout))
-        return layer_fwd_pair(X, prepared, Y, B, H, W, C, K, relu, in_scale, in_shift, out_scale, out_shift, residual, residual_relu, st);
+        return layer_fwd_pair(X, prepared, Y, B, H, W, C, K, layout, relu, in_scale, in_shift, out_scale, out_shift, residual, residual_relu, st);
     if (aligned && apart && on16(residual) && on16(in_scale) && on16(in_shift) && layer_cluster_preferred(B, H, W, C, K, layout))
         return layer_fwd_cluster(X, prepared, Y, B, H, W, C, K, layout, relu, in_scale, in_shift, out_scale, out_shift, residual, residual_relu, st);
     // The one-kernel layer: where it is the fastest; without scratch for the wide path, where there are few blocks of 64 output channels

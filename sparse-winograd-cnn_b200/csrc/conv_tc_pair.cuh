@@ -48,6 +48,7 @@ struct PrParams {
     int xpitch, xpart, whole;              // floats of a channel and of a whole image in a pixel stage; whole images are copied (pr_geometry)
     int nKB, nS, units;                    // blocks of N output channels, slots of 8 channels, units of 64 quads x N channels
     int relu, res_relu, in_place;          // in_place: Y holds the shortcut, its ReLU applied, and 16-byte pieces are added to it
+    uint32_t zero;                         // 0, which the compiler does not know
     uint32_t spin_limit;                   // polls before a wait gives up (wg2x2_set_wait_limit)
     int drop_load;                         // >= 0: the W producer of CTA 0 leaves out its drop_load-th stage (wg2x2_test_drop_load), else -1
 };
@@ -112,6 +113,30 @@ __device__ __forceinline__ void tmem_st_16x32(uint32_t taddr, const float *r)
                    "r"(__float_as_uint(r[12])), "r"(__float_as_uint(r[13])), "r"(__float_as_uint(r[14])), "r"(__float_as_uint(r[15])) : "memory");
 }
 
+// The same with pairs of columns: r[4 q + 2 d + p] = lane l / 4 + 8 d of column 8 q + 2 (l % 4) + p
+__device__ __forceinline__ void tmem_ld_16x32_pairs(uint32_t taddr, float *r)
+{
+    uint32_t u[16];
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]), "=r"(u[9]), "=r"(u[10]),
+                   "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
+                 : "r"(taddr));
+#pragma unroll
+    for (int q = 0; q < 16; ++q) r[q] = __uint_as_float(u[q]);
+}
+__device__ __forceinline__ void tmem_st_16x32_pairs(uint32_t taddr, const float *r)
+{
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+                 ::"r"(taddr), "f"(r[0]), "f"(r[1]), "f"(r[2]), "f"(r[3]), "f"(r[4]), "f"(r[5]), "f"(r[6]), "f"(r[7]), "f"(r[8]), "f"(r[9]), "f"(r[10]), "f"(r[11]),
+                   "f"(r[12]), "f"(r[13]), "f"(r[14]), "f"(r[15]) : "memory");
+}
+__device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1, int c2, int c3, int c4)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4) : "memory");
+}
+
 // Where a thread's quad lies, as bits: rows 0 .. 5 of the window inside the image; the quad's left / right neighbour does not exist;
 // an outer pixel has to be loaded (the neighbouring quad is another warp's)
 constexpr uint32_t kPrNoLeft = 1u << 6, kPrNoRight = 1u << 7, kPrEdge = 1u << 8;
@@ -131,6 +156,22 @@ __device__ __forceinline__ void pr_lds2(float &x, float &y, uint32_t at, uint32_
 __device__ __forceinline__ void pr_lds1(float &x, uint32_t at, uint32_t ok)
 {
     asm("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\tmov.b32 %0, 0;\n\t@p ld.shared.f32 %0, [%1];\n\t}" : "=&f"(x) : "r"(at), "r"(ok) : "memory");
+}
+__device__ __forceinline__ float2 pr_lds2(uint32_t at)
+{
+    float2 v;
+    asm("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(at) : "memory");
+    return v;
+}
+// Two channels of a pixel from and to memory
+__device__ __forceinline__ void pr_ldg2(float &x, float &y, const float *p, bool ok)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %3, 0;\n\tmov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\t@p ld.global.v2.f32 {%0,%1}, [%2];\n\t}"
+                 : "=&f"(x), "=&f"(y) : "l"(p), "r"((int)ok));
+}
+__device__ __forceinline__ void pr_stg2(float *p, float x, float y, bool ok)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %3, 0;\n\t@p st.global.v2.f32 [%0], {%1,%2};\n\t}" ::"l"(p), "f"(x), "f"(y), "r"((int)ok) : "memory");
 }
 // Four pixels of a row from and to memory, `cols` of them inside the image, none where `ok` is not set: predicates, no branches, so that a
 // row's eight accesses go out together
@@ -218,10 +259,14 @@ __device__ __forceinline__ int pr_offset(const PrParams &prm, const PrSpan &sp, 
     return ch * prm.xpitch + (part == 0 ? 0 : prm.whole ? part * prm.xpart : pr_room((prm.H - sp.y0) * prm.W) + (part - 1) * prm.xpart);
 }
 
+// VEC: 4, 2, 1 = NCHW, floats that can be accessed at once by the row length; kPrNhwc = channels last
+constexpr int kPrNhwc = 0;
+
 template <int VEC, bool AFFINE, bool EXTRAS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPrThreads, 1)
-layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, PrParams prm)
+layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, const __grid_constant__ CUtensorMap mapX, PrParams prm)
 {
+    constexpr bool NHWC = VEC == kPrNhwc;
     constexpr int N = kPrN, kStageBytes = kPrStageBytes;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -349,41 +394,65 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, PrParams prm)
             if (!ok) let_them_land();
         } else if (warp > 4) {
             // ------------------------------ X producers -----------------------------------
-            // Eight channels of the unit's pixels per slot, as plain copies of contiguous memory: one per channel and image, or per image
-            // where whole images are taken.  Copies go by 16 bytes: they start up to three floats early and end up to three late, inside
-            // the tensor all the same (its size is a multiple of 16 bytes, as C is one of 4).
-            // A lane has the same copy to make in every slot of a unit, 8 channels further on (8 H W floats: no other remainder).
-            const int per = prm.whole ? 1 : 8;
-            const long long step = 8LL * prm.H * prm.W;
-            int xs = 0, xf = 0;
-            uint32_t ph = 1;
-            bool ok = true;
-            for (int iu = 0; iu < my_units && ok; ++iu) {
-                const PrSpan sp = pr_span(prm, ((pair + iu * npairs) / prm.nKB) * (2 * kPrQuads) + (int)rank * kPrQuads);
-                const int part = lane / per, ch = lane - part * per;
-                const bool mine = part < sp.n && lane % 3 == warp - 5;
-                const int y0 = part == 0 ? sp.y0 : 0, floats = ((part == sp.n - 1 ? sp.y1 : prm.H) - y0) * prm.W;
-                const long long at = ((long long)(sp.b0 + part) * prm.C + ch) * prm.H * prm.W + (long long)y0 * prm.W;
-                const int rem = (int)(at & 3);
-                const float *src = prm.X + (at - rem);
-                const uint32_t dst = xbase + 4u * (uint32_t)pr_offset(prm, sp, part, ch);
-                for (int sl = 0; sl < nS; ++sl) {
-                    ok = mbar_wait_warp(xempty_bar(xs), ph, abort_flag, 0x900u | xs, prm.spin_limit);
-                    if (!ok) break;
-                    const int chans = min(8, prm.C - 8 * sl);
-                    const uint32_t bytes = mine && ch < chans ? 4u * (uint32_t)((rem + floats * (prm.whole ? chans : 1) + 3) & ~3) : 0u;
-                    const uint32_t all = __reduce_add_sync(0xffffffffu, bytes);
-                    if (lane == 0) mbar_expect_tx(xfull_bar(xf), all);
-                    __syncwarp();
-                    if (bytes)
-                        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                                     ::"r"(dst + xs * prm.xbytes), "l"(src), "r"(bytes), "r"(xfull_bar(xf)) : "memory");
-                    src += step;
-                    if (++xs == prm.nX) { xs = 0; ph ^= 1u; }
-                    if (++xf == 2 * prm.nX) xf = 0;
+            if constexpr (NHWC) {
+                // Eight channels of the windows of every row of quads that the unit touches, one box each: [row of the window][column of a
+                // quad][quad, with one more on either side][channel], zeros outside the image
+                int xs = 0, xf = 0;
+                uint32_t ph = 1;
+                bool ok = true;
+                for (int iu = 0; iu < my_units && ok; ++iu) {
+                    const int q0 = ((pair + iu * npairs) / prm.nKB) * (2 * kPrQuads) + (int)rank * kPrQuads, q1 = min(q0 + kPrQuads, prm.quads) - 1;
+                    const int t = q0 / prm.nQW + lane, b = t / prm.nQH, y = 4 * (t - b * prm.nQH) - 1;
+                    const bool mine = q1 >= q0 && t <= q1 / prm.nQW && lane % 3 == warp - 5;
+                    const uint32_t bytes = (uint32_t)__popc(__ballot_sync(0xffffffffu, mine)) * (uint32_t)prm.xpitch, dst = xbase + (uint32_t)(lane * prm.xpitch);
+                    for (int sl = 0; sl < nS; ++sl) {
+                        ok = mbar_wait_warp(xempty_bar(xs), ph, abort_flag, 0x900u | xs, prm.spin_limit);
+                        if (!ok) break;
+                        if (lane == 0) mbar_expect_tx(xfull_bar(xf), bytes);
+                        __syncwarp();
+                        if (mine) tma_load_5d(dst + xs * prm.xbytes, &mapX, xfull_bar(xf), 8 * sl, -1, 0, y, b);
+                        if (++xs == prm.nX) { xs = 0; ph ^= 1u; }
+                        if (++xf == 2 * prm.nX) xf = 0;
+                    }
                 }
+                if (!ok) let_them_land();
+            } else {
+                // Eight channels of the unit's pixels per slot, as plain copies of contiguous memory: one per channel and image, or per image
+                // where whole images are taken.  Copies go by 16 bytes: they start up to three floats early and end up to three late, inside
+                // the tensor all the same (its size is a multiple of 16 bytes, as C is one of 4).
+                // A lane has the same copy to make in every slot of a unit, 8 channels further on (8 H W floats: no other remainder).
+                const int per = prm.whole ? 1 : 8;
+                const long long step = 8LL * prm.H * prm.W;
+                int xs = 0, xf = 0;
+                uint32_t ph = 1;
+                bool ok = true;
+                for (int iu = 0; iu < my_units && ok; ++iu) {
+                    const PrSpan sp = pr_span(prm, ((pair + iu * npairs) / prm.nKB) * (2 * kPrQuads) + (int)rank * kPrQuads);
+                    const int part = lane / per, ch = lane - part * per;
+                    const bool mine = part < sp.n && lane % 3 == warp - 5;
+                    const int y0 = part == 0 ? sp.y0 : 0, floats = ((part == sp.n - 1 ? sp.y1 : prm.H) - y0) * prm.W;
+                    const long long at = ((long long)(sp.b0 + part) * prm.C + ch) * prm.H * prm.W + (long long)y0 * prm.W;
+                    const int rem = (int)(at & 3);
+                    const float *src = prm.X + (at - rem);
+                    const uint32_t dst = xbase + 4u * (uint32_t)pr_offset(prm, sp, part, ch);
+                    for (int sl = 0; sl < nS; ++sl) {
+                        ok = mbar_wait_warp(xempty_bar(xs), ph, abort_flag, 0x900u | xs, prm.spin_limit);
+                        if (!ok) break;
+                        const int chans = min(8, prm.C - 8 * sl);
+                        const uint32_t bytes = mine && ch < chans ? 4u * (uint32_t)((rem + floats * (prm.whole ? chans : 1) + 3) & ~3) : 0u;
+                        const uint32_t all = __reduce_add_sync(0xffffffffu, bytes);
+                        if (lane == 0) mbar_expect_tx(xfull_bar(xf), all);
+                        __syncwarp();
+                        if (bytes)
+                            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                                         ::"r"(dst + xs * prm.xbytes), "l"(src), "r"(bytes), "r"(xfull_bar(xf)) : "memory");
+                        src += step;
+                        if (++xs == prm.nX) { xs = 0; ph ^= 1u; }
+                        if (++xf == 2 * prm.nX) xf = 0;
+                    }
+                }
+                if (!ok) let_them_land();
             }
-            if (!ok) let_them_land();
         }
     } else {
         // the quad of this thread in a unit, by lane: eight quads per warp, four lanes (channels) per quad
@@ -407,16 +476,20 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, PrParams prm)
             const uint32_t a_tmem = tmem_base + ((uint32_t)(sub * 32) << 16) + (uint32_t)(kPrACol0 + team * kPrGroupCols);
             const uint32_t full0 = mapa_rank0(full_bar(team));
             int iu = 0, sl = team, cols = 0;
-            uint32_t flags = 0, quad = 0;                       // quad: byte offset of window row 0 of channel cl of this thread's quad in a stage
+            uint32_t flags = 0, quad = 0;                       // quad: byte offset of this thread's window in a stage
             long long at0 = 0;
             auto enter = [&]() {
                 int b, qr, qc;
                 const bool valid = locate(iu, b, qr, qc);
-                const PrSpan sp = pr_span(prm, ((pair + iu * npairs) / prm.nKB) * (2 * kPrQuads) + (int)rank * kPrQuads);
-                const int part = b - sp.b0, y0 = part == 0 ? sp.y0 : 0, ch = cl;
-                at0 = ((long long)b * prm.C + ch) * plane + (long long)y0 * prm.W;
-                const int off = pr_offset(prm, sp, part, ch);
-                quad = valid ? 4u * (uint32_t)(off + (4 * qr - 1 - y0) * prm.W + 4 * qc) : 0u;
+                const int q0 = ((pair + iu * npairs) / prm.nKB) * (2 * kPrQuads) + (int)rank * kPrQuads;
+                if constexpr (NHWC) {
+                    quad = (valid ? (uint32_t)((b * prm.nQH + qr - q0 / prm.nQW) * prm.xpitch + 32 * qc) : 0u) + 8u * cl;
+                } else {
+                    const PrSpan sp = pr_span(prm, q0);
+                    const int part = b - sp.b0, y0 = part == 0 ? sp.y0 : 0;
+                    at0 = ((long long)b * prm.C + cl) * plane + (long long)y0 * prm.W;
+                    quad = valid ? 4u * (uint32_t)(pr_offset(prm, sp, part, cl) + (4 * qr - 1 - y0) * prm.W + 4 * qc) : 0u;
+                }
                 flags = 0;
 #pragma unroll
                 for (int r = 0; r < 6; ++r) {
@@ -437,43 +510,77 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, PrParams prm)
             for (int n = team; n < total; n += 2) {
                 bool ok = mbar_wait_warp(xfull_bar(xf), xph, abort_flag, 0xB00u | xf, prm.spin_limit);
                 if (!ok) break;
-                float d[2][6][4], ed[2][6];                          // [channel][row]
-                float sc[2], tc[2];
-#pragma unroll
-                for (int p = 0; p < 2; ++p) {
-                    const int c = 8 * sl + 4 * p;
-                    const bool chan = c < prm.C;                     // C is a multiple of 4: the same for the four lanes of a quad
-                    uint32_t at = xbase + xs * prm.xbytes + quad + p * (uint32_t)(16 * prm.xpitch);
-                    if (VEC < 4 && !prm.whole) at += 4u * (uint32_t)((at0 + (long long)c * plane) & 3);   // where the copy's first 16 bytes begin
-                    pr_window<VEC>(d[p], ed[p], at, prm.W, qg == 0 ? -4 : 16, chan ? flags : 0u, cols);
-                    if (AFFINE) { sc[p] = chan ? __ldg(prm.in_scale + c + cl) : 1.f; tc[p] = chan ? __ldg(prm.in_shift + c + cl) : 0.f; }
-                }
-                // the windows with their outer columns, from the neighbouring quads' lanes where those are in this warp
-                float2 m[2][6][2], lr[2][6];                        // [channel][row]: columns 0 1 | 2 3, and the outer two
-#pragma unroll
-                for (int p = 0; p < 2; ++p)
+                // [channel][row]: columns 0 1 | 2 3, and the outer two; channels last: [row][column], both channels
+                float2 m[2][6][2], lr[2][6], win[6][6];
+                uint32_t loaded = 0;                                 // a bit of every load that nothing else waits for in front of the stage's release
+                if constexpr (NHWC) {
+                    const uint32_t at = xbase + xs * prm.xbytes + quad, px = 32u * (uint32_t)(prm.nQW + 2);
 #pragma unroll
                     for (int r = 0; r < 6; ++r) {
-                        if (AFFINE) {
-                            const float tr = (flags >> r) & 1u ? tc[p] : 0.f;     // pixels outside the image stay zero
+                        const uint32_t ar = at + 4u * r * px;
+                        win[r][0] = pr_lds2(ar + 3u * px);
 #pragma unroll
-                            for (int x = 0; x < 4; ++x) d[p][r][x] = fmaf(sc[p], d[p][r][x], VEC == 4 || x < cols ? tr : 0.f);
-                            ed[p][r] = fmaf(sc[p], ed[p][r], flags & kPrEdge ? tr : 0.f);
+                        for (int x = 0; x < 4; ++x) win[r][1 + x] = pr_lds2(ar + (uint32_t)x * px + 32u);
+                        win[r][5] = pr_lds2(ar + 64u);
+#pragma unroll
+                        for (int x = 0; x < 6; ++x) loaded ^= __float_as_uint(win[r][x].x);
+                    }
+                    if (AFFINE) {
+                        const int c = 8 * sl + 2 * cl;
+                        const float2 sc = c < prm.C ? make_float2(__ldg(prm.in_scale + c), __ldg(prm.in_scale + c + 1)) : make_float2(1.f, 1.f);
+                        const float2 tc = c < prm.C ? make_float2(__ldg(prm.in_shift + c), __ldg(prm.in_shift + c + 1)) : make_float2(0.f, 0.f);
+#pragma unroll
+                        for (int r = 0; r < 6; ++r)
+#pragma unroll
+                            for (int x = 0; x < 6; ++x) {
+                                // pixels outside the image stay zero
+                                const bool in = ((flags >> r) & 1u) && !(x == 0 && (flags & kPrNoLeft)) && !(x == 5 && (flags & kPrNoRight));
+                                win[r][x] = make_float2(fmaf(sc.x, win[r][x].x, in ? tc.x : 0.f), fmaf(sc.y, win[r][x].y, in ? tc.y : 0.f));
+                            }
+                    }
+                } else {
+                    float d[2][6][4], ed[2][6];                          // [channel][row]
+                    float sc[2], tc[2];
+#pragma unroll
+                    for (int p = 0; p < 2; ++p) {
+                        const int c = 8 * sl + 4 * p;
+                        const bool chan = c < prm.C;                     // C is a multiple of 4: the same for the four lanes of a quad
+                        uint32_t at = xbase + xs * prm.xbytes + quad + p * (uint32_t)(16 * prm.xpitch);
+                        if (VEC < 4 && !prm.whole) at += 4u * (uint32_t)((at0 + (long long)c * plane) & 3);   // where the copy's first 16 bytes begin
+                        pr_window<VEC>(d[p], ed[p], at, prm.W, qg == 0 ? -4 : 16, chan ? flags : 0u, cols);
+#pragma unroll
+                        for (int r = 0; r < 6; ++r) loaded ^= __float_as_uint(ed[p][r]) ^ (VEC == 1 ? __float_as_uint(d[p][r][1]) ^ __float_as_uint(d[p][r][2]) : 0u);
+                        if (AFFINE) { sc[p] = chan ? __ldg(prm.in_scale + c + cl) : 1.f; tc[p] = chan ? __ldg(prm.in_shift + c + cl) : 0.f; }
+                    }
+                    // the windows with their outer columns, from the neighbouring quads' lanes where those are in this warp
+#pragma unroll
+                    for (int p = 0; p < 2; ++p)
+#pragma unroll
+                        for (int r = 0; r < 6; ++r) {
+                            if (AFFINE) {
+                                const float tr = (flags >> r) & 1u ? tc[p] : 0.f;     // pixels outside the image stay zero
+#pragma unroll
+                                for (int x = 0; x < 4; ++x) d[p][r][x] = fmaf(sc[p], d[p][r][x], VEC == 4 || x < cols ? tr : 0.f);
+                                ed[p][r] = fmaf(sc[p], ed[p][r], flags & kPrEdge ? tr : 0.f);
+                            }
+                            lr[p][r].x = __shfl_up_sync(0xffffffffu, d[p][r][3], 4);
+                            lr[p][r].y = __shfl_down_sync(0xffffffffu, d[p][r][0], 4);
+                            m[p][r][0] = make_float2(d[p][r][0], d[p][r][1]);
+                            m[p][r][1] = make_float2(d[p][r][2], d[p][r][3]);
                         }
-                        lr[p][r].x = __shfl_up_sync(0xffffffffu, d[p][r][3], 4);
-                        lr[p][r].y = __shfl_down_sync(0xffffffffu, d[p][r][0], 4);
-                        m[p][r][0] = make_float2(d[p][r][0], d[p][r][1]);
-                        m[p][r][1] = make_float2(d[p][r][2], d[p][r][3]);
-                    }
 #pragma unroll
-                for (int p = 0; p < 2; ++p)
+                    for (int p = 0; p < 2; ++p)
 #pragma unroll
-                    for (int r = 0; r < 6; ++r) {
-                        lr[p][r].x = flags & kPrNoLeft ? 0.f : (qg == 0 ? ed[p][r] : lr[p][r].x);
-                        lr[p][r].y = flags & kPrNoRight ? 0.f : (qg == 7 ? ed[p][r] : lr[p][r].y);
-                    }
+                        for (int r = 0; r < 6; ++r) {
+                            lr[p][r].x = flags & kPrNoLeft ? 0.f : (qg == 0 ? ed[p][r] : lr[p][r].x);
+                            lr[p][r].y = flags & kPrNoRight ? 0.f : (qg == 7 ? ed[p][r] : lr[p][r].y);
+                        }
+                }
+                // The stage is handed back once every load has delivered.  An arrival does not wait for loads that have only been issued, and behind
+                // tensor-memory stores those may be hundreds of clocks away from shared memory: the shuffles wait for most of them, the
+                // arrival's address for the others.
                 __syncwarp();
-                if (lane == 0) mbar_arrive(xempty_bar(xs));          // in registers: the stage is handed back
+                if (lane == 0) mbar_arrive(xempty_bar(xs) + (loaded & prm.zero));
                 xs += 2; if (xs >= prm.nX) xs -= prm.nX;
                 xf += 2; if (xf >= 2 * prm.nX) { xf -= 2 * prm.nX; xph ^= 1u; }
 #pragma unroll
@@ -485,22 +592,35 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, PrParams prm)
                     for (int i = 2 * h; i < 2 * h + 2; ++i) {
 #pragma unroll
                         for (int dy = 0; dy < 2; ++dy) {
-                            // Winograd row i of the two tiles: columns 1 2 | 3 4 | 0 5 of the window
+                            const int y = 2 * dy;
+                            float o[16];                             // [j][channel][dx], channels last [j][dx][channel]
                             auto rows = [&](float2 d0, float2 d1, float2 d2, float2 d3) {
                                 return i == 0 ? sub2(d0, d2) : i == 1 ? add2(d1, d2) : i == 2 ? sub2(d2, d1) : sub2(d1, d3);
                             };
-                            const int y = 2 * dy;
-                            float o[16];                             // [j][channel][dx]
+                            if constexpr (NHWC) {
+                                float2 r[6];                         // Winograd row i of the two tiles
 #pragma unroll
-                            for (int p = 0; p < 2; ++p) {
-                                const float2 r12 = rows(m[p][y][0], m[p][y + 1][0], m[p][y + 2][0], m[p][y + 3][0]),
-                                             r34 = rows(m[p][y][1], m[p][y + 1][1], m[p][y + 2][1], m[p][y + 3][1]),
-                                             r05 = rows(lr[p][y], lr[p][y + 1], lr[p][y + 2], lr[p][y + 3]);
-                                const float2 d = sub2(r12, r34);
-                                o[2 * p] = fmaxf(r05.x - r12.y, lo); o[2 * p + 1] = fmaxf(d.y, lo);
-                                o[4 + 2 * p] = fmaxf(r12.x + r12.y, lo); o[5 + 2 * p] = fmaxf(r34.x + r34.y, lo);
-                                o[8 + 2 * p] = fmaxf(r12.y - r12.x, lo); o[9 + 2 * p] = fmaxf(r34.y - r34.x, lo);
-                                o[12 + 2 * p] = fmaxf(d.x, lo); o[13 + 2 * p] = fmaxf(r34.x - r05.y, lo);
+                                for (int x = 0; x < 6; ++x) r[x] = rows(win[y][x], win[y + 1][x], win[y + 2][x], win[y + 3][x]);
+#pragma unroll
+                                for (int dx = 0; dx < 2; ++dx) {
+                                    const float2 v[4] = {sub2(r[2 * dx], r[2 * dx + 2]), add2(r[2 * dx + 1], r[2 * dx + 2]), sub2(r[2 * dx + 2], r[2 * dx + 1]),
+                                                         sub2(r[2 * dx + 1], r[2 * dx + 3])};
+#pragma unroll
+                                    for (int j = 0; j < 4; ++j) { o[4 * j + 2 * dx] = fmaxf(v[j].x, lo); o[4 * j + 2 * dx + 1] = fmaxf(v[j].y, lo); }
+                                }
+                            } else {
+                                // columns 1 2 | 3 4 | 0 5 of the window
+#pragma unroll
+                                for (int p = 0; p < 2; ++p) {
+                                    const float2 r12 = rows(m[p][y][0], m[p][y + 1][0], m[p][y + 2][0], m[p][y + 3][0]),
+                                                 r34 = rows(m[p][y][1], m[p][y + 1][1], m[p][y + 2][1], m[p][y + 3][1]),
+                                                 r05 = rows(lr[p][y], lr[p][y + 1], lr[p][y + 2], lr[p][y + 3]);
+                                    const float2 d = sub2(r12, r34);
+                                    o[2 * p] = fmaxf(r05.x - r12.y, lo); o[2 * p + 1] = fmaxf(d.y, lo);
+                                    o[4 + 2 * p] = fmaxf(r12.x + r12.y, lo); o[5 + 2 * p] = fmaxf(r34.x + r34.y, lo);
+                                    o[8 + 2 * p] = fmaxf(r12.y - r12.x, lo); o[9 + 2 * p] = fmaxf(r34.y - r34.x, lo);
+                                    o[12 + 2 * p] = fmaxf(d.x, lo); o[13 + 2 * p] = fmaxf(r34.x - r05.y, lo);
+                                }
                             }
                             if (i == 1) {
                                 // Position (1, 1), of non-negative pixels the largest, is rounded to TF32 (half a unit of the last kept
@@ -510,7 +630,8 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, PrParams prm)
 #pragma unroll
                                 for (int x = 4; x < 8; ++x) o[x] = __uint_as_float(__float_as_uint(o[x]) + 0x1000u);
                             }
-                            tmem_st_16x32(a_tmem + ((uint32_t)(16 * dy) << 16) + (uint32_t)(32 * i), o);
+                            const uint32_t to = a_tmem + ((uint32_t)(16 * dy) << 16) + (uint32_t)(32 * i);
+                            if (NHWC) tmem_st_16x32_pairs(to, o); else tmem_st_16x32(to, o);
                         }
                     }
                 }
@@ -532,23 +653,33 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, PrParams prm)
             const int half = (warp - 8) >> 2;                    // which half of the block's output channels
             const uint32_t acce0 = mapa_rank0(acce_bar(0)), acce1 = mapa_rank0(acce_bar(1));
             const long long plane = (long long)prm.H * prm.W;
-            // this thread's part of unit iu: rows 4 qr .. of its quad in channels k0, k0 + 4, ...
+            // this thread's part of unit iu: rows 4 qr .. of its quad in channels k0, k0 + 4, ... (channels last: k0, k0 + 1, k0 + 8, ...)
             struct Where { long long off; int k0, rows, cols; };
             auto place = [&](int iu) {
                 int b, qr, qc;
                 const bool valid = locate(iu, b, qr, qc);
                 Where w;
-                w.k0 = ((pair + iu * npairs) % prm.nKB) * N + half * (N / 2) + cl;
+                w.k0 = ((pair + iu * npairs) % prm.nKB) * N + half * (N / 2) + (NHWC ? 2 * cl : cl);
                 w.cols = prm.W - 4 * qc;
                 w.rows = valid ? prm.H - 4 * qr : 0;
-                w.off = ((long long)b * prm.K + w.k0) * plane + (long long)(4 * qr) * prm.W + 4 * qc;
+                w.off = NHWC ? (((long long)b * prm.H + 4 * qr) * prm.W + 4 * qc) * prm.K + w.k0
+                             : ((long long)b * prm.K + w.k0) * plane + (long long)(4 * qr) * prm.W + 4 * qc;
                 return w;
             };
             auto store = [&](const Where &w, int y, const float (&v)[2][N / 4]) {       // row y of the quad, v as [e][channel, dx]
+                if constexpr (NHWC) {
+                    float *yp = prm.Y + w.off + (long long)y * prm.W * prm.K;
+#pragma unroll
+                    for (int x = 0; x < 4; ++x, yp += prm.K)
+#pragma unroll
+                        for (int j = 0; j < N / 16; ++j)
+                            pr_stg2(yp + 8 * j, v[x & 1][4 * j + (x & 2)], v[x & 1][4 * j + (x & 2) + 1], y < w.rows && w.k0 + 8 * j < prm.K);
+                    return;
+                }
                 float *yp = prm.Y + w.off + (long long)y * prm.W;
 #pragma unroll
                 for (int c = 0; c < N / 8; ++c, yp += 4 * plane)
-                    pr_stg<VEC>(yp, v[0][2 * c], v[1][2 * c], v[0][2 * c + 1], v[1][2 * c + 1], w.cols, y < w.rows && w.k0 + 4 * c < prm.K);
+                    pr_stg<NHWC ? 1 : VEC>(yp, v[0][2 * c], v[1][2 * c], v[0][2 * c + 1], v[1][2 * c + 1], w.cols, y < w.rows && w.k0 + 4 * c < prm.K);
             };
             auto add = [&](const Where &w, int y, const float (&v)[2][N / 4]) {         // the same, added to what is there
                 float *yp = prm.Y + w.off + (long long)y * prm.W;
@@ -560,7 +691,10 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, PrParams prm)
             // v[e] of rows dy of output row a
             auto fetch = [&](int a, int dy, float (&v)[2][N / 4]) {
 #pragma unroll
-                for (int e = 0; e < 2; ++e) tmem_ld_16x32(t_half + ((uint32_t)(16 * dy) << 16) + (uint32_t)((2 * a + e) * N), v[e]);
+                for (int e = 0; e < 2; ++e) {
+                    const uint32_t from = t_half + ((uint32_t)(16 * dy) << 16) + (uint32_t)((2 * a + e) * N);
+                    if (NHWC) tmem_ld_16x32_pairs(from, v[e]); else tmem_ld_16x32(from, v[e]);
+                }
             };
             auto hand_back = [&](int a) {                        // the accumulators of output row a are in registers
                 tc_fence_before();
@@ -569,34 +703,44 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, PrParams prm)
             };
             // the shortcut's row y, as v
             auto shortcut = [&](const Where &w, int y, float (&r)[2][N / 4]) {
+                if constexpr (NHWC) {
+                    const float *rp = prm.residual + w.off + (long long)y * prm.W * prm.K;
+#pragma unroll
+                    for (int x = 0; x < 4; ++x, rp += prm.K)
+#pragma unroll
+                        for (int j = 0; j < N / 16; ++j)
+                            pr_ldg2(r[x & 1][4 * j + (x & 2)], r[x & 1][4 * j + (x & 2) + 1], rp + 8 * j, y < w.rows && w.k0 + 8 * j < prm.K);
+                    return;
+                }
                 const float *rp = prm.residual + w.off + (long long)y * prm.W;
 #pragma unroll
                 for (int c = 0; c < N / 8; ++c, rp += 4 * plane) {
                     float t[4];
-                    pr_ldg<VEC>(t, rp, w.cols, y < w.rows && w.k0 + 4 * c < prm.K);
+                    pr_ldg<NHWC ? 1 : VEC>(t, rp, w.cols, y < w.rows && w.k0 + 4 * c < prm.K);
                     r[0][2 * c] = t[0]; r[1][2 * c] = t[1]; r[0][2 * c + 1] = t[2]; r[1][2 * c + 1] = t[3];
                 }
             };
             bool ok = true;
             if constexpr (EXTRAS && VEC < 4) {
                 // The shortcut in narrow pieces: added in front of the stores (8- and 4-byte reductions behind them take longer than its
-                // latency: 103 against 90 us for 128 x 256 x 14 x 14), also where Y lies over it.  A row's loads go out when the row before has been added, the first row's
-                // of a unit while that unit is still being multiplied, and the others into L2 by then.
+                // latency: 103 against 90 us for 128 x 256 x 14 x 14), also where Y lies over it.  A row's loads go out when the row before has
+                // been added, the first row's of a unit while that unit is still being multiplied, and the others into L2 by then.
                 float r[2][N / 4], scale = 1.f, shift = 0.f;
                 Where w = my_units > 0 ? place(0) : Where{};
                 // lane l: the affine map of the half's channel l (N / 2 of them)
                 auto maps = [&]() {
-                    const int k = w.k0 - cl + lane;
+                    const int k = w.k0 - (NHWC ? 2 * cl : cl) + lane;
                     if (prm.out_scale && lane < N / 2 && k < prm.K) { scale = __ldg(prm.out_scale + k); shift = __ldg(prm.out_shift + k); }
                 };
                 auto ahead = [&]() {
                     shortcut(w, 0, r);
 #pragma unroll 1
-                    for (int y = 1; y < 4; ++y)
+                    for (int y = 1; y < 4; ++y) {
+                        const float *rp = prm.residual + w.off + (long long)y * prm.W * (NHWC ? prm.K : 1);
 #pragma unroll
-                        for (int c = 0; c < N / 8; ++c)
-                            if (y < w.rows && w.k0 + 4 * c < prm.K)
-                                asm volatile("prefetch.global.L2 [%0];" ::"l"(prm.residual + w.off + (long long)y * prm.W + (long long)(4 * c) * plane));
+                        for (int c = 0; c < (NHWC ? 4 : N / 8); ++c, rp += NHWC ? prm.K : 4 * plane)       // (channels last: a pixel's half is one line)
+                            if (y < w.rows && w.k0 + (NHWC ? 0 : 4 * c) < prm.K) asm volatile("prefetch.global.L2 [%0];" ::"l"(rp));
+                    }
                 };
                 if (my_units > 0) maps();
                 if (prm.residual && my_units > 0) ahead();
@@ -613,15 +757,17 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, PrParams prm)
                         tmem_ld_wait();
                         if (dy == 1) hand_back(a);
 #pragma unroll
-                        for (int c = 0; c < N / 8; ++c) {
+                        for (int c = 0; c < N / 8; ++c) {            // the c-th channel of this thread: two values per e
+                            const int at = NHWC ? 4 * (c >> 1) + (c & 1) : 2 * c, step = NHWC ? 2 : 1, ch = NHWC ? 8 * (c >> 1) + 2 * cl + (c & 1) : 4 * c + cl;
                             if (prm.out_scale) {
-                                const float s1 = __shfl_sync(0xffffffffu, scale, 4 * c + cl), b1 = __shfl_sync(0xffffffffu, shift, 4 * c + cl);
+                                const float s1 = __shfl_sync(0xffffffffu, scale, ch), b1 = __shfl_sync(0xffffffffu, shift, ch);
 #pragma unroll
-                                for (int x = 0; x < 4; ++x) v[x & 1][2 * c + (x >> 1)] = fmaf(v[x & 1][2 * c + (x >> 1)], s1, b1);
+                                for (int x = 0; x < 4; ++x) v[x & 1][at + step * (x >> 1)] = fmaf(v[x & 1][at + step * (x >> 1)], s1, b1);
                             }
                             if (prm.residual) {
 #pragma unroll
-                                for (int x = 0; x < 4; ++x) v[x & 1][2 * c + (x >> 1)] += prm.res_relu ? relu_nan(r[x & 1][2 * c + (x >> 1)]) : r[x & 1][2 * c + (x >> 1)];
+                                for (int x = 0; x < 4; ++x)
+                                    v[x & 1][at + step * (x >> 1)] += prm.res_relu ? relu_nan(r[x & 1][at + step * (x >> 1)]) : r[x & 1][at + step * (x >> 1)];
                             }
                         }
                         const Where here = w;
@@ -704,20 +850,26 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, PrParams prm)
 
 // Shared memory: the pixels of eight channels of 32 quads, wherever these begin, per stage; three stages if a unit's weights then
 // still stay resident (or the ring of those has four), else two; the rest for weights.
-static bool pr_geometry(PrParams &p)
+static bool pr_geometry(PrParams &p, int layout)
 {
     constexpr int wstage = kPrStageBytes;
+    // quad rows that 32 quads can touch
+    const int qrows = kPrQuads % p.nQW == 0 ? kPrQuads / p.nQW : (kPrQuads - 2) / p.nQW + 2;
     const long long per_image = (long long)p.nQH * p.nQW, HW = (long long)p.H * p.W;
     if (HW * 32 > 0x7fffffffLL) return false;
     const int images = per_image >= kPrQuads ? (per_image % kPrQuads ? 2 : 1) : kPrQuads % per_image == 0 ? (int)(kPrQuads / per_image) : (int)((kPrQuads - 2) / per_image) + 2;
     long long floats;
     p.whole = images * 8 > 32;
-    if (p.whole) {
+    if (layout == WG2X2_NHWC) {                                   // a box per quad row
+        if (p.W % 4 || p.K % 4 || p.nQW + 2 > 256) return false;
+        p.xpitch = 6 * 4 * (p.nQW + 2) * 32;
+        p.xpart = p.whole = 0;
+        floats = (long long)qrows * (p.xpitch / 4);
+    } else if (p.whole) {
         p.xpitch = (int)HW; p.xpart = (int)(8 * HW);
         floats = (long long)images * p.xpart + 4;
     } else {
-        // quad rows that 32 quads can touch, four rows of pixels each, and one above and one below (none where an image ends)
-        const int qrows = kPrQuads % p.nQW == 0 ? kPrQuads / p.nQW : (kPrQuads - 2) / p.nQW + 2;
+        // four rows of pixels per quad row, and one above and one below (none where an image ends)
         p.xpart = pr_room((int)HW);
         const long long rows = std::min<long long>(4LL * qrows + 2, (long long)images * p.H);
         long long pitch = rows * p.W + 8LL * images;
@@ -738,7 +890,7 @@ static bool pr_geometry(PrParams &p)
 }
 
 // Sizes of the kernel for a layer; false: not one that it takes
-static bool pr_sizes(PrParams &p, int B, int H, int W, int C, int K)
+static bool pr_sizes(PrParams &p, int B, int H, int W, int C, int K, int layout)
 {
     if (!tc_shape_supported(C, K)) return false;
     p.B = B; p.H = H; p.W = W; p.C = C; p.K = K;
@@ -748,15 +900,15 @@ static bool pr_sizes(PrParams &p, int B, int H, int W, int C, int K)
     const long long units = cdivll(quads, 2 * kPrQuads) * p.nKB;
     if (quads > 0x7fffffffLL - 2 * kPrQuads || units * p.nS > 0x7fffffffLL) return false;
     p.quads = (int)quads; p.units = (int)units;
-    return pr_geometry(p);
+    return pr_geometry(p, layout);
 }
-static bool pair_supported(int B, int H, int W, int C, int K)
+static bool pair_supported(int B, int H, int W, int C, int K, int layout)
 {
     PrParams p;
-    return pr_sizes(p, B, H, W, C, K);
+    return pr_sizes(p, B, H, W, C, K, layout);
 }
 
-int layer_fwd_pair(const float *X, const void *prepared, float *Y, int B, int H, int W, int C, int K, int relu,
+int layer_fwd_pair(const float *X, const void *prepared, float *Y, int B, int H, int W, int C, int K, int layout, int relu,
                    const float *in_scale, const float *in_shift, const float *out_scale, const float *out_shift,
                    const float *residual, int res_relu, cudaStream_t st)
 {
@@ -764,13 +916,13 @@ int layer_fwd_pair(const float *X, const void *prepared, float *Y, int B, int H,
     if ((in_scale == nullptr) != (in_shift == nullptr) || (out_scale == nullptr) != (out_shift == nullptr)) return WG2X2_ERR_BAD_ARG;
     if (misaligned16(X) || misaligned16(prepared) || misaligned16(Y) || misaligned16(residual)) return WG2X2_ERR_BAD_ARG;
     PrParams p;
-    if (!pr_sizes(p, B, H, W, C, K)) return WG2X2_ERR_UNSUPPORTED;
+    if (!pr_sizes(p, B, H, W, C, K, layout)) return WG2X2_ERR_UNSUPPORTED;
     p.X = X; p.Y = Y;
     p.in_scale = in_scale; p.in_shift = in_shift; p.out_scale = out_scale; p.out_shift = out_shift; p.residual = residual;
     p.masks = reinterpret_cast<const unsigned long long *>(static_cast<const unsigned char *>(prepared) + align_up((size_t)16 * K * C * sizeof(float), 256));
     p.relu = relu; p.res_relu = res_relu;
     // Y over the shortcut: a thread adds its elements to those there
-    p.in_place = W % 4 == 0 && residual == Y;      // (a NULL Y was refused)
+    p.in_place = layout == WG2X2_NCHW && W % 4 == 0 && residual == Y;      // (a NULL Y was refused)
     if (p.in_place) {
         if (res_relu) {
             const long long n4 = (long long)B * K * H * W / 4;
@@ -779,6 +931,7 @@ int layer_fwd_pair(const float *X, const void *prepared, float *Y, int B, int H,
         }
         p.residual = nullptr;
     }
+    p.zero = 0;
     p.spin_limit = wait_limit();
     p.drop_load = take_drop_load();
     CUtensorMap mapW;
@@ -788,6 +941,15 @@ int layer_fwd_pair(const float *X, const void *prepared, float *Y, int B, int H,
         const cuuint32_t box[3] = {16, kPrN / 2, 16};
         if (!tensor_map_f32(&mapW, 3, static_cast<const float *>(prepared), dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B)) return WG2X2_ERR_LAUNCH;
     }
+    CUtensorMap mapX = mapW;                                      // (NCHW: not looked at)
+    if (layout == WG2X2_NHWC) {
+        // a row of the image as [column of a quad][quad][channel]
+        const cuuint64_t px = (cuuint64_t)C * 4;
+        const cuuint64_t dims[5] = {(cuuint64_t)C, (cuuint64_t)p.nQW, 4, (cuuint64_t)H, (cuuint64_t)B};
+        const cuuint64_t strides[4] = {4 * px, px, px * W, px * W * H};
+        const cuuint32_t box[5] = {8, (cuuint32_t)(p.nQW + 2), 4, 6, 1};
+        if (!tensor_map_f32(&mapX, 5, X, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE)) return WG2X2_ERR_LAUNCH;
+    }
     // a grid that divides the units evenly: every pair runs the same number of them, or one fewer
     const int pairs = cdiv(p.units, cdiv(p.units, kNumSMs / 2));
     const bool extras = out_scale || residual, affine = in_scale != nullptr;
@@ -796,16 +958,16 @@ int layer_fwd_pair(const float *X, const void *prepared, float *Y, int B, int H,
         return extras ? (affine ? layer_fwd_pair_kernel<V, true, true> : layer_fwd_pair_kernel<V, false, true>)
                       : (affine ? layer_fwd_pair_kernel<V, true, false> : layer_fwd_pair_kernel<V, false, false>);
     };
-    auto *kernel = W % 4 == 0 ? pick(std::integral_constant<int, 4>{}) : W % 2 == 0 ? pick(std::integral_constant<int, 2>{}) : pick(std::integral_constant<int, 1>{});
-    return launch(kernel, dim3((unsigned)(2 * pairs)), kPrThreads, (size_t)p.nW * kPrStageBytes + (size_t)p.nX * p.xbytes + kCtrlBytes + 1024, st, mapW, p);
+    auto *kernel = layout == WG2X2_NHWC ? pick(std::integral_constant<int, kPrNhwc>{}) : W % 4 == 0 ? pick(std::integral_constant<int, 4>{}) : W % 2 == 0 ? pick(std::integral_constant<int, 2>{}) : pick(std::integral_constant<int, 1>{});
+    return launch(kernel, dim3((unsigned)(2 * pairs)), kPrThreads, (size_t)p.nW * kPrStageBytes + (size_t)p.nX * p.xbytes + kCtrlBytes + 1024, st, mapW, mapX, p);
 }
 
 // Microseconds of the layer on pairs of SMs (plain, 1 .. 128 images of 7 .. 56 pixels, 32 .. 512 channels: within a tenth of the
 // measured): rounds of units, each a walk over the input channels and the change of accumulators at its end.
-static double pair_us(int B, int H, int W, int C, int K)
+static double pair_us(int B, int H, int W, int C, int K, int layout)
 {
     const double rounds = (double)cdivll(cdivll((long long)B * cdiv(H, 4) * cdiv(W, 4), 2 * kPrQuads) * cdiv(K, 64), kNumSMs / 2);
-    return 6.4 + rounds * (3.5 + (W % 4 == 0 ? 0.71 : W % 2 == 0 ? 0.79 : 1.21) * cdiv(C, 8));
+    return 6.4 + rounds * (3.5 + (layout == WG2X2_NHWC ? 0.83 : W % 4 == 0 ? 0.71 : W % 2 == 0 ? 0.79 : 1.21) * cdiv(C, 8));
 }
 
 // Against all other paths, for any NCHW image.  It wins where its units fill the SMs at
@@ -813,8 +975,8 @@ static double pair_us(int B, int H, int W, int C, int K)
 // 128 x 256 x 14 x 14 93 -> 68, 64 x 64 x 56 x 56 45 -> 34), with fewer units up to four times as long.
 bool layer_pair_preferred(int B, int H, int W, int C, int K, int layout)
 {
-    if (layout != WG2X2_NCHW || !tc_shape_supported(C, K) || !pair_supported(B, H, W, C, K)) return false;
+    if (!pair_supported(B, H, W, C, K, layout)) return false;
     const long long P = (long long)B * ((H + 1) / 2) * ((W + 1) / 2);
     if (P > 0x7fffffffLL - kBlockM) return false;
-    return pair_us(B, H, W, C, K) < 0.95 * fmin(unpaired_us(B, H, W, C, K, layout), cl_cut(P, C, K).us);
+    return pair_us(B, H, W, C, K, layout) < 0.95 * fmin(unpaired_us(B, H, W, C, K, layout), cl_cut(P, C, K).us);
 }

@@ -137,8 +137,8 @@ def fused_preferred(B, H, W, C, K, layout="NCHW"):
 
 def layer_fwd_prepared(x, prepared, K, relu=True, layout="NHWC", out=None, V_scratch=None, out_scale=None, out_shift=None,
                        residual=None, workspace=None, in_scale=None, in_shift=None, residual_relu=False):
-    """Whole layer with prepared weights: one kernel where supported and faster (V never stored: a kernel of its own for few
-    tiles, NCHW ones for many tiles and for few channels), else transform + product through V_scratch (allocated here when not given); layers
+    """Whole layer with prepared weights: one kernel where supported and faster (V never stored: kernels of their own for few
+    and for many tiles, an NCHW one for few channels), else transform + product through V_scratch (allocated here when not given); layers
     with many channels take the wide product path through `workspace` (allocated here when not given;
     layer_fwd_prepared_workspace_bytes).  in_scale / in_shift (C,): affine map of the pixels in front of the transform, the
     padding stays zero; residual_relu: the shortcut passes through a ReLU first."""

@@ -1,6 +1,6 @@
 """The layer on pairs of SMs (csrc/conv_tc_pair.cuh) through layer_fwd_prepared, at sizes where its cuts can go wrong: row lengths of
 each alignment, quads that cross rows and images, images copied whole, channel counts that end inside a slot, a weight stage or a block
-of outputs, weights that stay in shared memory and weights that stream, a last unit with one CTA's quads only."""
+of outputs, weights that stay in shared memory and weights that stream, a last unit with one CTA's quads only; both layouts."""
 import numpy as np
 import pytest
 
@@ -20,43 +20,48 @@ SHAPES = [
     (17, 256, 256, 28, 31),    # weights stream through their ring
     (24, 64, 64, 65, 64),      # wide rows
 ]
+# channels last: rows of whole quads
+CASES = [(s, "NCHW") for s in SHAPES] + [(s, "NHWC") for s in ((96, 64, 64, 40, 56), (40, 100, 80, 41, 20), (513, 64, 128, 11, 12), (17, 256, 256, 27, 32),
+                                                               (24, 64, 64, 65, 64), (900, 36, 72, 7, 8), (2000, 64, 68, 5, 4))]
 
 
-def _inputs(shape):
+def _inputs(shape, layout="NCHW"):
     import torch
     B, C, K, H, W = shape
     g = torch.Generator(device="cuda").manual_seed(sum(shape))
     rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
-    return rnd, rnd(B, C, H, W), rnd(16, C, K) * (1.0 / (16 * C)) ** 0.5
+    return rnd, rnd(B, C, H, W) if layout == "NCHW" else rnd(B, H, W, C), rnd(16, C, K) * (1.0 / (16 * C)) ** 0.5
 
 
 def _images(B):
     return sorted({0, B // 2, B - 1})      # the oracle computes these
 
 
-@pytest.mark.parametrize("shape", SHAPES)
-def test_against_the_oracle(oracle, shape):
+@pytest.mark.parametrize("shape,layout", CASES)
+def test_against_the_oracle(oracle, shape, layout):
     import torch
     import wg2x2
     from wg2x2._lib import lib
     B, C, K, H, W = shape
-    assert lib.wg2x2_layer_fwd_pair_preferred(B, H, W, C, K, 1)
-    rnd, x, w = _inputs(shape)
+    assert lib.wg2x2_layer_fwd_pair_preferred(B, H, W, C, K, 1 if layout == "NCHW" else 0)
+    rnd, x, w = _inputs(shape, layout)
     prepared = wg2x2.prepare_weights(w)
-    si, ti, so, to, r = 1 + 0.2 * rnd(C), 0.3 * rnd(C), 1 + 0.2 * rnd(K), 0.3 * rnd(K), rnd(B, K, H, W)
+    si, ti, so, to = 1 + 0.2 * rnd(C), 0.3 * rnd(C), 1 + 0.2 * rnd(K), 0.3 * rnd(K)
+    r = rnd(B, K, H, W) if layout == "NCHW" else rnd(B, H, W, K)
     pick = _images(B)
-    nhwc = lambda t: np.ascontiguousarray(t[pick].permute(0, 2, 3, 1).cpu().numpy())
+    nhwc = lambda t: np.ascontiguousarray((t[pick].permute(0, 2, 3, 1) if layout == "NCHW" else t[pick]).cpu().numpy())
+    ch = lambda t: t.view(1, -1, 1, 1) if layout == "NCHW" else t
 
     def want(a, relu):
         v = oracle.imtrans_fwd(a, relu=relu)
         return oracle.conv_fwd(v, w.cpu().numpy(), H, W)
 
     for relu in (True, False):
-        y = wg2x2.layer_fwd_prepared(x, prepared, K, relu=relu, layout="NCHW")
+        y = wg2x2.layer_fwd_prepared(x, prepared, K, relu=relu, layout=layout)
         assert wg2x2.last_device_status()[0] == 0
         assert oracle.max_rel(nhwc(y), want(nhwc(x), relu)) <= TOL_TF32
-    main = want(nhwc(x * si.view(1, -1, 1, 1) + ti.view(1, -1, 1, 1)), True) * so.cpu().numpy() + to.cpu().numpy()
-    kw = dict(relu=True, layout="NCHW", in_scale=si, in_shift=ti, out_scale=so, out_shift=to)
+    main = want(nhwc(x * ch(si) + ch(ti)), True) * so.cpu().numpy() + to.cpu().numpy()
+    kw = dict(relu=True, layout=layout, in_scale=si, in_shift=ti, out_scale=so, out_shift=to)
     # no shortcut, one of its own, one that Y lies over
     assert oracle.max_rel(nhwc(wg2x2.layer_fwd_prepared(x, prepared, K, **kw)), main) <= TOL_TF32
     for res_relu in (False, True):
@@ -71,18 +76,36 @@ def test_against_the_oracle(oracle, shape):
     assert wg2x2.last_device_status()[0] == 0
 
 
+@pytest.mark.parametrize("shape,layout", [((96, 64, 64, 40, 56), "NHWC"), ((128, 64, 64, 28, 28), "NHWC"), ((64, 64, 64, 56, 56), "NCHW"), ((65, 96, 96, 27, 27), "NCHW")])
+def test_every_element_of_many_launches(shape, layout):
+    """Against the FP32 kernels: a stage of pixels handed back before its last load has delivered shows in a few pixels of some launches."""
+    import torch
+    import wg2x2
+    B, C, K, H, W = shape
+    rnd, x, w = _inputs(shape, layout)
+    prepared = wg2x2.prepare_weights(w)
+    ch = lambda t: t.view(1, -1, 1, 1) if layout == "NCHW" else t
+    si, ti, r = 1 + 0.2 * rnd(C), 0.3 * rnd(C), torch.randn_like(x[:, :1] if layout == "NCHW" else x[..., :1]).expand(*((B, K, H, W) if layout == "NCHW" else (B, H, W, K))).contiguous()
+    fp32 = lambda a: wg2x2.conv_fwd(wg2x2.imtrans_fwd(a, relu=True, layout=layout), w, H, W, layout=layout, math="fp32")
+    plain, main = fp32(x), fp32(x * ch(si) + ch(ti)) + r
+    for _ in range(12):
+        for want, kw in ((plain, {}), (main, dict(in_scale=si, in_shift=ti, residual=r))):
+            y = wg2x2.layer_fwd_prepared(x, prepared, K, relu=True, layout=layout, **kw)
+            assert float((y - want).abs().max()) <= TOL_TF32 * float(want.abs().max())
+
+
 def test_output_is_written_exactly():
     """Nothing beyond Y is touched, and all of Y is."""
     import torch
     import wg2x2
-    for shape in SHAPES:
+    for shape, layout in CASES:
         B, C, K, H, W = shape
-        rnd, x, w = _inputs(shape)
+        rnd, x, w = _inputs(shape, layout)
         n = B * K * H * W
         room = torch.full((n + 64,), 12345.0, device="cuda")
-        y = room[32:32 + n].view(B, K, H, W)
+        y = room[32:32 + n].view((B, K, H, W) if layout == "NCHW" else (B, H, W, K))
         y.fill_(float("nan"))
-        wg2x2.layer_fwd_prepared(x, wg2x2.prepare_weights(w), K, layout="NCHW", out=y)
+        wg2x2.layer_fwd_prepared(x, wg2x2.prepare_weights(w), K, layout=layout, out=y)
         assert bool(torch.isfinite(y).all()) and bool((room[:32] == 12345.0).all()) and bool((room[32 + n:] == 12345.0).all())
 
 
