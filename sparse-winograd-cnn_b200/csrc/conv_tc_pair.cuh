@@ -1,5 +1,6 @@
-// Winograd-ReLU layer forward, X -> Y in one kernel, on pairs of SMs (NCHW in and out, any image size): neither the transformed
-// input V nor the sixteen Winograd-domain products ever exist outside an SM.  Included by conv_tc.cu.
+// Winograd-ReLU layer forward, X -> Y in one kernel, on pairs of SMs (NCHW, any image size, and channels last where a
+// row of quads is whole, W % 4 == 0 and K % 4 == 0): neither the transformed input V nor the
+// sixteen Winograd-domain products ever exist outside an SM.  Included by conv_tc.cu.
 //
 // As in conv_tc_fused.cuh both transforms ride on the tensor core's operands: the A operand of every MMA (position (i, j) of B^T d B,
 // after the ReLU) is written into tensor memory by transform warps, and position (i, j) is accumulated with the sign
@@ -11,19 +12,24 @@
 //     of 56 x 56 are 196 units of 256 tiles in three rounds on 74 pairs, where whole rows of tiles need four;
 //   * a thread forms all sixteen positions of a quad's four tiles from one 6 x 6 window: 36 loads for 64 values, and one
 //     tcgen05.st of 16 lanes x 32 columns per Winograd row and row of tiles;
-//   * pixels come as plain bulk copies of the rows' contiguous memory, so the image needs no row length of 16-byte pieces;
-//   * Y leaves from registers, 16 bytes a thread where rows allow; the shortcut is added behind the stores.
+//   * pixels come as plain bulk copies of the rows' contiguous memory, so that an NCHW image needs no row length of 16-byte pieces; channels
+//     last as one TMA box of 8 channels per row of quads, read by thread pairs as two channels at a time;
+//   * Y leaves from registers, 16 bytes a thread where rows allow; the shortcut is added in front of the stores, or behind them in L2 where
+//     rows are of 16-byte pieces and a pair has more than one unit.
 // A unit walks the input channels in slots of 8: transform team n % 2 fills A group n % 2 (16 positions x 8 columns), four issuers,
 // one per accumulator, take it from there.
 //
 // What it measured (us, this against the fastest of the other paths): 64 x 64 x 56 x 56 45 -> 34, 256 images of it 137 -> 105,
-// 256 x 128 x 28 x 28 138 -> 97, 128 x 256 x 14 x 14 93 -> 68, 64 x 256 x 40 x 40 341 -> 170.  What bounds it: a slot's MMAs take 1152
+// 256 x 128 x 28 x 28 138 -> 97, 128 x 256 x 14 x 14 93 -> 68, 64 x 256 x 40 x 40 341 -> 170;
+// channels last 32 x 128 x 28 x 28 37 -> 22.  What bounds it: a slot's MMAs take 1152
 // clocks, a slot takes about 1600.  With the MMAs at full rate tensor memory takes one store of 1 KB per subpartition and MMA (16 of 36
 // such gaps are needed, so that stores are slow and the warps behind them wait), a transform warp's own chain of loads, shuffles, 288
 // arithmetic instructions and eight stores is 2700 clocks for its two slots, and issue slots are 57 % busy.  At the end of a unit the
 // stores of one output row hold the other's accumulators: 4000 - 5000 clocks, when all SMs store at once.
-// Tried: pixels by loads into registers (latency: 111 against 97 us at 28 x 28), sixteen transform warps of one channel each (stores of 256
-// bytes: 106), three teams (101), one issuer per output row (two in all: 141), a full barrier per half group (126).
+// Tried, at 256 x 128 x 28 x 28 with 97 .. 100 us as it is: pixels by loads into registers (latency: 111), sixteen transform warps of one
+// channel each (stores of 256 bytes: 106), three teams (101 .. 105), issuers that look ahead for the next slot's barrier (104, with three
+// teams 113), one issuer per output row (two in all: 141), a full barrier per half group (126); at 256 x 64 x 56 x 56, 108 as it is, an
+// epilogue that takes three of the four quarter rows into registers before its first store (111).
 #pragma once
 
 constexpr int kPrThreads = 768;                    // 4 issuing, 4 loading, 8 epilogue, 8 transform warps
@@ -47,7 +53,8 @@ struct PrParams {
     int nW, nX, xbytes;                    // stages of weights and pixels, bytes of a pixel stage
     int xpitch, xpart, whole;              // floats of a channel and of a whole image in a pixel stage; whole images are copied (pr_geometry)
     int nKB, nS, units;                    // blocks of N output channels, slots of 8 channels, units of 64 quads x N channels
-    int relu, res_relu, in_place;          // in_place: Y holds the shortcut, its ReLU applied, and 16-byte pieces are added to it
+    int relu, res_relu, front;             // front: the shortcut is added in front of the stores
+    int in_place;                          // in_place: Y holds the shortcut, its ReLU applied, and 16-byte pieces are added to it
     uint32_t zero;                         // 0, which the compiler does not know
     uint32_t spin_limit;                   // polls before a wait gives up (wg2x2_set_wait_limit)
     int drop_load;                         // >= 0: the W producer of CTA 0 leaves out its drop_load-th stage (wg2x2_test_drop_load), else -1
@@ -721,9 +728,10 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, const __grid_con
                 }
             };
             bool ok = true;
-            if constexpr (EXTRAS && VEC < 4) {
-                // The shortcut in narrow pieces: added in front of the stores (8- and 4-byte reductions behind them take longer than its
-                // latency: 103 against 90 us for 128 x 256 x 14 x 14), also where Y lies over it.  A row's loads go out when the row before has
+            if (EXTRAS && (VEC < 4 || prm.front)) {
+                // The shortcut in narrow pieces, or with one unit per pair: added in front of the stores (8- and 4-byte reductions behind them
+                // take longer than its latency, 103 against 90 us for 128 x 256 x 14 x 14, and with no unit to follow nothing hides them,
+                // 29.2 against 26.0 for 16 x 96 x 40 x 36), also where Y lies over it.  A row's loads go out when the row before has
                 // been added, the first row's of a unit while that unit is still being multiplied, and the others into L2 by then.
                 float r[2][N / 4], scale = 1.f, shift = 0.f;
                 Where w = my_units > 0 ? place(0) : Where{};
@@ -922,7 +930,8 @@ int layer_fwd_pair(const float *X, const void *prepared, float *Y, int B, int H,
     p.masks = reinterpret_cast<const unsigned long long *>(static_cast<const unsigned char *>(prepared) + align_up((size_t)16 * K * C * sizeof(float), 256));
     p.relu = relu; p.res_relu = res_relu;
     // Y over the shortcut: a thread adds its elements to those there
-    p.in_place = layout == WG2X2_NCHW && W % 4 == 0 && residual == Y;      // (a NULL Y was refused)
+    p.front = p.units <= kNumSMs / 2;
+    p.in_place = layout == WG2X2_NCHW && W % 4 == 0 && !p.front && residual == Y;      // (a NULL Y was refused)
     if (p.in_place) {
         if (res_relu) {
             const long long n4 = (long long)B * K * H * W / 4;
@@ -962,21 +971,25 @@ int layer_fwd_pair(const float *X, const void *prepared, float *Y, int B, int H,
     return launch(kernel, dim3((unsigned)(2 * pairs)), kPrThreads, (size_t)p.nW * kPrStageBytes + (size_t)p.nX * p.xbytes + kCtrlBytes + 1024, st, mapW, mapX, p);
 }
 
-// Microseconds of the layer on pairs of SMs (plain, 1 .. 128 images of 7 .. 56 pixels, 32 .. 512 channels: within a tenth of the
-// measured): rounds of units, each a walk over the input channels and the change of accumulators at its end.
+// Microseconds of the layer on pairs of SMs (plain, both layouts, 1 .. 256 images of 7 .. 64 pixels, 16 .. 512 channels: within a fifth of
+// the measured): rounds of units, each a walk over the input channels and the change of accumulators at its end, which takes
+// long where rows are stored pixel by pixel.  (Images of at most ten quads lie whole in shared memory, their channels on the same banks.)
 static double pair_us(int B, int H, int W, int C, int K, int layout)
 {
     const double rounds = (double)cdivll(cdivll((long long)B * cdiv(H, 4) * cdiv(W, 4), 2 * kPrQuads) * cdiv(K, 64), kNumSMs / 2);
-    return 6.4 + rounds * (3.5 + (layout == WG2X2_NHWC ? 0.83 : W % 4 == 0 ? 0.71 : W % 2 == 0 ? 0.79 : 1.21) * cdiv(C, 8));
+    return layout == WG2X2_NHWC ? 6.5 + rounds * (1.5 + 0.98 * cdiv(C, 8)) : 6.3 + rounds * ((W % 2 ? 9.5 : 3.2) + (cdiv(H, 4) * cdiv(W, 4) <= 10 ? 1.05 : 0.82) * cdiv(C, 8));
 }
 
-// Against all other paths, for any NCHW image.  It wins where its units fill the SMs at
-// least once: over 172 layers of 1 .. 128 images it takes 0.50 .. 0.95 of the time in 75 (64 x 256 x 40 x 40 341 -> 170 us,
-// 128 x 256 x 14 x 14 93 -> 68, 64 x 64 x 56 x 56 45 -> 34), with fewer units up to four times as long.
+// Against all other paths.  It wins where its units fill the SMs at least once: over 172 NCHW layers of 1 .. 128 images it takes 0.50 ..
+// 0.95 of the time in 75 (64 x 256 x 40 x 40 341 -> 170 us, 128 x 256 x 14 x 14 93 -> 68, 64 x 64 x 56 x 56 45 -> 34), with fewer units up
+// to four times as long.  Over 110 layers of both layouts that this rule picks the geometric mean is 1.7 times as fast, with a shortcut
+// too.  The factors are the margins that the estimates need: channels last, 0.95 takes 46 x 96 x 192 x 12 x 12 too, 19.9 us (24.9 with a
+// shortcut) against 18.7 (19.7), and nothing else that 0.85 leaves.  A layer of fewer than 16 units is a call of a few microseconds, for
+// which the estimates themselves (60 ns, asked twice) would count.
 bool layer_pair_preferred(int B, int H, int W, int C, int K, int layout)
 {
-    if (!pair_supported(B, H, W, C, K, layout)) return false;
+    if (cdivll((long long)B * cdiv(H, 4) * cdiv(W, 4), 2 * kPrQuads) * cdiv(K, 64) < 16 || !pair_supported(B, H, W, C, K, layout)) return false;
     const long long P = (long long)B * ((H + 1) / 2) * ((W + 1) / 2);
     if (P > 0x7fffffffLL - kBlockM) return false;
-    return pair_us(B, H, W, C, K, layout) < 0.95 * fmin(unpaired_us(B, H, W, C, K, layout), cl_cut(P, C, K).us);
+    return pair_us(B, H, W, C, K, layout) < (layout == WG2X2_NHWC ? 0.85 : 0.95) * fmin(unpaired_us(B, H, W, C, K, layout), cl_cut(P, C, K).us);
 }

@@ -15,8 +15,8 @@ SHAPES = [
     (65, 96, 96, 27, 27),      # odd rows: copies from any 4-byte boundary
     (130, 44, 72, 14, 14),     # rows of 8-byte pieces, quads beyond the image on two sides
     (513, 64, 128, 11, 12),    # nine quads an image: images copied whole
-    (1100, 48, 136, 9, 10),
-    (600, 72, 64, 10, 11),     # the same with odd rows
+    (1400, 64, 120, 9, 10),
+    (1100, 92, 124, 12, 11),   # the same with odd rows, and a slot of four channels
     (17, 256, 256, 28, 31),    # weights stream through their ring
     (24, 64, 64, 65, 64),      # wide rows
 ]
