@@ -47,6 +47,8 @@ NCU_TRAFFIC = {
     ("cfg2", 64, "NCHW", "conv"): (224.7e6, "ncu capture, profiles/conv_fwd_tc_kernel_cfg2.md"),
     ("cfg2", 64, "NCHW", "fused"): (60.0e6, "ncu capture, profiles/layer_fwd_fused_kernel_cfg2.md (X read once; most of Y is still "
                                             "dirty in L2 when the launch ends, so it is below the algorithmic X + W + Y)"),
+    ("cfg2", 64, "NCHW", "pair"): (58.1e6, "ncu capture, profiles/layer_fwd_pair_kernel_cfg2.md (X read once; most of Y is still "
+                                           "dirty in L2 when the launch ends, so it is below the algorithmic X + W + Y)"),
 }
 
 
@@ -316,9 +318,12 @@ class LayerFwd:
         self.prepared = wg2x2.prepare_weights(self.Wt) if math == "tf32" else None
         cws_n = lib.wg2x2_conv_fwd_prepared_workspace_bytes(B, nH, nW, C, K) if self.prepared is not None else 0
         self.cws = torch.empty(cws_n, dtype=torch.uint8, device=ctx.dev) if cws_n else None   # products of the wide path (C, K >= 256)
-        fused_ok = self.prepared is not None and layout == "NCHW" and wg2x2.fused_supported(B, H, W, C, K, "NCHW")
+        # one kernel per layer: where the library's own call takes one ("auto"), or the unpaired one by name ("fused")
+        one = self.prepared is not None and layout == "NCHW"
+        self.use_pair = one and path == "auto" and bool(lib.wg2x2_layer_fwd_pair_preferred(B, H, W, C, K, 1))
+        fused_ok = one and wg2x2.fused_supported(B, H, W, C, K, "NCHW")
         fused_pays = K <= 128 or (K <= 256 and C <= 64)          # the rule of wg2x2_layer_fwd_prepared for a layer of many tiles
-        self.use_fused = fused_ok and (path == "fused" or (path == "auto" and fused_pays))
+        self.use_fused = self.use_pair or (fused_ok and (path == "fused" or (path == "auto" and fused_pays)))
         self.bytesX, self.bytesV, self.bytesY, self.bytesW = 4 * B * C * H * W, 64 * self.P * C, 4 * B * K * H * W, 64 * C * K
         self.flops = 2.0 * 16 * self.P * C * K
         self._fused_calls = None
@@ -335,19 +340,23 @@ class LayerFwd:
 
     def fused(self, i):
         # straight through the C ABI with the arguments built once: the timed loop is one foreign call per step, as in the
-        # reference's op Compute (the Python wrapper's argument checks would cost a third of a 47 us step on the host)
+        # reference's op Compute (the Python wrapper's argument checks would cost a third of a 33 us step on the host)
         if self._fused_calls is None:
             lib = self.wg._lib.lib
             wl = self.wl
             stream = ctypes.c_void_p(self.ctx.torch.cuda.current_stream().cuda_stream)
             P = ctypes.c_void_p
+            # the entry point that chooses the kernel by the layer's sizes; a layer that it runs on pairs of SMs needs no scratch
             self._fused_calls = [
+                (lib.wg2x2_layer_fwd_prepared_ex, (P(x.data_ptr()), None, None, P(self.prepared.data_ptr()), P(self.Y.data_ptr()), None, wl["B"],
+                                                   wl["H"], wl["W"], wl["C"], wl["K"], 1, 1, None, None, None, 0, None, 0, stream))
+                for x in self.Xs] if self.use_pair else [
                 (lib.wg2x2_layer_fwd_fused, (P(x.data_ptr()), P(self.prepared.data_ptr()), P(self.Y.data_ptr()), wl["B"], wl["H"], wl["W"],
                                              wl["C"], wl["K"], 1, None, None, None, stream)) for x in self.Xs]
         fn, a = self._fused_calls[i % self.nbuf]
         rc = fn(*a)
         if rc != 0:
-            raise RuntimeError("wg2x2_layer_fwd_fused returned %d" % rc)
+            raise RuntimeError("the one-kernel layer returned %d" % rc)
 
     def step(self, i):
         if self.use_fused:
@@ -368,14 +377,18 @@ class LayerFwd:
         if self.use_fused:
             ms = each_launch_ms(torch, self.fused, n_each)
             fb = self.bytesX + self.bytesW + self.bytesY
-            roof = dict(kernel="layer_fwd_fused_kernel (transform + ReLU + products + output transform, one launch = the whole layer)",
-                        bound="hbm", achieved=fb / (ms * 1e-3) / 1e9, peak=pk["hbm_gbs"], unit="GB/s", peak_source=pk["source"],
-                        algorithmic_bytes=fb, tensor_tflops_algorithmic=self.flops / (ms * 1e-3) / 1e12,
-                        tensor_tflops_issued=2.25 * self.flops / (ms * 1e-3) / 1e12, kernels_ms={"layer_fwd_fused": ms},
+            name = "layer_fwd_pair" if self.use_pair else "layer_fwd_fused"
+            roof = dict(kernel=name + "_kernel (transform + ReLU + products + output transform, one launch = the whole layer)")
+            if self.flops / (tf32_peak * 1e12) > fb / (pk["hbm_gbs"] * 1e9):
+                roof.update(bound="tensor", achieved=self.flops / (ms * 1e-3) / 1e12, peak=tf32_peak, unit="TFLOP/s", peak_source=pk["source"] + " bf16 / 2")
+            else:
+                roof.update(bound="hbm", achieved=fb / (ms * 1e-3) / 1e9, peak=pk["hbm_gbs"], unit="GB/s", peak_source=pk["source"])
+            roof.update(algorithmic_bytes=fb, tensor_tflops_algorithmic=self.flops / (ms * 1e-3) / 1e12,
+                        tensor_tflops_issued=2.25 * self.flops / (ms * 1e-3) / 1e12, kernels_ms={name: ms},
                         note="only X, W and Y cross HBM; the kernel is paced by the SM, not by HBM (36 signed MMAs per 8 channels instead "
                              "of 16, transform warps in step with them).  kernels_ms is a launch bracketed by events on its own; back to "
                              "back the launches overlap their neighbours' tails (programmatic dependent launch), so ms_per_step can be below it")
-            which = "fused"
+            which = "pair" if self.use_pair else "fused"
         else:
             ms1 = each_launch_ms(torch, self.imtrans, n_each)
             ms2 = each_launch_ms(torch, self.conv, n_each)
@@ -435,7 +448,7 @@ def sub_layer_fwd(ctx, name, args, steps):
     roof, _ = L.roofline(pk, n_each=12)
     roof["traffic"] = None
     rec = {"ms_per_step": ms, "steps": steps, "img_s": ctx.world * wl["B"] / (ms * 1e-3), "layer": wl, "layout": "NCHW", "dtype": "tf32",
-           "path": "one fused kernel" if L.use_fused else ("input transform, then products as GEMMs with 256 output channels per unit "
+           "path": "one kernel on pairs of SMs" if L.use_pair else "one fused kernel" if L.use_fused else ("input transform, then products as GEMMs with 256 output channels per unit "
                                                           "into scratch + output transform pass" if L.cws is not None else "two kernels, V through HBM"),
            "layer_tflops": L.flops / (ms * 1e-3) / 1e12, "layer_gbs": L.layer_bytes() / (ms * 1e-3) / 1e9,
            "strict_layer_bound_ms": 1e3 * max((L.bytesX + L.bytesW + L.bytesY) / (pk["hbm_gbs"] * 1e9), L.flops / (pk["bf16_tflops"] / 2 * 1e12)),
@@ -446,7 +459,7 @@ def sub_layer_fwd(ctx, name, args, steps):
         w2 = (0.05 * np.random.default_rng(2).standard_normal((16, wl["C"], wl["K"]))).astype(np.float32)
         rec["skip_rate_magnitude_mask"] = zero_block_fraction(gen_prune_mask(w2, wl["density"]))   # the reference's top-|w| mask, same density
         rec["skip_note"] = "unstructured masks leave no 64 x 32 block empty: tensor-pipe figures are from dense flops"
-    if not L.use_fused and wl["C"] >= 256:       # tensor-bound shape: the vendor library's rate on the same 16 products, for scale
+    if wl["C"] >= 256:       # tensor-bound shape: the vendor library's rate on the same 16 products, for scale
         P = wl["B"] * ((wl["H"] + 1) // 2) * ((wl["W"] + 1) // 2)
         rec["library_tf32"] = library_tf32(ctx, [(16, P, wl["C"], wl["K"])])
     del L
@@ -680,7 +693,7 @@ def run_layer(args, ctx):
         # one launch per step: the kernel's average launch duration over the timed region is ms_per_step; the duration of a
         # launch bracketed by its own events (no overlap with its neighbours' launch latency) is kept beside it
         roof["achieved_isolated_launch"], roof["frac_isolated_launch"] = roof["achieved"], roof["frac"]
-        roof["achieved"] = roof["algorithmic_bytes"] / (ms_step * 1e-3) / 1e9
+        roof["achieved"] = (roof["algorithmic_bytes"] / 1e9 if roof["bound"] == "hbm" else L.flops / 1e12) / (ms_step * 1e-3)
         roof["frac"] = roof["achieved"] / roof["peak"]
         roof["duration_ms"] = ms_step
     traffic = NCU_TRAFFIC.get((args.workload, B, args.layout, which))
@@ -702,7 +715,8 @@ def run_layer(args, ctx):
                    "l2": "%d rotating input buffers (%.0f MB); %.0f MB moved per step" % (L.nbuf, L.nbuf * L.bytesX / 1e6, L.layer_bytes() / 1e6),
                    "weights": "prepared once outside the timed region (wg2x2_weights_prepare)",
                    "timing": "two CUDA events around the steps; per-kernel durations from a separate pass afterwards",
-                   "path": "one fused kernel (wg2x2_layer_fwd_fused)" if L.use_fused else "two kernels, V through HBM"},
+                   "path": "one kernel (wg2x2_layer_fwd_prepared_ex, on pairs of SMs)" if L.use_pair else
+                           "one fused kernel (wg2x2_layer_fwd_fused)" if L.use_fused else "two kernels, V through HBM"},
         "layer_gbs": L.layer_bytes() * ctx.world / (ms_step * 1e-3) / 1e9,
         "layer_tflops": L.flops * ctx.world / (ms_step * 1e-3) / 1e12,
         "roofline": roof, "clocks": clocks, "gpu_launches": args.steps * (1 if L.use_fused else 2),
@@ -839,8 +853,8 @@ def main():
     ap.add_argument("--batch", type=int, default=0, help="override the per-GPU batch of the workload (profiling on a small case)")
     ap.add_argument("--e2e-chunks", type=int, default=2, help="chunks of the host-buffer pipeline")
     ap.add_argument("--path", default="auto", choices=["auto", "fused", "two-kernel"],
-                    help="layer forward: the one-kernel path (X -> Y, V never stored), the two kernels, or (auto) the one "
-                         "kernel for K <= 128, or K <= 256 with C <= 64")
+                    help="layer forward: the unpaired one-kernel path (X -> Y, V never stored), the two kernels, or (auto) the kernel "
+                         "on pairs of SMs where the library prefers it, else the unpaired one for K <= 128, or K <= 256 with C <= 64")
     ap.add_argument("--fused", action="store_true", help="same as --path fused")
     ap.add_argument("--net-layout", default="NCHW", choices=["NHWC", "NCHW"],
                     help="cfg4: physical layout of the activations (NCHW: the 56x56 and 28x28 layers run as one kernel each)")
