@@ -519,7 +519,7 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, const __grid_con
                 if (!ok) break;
                 // [channel][row]: columns 0 1 | 2 3, and the outer two; channels last: [row][column], both channels
                 float2 m[2][6][2], lr[2][6], win[6][6];
-                uint32_t loaded = 0;                                 // a bit of every load that nothing else waits for in front of the stage's release
+                uint32_t loaded = 0;                                 // a register of every load
                 if constexpr (NHWC) {
                     const uint32_t at = xbase + xs * prm.xbytes + quad, px = 32u * (uint32_t)(prm.nQW + 2);
 #pragma unroll
@@ -556,7 +556,11 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, const __grid_con
                         if (VEC < 4 && !prm.whole) at += 4u * (uint32_t)((at0 + (long long)c * plane) & 3);   // where the copy's first 16 bytes begin
                         pr_window<VEC>(d[p], ed[p], at, prm.W, qg == 0 ? -4 : 16, chan ? flags : 0u, cols);
 #pragma unroll
-                        for (int r = 0; r < 6; ++r) loaded ^= __float_as_uint(ed[p][r]) ^ (VEC == 1 ? __float_as_uint(d[p][r][1]) ^ __float_as_uint(d[p][r][2]) : 0u);
+                        for (int r = 0; r < 6; ++r) {
+                            loaded ^= __float_as_uint(ed[p][r]);
+#pragma unroll
+                            for (int x = 0; x < 4; x += VEC) loaded ^= __float_as_uint(d[p][r][x]);
+                        }
                         if (AFFINE) { sc[p] = chan ? __ldg(prm.in_scale + c + cl) : 1.f; tc[p] = chan ? __ldg(prm.in_shift + c + cl) : 0.f; }
                     }
                     // the windows with their outer columns, from the neighbouring quads' lanes where those are in this warp
@@ -583,11 +587,11 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, const __grid_con
                             lr[p][r].y = flags & kPrNoRight ? 0.f : (qg == 7 ? ed[p][r] : lr[p][r].y);
                         }
                 }
-                // The stage is handed back once every load has delivered.  An arrival does not wait for loads that have only been issued, and behind
-                // tensor-memory stores those may be hundreds of clocks away from shared memory: the shuffles wait for most of them, the
-                // arrival's address for the others.
-                __syncwarp();
-                if (lane == 0) mbar_arrive(xempty_bar(xs) + (loaded & prm.zero));
+                // The stage is handed back once every load of every lane has delivered.  An arrival does not wait for loads that have only been
+                // issued, and behind tensor-memory stores those may be hundreds of clocks away from shared memory: the arrival's address
+                // depends on a vote over all that they brought (which is always 0).
+                const uint32_t none = __any_sync(0xffffffffu, (loaded & prm.zero) != 0u) ? 8u : 0u;
+                if (lane == 0) mbar_arrive(xempty_bar(xs) + none);
                 xs += 2; if (xs >= prm.nX) xs -= prm.nX;
                 xf += 2; if (xf >= 2 * prm.nX) { xf -= 2 * prm.nX; xph ^= 1u; }
 #pragma unroll

@@ -76,7 +76,9 @@ def test_against_the_oracle(oracle, shape, layout):
     assert wg2x2.last_device_status()[0] == 0
 
 
-@pytest.mark.parametrize("shape,layout", [((96, 64, 64, 40, 56), "NHWC"), ((128, 64, 64, 28, 28), "NHWC"), ((64, 64, 64, 56, 56), "NCHW"), ((65, 96, 96, 27, 27), "NCHW")])
+@pytest.mark.parametrize("shape,layout", [((96, 64, 64, 40, 56), "NHWC"), ((128, 64, 64, 28, 28), "NHWC"), ((64, 64, 64, 56, 56), "NCHW"), ((65, 96, 96, 27, 27), "NCHW"),
+                                          # rows of 8-byte pieces with weights streaming, images copied whole in rows of each alignment
+                                          ((128, 256, 256, 14, 14), "NCHW"), ((513, 64, 128, 11, 12), "NCHW"), ((1400, 64, 120, 9, 10), "NCHW"), ((1100, 92, 124, 12, 11), "NCHW")])
 def test_every_element_of_many_launches(shape, layout):
     """Against the FP32 kernels: a stage of pixels handed back before its last load has delivered shows in a few pixels of some launches."""
     import torch
