@@ -477,7 +477,7 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, const __grid_con
             // Team t fills the slots n with n % 2 = t, always into A group t.  A thread walks its quad's channels, two a slot (cl and cl + 4).
             asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPrRegsXf));
             const int team = (warp - 16) >> 2;
-            const float lo = prm.relu ? 0.f : -__int_as_float(0x7f800000);
+            const float lo = prm.relu ? 0.f : __int_as_float(0x7fffffff);      // the larger of a number and NaN is the number: without a ReLU all stay
             const long long plane = (long long)prm.H * prm.W;
             const int total = my_units * nS;
             const uint32_t a_tmem = tmem_base + ((uint32_t)(sub * 32) << 16) + (uint32_t)(kPrACol0 + team * kPrGroupCols);
@@ -639,7 +639,8 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, const __grid_con
                                 // instead of 16, whose longer sums cost up to 1.3 % of the error against 64 bits (512 channels:
                                 // 4.69e-4 -> 4.75e-4 relative); with this one it is 4.58e-4.  All rounded: 2.96e-4, 3 to 18 % slower.
 #pragma unroll
-                                for (int x = 4; x < 8; ++x) o[x] = __uint_as_float(__float_as_uint(o[x]) + 0x1000u);
+                                for (int x = 4; x < 8; ++x)
+                                    if (fabsf(o[x]) < __int_as_float(0x7f800000)) o[x] = __uint_as_float(__float_as_uint(o[x]) + 0x1000u);     // (infinities and NaN stay)
                             }
                             const uint32_t to = a_tmem + ((uint32_t)(16 * dy) << 16) + (uint32_t)(32 * i);
                             if (NHWC) tmem_st_16x32_pairs(to, o); else tmem_st_16x32(to, o);

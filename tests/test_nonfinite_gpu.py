@@ -123,6 +123,56 @@ def test_shortcut_reaches_the_output(shape, layout):
     assert torch.equal(torch.nan_to_num(got, 0.0), torch.nan_to_num(want, 0.0))
 
 
+def _layer_like(x, w, H, W, relu):
+    """The layer's output in float64 by additions only, a zero coefficient being no operand: x (B, C, H, W), w (16, C, K) -> (B, K, H, W)."""
+    nH, nW = (H + 1) // 2, (W + 1) // 2
+    d = F.pad(x.double(), (1, 2 * nW - W + 1, 1, 2 * nH - H + 1)).unfold(2, 4, 2).unfold(3, 4, 2)                       # (B, C, nH, nW, 4, 4)
+    rows = lambda q: (q[0] - q[2], q[1] + q[2], q[2] - q[1], q[1] - q[3])
+    v = [p for r in rows(d.unbind(4)) for p in rows(r.unbind(4))]
+    if relu:
+        v = [torch.where(p > 0, p, 0.0) for p in v]            # drops NaN, as fmax does
+    m = torch.stack([torch.einsum("bchw,ck->bkhw", p, q.double()) for p, q in zip(v, w)]).unflatten(0, (4, 4))
+    cols = lambda q: torch.stack((q[0] + q[1] + q[2], q[1] - q[2] - q[3]), -1)
+    a = cols(m.unbind(0))                                      # (4, B, K, nH, nW, 2), rows transformed
+    return cols(a.unbind(0)).permute(0, 1, 2, 4, 3, 5).reshape(x.shape[0], w.shape[2], 2 * nH, 2 * nW)[:, :, :H, :W]
+
+
+# the layer on pairs of SMs: rows of each alignment, images copied whole, channels last
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,layout", [((64, 64, 64, 56, 56), "NCHW"), ((130, 44, 72, 14, 14), "NCHW"), ((65, 96, 96, 27, 27), "NCHW"), ((1400, 64, 120, 9, 10), "NCHW"),
+                                          ((513, 64, 128, 11, 12), "NCHW"), ((128, 64, 64, 28, 28), "NHWC"), ((40, 100, 80, 41, 20), "NHWC")])
+@pytest.mark.parametrize("affine", [False, True])
+@pytest.mark.parametrize("relu", [False, True])
+def test_image_reaches_the_layer(shape, layout, affine, relu):
+    """NaN and infinities in pixels: without the ReLU NaN comes out as NaN, with it NaN is dropped, and an infinity alone stays one."""
+    import wg2x2
+    from wg2x2._lib import lib
+    B, C, K, H, W = shape
+    assert lib.wg2x2_layer_fwd_pair_preferred(B, H, W, C, K, 1 if layout == "NCHW" else 0)
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    clean, w = rnd(B, C, H, W), rnd(16, C, K) / C ** 0.5
+    w[:, :, ::2] = w[:, :, ::2].abs()         # where all terms have one sign an infinity comes out as itself
+    si, ti = 1 + 0.2 * rnd(C), 0.3 * rnd(C)
+    kw = dict(in_scale=si, in_shift=ti) if affine else {}
+    prepared = wg2x2.prepare_weights(w)
+    inf = 0x7F800000
+    cases = [{(i, 3 + i, 5, 6 - i): n for i, n in enumerate(NANS)},
+             {(0, 0, 0, 0): inf, (1, C - 1, H - 1, W - 1): 0xFF800000 - (1 << 32), (2, 7, 4, 3): inf, (3, 8, 3, 4): 0xFF800000 - (1 << 32)},
+             {(0, 2, 1, 1): inf, (0, 2, 1, 2): 0xFF800000 - (1 << 32), (1, 5, 3, 3): inf, (1, 5, 4, 3): inf}]             # inf - inf inside a tile
+    for case in cases:
+        x = clean.clone()
+        for at, bits in case.items():
+            _put(x, at, bits)
+        y = wg2x2.layer_fwd_prepared(x if layout == "NCHW" else x.permute(0, 2, 3, 1).contiguous(), prepared, K, relu=relu, layout=layout, **kw)
+        y = (y if layout == "NCHW" else y.permute(0, 3, 1, 2))[:6]
+        want = _layer_like(x[:6].double() * si.view(1, -1, 1, 1) + ti.view(1, -1, 1, 1) if affine else x[:6], w, H, W, relu)
+        assert not want.isfinite().all() or relu and case is cases[0]
+        assert torch.equal(y.isnan(), want.isnan()) and torch.equal(y[y.isinf()].double(), want[want.isinf()])
+        fine = want.isfinite()
+        assert float((y[fine] - want[fine]).abs().max()) <= 5e-3 * float(want[fine].abs().max())
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("n", [1, 31, 32, 33, 49, 196])
 def test_relu_mean(n):
