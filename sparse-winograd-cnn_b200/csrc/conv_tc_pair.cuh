@@ -540,9 +540,9 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, const __grid_con
                         for (int r = 0; r < 6; ++r)
 #pragma unroll
                             for (int x = 0; x < 6; ++x) {
-                                // pixels outside the image stay zero
+                                // pixels outside the image stay zero, whatever the scale
                                 const bool in = ((flags >> r) & 1u) && !(x == 0 && (flags & kPrNoLeft)) && !(x == 5 && (flags & kPrNoRight));
-                                win[r][x] = make_float2(fmaf(sc.x, win[r][x].x, in ? tc.x : 0.f), fmaf(sc.y, win[r][x].y, in ? tc.y : 0.f));
+                                if (in) win[r][x] = make_float2(fmaf(sc.x, win[r][x].x, tc.x), fmaf(sc.y, win[r][x].y, tc.y));
                             }
                     }
                 } else {
@@ -569,10 +569,11 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, const __grid_con
 #pragma unroll
                         for (int r = 0; r < 6; ++r) {
                             if (AFFINE) {
-                                const float tr = (flags >> r) & 1u ? tc[p] : 0.f;     // pixels outside the image stay zero
+                                const bool row = (flags >> r) & 1u;                   // pixels outside the image stay zero, whatever the scale
 #pragma unroll
-                                for (int x = 0; x < 4; ++x) d[p][r][x] = fmaf(sc[p], d[p][r][x], VEC == 4 || x < cols ? tr : 0.f);
-                                ed[p][r] = fmaf(sc[p], ed[p][r], flags & kPrEdge ? tr : 0.f);
+                                for (int x = 0; x < 4; ++x)
+                                    if (row && (VEC == 4 || x < cols)) d[p][r][x] = fmaf(sc[p], d[p][r][x], tc[p]);
+                                if (row && (flags & kPrEdge)) ed[p][r] = fmaf(sc[p], ed[p][r], tc[p]);
                             }
                             lr[p][r].x = __shfl_up_sync(0xffffffffu, d[p][r][3], 4);
                             lr[p][r].y = __shfl_down_sync(0xffffffffu, d[p][r][0], 4);

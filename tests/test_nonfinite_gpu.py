@@ -138,9 +138,12 @@ def _layer_like(x, w, H, W, relu):
 
 
 # the layer on pairs of SMs: rows of each alignment, images copied whole, channels last
+PAIR_LAYERS = [((64, 64, 64, 56, 56), "NCHW"), ((130, 44, 72, 14, 14), "NCHW"), ((65, 96, 96, 27, 27), "NCHW"), ((1400, 64, 120, 9, 10), "NCHW"),
+               ((513, 64, 128, 11, 12), "NCHW"), ((128, 64, 64, 28, 28), "NHWC"), ((40, 100, 80, 41, 20), "NHWC")]
+
+
 @pytest.mark.gpu
-@pytest.mark.parametrize("shape,layout", [((64, 64, 64, 56, 56), "NCHW"), ((130, 44, 72, 14, 14), "NCHW"), ((65, 96, 96, 27, 27), "NCHW"), ((1400, 64, 120, 9, 10), "NCHW"),
-                                          ((513, 64, 128, 11, 12), "NCHW"), ((128, 64, 64, 28, 28), "NHWC"), ((40, 100, 80, 41, 20), "NHWC")])
+@pytest.mark.parametrize("shape,layout", PAIR_LAYERS)
 @pytest.mark.parametrize("affine", [False, True])
 @pytest.mark.parametrize("relu", [False, True])
 def test_image_reaches_the_layer(shape, layout, affine, relu):
@@ -171,6 +174,24 @@ def test_image_reaches_the_layer(shape, layout, affine, relu):
         assert torch.equal(y.isnan(), want.isnan()) and torch.equal(y[y.isinf()].double(), want[want.isinf()])
         fine = want.isfinite()
         assert float((y[fine] - want[fine]).abs().max()) <= 5e-3 * float(want[fine].abs().max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,layout", PAIR_LAYERS)
+def test_padding_stays_zero_under_any_scale(shape, layout):
+    """An infinite in_scale (a variance of zero) makes infinities of the channel's pixels, and the padding beside them is still zero."""
+    import wg2x2
+    B, C, K, H, W = shape
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+    x, w, si, ti = rnd(B, C, H, W).abs(), rnd(16, C, K).abs() / C, 1 + 0.2 * rnd(C), rnd(C)
+    si[5], x[1:, 5], ti[5] = float("inf"), 1.0, 0.0
+    x[0, 5] = -1.0
+    x[0, 5, 0, 0], x[0, 5, H - 1, W - 1], x[0, 5, 0, W // 2], x[0, 5, H // 2, 0] = 1.0, 1.0, 1.0, 1.0
+    y = wg2x2.layer_fwd_prepared(x if layout == "NCHW" else x.permute(0, 2, 3, 1).contiguous(), wg2x2.prepare_weights(w), K, layout=layout, in_scale=si, in_shift=ti)
+    y = (y if layout == "NCHW" else y.permute(0, 3, 1, 2))[:3]
+    want = _layer_like(x[:3].double() * si.view(1, -1, 1, 1) + ti.view(1, -1, 1, 1), w, H, W, True)
+    assert want.isinf().any() and torch.equal(y.isnan(), want.isnan()) and torch.equal(y[y.isinf()].double(), want[want.isinf()])
 
 
 @pytest.mark.gpu
