@@ -297,9 +297,9 @@ int wg2x2_layer_fwd_prepared_ex(const float *X, const float *in_scale, const flo
     // Y over X: only with V in between is all of X read before any of Y is written
     const uintptr_t x0 = reinterpret_cast<uintptr_t>(X), y0 = reinterpret_cast<uintptr_t>(Y);
     const uintptr_t pixels = sizeof(float) * (uintptr_t)B * H * W;
-    const bool apart = x0 + pixels * C <= y0 || y0 + pixels * K <= x0 || !V_scratch;
+    const bool disjoint = x0 + pixels * C <= y0 || y0 + pixels * K <= x0, apart = disjoint || !V_scratch;
     const bool extras_on16 = on16(out_scale) && on16(out_shift) && on16(residual);
-    if (aligned && apart && extras_on16 && layer_pair_preferred(B, H, W, C, K, layout))
+    if (aligned && disjoint && extras_on16 && layer_pair_preferred(B, H, W, C, K, layout))
         return layer_fwd_pair(X, prepared, Y, B, H, W, C, K, layout, relu, in_scale, in_shift, out_scale, out_shift, residual, residual_relu, st);
     if (aligned && apart && on16(residual) && on16(in_scale) && on16(in_shift) && layer_cluster_preferred(B, H, W, C, K, layout))
         return layer_fwd_cluster(X, prepared, Y, B, H, W, C, K, layout, relu, in_scale, in_shift, out_scale, out_shift, residual, residual_relu, st);

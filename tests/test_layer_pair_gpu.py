@@ -111,6 +111,26 @@ def test_output_is_written_exactly():
         assert bool(torch.isfinite(y).all()) and bool((room[:32] == 12345.0).all()) and bool((room[32 + n:] == 12345.0).all())
 
 
+@pytest.mark.parametrize("shape,layout", [((96, 64, 64, 40, 56), "NHWC"), ((65, 96, 96, 27, 27), "NCHW"), ((130, 72, 72, 14, 14), "NCHW")])
+def test_output_over_the_input_needs_scratch(shape, layout):
+    """Layers that only transform and products in memory could compute over their own input: refused without V_scratch, X left as it is."""
+    import torch
+    import wg2x2
+    from wg2x2._lib import lib
+    B, C, K, H, W = shape
+    assert lib.wg2x2_layer_fwd_pair_preferred(B, H, W, C, K, 1 if layout == "NCHW" else 0)
+    rnd, x, w = _inputs(shape, layout)
+    prepared, y, n = wg2x2.prepare_weights(w), x.clone(), lambda t: None if t is None else t.data_ptr()
+    call = lambda v: lib.wg2x2_layer_fwd_prepared_ex(n(y), None, None, n(prepared), n(y), n(v), B, H, W, C, K, 1 if layout == "NCHW" else 0, 1,
+                                                     None, None, None, 0, None, 0, torch.cuda.current_stream().cuda_stream)
+    assert call(None) == -2
+    torch.cuda.synchronize()
+    assert torch.equal(x, y)
+    assert call(torch.empty((16, B, (H + 1) // 2, (W + 1) // 2, C), device="cuda")) == 0
+    want = wg2x2.layer_fwd_prepared(x, prepared, K, layout=layout)
+    assert float((y - want).abs().max()) <= TOL_TF32 * float(want.abs().max())
+
+
 def test_zero_blocks_are_skipped_right(oracle):
     import wg2x2
     shape = (64, 160, 128, 28, 28)
