@@ -229,9 +229,10 @@ size_t wg2x2_layer_fwd_prepared_workspace_bytes(int B, int H, int W, int C, int 
  * passes through a ReLU before it is added.  Layers of few tiles run as one kernel on clusters of four CTAs in either
  * layout and at any image size (X, Y, residual, in_scale and in_shift 16-byte aligned) and read neither scratch buffer.
  * wg2x2_layer_fwd_prepared_scratch: the bytes of V_scratch and workspace with which the call is fastest (0: not used);
- * `aligned`: whether all of those pointers, out_scale and out_shift are on 16-byte boundaries.
+ * `aligned`: whether all of those pointers are on 16-byte boundaries.
  * out_scale, out_shift and residual may be at any alignment where the one-kernel layer is supported (X and Y aligned) and C < 256 or
- * K < 256; that layer is then taken and needs no scratch.  Y may lie over X where V_scratch is given: the transform is then always a
+ * K < 256; out_scale and out_shift also where the layer runs on pairs of SMs, with C < 256, K < 256 or no V_scratch.  Such a layer is
+ * then taken and needs no scratch.  Y may lie over X where V_scratch is given: the transform is then always a
  * kernel of its own.  (wg2x2_layer_fwd_prepared_scratch: `aligned` = 0 for such a call.)
  */
 int wg2x2_layer_fwd_prepared_ex(const float *X, const float *in_scale, const float *in_shift, const void *prepared, float *Y,
@@ -244,8 +245,8 @@ int wg2x2_layer_fwd_fused_supported(int B, int H, int W, int C, int K, int layou
 /* 1 where the one-kernel NCHW layer is preferred to transform, products and output transform through both scratch buffers (it reads
  * neither); 0 where those are, or the whole layer on clusters. */
 int wg2x2_layer_fwd_fused_preferred(int B, int H, int W, int C, int K, int layout);
-/* 1 where wg2x2_layer_fwd_prepared[_ws|_ex] runs the layer on pairs of SMs, also in one kernel and without scratch (X, Y, residual,
- * out_scale and out_shift 16-byte aligned, Y not over X), before it looks at any of the others: many tiles, NCHW at any image size,
+/* 1 where wg2x2_layer_fwd_prepared[_ws|_ex] runs the layer on pairs of SMs, also in one kernel and without scratch (X, Y and
+ * residual 16-byte aligned, Y not over X), before it looks at any of the others: many tiles, NCHW at any image size,
  * NHWC with W and K multiples of 4. */
 int wg2x2_layer_fwd_pair_preferred(int B, int H, int W, int C, int K, int layout);
 /* The one-kernel layer forward on its own (NCHW in and out); WG2X2_ERR_UNSUPPORTED outside the shapes above.

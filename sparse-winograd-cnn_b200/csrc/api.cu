@@ -299,7 +299,8 @@ int wg2x2_layer_fwd_prepared_ex(const float *X, const float *in_scale, const flo
     const uintptr_t pixels = sizeof(float) * (uintptr_t)B * H * W;
     const bool disjoint = x0 + pixels * C <= y0 || y0 + pixels * K <= x0, apart = disjoint || !V_scratch;
     const bool extras_on16 = on16(out_scale) && on16(out_shift) && on16(residual);
-    if (aligned && disjoint && extras_on16 && layer_pair_preferred(B, H, W, C, K, layout))
+    // (it reads out_scale and out_shift by single floats; with C, K >= 256 and scratch, off 16 bytes, they are refused below as ever)
+    if (aligned && disjoint && on16(residual) && (extras_on16 || C < 256 || K < 256 || !V_scratch) && layer_pair_preferred(B, H, W, C, K, layout))
         return layer_fwd_pair(X, prepared, Y, B, H, W, C, K, layout, relu, in_scale, in_shift, out_scale, out_shift, residual, residual_relu, st);
     if (aligned && apart && on16(residual) && on16(in_scale) && on16(in_shift) && layer_cluster_preferred(B, H, W, C, K, layout))
         return layer_fwd_cluster(X, prepared, Y, B, H, W, C, K, layout, relu, in_scale, in_shift, out_scale, out_shift, residual, residual_relu, st);

@@ -111,6 +111,32 @@ def test_output_is_written_exactly():
         assert bool(torch.isfinite(y).all()) and bool((room[:32] == 12345.0).all()) and bool((room[32 + n:] == 12345.0).all())
 
 
+@pytest.mark.parametrize("shape,layout", [((96, 64, 64, 40, 56), "NHWC"), ((65, 96, 96, 27, 27), "NCHW"), ((130, 256, 72, 14, 14), "NCHW"), ((64, 64, 64, 56, 56), "NCHW")])
+def test_maps_at_any_alignment(shape, layout):
+    """out_scale and out_shift off 16 bytes: with the scratch that the query names for the other pointers on 16 bytes (none), the same bits."""
+    import ctypes
+    import torch
+    import wg2x2
+    from wg2x2._lib import lib
+    B, C, K, H, W = shape
+    code, n = 1 if layout == "NCHW" else 0, lambda t: None if t is None else t.data_ptr()
+    assert lib.wg2x2_layer_fwd_pair_preferred(B, H, W, C, K, code)
+    nv, nw = ctypes.c_size_t(1), ctypes.c_size_t(1)
+    lib.wg2x2_layer_fwd_prepared_scratch(B, H, W, C, K, code, 1, ctypes.byref(nv), ctypes.byref(nw))
+    assert nv.value == nw.value == 0
+    rnd, x, w = _inputs(shape, layout)
+    r = rnd(B, K, H, W) if layout == "NCHW" else rnd(B, H, W, K)
+    prepared, so, to = wg2x2.prepare_weights(w), 1 + 0.2 * rnd(K), 0.3 * rnd(K)
+    off = lambda t: torch.empty(t.numel() + 1, device="cuda")[1:].copy_(t)
+    for res in (None, r):
+        want = wg2x2.layer_fwd_prepared(x, prepared, K, layout=layout, out_scale=so, out_shift=to, residual=res)
+        for s, t in ((off(so), to), (so, off(to)), (off(so), off(to))):
+            y = torch.empty_like(want)
+            assert lib.wg2x2_layer_fwd_prepared_ex(n(x), None, None, n(prepared), n(y), None, B, H, W, C, K, code, 1, n(s), n(t), n(res), 0, None, 0,
+                                                   torch.cuda.current_stream().cuda_stream) == 0
+            assert torch.equal(y, want) and torch.equal(wg2x2.layer_fwd_prepared(x, prepared, K, layout=layout, out_scale=s, out_shift=t, residual=res), want)
+
+
 @pytest.mark.parametrize("shape,layout", [((96, 64, 64, 40, 56), "NHWC"), ((65, 96, 96, 27, 27), "NCHW"), ((130, 72, 72, 14, 14), "NCHW")])
 def test_output_over_the_input_needs_scratch(shape, layout):
     """Layers that only transform and products in memory could compute over their own input: refused without V_scratch, X left as it is."""
