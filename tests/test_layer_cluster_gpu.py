@@ -35,12 +35,15 @@ def test_layer_of_few_tiles(oracle, shape, layout):
     assert wg2x2.last_device_status()[0] == 0
 
 
-# residual_relu where the other paths run: one-kernel NCHW layer, wide path, transform + row-walk kernel
-@pytest.mark.parametrize("shape,layout", [((16, 56, 56, 64, 64), "NCHW"), ((48, 14, 14, 256, 256), "NCHW"), ((48, 14, 14, 256, 256), "NHWC"),
-                                          ((24, 48, 48, 64, 64), "NHWC"), ((40, 49, 49, 32, 64), "NCHW"), ((40, 13, 15, 256, 256), "NCHW")])
-def test_residual_relu_of_the_other_paths(shape, layout):
+# residual_relu where the other paths run: one-kernel NCHW layer, wide path, transform + row-walk kernel, pairs of SMs
+@pytest.mark.parametrize("shape,layout,kernel", [((16, 56, 56, 64, 64), "NCHW", "one"), ((24, 14, 14, 256, 256), "NCHW", "wide"), ((48, 14, 14, 256, 256), "NHWC", "wide"),
+                                                 ((24, 48, 46, 64, 64), "NHWC", "walk"), ((40, 49, 49, 32, 64), "NCHW", "walk"), ((40, 13, 15, 256, 256), "NCHW", "wide"),
+                                                 ((48, 14, 14, 256, 256), "NCHW", "pairs"), ((24, 48, 48, 64, 64), "NHWC", "pairs")])
+def test_residual_relu_of_the_other_paths(shape, layout, kernel):
     import torch
     import wg2x2
+    from conftest import kernel_of
+    assert kernel_of(*shape, layout) == kernel
     B, H, W, C, K = shape
     g = torch.Generator(device="cuda").manual_seed(sum(shape))
     rnd = lambda *s: torch.randn(s, generator=g, device="cuda")

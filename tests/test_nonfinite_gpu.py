@@ -100,14 +100,19 @@ def test_round_tf32_values():
 
 
 # every kernel that adds relu(shortcut): few tiles (NCHW of even and odd width, NHWC with and without whole groups of four channels), the
-# one-kernel layer, the wide path's output transforms, the row-walk kernel (NHWC in whole blocks and not, NCHW)
+# one-kernel layer, the wide path's output transforms, the row-walk kernel (NHWC in whole blocks and not, NCHW), the layer on pairs of SMs
+# (in front of the stores: rows of 8- and 4-byte pieces, channels last, one unit a pair; behind them)
 @pytest.mark.gpu
-@pytest.mark.parametrize("shape,layout", [
-    ((1, 56, 56, 64, 64), "NCHW"), ((2, 9, 13, 32, 36), "NCHW"), ((2, 9, 13, 32, 36), "NHWC"), ((7, 7, 7, 128, 130), "NHWC"),
-    ((16, 56, 56, 64, 64), "NCHW"), ((48, 14, 14, 256, 256), "NCHW"), ((48, 14, 14, 256, 256), "NHWC"), ((12, 13, 15, 256, 264), "NCHW"),
-    ((24, 48, 48, 64, 64), "NHWC"), ((24, 48, 48, 64, 66), "NHWC"), ((40, 49, 49, 32, 64), "NCHW")])
-def test_shortcut_reaches_the_output(shape, layout):
+@pytest.mark.parametrize("shape,layout,kernel", [
+    ((1, 56, 56, 64, 64), "NCHW", "clusters"), ((2, 9, 13, 32, 36), "NCHW", "clusters"), ((2, 9, 13, 32, 36), "NHWC", "clusters"), ((7, 7, 7, 128, 130), "NHWC", "clusters"),
+    ((16, 56, 56, 64, 64), "NCHW", "one"), ((24, 14, 14, 256, 256), "NCHW", "wide"), ((48, 14, 14, 256, 256), "NHWC", "wide"), ((12, 13, 15, 256, 264), "NCHW", "wide"),
+    ((24, 48, 46, 64, 64), "NHWC", "walk"), ((24, 48, 48, 64, 66), "NHWC", "walk"), ((40, 49, 49, 32, 64), "NCHW", "walk"),
+    ((48, 14, 14, 256, 256), "NCHW", "pairs"), ((65, 27, 27, 96, 96), "NCHW", "pairs"), ((24, 48, 48, 64, 64), "NHWC", "pairs"), ((16, 40, 36, 96, 96), "NCHW", "pairs"),
+    ((64, 56, 56, 64, 64), "NCHW", "pairs")])
+def test_shortcut_reaches_the_output(shape, layout, kernel):
     import wg2x2
+    from conftest import kernel_of
+    assert kernel_of(*shape, layout) == kernel
     B, H, W, C, K = shape
     g = torch.Generator(device="cuda").manual_seed(sum(shape))
     rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
