@@ -96,8 +96,45 @@ def test_every_element_of_many_launches(shape, layout):
             assert float((y - want).abs().max()) <= TOL_TF32 * float(want.abs().max())
 
 
+def _operands64(x, w, H, W, relu, rounded):
+    """The layer in float64 sums over the operands that the tensor cores see: weights rounded to TF32, V by FP32 additions and cut to TF32,
+    position (1, 1) rounded where `rounded`.  x (B, C, H, W) -> (B, K, H, W)"""
+    import torch
+    import torch.nn.functional as F
+    import wg2x2
+    nH, nW = (H + 1) // 2, (W + 1) // 2
+    d = F.pad(x, (1, 2 * nW - W + 1, 1, 2 * nH - H + 1)).unfold(2, 4, 2).unfold(3, 4, 2)
+    rows = lambda q: (q[0] - q[2], q[1] + q[2], q[2] - q[1], q[1] - q[3])
+    v = [p for r in rows(d.unbind(4)) for p in rows(r.unbind(4))]
+    if relu:
+        v = [p.clamp(min=0) for p in v]
+    cut = lambda p: (p.contiguous().view(torch.int32) & -0x2000).view(torch.float32)
+    v = [wg2x2.round_tf32(p.contiguous()) if t == 5 and rounded else cut(p) for t, p in enumerate(v)]
+    m = torch.stack([torch.einsum("bchw,ck->bkhw", p.double(), wg2x2.round_tf32(q.contiguous()).double()) for p, q in zip(v, w)]).unflatten(0, (4, 4))
+    cols = lambda q: torch.stack((q[0] + q[1] + q[2], q[1] - q[2] - q[3]), -1)
+    return cols(cols(m.unbind(0)).unbind(0)).permute(0, 1, 2, 4, 3, 5).reshape(x.shape[0], w.shape[2], 2 * nH, 2 * nW)[:, :, :H, :W]
+
+
+@pytest.mark.parametrize("shape,layout", [((64, 64, 64, 56, 56), "NCHW"), ((130, 44, 72, 14, 14), "NCHW"), ((65, 96, 96, 27, 27), "NCHW"), ((128, 64, 64, 28, 28), "NHWC")])
+@pytest.mark.parametrize("relu", [True, False])
+def test_operands_are_rounded_as_stated(shape, layout, relu):
+    """An accumulator takes 9 C / 8 FP32 additions, each off by a unit in the last place of what it holds at most; that is far less than what
+    the rounding of the operands does, and than what cutting position (1, 1) instead would change."""
+    import torch
+    import wg2x2
+    B, C, K, H, W = shape
+    rnd, x, w = _inputs(shape, layout)
+    y = wg2x2.layer_fwd_prepared(x, wg2x2.prepare_weights(w), K, relu=relu, layout=layout)[:8].double()
+    a = x[:8] if layout == "NCHW" else x[:8].permute(0, 3, 1, 2)
+    y = y if layout == "NCHW" else y.permute(0, 3, 1, 2)
+    want, other = (_operands64(a, w, H, W, relu, rounded) for rounded in (True, False))
+    rel = lambda p, q: float((p - q).norm() / q.norm())
+    bound = 9 * C / 8 * 2.0 ** -23
+    assert rel(other, want) > 4 * bound and rel(y, want) <= bound
+
+
 def test_output_is_written_exactly():
-    """Nothing beyond Y is touched, and all of Y is."""
+    """Nothing beyond Y is touched, and all of Y is: plain, with a shortcut in front of the stores or behind them, and with Y over it."""
     import torch
     import wg2x2
     for shape, layout in CASES:
@@ -106,9 +143,13 @@ def test_output_is_written_exactly():
         n = B * K * H * W
         room = torch.full((n + 64,), 12345.0, device="cuda")
         y = room[32:32 + n].view((B, K, H, W) if layout == "NCHW" else (B, H, W, K))
-        y.fill_(float("nan"))
-        wg2x2.layer_fwd_prepared(x, wg2x2.prepare_weights(w), K, layout=layout, out=y)
-        assert bool(torch.isfinite(y).all()) and bool((room[:32] == 12345.0).all()) and bool((room[32 + n:] == 12345.0).all())
+        r, prepared, plain = torch.randn_like(y), wg2x2.prepare_weights(w), None
+        for residual in (None, r, y):
+            y.copy_(r) if residual is y else y.fill_(float("nan"))
+            wg2x2.layer_fwd_prepared(x, prepared, K, layout=layout, out=y, residual=residual)
+            assert bool(torch.isfinite(y).all()) and bool((room[:32] == 12345.0).all()) and bool((room[32 + n:] == 12345.0).all())
+            plain = y.clone() if plain is None else plain
+            assert residual is None or torch.equal(y, plain + r)         # one addition, of the same two numbers in either order
 
 
 @pytest.mark.parametrize("shape,layout", [((96, 64, 64, 40, 56), "NHWC"), ((65, 96, 96, 27, 27), "NCHW"), ((130, 256, 72, 14, 14), "NCHW"), ((64, 64, 64, 56, 56), "NCHW")])
@@ -172,13 +213,12 @@ def test_zero_blocks_are_skipped_right(oracle):
     assert oracle.max_rel(nhwc(y), oracle.conv_fwd(oracle.imtrans_fwd(nhwc(x), relu=True), w.cpu().numpy(), H, W)) <= TOL_TF32
 
 
-@pytest.mark.parametrize("nth", [0, 3])
-def test_times_out_and_recovers(nth):
+@pytest.mark.parametrize("shape,nth", [(SHAPES[0], 0), (SHAPES[0], 3), (SHAPES[7], 0), (SHAPES[7], 20)])        # weights resident, weights streaming
+def test_times_out_and_recovers(shape, nth):
     """CTA 0's weight producer stops before one load, with nothing in flight, under a limit of a few thousand polls."""
     import torch
     import wg2x2
     from wg2x2._lib import lib
-    shape = SHAPES[0]
     rnd, x, w = _inputs(shape)
     prepared, K = wg2x2.prepare_weights(w), shape[2]
     want = wg2x2.layer_fwd_prepared(x, prepared, K, layout="NCHW")
