@@ -6,10 +6,11 @@
 // after the ReLU) is written into tensor memory by transform warps, and position (i, j) is accumulated with the sign
 // At[a][i] At[e][j] straight into the output accumulators (a, e) it contributes to, 36 MMAs per 8 input channels.  What differs:
 //   * tcgen05 cta_group::2: two CTAs share an M = 256, N = 64 unit, each holding half of every weight tile, so that the weight
-//     tiles' reads from shared memory, half of that kernel's shared-memory time, are halved; with up to 96 input channels and
-//     64 outputs all weights stay in shared memory for the whole launch;
+//     tiles' reads from shared memory, half of that kernel's shared-memory time, are halved; with up to 64 outputs all weights stay in
+//     shared memory for the whole launch where they fit beside the pixels: up to 64 input channels (channels last a little fewer in rows of
+//     few quads), up to 80 for two images' sizes in five;
 //   * tiles go to tensor-memory lanes densely, in quads of 2 x 2 (4 x 4 output pixels), whatever image and row they lie in: 64 images
-//     of 56 x 56 are 196 units of 256 tiles in three rounds on 74 pairs, where whole rows of tiles need four;
+//     of 56 x 56 are 196 units of 256 tiles in three rounds on 66 pairs, where whole rows of tiles need four;
 //   * a thread forms all sixteen positions of a quad's four tiles from one 6 x 6 window: 36 loads for 64 values, and one
 //     tcgen05.st of 16 lanes x 32 columns per Winograd row and row of tiles;
 //   * pixels come as plain bulk copies of the rows' contiguous memory, so that an NCHW image needs no row length of 16-byte pieces; channels
@@ -341,7 +342,6 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, const __grid_con
             const uint32_t idesc_a = idesc ^ ((uint32_t)a << 14), idesc_e = idesc ^ ((uint32_t)e << 14), idesc_ae = idesc ^ ((uint32_t)(a ^ e) << 14);   // bit 14: negate B
             const uint64_t bdesc0 = make_desc_k_sw64(base);
             const uint32_t b_hi = (uint32_t)(bdesc0 >> 32), b_lo0 = (uint32_t)bdesc0;
-            const int nC32 = (prm.C + 31) >> 5;
             int stage = 0; uint32_t wph = 0;
             uint32_t n = 0;                                               // slots so far
             bool ok = true;
