@@ -342,12 +342,10 @@ layer_fwd_fused_kernel(const __grid_constant__ CUtensorMap mapXd, const __grid_c
                         const bool neg_e = (e == 1 && jj >= 1);                      // At[1][j] = -1 for j = 2, 3
                         const uint32_t idesc = (neg_a != neg_e) ? idesc_neg : idesc_pos;
                         const uint32_t aj = a_tmem + (uint32_t)((e + jj) * 32), bj = b_lo + (uint32_t)((e + jj) * (kFuWTile >> 4));
-#ifndef WG_KO_MMA  // (development knock-out: no MMAs, results wrong)
                         if (leader) {
                             umma_tf32_ts_x2(d_tmem, aj, bj, b_hi, idesc, (jj == 0 && sl == first_slot) ? 0u : 1u);
                             umma_tf32_ts_x2(d_tmem, aj + 16u, bj + 4u, b_hi, idesc, 1u);
                         }
-#endif
                     }
                 } else if (active) {
                     // Winograd rows 1 and 2, 16 channels: tile (i - 1) * 4 + j at columns 16 * tile, weights in rows of 64 bytes
@@ -363,9 +361,7 @@ layer_fwd_fused_kernel(const __grid_constant__ CUtensorMap mapXd, const __grid_c
                             const uint32_t idesc = (neg_a != neg_e) ? idesc_neg : idesc_pos;
                             const int tile = (ii - 1) * 4 + e + jj;
                             const uint32_t aj = a_tmem + (uint32_t)(tile * 16), bj = b_lo + (uint32_t)(tile * (kFuW2Tile >> 4));
-#ifndef WG_KO_MMA
                             if (leader) umma_tf32_ts_x2(d_tmem, aj, bj, b2_hi, idesc, (ii == 1 && jj == 0 && sl == first_slot) ? 0u : 1u);
-#endif
                         }
                     }
                 }
@@ -393,9 +389,6 @@ layer_fwd_fused_kernel(const __grid_constant__ CUtensorMap mapXd, const __grid_c
                     if (!mbar_wait_sleepy(xempty_bar(xb), xph ^ 1u, abort_flag, 0x900u | xb, 100, prm.spin_limit)) { ok = false; break; }
                     TC_TRACE(trx); ++trx;
                     const uint32_t dst = xbase + xb * kFuXbufBytes;
-#ifdef WG_KO_X     // development knock-out: no input loads (results wrong)
-                    mbar_arrive(xfull_bar(xj)); (void)dst; (void)x0; (void)th0; (void)b0;
-#else
                     if (st >= 2 * nC32 && st < 6 * nC32) {         // phase B: rows d1, d2 of 8 channels, dense
                         mbar_expect_tx(xfull_bar(xj), prm.xbytes1);
                         tma_load_4d(dst, &mapXd, xfull_bar(xj), x0, 2 * th0, (st - 2 * nC32) * 8, b0);
@@ -404,7 +397,6 @@ layer_fwd_fused_kernel(const __grid_constant__ CUtensorMap mapXd, const __grid_c
                         mbar_expect_tx(xfull_bar(xj), prm.xbytes2);
                         tma_load_4d(dst, &mapXs, xfull_bar(xj), x0, 2 * th0 - (first ? 1 : 0), (first ? st : st - 6 * nC32) * 16, b0);
                     }
-#endif
                     if (++xb == kFuXbufs) { xb = 0; xph ^= 1u; }
                     if (++xj == kFuXfull) xj = 0;
                 }
@@ -423,14 +415,10 @@ layer_fwd_fused_kernel(const __grid_constant__ CUtensorMap mapXd, const __grid_c
                     if (!mbar_wait_sleepy(free_bar(s), ph ^ 1u, abort_flag, 0xA00u | s, 100, prm.spin_limit)) { ok = false; break; }
                     // test hook: this slot's weights never arrive (nothing is put in flight), so the issuers' wait on it runs out
                     if (blockIdx.x == 0 && nload++ == prm.drop_load) { ok = false; break; }
-#ifdef WG_KO_W     // development knock-out: no weight loads (results wrong)
-                    mbar_arrive(full_bar(s));
-#else
                     mbar_expect_tx(full_bar(s), kFuWBytes);
                     if (sl < nC32)          tma_load_3d(wbase + s * kFuWBytes, &mapW, full_bar(s), sl * 32, kb * kBlockN, 0);
                     else if (sl < 3 * nC32) tma_load_3d(wbase + s * kFuWBytes, &mapW2, full_bar(s), (sl - nC32) * 16, kb * kBlockN, 4);
                     else                    tma_load_3d(wbase + s * kFuWBytes, &mapW, full_bar(s), (sl - 3 * nC32) * 32, kb * kBlockN, 12);
-#endif
                     if (++s == kFuWStages) { s = 0; ph ^= 1u; }
                 }
             }
@@ -542,18 +530,10 @@ layer_fwd_fused_kernel(const __grid_constant__ CUtensorMap mapXd, const __grid_c
                 constexpr bool kByLanes = decltype(by_lanes_tag)::value;
                 const float *pa = xq + c * chs;
                 const float *pb = pa + BW;
-#ifdef WG_KO_LDS   // development knock-out: no shared-memory loads (results wrong)
-                const float2 am = make_float2((float)c, s2), bm = make_float2(s2, 1.f);
-#else
                 const float2 am = lds_f2(xq_s + (uint32_t)(4 * c * chs));
                 const float2 bm = lds_f2(xq_s + (uint32_t)(4 * (c * chs + BW)));
-#endif
                 r1 = fmaf(s2, bm.x, am.x); r2 = fmaf(s2, bm.y, am.y);
-#ifdef WG_KO_SHFL  // development knock-out: no shuffles (results wrong)
-                r0 = r2 * 0.5f; r3 = r1 * 0.25f;
-#else
                 r0 = __shfl_sync(0xffffffffu, r2, src_l); r3 = __shfl_sync(0xffffffffu, r1, src_r);
-#endif
                 if (!kByLanes) {
                     if (need_l) r0 = fmaf(s2, pb[0], pa[0]);
                     if (need_r) r3 = fmaf(s2, pb[3], pa[3]);
@@ -585,12 +565,8 @@ layer_fwd_fused_kernel(const __grid_constant__ CUtensorMap mapXd, const __grid_c
                                 o[3][cq] = fmaxf(r1 - r3, lo);
                             }
                         }
-#ifdef WG_KO_ST    // development knock-out: one tensor-memory store instead of four (results wrong)
-                        { float z[4] = {o[0][0] + o[1][1], o[2][2] + o[3][3], o[0][1] + o[1][2], o[2][3] + o[3][0]}; tmem_st4(a_tmem + (uint32_t)(c4 * 4), z); }
-#else
 #pragma unroll
                         for (int j = 0; j < 4; ++j) tmem_st4(a_tmem + (uint32_t)(j * 32 + c4 * 4), o[j]);
-#endif
                         if (warp == 16 && lane == 0) TC_TRACE(512 + 8 * trt + 4 + q);
                     }
                 } else {
@@ -600,12 +576,8 @@ layer_fwd_fused_kernel(const __grid_constant__ CUtensorMap mapXd, const __grid_c
                     float m1[4][2], m2[4][2], e1[4][2], e2[4][2];   // [channel][left, right]: rows 1 and 2; e*: the outer pixels where lanes cannot supply them
 #pragma unroll
                     for (int cq = 0; cq < 4; ++cq) {
-#ifdef WG_KO_LDS   // development knock-out: no shared-memory loads (results wrong)
-                        const float2 am = make_float2((float)cq, lo), bm = make_float2(lo, 1.f);
-#else
                         const float2 am = lds_f2(xq_s + (uint32_t)(4 * cq * chs));
                         const float2 bm = lds_f2(xq_s + (uint32_t)(4 * (cq * chs + BW)));
-#endif
                         m1[cq][0] = am.x + bm.x; m1[cq][1] = am.y + bm.y;      // row 1 = d1 + d2
                         m2[cq][0] = bm.x - am.x; m2[cq][1] = bm.y - am.y;      // row 2 = d2 - d1
                         if (!decltype(by_lanes_tag)::value) {
@@ -620,11 +592,7 @@ layer_fwd_fused_kernel(const __grid_constant__ CUtensorMap mapXd, const __grid_c
 #pragma unroll
                         for (int cq = 0; cq < 4; ++cq) {
                             const float r1 = ii == 0 ? m1[cq][0] : m2[cq][0], r2 = ii == 0 ? m1[cq][1] : m2[cq][1];
-#ifdef WG_KO_SHFL  // development knock-out: no shuffles (results wrong)
-                            float r0 = r2 * 0.5f, r3 = r1 * 0.25f;
-#else
                             float r0 = __shfl_sync(0xffffffffu, r2, src_l), r3 = __shfl_sync(0xffffffffu, r1, src_r);
-#endif
                             if (!decltype(by_lanes_tag)::value) {
                                 if (need_l) r0 = ii == 0 ? e1[cq][0] : e2[cq][0];
                                 if (need_r) r3 = ii == 0 ? e1[cq][1] : e2[cq][1];
@@ -642,12 +610,8 @@ layer_fwd_fused_kernel(const __grid_constant__ CUtensorMap mapXd, const __grid_c
                                 o[3][cq] = fmaxf(r1 - r3, lo);
                             }
                         }
-#ifdef WG_KO_ST    // development knock-out: one tensor-memory store instead of four (results wrong)
-                        { float z[4] = {o[0][0] + o[1][1], o[2][2] + o[3][3], o[0][1] + o[1][2], o[2][3] + o[3][0]}; tmem_st4(a_tmem + (uint32_t)(ii * 64), z); }
-#else
 #pragma unroll
                         for (int j = 0; j < 4; ++j) tmem_st4(a_tmem + (uint32_t)((4 * ii + j) * 16), o[j]);
-#endif
                         if (warp == 16 && lane == 0) TC_TRACE(512 + 8 * trt + 4 + ii);
                     }
                 }
@@ -717,11 +681,7 @@ layer_fwd_fused_kernel(const __grid_constant__ CUtensorMap mapXd, const __grid_c
                     }
                     if (!mbar_wait_warp(yfree_bar(half), st_use & 1u, abort_flag, 0x500u | ew, prm.spin_limit)) { ok = false; break; }
                     float *stage = stage0 + ybox * (kFuYStageBytes / 4);
-#ifdef WG_KO_Y     // development knock-out: Y is neither staged nor stored (results wrong)
-                    if (false) {
-#else
                     if (live) {
-#endif
 #pragma unroll
                         for (int c = 0; c < 16; ++c) {
                             const int k = kbase + rd * 16 + c;
@@ -741,11 +701,7 @@ layer_fwd_fused_kernel(const __grid_constant__ CUtensorMap mapXd, const __grid_c
                     bool stored = true;
                     if (elected) {
                         stored = mbar_wait(ywritten_bar(half), st_use & 1u, abort_flag, 0x580u | ew, prm.spin_limit);
-#ifdef WG_KO_Y
-                        if (false) {
-#else
                         if (stored && kbase + rd * 16 < prm.K) {      // a box that starts beyond the last channel is not issued at all
-#endif
                             if (prm.accumulate) tma_reduce_add_4d(smem_u32(stage), &mapY, 2 * seg * prm.TW, 2 * rb * TH + a, kbase + rd * 16, g * prm.NB);
                             else tma_store_4d(smem_u32(stage), &mapY, 2 * seg * prm.TW, 2 * rb * TH + a, kbase + rd * 16, g * prm.NB);
                         }
