@@ -449,7 +449,7 @@ layer_fwd_fused_kernel(const __grid_constant__ CUtensorMap mapXd, const __grid_c
         const int BW = prm.BW;
         const int src_l = (lane & ~(LP - 1)) | ((tcol + LP - 1) & (LP - 1)), src_r = (lane & ~(LP - 1)) | ((tcol + 1) & (LP - 1));
         const bool need_l = !halo_by_lanes && (tcol == 0), need_r = !halo_by_lanes && ((tcol == prm.TW - 1) || (tcol == LP - 1));
-        const float lo = prm.relu ? 0.f : -__int_as_float(0x7f800000);
+        const float lo = prm.relu ? 0.f : __int_as_float(0x7fffffff);      // the larger of a number and NaN is the number: without a ReLU all stay
         const int spu = 2 * spu_slots;                          // steps per unit
         const int my_units = (prm.units - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
         const int total = my_units * spu;

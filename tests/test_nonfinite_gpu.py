@@ -148,15 +148,15 @@ PAIR_LAYERS = [((64, 64, 64, 56, 56), "NCHW"), ((130, 44, 72, 14, 14), "NCHW"), 
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("shape,layout", PAIR_LAYERS)
+@pytest.mark.parametrize("shape,layout,kernel", [(*p, "pairs") for p in PAIR_LAYERS] + [((16, 64, 64, 56, 56), "NCHW", "one"), ((48, 16, 16, 48, 48), "NCHW", "one")])
 @pytest.mark.parametrize("affine", [False, True])
 @pytest.mark.parametrize("relu", [False, True])
-def test_image_reaches_the_layer(shape, layout, affine, relu):
+def test_image_reaches_the_layer(shape, layout, kernel, affine, relu):
     """NaN and infinities in pixels: without the ReLU NaN comes out as NaN, with it NaN is dropped, and an infinity alone stays one."""
     import wg2x2
-    from wg2x2._lib import lib
+    from conftest import kernel_of
     B, C, K, H, W = shape
-    assert lib.wg2x2_layer_fwd_pair_preferred(B, H, W, C, K, 1 if layout == "NCHW" else 0)
+    assert kernel_of(B, H, W, C, K, layout) == kernel
     g = torch.Generator(device="cuda").manual_seed(sum(shape))
     rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
     clean, w = rnd(B, C, H, W), rnd(16, C, K) / C ** 0.5
