@@ -7,8 +7,8 @@
 // At[a][i] At[e][j] straight into the output accumulators (a, e) it contributes to, 36 MMAs per 8 input channels.  What differs:
 //   * tcgen05 cta_group::2: two CTAs share an M = 256, N = 64 unit, each holding half of every weight tile, so that the weight
 //     tiles' reads from shared memory, half of that kernel's shared-memory time, are halved; with up to 64 outputs all weights stay in
-//     shared memory for the whole launch where they fit beside the pixels: up to 64 input channels (channels last a little fewer in rows of
-//     few quads), up to 80 for two images' sizes in five;
+//     shared memory for the whole launch where they fit beside the pixels: up to 64 input channels (channels last not in every
+//     width), up to 80 in two image sizes of five;
 //   * tiles go to tensor-memory lanes densely, in quads of 2 x 2 (4 x 4 output pixels), whatever image and row they lie in: 64 images
 //     of 56 x 56 are 196 units of 256 tiles in three rounds on 66 pairs, where whole rows of tiles need four;
 //   * a thread forms all sixteen positions of a quad's four tiles from one 6 x 6 window: 36 loads for 64 values, and one
