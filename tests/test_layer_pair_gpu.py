@@ -213,7 +213,7 @@ def test_zero_blocks_are_skipped_right(oracle):
     assert oracle.max_rel(nhwc(y), oracle.conv_fwd(oracle.imtrans_fwd(nhwc(x), relu=True), w.cpu().numpy(), H, W)) <= TOL_TF32
 
 
-@pytest.mark.parametrize("shape,nth", [(SHAPES[0], 0), (SHAPES[0], 3), (SHAPES[7], 0), (SHAPES[7], 20)])        # weights resident, weights streaming
+@pytest.mark.parametrize("shape,nth", [(SHAPES[0], 0), (SHAPES[0], 3), (SHAPES[7], 0), (SHAPES[7], 10)])        # weights resident, weights streaming
 def test_times_out_and_recovers(shape, nth):
     """CTA 0's weight producer stops before one load, with nothing in flight, under a limit of a few thousand polls."""
     import torch
