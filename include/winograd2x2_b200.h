@@ -247,8 +247,10 @@ int wg2x2_layer_fwd_fused_supported(int B, int H, int W, int C, int K, int layou
 int wg2x2_layer_fwd_fused_preferred(int B, int H, int W, int C, int K, int layout);
 /* 1 where wg2x2_layer_fwd_prepared[_ws|_ex] runs the layer on pairs of SMs, also in one kernel and without scratch (X, Y and
  * residual 16-byte aligned, Y not over X), before it looks at any of the others: many tiles, NCHW at any image size,
- * NHWC with W and K multiples of 4. */
+ * NHWC with W and K multiples of 4.  It answers for any options of the call; _for answers for one: `affine`, whether in_scale and
+ * in_shift are given, `shortcut` 0 without a residual, 1 with one of its own, 2 with one that is Y, -1 for all of these. */
 int wg2x2_layer_fwd_pair_preferred(int B, int H, int W, int C, int K, int layout);
+int wg2x2_layer_fwd_pair_preferred_for(int B, int H, int W, int C, int K, int layout, int affine, int shortcut);
 /* The one-kernel layer forward on its own (NCHW in and out); WG2X2_ERR_UNSUPPORTED outside the shapes above.
  * residual may be Y itself: the result is then added into Y in place (the TMA unit does the addition);
  * otherwise residual is first copied to Y on the same stream and must not overlap it. */

@@ -37,7 +37,7 @@ int conv_fwd_tc_wide(const float *V, const void *prepared, float *Y, int B, int 
 bool fused_fwd_supported(int B, int H, int W, int C, int K, int layout);
 bool layer_fused_preferred(int B, int H, int W, int C, int K, int layout);
 bool layer_cluster_preferred(int B, int H, int W, int C, int K, int layout);
-bool layer_pair_preferred(int B, int H, int W, int C, int K, int layout);
+bool layer_pair_preferred(int B, int H, int W, int C, int K, int layout, bool affine, int shortcut);
 int layer_fwd_pair(const float *X, const void *prepared, float *Y, int B, int H, int W, int C, int K, int layout, int relu,
                    const float *in_scale, const float *in_shift, const float *out_scale, const float *out_shift,
                    const float *residual, int res_relu, cudaStream_t st);
@@ -259,7 +259,12 @@ int wg2x2_layer_fwd_fused_preferred(int B, int H, int W, int C, int K, int layou
 
 int wg2x2_layer_fwd_pair_preferred(int B, int H, int W, int C, int K, int layout)
 {
-    return (B > 0 && H > 0 && W > 0 && C > 0 && K > 0 && layer_pair_preferred(B, H, W, C, K, layout)) ? 1 : 0;
+    return wg2x2_layer_fwd_pair_preferred_for(B, H, W, C, K, layout, 0, -1);
+}
+
+int wg2x2_layer_fwd_pair_preferred_for(int B, int H, int W, int C, int K, int layout, int affine, int shortcut)
+{
+    return (B > 0 && H > 0 && W > 0 && C > 0 && K > 0 && layer_pair_preferred(B, H, W, C, K, layout, affine != 0, shortcut)) ? 1 : 0;
 }
 
 size_t wg2x2_layer_fwd_prepared_workspace_bytes(int B, int H, int W, int C, int K)
@@ -275,7 +280,7 @@ void wg2x2_layer_fwd_prepared_scratch(int B, int H, int W, int C, int K, int lay
 {
     *v_bytes = *workspace_bytes = 0;
     if (B <= 0 || H <= 0 || W <= 0 || C <= 0 || K <= 0 || !layout_ok(layout)) return;
-    if (aligned && (layer_pair_preferred(B, H, W, C, K, layout) || layer_cluster_preferred(B, H, W, C, K, layout) || layer_fused_preferred(B, H, W, C, K, layout)))
+    if (aligned && (layer_pair_preferred(B, H, W, C, K, layout, false, -1) || layer_cluster_preferred(B, H, W, C, K, layout) || layer_fused_preferred(B, H, W, C, K, layout)))
         return;
     const int nH = (H + 1) / 2, nW = (W + 1) / 2;
     *workspace_bytes = wg2x2_conv_fwd_prepared_workspace_bytes(B, nH, nW, C, K);
@@ -300,7 +305,8 @@ int wg2x2_layer_fwd_prepared_ex(const float *X, const float *in_scale, const flo
     const bool disjoint = x0 + pixels * C <= y0 || y0 + pixels * K <= x0, apart = disjoint || !V_scratch;
     const bool extras_on16 = on16(out_scale) && on16(out_shift) && on16(residual);
     // (it reads out_scale and out_shift by single floats; with C, K >= 256 and scratch, off 16 bytes, they are refused below as ever)
-    if (aligned && disjoint && on16(residual) && (extras_on16 || C < 256 || K < 256 || !V_scratch) && layer_pair_preferred(B, H, W, C, K, layout))
+    if (aligned && disjoint && on16(residual) && (extras_on16 || C < 256 || K < 256 || !V_scratch) &&
+        layer_pair_preferred(B, H, W, C, K, layout, in_scale != nullptr, !residual ? 0 : residual == Y ? 2 : 1))
         return layer_fwd_pair(X, prepared, Y, B, H, W, C, K, layout, relu, in_scale, in_shift, out_scale, out_shift, residual, residual_relu, st);
     if (aligned && apart && on16(residual) && on16(in_scale) && on16(in_shift) && layer_cluster_preferred(B, H, W, C, K, layout))
         return layer_fwd_cluster(X, prepared, Y, B, H, W, C, K, layout, relu, in_scale, in_shift, out_scale, out_shift, residual, residual_relu, st);

@@ -564,7 +564,10 @@ void layer_fwd_prepared(const Tensor &x, const Tensor &prep, const Tensor &Y, co
     // (Y over X needs V in between; extras off 16 bytes are the one-kernel layer's, or without the residual the cluster's and the pairs'; none
     // of them reads scratch.  C, K >= 256: refused off 16 bytes, by the path through scratch)
     const bool one_kernel = xy && !extras && (d.C < 256 || K < 256) && wg2x2_layer_fwd_fused_supported(d.B, d.H, d.W, d.C, K, layout);
-    const LayerScratch s(d, K, layout, xy && on16(residual) && (extras || d.C < 256 || K < 256) && on16(in_scale) && on16(in_shift), one_kernel, V, uws);
+    const bool own = xy && on16(residual) && (extras || d.C < 256 || K < 256);
+    const int shortcut = !residual.defined() ? 0 : residual.data_ptr() == Y.data_ptr() ? 2 : 1;
+    const bool none = one_kernel || (own && wg2x2_layer_fwd_pair_preferred_for(d.B, d.H, d.W, d.C, K, layout, in_scale.defined(), shortcut));
+    const LayerScratch s(d, K, layout, own && on16(in_scale) && on16(in_shift), none, V, uws);
     check(wg2x2_layer_fwd_prepared_ex(cptr(x), cptr(in_scale), cptr(in_shift), prep.data_ptr(), ptr(Y), s.v, d.B, d.H, d.W, d.C, K, layout, relu,
                                       cptr(out_scale), cptr(out_shift), cptr(residual), residual_relu, s.w, s.wn, stream),
           "wg2x2_layer_fwd_prepared_ex");

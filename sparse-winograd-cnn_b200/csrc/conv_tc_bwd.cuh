@@ -628,7 +628,7 @@ static int gg_cols(int n) { return n > 128 ? 256 : (n > 64 ? 128 : 64); }
 // take least.  A unit takes about (chunks of 32) x c + e microseconds, measured with c = 0.37 / 0.45 / 0.60 and e = 0.3 / 0.5 / 0.9
 // for 64 / 128 / 256 columns: wide units share the A tile among more columns, narrow ones put more SMs to work (one 14 x 14
 // image of 512 channels: 13.9 us with 256 columns, 10.4 with 64).
-static int gg_pick_cols(long long rows, int n, int contr)
+static int gg_pick_cols(long long rows, int n, int contr, double *us = nullptr)
 {
     const int widest = gg_cols(n);
     const double ch = cdiv(contr, 32);
@@ -640,6 +640,7 @@ static int gg_pick_cols(long long rows, int n, int contr)
         const double u = (double)cdivll(units, kNumSMs) * per;
         if (u < t) { t = u; best = N; }
     }
+    if (us) *us = t;
     return best;
 }
 

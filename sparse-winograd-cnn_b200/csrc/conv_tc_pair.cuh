@@ -637,8 +637,8 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, const __grid_con
                             if (i == 1) {
                                 // Position (1, 1), of non-negative pixels the largest, is rounded to TF32 (half a unit of the last kept
                                 // place, then the tensor core's cut), the others are cut: the accumulators take 36 MMAs per 8 channels
-                                // instead of 16, whose longer sums cost up to 1.3 % of the error against 64 bits (512 channels:
-                                // 4.69e-4 -> 4.75e-4 relative); with this one it is 4.58e-4.  All rounded: 2.96e-4, 3 to 18 % slower.
+                                // instead of 16, whose longer sums cost up to 1.3 % of the error against 64 bits; with this one it is below the former
+                                // paths' (64 x 512 x 14 x 14: 4.63e-4 -> 4.52e-4, relative).  All rounded: 2.96e-4, 3 to 18 % slower.
 #pragma unroll
                                 for (int x = 4; x < 8; ++x)
                                     if (fabsf(o[x]) < __int_as_float(0x7f800000)) o[x] = __uint_as_float(__float_as_uint(o[x]) + 0x1000u);     // (infinities and NaN stay)
@@ -916,12 +916,6 @@ static bool pr_sizes(PrParams &p, int B, int H, int W, int C, int K, int layout)
     p.quads = (int)quads; p.units = (int)units;
     return pr_geometry(p, layout);
 }
-static bool pair_supported(int B, int H, int W, int C, int K, int layout)
-{
-    PrParams p;
-    return pr_sizes(p, B, H, W, C, K, layout);
-}
-
 int layer_fwd_pair(const float *X, const void *prepared, float *Y, int B, int H, int W, int C, int K, int layout, int relu,
                    const float *in_scale, const float *in_shift, const float *out_scale, const float *out_shift,
                    const float *residual, int res_relu, cudaStream_t st)
@@ -979,23 +973,57 @@ int layer_fwd_pair(const float *X, const void *prepared, float *Y, int B, int H,
 
 // Microseconds of the layer on pairs of SMs (plain, both layouts, 1 .. 256 images of 7 .. 64 pixels, 16 .. 512 channels: within a fifth of
 // the measured): rounds of units, each a walk over the input channels and the change of accumulators at its end, which takes
-// long where rows are stored pixel by pixel.  (Images of at most ten quads lie whole in shared memory, their channels on the same banks.)
-static double pair_us(int B, int H, int W, int C, int K, int layout)
+// long where rows are stored pixel by pixel.  (Images that lie whole in shared memory have their channels on the same banks.)
+static double pair_us(const PrParams &p, int layout)
 {
-    const double rounds = (double)cdivll(cdivll((long long)B * cdiv(H, 4) * cdiv(W, 4), 2 * kPrQuads) * cdiv(K, 64), kNumSMs / 2);
-    return layout == WG2X2_NHWC ? 6.5 + rounds * (1.5 + 0.98 * cdiv(C, 8)) : 6.3 + rounds * ((W % 2 ? 9.5 : 3.2) + (cdiv(H, 4) * cdiv(W, 4) <= 10 ? 1.05 : 0.82) * cdiv(C, 8));
+    const double rounds = cdiv(p.units, kNumSMs / 2);
+    return layout == WG2X2_NHWC ? 6.5 + rounds * (1.5 + 0.98 * p.nS) : 6.3 + rounds * ((p.W % 2 ? 9.5 : 3.2) + (p.whole ? 1.05 : 0.82) * p.nS);
+}
+
+// The same layer with an affine map in front or a shortcut (0: none, 1: of its own, 2: under Y), against the wide path and the layer on
+// clusters with the same.  There the margins of the plain rule are too narrow: a shortcut costs a pair 5 .. 7 us a round and a map 0.1 ..
+// 0.24 us a slot, the others 5 .. 12 %.  Over the 900 of 3030 layers that the plain rule takes from those two paths, with map and shortcut:
+// 88 were more than 3 % slower than before without this test (111 x 128 x 10 x 10 24.8 -> 34.5 us), 12 are with it; what it turns away is on the
+// mean as fast either way.  (The estimates: within 5 .. 12 % of the measured, one standard deviation.)
+static bool options_lose(const PrParams &p, int layout, double clusters, bool wide, bool affine, int shortcut)
+{
+    const bool nhwc = layout == WG2X2_NHWC, w4 = p.W % 4 == 0, w2 = p.W % 2 == 0;
+    const double rounds = cdiv(p.units, kNumSMs / 2);
+    const double slot = nhwc ? 0.93 + (affine ? 0.24 : 0.) : w4 ? 0.83 + (affine ? 0.10 : 0.) : w2 ? 0.86 + (affine ? 0.19 : 0.) : 0.97 + (affine ? 0.17 : 0.);
+    const double last = !shortcut ? 0. : nhwc ? 4.9 : w4 ? (shortcut == 2 && rounds > 1. ? 1.2 : 6.8) : w2 ? 6.3 : 4.8;
+    const double us = (nhwc ? 6.4 : w2 ? 6.8 : 9.0) + rounds * ((nhwc ? 2.5 : w4 ? 2.4 : w2 ? 3.0 : 5.0) + last + slot * p.nS);
+    double other = clusters * (affine ? 1.07 : 1.02) * (shortcut == 2 ? 1.12 : shortcut ? 1.08 : 1.);
+    if (wide) {
+        const long long P = (long long)p.B * ((p.H + 1) / 2) * ((p.W + 1) / 2);
+        double products = 0.;
+        gg_pick_cols(P, p.K, p.C, &products);
+        const double mb = (4e-6 * p.B * p.H * p.W + 128e-6 * P) * ((double)p.C + p.K);
+        other = (nhwc ? 7.1 + 0.108 * mb + 0.68 * products : 9.0 + 0.130 * mb + 0.63 * products) * (p.C % 32 || p.K % 32 ? 1.12 : 1.) *
+                (affine && nhwc ? 1.08 : 1.) * (shortcut ? 1.07 : 1.);
+    }
+    return us >= other;
 }
 
 // Against all other paths.  It wins where its units fill the SMs at least once: over 172 NCHW layers of 1 .. 128 images it takes 0.50 ..
 // 0.95 of the time in 75 (64 x 256 x 40 x 40 341 -> 170 us, 128 x 256 x 14 x 14 93 -> 68, 64 x 64 x 56 x 56 45 -> 34), with fewer units up
-// to four times as long.  Over 110 layers of both layouts that this rule picks the geometric mean is 1.7 times as fast, with a shortcut
-// too.  The factors are the margins that the estimates need: channels last, 0.95 takes 46 x 96 x 192 x 12 x 12 too, 19.9 us (24.9 with a
+// to four times as long.  Over 3030 layers of both layouts that this rule picks plain the geometric mean is 1.65 times as fast.  The factors
+// are the margins that the estimates need: channels last, 0.95 takes 46 x 96 x 192 x 12 x 12 too, 19.9 us (24.9 with a
 // shortcut) against 18.7 (19.7), and nothing else that 0.85 leaves.  A layer of fewer than 16 units is a call of a few microseconds, for
-// which the estimates themselves (60 ns, asked twice) would count.
-bool layer_pair_preferred(int B, int H, int W, int C, int K, int layout)
+// which the estimates themselves (60 ns, asked twice) would count.  shortcut: as above; -1: whatever options the call has.
+bool layer_pair_preferred(int B, int H, int W, int C, int K, int layout, bool affine, int shortcut)
 {
-    if (cdivll((long long)B * cdiv(H, 4) * cdiv(W, 4), 2 * kPrQuads) * cdiv(K, 64) < 16 || !pair_supported(B, H, W, C, K, layout)) return false;
+    PrParams p;
+    if (cdivll((long long)B * cdiv(H, 4) * cdiv(W, 4), 2 * kPrQuads) * cdiv(K, 64) < 16 || !pr_sizes(p, B, H, W, C, K, layout)) return false;
     const long long P = (long long)B * ((H + 1) / 2) * ((W + 1) / 2);
     if (P > 0x7fffffffLL - kBlockM) return false;
-    return pair_us(B, H, W, C, K, layout) < (layout == WG2X2_NHWC ? 0.85 : 0.95) * fmin(unpaired_us(B, H, W, C, K, layout), cl_cut(P, C, K).us);
+    const double unpaired = unpaired_us(B, H, W, C, K, layout), clusters = cl_cut(P, C, K).us;
+    if (pair_us(p, layout) >= (layout == WG2X2_NHWC ? 0.85 : 0.95) * fmin(unpaired, clusters)) return false;
+    double us = 0.;
+    const bool few = clusters < 0.97 * unpaired;                  // (layer_cluster_preferred)
+    const bool wide = !few && !fused_beats_wide(B, H, W, C, K, layout, &us) && conv_fwd_wide_preferred(P, C, K);
+    if (!few && !wide) return true;
+    for (int a = 0; a < 2; ++a)
+        for (int s = 0; s < 3; ++s)
+            if ((a || s) && (shortcut < 0 || (affine == (a != 0) && shortcut == s)) && options_lose(p, layout, clusters, wide, a != 0, s)) return false;
+    return true;
 }

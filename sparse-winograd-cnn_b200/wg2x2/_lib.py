@@ -66,6 +66,7 @@ _SIGS = {
     "wg2x2_layer_fwd_fused_supported": (_i, [_i, _i, _i, _i, _i, _i]),
     "wg2x2_layer_fwd_fused_preferred": (_i, [_i, _i, _i, _i, _i, _i]),
     "wg2x2_layer_fwd_pair_preferred": (_i, [_i, _i, _i, _i, _i, _i]),
+    "wg2x2_layer_fwd_pair_preferred_for": (_i, [_i, _i, _i, _i, _i, _i, _i, _i]),
     "wg2x2_maxpool3x3s2_same_nhwc_in": (_i, [_p, _p, _p, _p, _p, _i, _i, _i, _i, _p]),
     "wg2x2_maxpool3x3s2_same": (_i, [_p, _p, _p, _p, _p, _i, _i, _i, _i, _p]),
     "wg2x2_stem_prepared_floats": (_i, []),

@@ -21,12 +21,12 @@ def oracle():
     return wg_oracle
 
 
-def kernel_of(B, H, W, C, K, layout):
-    """Which way layer_fwd_prepared takes an aligned layer: "pairs", "clusters" or "one" (kernel), or through memory "wide" or "walk"."""
+def kernel_of(B, H, W, C, K, layout, affine=0, shortcut=0):
+    """Which way layer_fwd_prepared takes an aligned layer with these options: "pairs", "clusters" or "one" (kernel), or through memory "wide" or "walk"."""
     import ctypes
     from wg2x2._lib import lib
     code = 1 if layout == "NCHW" else 0
-    if lib.wg2x2_layer_fwd_pair_preferred(B, H, W, C, K, code):
+    if lib.wg2x2_layer_fwd_pair_preferred_for(B, H, W, C, K, code, affine, shortcut):
         return "pairs"
     v, ws = ctypes.c_size_t(), ctypes.c_size_t()
     lib.wg2x2_layer_fwd_prepared_scratch(B, H, W, C, K, code, 1, ctypes.byref(v), ctypes.byref(ws))

@@ -198,6 +198,33 @@ def test_output_over_the_input_needs_scratch(shape, layout):
     assert float((y - want).abs().max()) <= TOL_TF32 * float(want.abs().max())
 
 
+@pytest.mark.parametrize("shape,layout", [((111, 128, 128, 10, 10), "NCHW"), ((48, 256, 256, 14, 14), "NCHW"), ((128, 256, 256, 14, 14), "NCHW"), ((46, 96, 192, 12, 12), "NHWC")])
+def test_rule_sees_the_options(shape, layout):
+    """Plain layers that run on pairs of SMs, and with a map or a shortcut on the path that is then the faster: what the queries say fits together,
+    and either kernel's results agree."""
+    import ctypes
+    import torch
+    import wg2x2
+    from wg2x2._lib import lib
+    B, C, K, H, W = shape
+    sizes = (B, H, W, C, K, 1 if layout == "NCHW" else 0)
+    for_ = {(a, s): lib.wg2x2_layer_fwd_pair_preferred_for(*sizes, a, s) for a in (0, 1) for s in (0, 1, 2)}
+    every = int(all(for_.values()))
+    assert lib.wg2x2_layer_fwd_pair_preferred(*sizes) == lib.wg2x2_layer_fwd_pair_preferred_for(*sizes, 0, -1) == every
+    assert for_[0, 0] == (layout == "NCHW") and every == (shape == (128, 256, 256, 14, 14))
+    nv, nw = ctypes.c_size_t(), ctypes.c_size_t()
+    lib.wg2x2_layer_fwd_prepared_scratch(*sizes, 1, ctypes.byref(nv), ctypes.byref(nw))
+    assert (nv.value == 0) == bool(every)         # what the query names is enough for any options
+    rnd, x, w = _inputs(shape, layout)
+    prepared, r = wg2x2.prepare_weights(w), rnd(B, K, H, W) if layout == "NCHW" else rnd(B, H, W, K)
+    plain = wg2x2.layer_fwd_prepared(x, prepared, K, layout=layout)
+    kw = dict(layout=layout, residual=r, in_scale=torch.ones(C, device="cuda"), in_shift=torch.zeros(C, device="cuda"))
+    tol = 2e-3 * float(plain.abs().max())          # another kernel: one rounds where the other cuts
+    assert float((wg2x2.layer_fwd_prepared(x, prepared, K, **kw) - (plain + r)).abs().max()) <= tol
+    got = wg2x2.layer_fwd_prepared(x, prepared, K, out=r, **dict(kw, residual=r))
+    assert got.data_ptr() == r.data_ptr() and bool(torch.isfinite(got).all())
+
+
 def test_zero_blocks_are_skipped_right(oracle):
     import wg2x2
     shape = (64, 160, 128, 28, 28)

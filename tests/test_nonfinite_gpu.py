@@ -112,7 +112,7 @@ def test_round_tf32_values():
 def test_shortcut_reaches_the_output(shape, layout, kernel):
     import wg2x2
     from conftest import kernel_of
-    assert kernel_of(*shape, layout) == kernel
+    assert kernel_of(*shape, layout, shortcut=1) == kernel
     B, H, W, C, K = shape
     g = torch.Generator(device="cuda").manual_seed(sum(shape))
     rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
@@ -156,7 +156,7 @@ def test_image_reaches_the_layer(shape, layout, kernel, affine, relu):
     import wg2x2
     from conftest import kernel_of
     B, C, K, H, W = shape
-    assert kernel_of(B, H, W, C, K, layout) == kernel
+    assert kernel_of(B, H, W, C, K, layout, affine=affine) == kernel
     g = torch.Generator(device="cuda").manual_seed(sum(shape))
     rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
     clean, w = rnd(B, C, H, W), rnd(16, C, K) / C ** 0.5
