@@ -101,6 +101,13 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b)
         : "=f"(o.x), "=f"(o.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
     return o;
 }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
+{
+    float2 o;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\tfma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "=f"(o.x), "=f"(o.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return o;
+}
 // 16 lanes x 32 columns: r[2 q], r[2 q + 1] = lanes l / 4 and l / 4 + 8 of column 4 q + l % 4
 __device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, float *r)
 {
@@ -536,14 +543,15 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, const __grid_con
                         const int c = 8 * sl + 2 * cl;
                         const float2 sc = c < prm.C ? make_float2(__ldg(prm.in_scale + c), __ldg(prm.in_scale + c + 1)) : make_float2(1.f, 1.f);
                         const float2 tc = c < prm.C ? make_float2(__ldg(prm.in_shift + c), __ldg(prm.in_shift + c + 1)) : make_float2(0.f, 0.f);
+                        // pixels outside the image stay zero, whatever the scale
 #pragma unroll
-                        for (int r = 0; r < 6; ++r)
+                        for (int r = 0; r < 6; ++r) {
+                            const bool row = (flags >> r) & 1u;
+                            const float2 sr = make_float2(row ? sc.x : 0.f, row ? sc.y : 0.f), tr = make_float2(row ? tc.x : 0.f, row ? tc.y : 0.f);
 #pragma unroll
-                            for (int x = 0; x < 6; ++x) {
-                                // pixels outside the image stay zero, whatever the scale
-                                const bool in = ((flags >> r) & 1u) && !(x == 0 && (flags & kPrNoLeft)) && !(x == 5 && (flags & kPrNoRight));
-                                if (in) win[r][x] = make_float2(fmaf(sc.x, win[r][x].x, tc.x), fmaf(sc.y, win[r][x].y, tc.y));
-                            }
+                            for (int x = 0; x < 6; ++x)
+                                if (!(x == 0 && (flags & kPrNoLeft)) && !(x == 5 && (flags & kPrNoRight))) win[r][x] = fma2(sr, win[r][x], tr);
+                        }
                     }
                 } else {
                     float d[2][6][4], ed[2][6];                          // [channel][row]
@@ -569,11 +577,13 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, const __grid_con
 #pragma unroll
                         for (int r = 0; r < 6; ++r) {
                             if (AFFINE) {
-                                const bool row = (flags >> r) & 1u;                   // pixels outside the image stay zero, whatever the scale
+                                // pixels outside the image stay zero, whatever the scale (an outer pixel that was not loaded is not looked at)
+                                const bool row = (flags >> r) & 1u;
+                                const float sr = row ? sc[p] : 0.f, tr = row ? tc[p] : 0.f;
 #pragma unroll
                                 for (int x = 0; x < 4; ++x)
-                                    if (row && (VEC == 4 || x < cols)) d[p][r][x] = fmaf(sc[p], d[p][r][x], tc[p]);
-                                if (row && (flags & kPrEdge)) ed[p][r] = fmaf(sc[p], ed[p][r], tc[p]);
+                                    if (VEC == 4 || x < cols) d[p][r][x] = fmaf(sr, d[p][r][x], tr);
+                                ed[p][r] = fmaf(sr, ed[p][r], tr);
                             }
                             lr[p][r].x = __shfl_up_sync(0xffffffffu, d[p][r][3], 4);
                             lr[p][r].y = __shfl_down_sync(0xffffffffu, d[p][r][0], 4);
