@@ -549,8 +549,9 @@ layer_fwd_pair_kernel(const __grid_constant__ CUtensorMap mapW, const __grid_con
                             const bool row = (flags >> r) & 1u;
                             const float2 sr = make_float2(row ? sc.x : 0.f, row ? sc.y : 0.f), tr = make_float2(row ? tc.x : 0.f, row ? tc.y : 0.f);
 #pragma unroll
-                            for (int x = 0; x < 6; ++x)
-                                if (!(x == 0 && (flags & kPrNoLeft)) && !(x == 5 && (flags & kPrNoRight))) win[r][x] = fma2(sr, win[r][x], tr);
+                            for (int x = 0; x < 6; ++x) win[r][x] = fma2(sr, win[r][x], tr);
+                            if (flags & kPrNoLeft) win[r][0] = make_float2(0.f, 0.f);
+                            if (flags & kPrNoRight) win[r][5] = make_float2(0.f, 0.f);
                         }
                     }
                 } else {
