@@ -992,15 +992,15 @@ static double pair_us(const PrParams &p, int layout)
 }
 
 // The same layer with an affine map in front or a shortcut (0: none, 1: of its own, 2: under Y), against the wide path and the layer on
-// clusters with the same.  There the margins of the plain rule are too narrow: a shortcut costs a pair 5 .. 7 us a round and a map 0.1 ..
-// 0.24 us a slot, the others 5 .. 12 %.  Over the 900 of 3030 layers that the plain rule takes from those two paths, with map and shortcut:
-// 88 were more than 3 % slower than before without this test (111 x 128 x 10 x 10 24.8 -> 34.5 us), 12 are with it; what it turns away is on the
-// mean as fast either way.  (The estimates: within 5 .. 12 % of the measured, one standard deviation.)
+// clusters with the same.  There the margins of the plain rule are too narrow: a shortcut costs a pair 5 .. 7 us a round and a map 0.04 ..
+// 0.16 us a slot, the others 5 .. 12 % (the estimates are within 5 .. 12 % of the measured, one standard deviation).  Of 1272 drawn layers
+// that the plain rule takes, 25 were more than 3 % slower than before with map and shortcut, the worst 0.80 of the speed (in another draw 111 x 128 x
+// 10 x 10 24.8 -> 34.5 us); with this test 4 of 1206 are, the worst 0.89, and the 66 it turns away are on the mean as fast either way.
 static bool options_lose(const PrParams &p, int layout, double clusters, bool wide, bool affine, int shortcut)
 {
     const bool nhwc = layout == WG2X2_NHWC, w4 = p.W % 4 == 0, w2 = p.W % 2 == 0;
     const double rounds = cdiv(p.units, kNumSMs / 2);
-    const double slot = nhwc ? 0.93 + (affine ? 0.24 : 0.) : w4 ? 0.83 + (affine ? 0.10 : 0.) : w2 ? 0.86 + (affine ? 0.19 : 0.) : 0.97 + (affine ? 0.17 : 0.);
+    const double slot = nhwc ? 0.93 + (affine ? 0.08 : 0.) : w4 ? 0.83 + (affine ? 0.08 : 0.) : w2 ? 0.86 + (affine ? 0.18 : 0.) : 0.97 + (affine ? 0.15 : 0.);
     const double last = !shortcut ? 0. : nhwc ? 4.9 : w4 ? (shortcut == 2 && rounds > 1. ? 1.2 : 6.8) : w2 ? 6.3 : 4.8;
     const double us = (nhwc ? 6.4 : w2 ? 6.8 : 9.0) + rounds * ((nhwc ? 2.5 : w4 ? 2.4 : w2 ? 3.0 : 5.0) + last + slot * p.nS);
     double other = clusters * (affine ? 1.07 : 1.02) * (shortcut == 2 ? 1.12 : shortcut ? 1.08 : 1.);
